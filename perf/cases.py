@@ -88,7 +88,8 @@ def draw(rng):
         c = _case("", "eulerpsi", n, n, kind=kind, members=_spread(rng, 4, 64),
                   precision=rng.choice(["fp64", "fp32"]), steps=2, islands=rng.randint(0, 4))
     elif kind == "adjoint":
-        c = _case("", "eulerpsi", _spread(rng, 48, 512), _spread(rng, 48, 512), kind=kind,
+        nx = _spread(rng, 64, 512)
+        c = _case("", "eulerpsi", nx, min(512, int(nx * rng.uniform(0.6, 1.6))), kind=kind,
                   steps=rng.randint(8, 20))
     else:
         model = rng.choice(["eulerpsi", "qg", "rsw", "euler", "boussinesq"])
@@ -96,7 +97,7 @@ def draw(rng):
         small = model in ("euler", "boussinesq")
         lo, hi = (40, 640) if small else (64, 1536)
         nx = _spread(rng, lo, hi)
-        ny = min(hi, max(lo, int(nx * rng.uniform(0.4, 1.6))))
+        ny = min(hi, max(lo, int(nx * rng.uniform(0.6, 1.6))))
         c = _case("", model, nx, ny, precision=precision, steps=rng.randint(2, 4),
                   islands=rng.randint(0, 3 if small else 6), noslip=rng.random() < 0.25,
                   xperiodic=model in ("rsw", "euler", "boussinesq") and rng.random() < 0.5,
