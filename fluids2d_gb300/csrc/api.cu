@@ -389,7 +389,7 @@ static int rec_diag(f2d_model_s* m, int par, cudaStream_t s, int warm = -1)
         int e = ensure_ns(m);
         if (e) return e;
         int fixed = 0;
-        CKI(ns_record(m->ns, s, m->s2, eager_mode(), &fixed));
+        CKI(ns_record(m->ns, s, &fixed));
         if (g.xper) CKI(launch_fill_periodic(0, fb(m, "p"), g, s));
         CKI(launch_euler_project(m->prec, fb(m, "u.x", par), fb(m, "u.y", par),
                                  (const double*)fb(m, "p"), m->d_code, g, s));
@@ -1657,6 +1657,7 @@ int f2d_sync(f2d_model m)
         CK(cudaMemcpy(&m->sc->status, &zero, sizeof(int), cudaMemcpyHostToDevice));
         std::string msg = "device status:";
         if (st & ST_TMA_TIMEOUT) msg += " TMA tile load timed out;";
+        if (st & ST_GRID_TIMEOUT) msg += " a solver's grid barrier timed out;";
         if (st & ST_STAGE_ALIGN) msg += " TMA staging buffer misaligned;";
         if (st & ST_PCG_MAXIT) msg += " Poisson solve reached max iterations;";
         if (st & ST_NONFINITE) msg += " non-finite value (residual or time step);";

@@ -38,6 +38,7 @@ enum : int {
     ST_PCG_MAXIT = 2,      // the Poisson solve stopped at max iterations
     ST_NONFINITE = 4,      // a non-finite value reached a reduction
     ST_STAGE_ALIGN = 8,    // a TMA staging buffer was not 128-byte aligned (nothing loaded)
+    ST_GRID_TIMEOUT = 16,  // a grid barrier of a persistent solve was not passed within 2 s
 };
 
 // min(x, cap) with Python's min semantics (the reference's set_dt,

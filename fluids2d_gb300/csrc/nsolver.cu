@@ -14,7 +14,7 @@
 // the solution is returned with zero mean: the pressure is defined up to a
 // constant, and only its gradient enters the model.
 //
-// Preconditioner: cell-centred V-cycle with red-black Gauss-Seidel (nu sweeps
+// Preconditioner: cell-centred V-cycle with red-black Gauss-Seidel (2 sweeps
 // per leg, symmetric order), coarse cells = 2x2 agglomerates (fluid if any
 // child is), restriction = sum of the children's residuals, prolongation =
 // the parent's value, coarse couplings = half the sum of the fine face
@@ -22,426 +22,796 @@
 // R A P for this R and P; with piecewise-constant P it is twice too stiff for
 // smooth errors, and the coarse correction comes out halved - half the sum is
 // the re-discretised coupling where the face is fully open and keeps the
-// partial openings of masked faces.) Coarsest level by (R,B)^k (B,R)^k in one
-// thread block. The FP32 form runs the cycle in FP32 (levels, couplings and
-// smoothing in float; its right-hand side is the FP64 Krylov residual
-// rounded, its result converted back), while the Krylov vectors, the
-// operator products, the dot products and the zero-mean projections stay
-// FP64. Single component assumed (a
-// fluid domain made of several disconnected parts would need a projection
-// per part).
+// partial openings of masked faces.) The first level of at most 2048 cells is
+// solved exactly with its precomputed dense pseudo-inverse. The FP32 form runs the cycle in FP32
+// (levels, couplings and smoothing in float; its right-hand side is the FP64
+// Krylov residual rounded, its result converted back), while the Krylov
+// vectors, the operator products, the dot products and the zero-mean
+// projections stay FP64.
+//
+// The solve is one cooperative kernel (persist.cuh), one block per SM. CG in
+// the form of Chronopoulos and Gear (s-step methods for symmetric linear
+// systems, J. Comput. Appl. Math. 25, 1989; here s = 1): with w = A z the two
+// inner products <r, z> and <z, w> come from one pass, s = A p by the same
+// recurrence as p, so an iteration has 2 (grid levels) + 1 barriers:
+//   A   update s, r, p, x (r also on the tile's halo, recomputed), <r, r>,
+//       and the pre-smoothing, residual and restriction of level 0
+//   D_l the down legs of the other grid levels
+//   the dense level
+//   U_l the up legs
+//   B   the up leg of level 0 with z one cell past the tile, w = A z, the
+//       two inner products
+// A leg works on a tile and a halo of the 4 (B: 5) cells its half sweeps
+// reach over, in shared memory, so a leg needs one barrier; tile sizes are
+// chosen per level so that the chip is filled (pick_tile).
+// What bounds it: at 40^2 and 64^2 the barriers, at 512^2 the FP64 pipe.
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
+#include <numeric>
 
-#include "graph_while.cuh"
 #include "nsolver.cuh"
+#include "persist.cuh"
 
 namespace f2d {
 
-__device__ __forceinline__ long long cidx(const NLevel& L, int J, int I)
+constexpr int NS_H = 5;  // halo of the widest leg
+
+// A staged region of a tile: rows J0 - h .. J0 + th + h - 1, columns alike
+template <typename S>
+struct NReg {
+    S *x, *b, *fx, *fy, *inv;
+    uint8_t* code;
+    int J0, I0, h, W, RH;
+    float rW;
+};
+
+// level-0 tables in the cycle's precision (shared memory)
+template <typename S>
+struct NTab {
+    S cxi[9], cyi[9], inv[9], cs[9];
+};
+
+__device__ __forceinline__ int n_open(uint8_t c)
 {
-    return L.off + (long long)J * L.pitch + I;
+    return 3 * (((c >> 1) & 1) + ((c >> 2) & 1)) + ((c >> 3) & 1) + ((c >> 4) & 1);
 }
 
-// A x at fluid cell (J, I); also the sum of its couplings. S: the value
-// and coupling type of the level (the FP32 cycle's levels are float)
-template <typename S>
-__device__ __forceinline__ S n_apply(const NLevel& L, const S* __restrict__ x, int J, int I,
-                                     S* csum)
+// wrapped column of a region cell; false outside the level
+__device__ __forceinline__ bool n_cell(const NLevel& L, int J, int& I)
 {
-    const S* __restrict__ fx = (const S*)L.fx;
-    const S* __restrict__ fy = (const S*)L.fy;
-    const long long k = cidx(L, J, I);
-    const S xc = x[k];
-    const S cw = fx[k], cs = fy[k];
-    S ce = S(0), cn = S(0), xw = S(0), xe = S(0), xs = S(0), xn = S(0);
-    if (I > 0) xw = x[k - 1];
-    else if (L.per) xw = x[cidx(L, J, L.nxn - 1)];
-    if (I + 1 < L.nxn) {
-        ce = fx[k + 1];
-        xe = x[k + 1];
-    } else if (L.per) {
-        const long long k0 = cidx(L, J, 0);
-        ce = fx[k0];
-        xe = x[k0];
+    if (J < 0 || J >= L.nyn) return false;
+    if (L.per) {
+        // a tile wider than the level wraps more than once
+        while (I < 0) I += L.nxn;
+        while (I >= L.nxn) I -= L.nxn;
+        return true;
     }
-    if (J > 0) xs = x[k - L.pitch];
-    if (J + 1 < L.nyn) {
-        cn = fy[k + L.pitch];
-        xn = x[k + L.pitch];
+    return I >= 0 && I < L.nxn;
+}
+
+// the Gauss-Seidel value of region cell e (0 at cells without couplings)
+template <typename S, bool L0>
+__device__ __forceinline__ S n_gs(const NReg<S>& R, const NTab<S>& T, int e)
+{
+    if constexpr (L0) {
+        const uint8_t c = R.code[e];
+        const int k = n_open(c);
+        const S xw = c & 2 ? R.x[e - 1] : S(0), xe = c & 4 ? R.x[e + 1] : S(0);
+        const S xs = c & 8 ? R.x[e - R.W] : S(0), xn = c & 16 ? R.x[e + R.W] : S(0);
+        // b holds b / (coupling sum)
+        return T.cxi[k] * (xw + xe) + (T.cyi[k] * (xs + xn) - R.b[e]);
+    } else {
+        S v = R.fx[e] * R.x[e - 1] - R.b[e];
+        v = R.fx[e + 1] * R.x[e + 1] + v;
+        v = R.fy[e] * R.x[e - R.W] + v;
+        v = R.fy[e + R.W] * R.x[e + R.W] + v;
+        return v * R.inv[e];
     }
-    if (csum) *csum = (cw + ce) + (cs + cn);
-    return (cw * (xw - xc) + ce * (xe - xc)) + (cs * (xs - xc) + cn * (xn - xc));
 }
 
-__device__ __forceinline__ bool cell(const NLevel& L, int& J, int& I)
+// residual b - A x at region cell e = (coupling sum) (x - Gauss-Seidel value)
+template <typename S, bool L0>
+__device__ __forceinline__ S n_res(const NReg<S>& R, const NTab<S>& T, int e)
 {
-    I = blockIdx.x * blockDim.x + threadIdx.x;
-    J = blockIdx.y * blockDim.y + threadIdx.y;
-    return J < L.nyn && I < L.nxn;
+    if constexpr (L0) {
+        return T.cs[n_open(R.code[e])] * (R.x[e] - n_gs<S, true>(R, T, e));
+    } else {
+        S v = R.fx[e] * R.x[e - 1] - R.b[e];
+        v = R.fx[e + 1] * R.x[e + 1] + v;
+        v = R.fy[e] * R.x[e - R.W] + v;
+        v = R.fy[e + R.W] * R.x[e + R.W] + v;
+        const S cs = (R.fx[e] + R.fx[e + 1]) + (R.fy[e] + R.fy[e + R.W]);
+        return cs * R.x[e] - v;
+    }
 }
 
-// ---- multigrid -------------------------------------------------------------
-template <typename S>
-__device__ __forceinline__ void n_smooth_cell(const NLevel& L, int J, int I)
+// Half sweep of one colour over the cells within rad of the tile, next to a
+// seam (a periodic level of odd width: the cells at both ends of the wrap are
+// of one colour). Every value is formed before any is written, which is
+// Jacobi across the seam and keeps the cycle symmetric.
+constexpr int NS_SEAM_T = 32;  // tile rows and columns of such a level, at most
+template <typename S, bool L0>
+__device__ __noinline__ void n_half_seam(NReg<S> R, const NTab<S>& T, const NLevel& L, int color,
+                                         int rad)
 {
-    S* __restrict__ x = (S*)L.x;
-    const S* __restrict__ b = (const S*)L.b;
-    const long long k = cidx(L, J, I);
-    if (!L.m[k]) return;
-    S cs;
-    const S ax = n_apply<S>(L, x, J, I, &cs);
-    // A x = sum c_n x_n - cs x_c = b  ->  x_c = (sum c_n x_n - b) / cs
-    if (cs > S(0)) x[k] = ((ax + cs * x[k]) - b[k]) / cs;
-}
-
-// one thread per cell of the colour: thread column I' of row J takes cell
-// I = 2 I' + ((J + color) & 1)
-template <typename S>
-__global__ void k_ns_smooth(const NLevel* __restrict__ levs, int l, int color)
-{
-    const NLevel L = levs[l];
-    const int J = blockIdx.y * blockDim.y + threadIdx.y;
-    const int I = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + ((J + color) & 1);
-    if (J >= L.nyn || I >= L.nxn) return;
-    n_smooth_cell<S>(L, J, I);
-}
-
-// coarse b = sum of the fluid children's residuals; coarse x = 0
-template <typename S>
-__global__ void k_ns_restrict(const NLevel* __restrict__ levs, int l)
-{
-    const NLevel F = levs[l], C = levs[l + 1];
-    int J, I;
-    if (!cell(C, J, I)) return;
-    const S* __restrict__ fxv = (const S*)F.x;
-    const S* __restrict__ fb = (const S*)F.b;
-    S v = S(0);
-    for (int a = 0; a < 2; ++a)
-        for (int c = 0; c < 2; ++c) {
-            const int fj = 2 * J + a, fi = 2 * I + c;
-            if (fj >= F.nyn || fi >= F.nxn) continue;
-            const long long k = cidx(F, fj, fi);
-            if (F.m[k]) v += fb[k] - n_apply<S>(F, fxv, fj, fi, nullptr);
+    constexpr int N = NS_SEAM_T + 2 * (NS_H - 1), MAXC = (N * N + PS_NT - 1) / PS_NT;
+    const int o = R.h - rad, nr = L.th + 2 * rad;
+    const int wc = L.tw + 2 * rad;
+    const float rw = 1.0f / (float)wc;
+    S v[MAXC];
+#pragma unroll
+    for (int q = 0; q < MAXC; ++q) {
+        const int k = threadIdx.x + q * PS_NT;
+        v[q] = S(0);
+        if (k < nr * wc) {
+            const int a = fdiv(k, rw);
+            v[q] = n_gs<S, L0>(R, T, (o + a) * R.W + o + k - a * wc);
         }
-    const long long kc = cidx(C, J, I);
-    ((S*)C.b)[kc] = C.m[kc] ? v : S(0);
-    ((S*)C.x)[kc] = S(0);
-}
-
-template <typename S>
-__global__ void k_ns_prolong(const NLevel* __restrict__ levs, int l)
-{
-    const NLevel F = levs[l], C = levs[l + 1];
-    int J, I;
-    if (!cell(F, J, I)) return;
-    const long long k = cidx(F, J, I);
-    if (F.m[k]) ((S*)F.x)[k] += ((const S*)C.x)[cidx(C, J >> 1, I >> 1)];
-}
-
-template <typename S>
-__global__ void k_ns_zero(const NLevel* __restrict__ levs, int l)
-{
-    const NLevel L = levs[l];
-    int J, I;
-    if (cell(L, J, I)) ((S*)L.x)[cidx(L, J, I)] = S(0);
-}
-
-// coarsest level: (R,B)^k (B,R)^k from x = 0, one block
-template <typename S>
-__global__ void __launch_bounds__(1024) k_ns_coarse(const NLevel* __restrict__ levs, int l,
-                                                    int ksweeps)
-{
-    const NLevel L = levs[l];
-    const int n = L.nyn * L.nxn;
-    for (int e = threadIdx.x; e < n; e += blockDim.x)
-        ((S*)L.x)[cidx(L, e / L.nxn, e % L.nxn)] = S(0);
+    }
     __syncthreads();
-    for (int s = 0; s < 2 * ksweeps; ++s) {
-        for (int h = 0; h < 2; ++h) {
-            const int color = s < ksweeps ? h : 1 - h;
-            for (int e = threadIdx.x; e < n; e += blockDim.x) {
-                const int J = e / L.nxn, I = e % L.nxn;
-                if (((J + I) & 1) == color) n_smooth_cell<S>(L, J, I);
+#pragma unroll
+    for (int q = 0; q < MAXC; ++q) {
+        const int k = threadIdx.x + q * PS_NT;
+        if (k >= nr * wc) continue;
+        const int a = fdiv(k, rw), r = o + a, c = o + k - a * wc;
+        int I = R.I0 - R.h + c;
+        const int J = R.J0 - R.h + r;
+        if (n_cell(L, J, I) && ((J + I) & 1) == color) R.x[r * R.W + c] = v[q];
+    }
+    __syncthreads();
+}
+
+// Half sweep of one colour over the cells within rad of the tile
+template <typename S, bool L0>
+__device__ __forceinline__ void n_half(const NReg<S>& R, const NTab<S>& T, const NLevel& L,
+                                       int color, int rad)
+{
+    if (L.seam) {
+        n_half_seam<S, L0>(R, T, L, color, rad);
+        return;
+    }
+    const int o = R.h - rad, nr = L.th + 2 * rad;
+    const int wc = L.tw / 2 + rad;
+    const float rw = 1.0f / (float)wc;
+    for (int k = threadIdx.x; k < nr * wc; k += PS_NT) {
+        const int a = fdiv(k, rw), r = o + a;
+        // J0, I0 are even: the colour of region cell (r, c) is r + c
+        const int c = o + 2 * (k - a * wc) + ((r + o + color) & 1);
+        const int e = r * R.W + c;
+        R.x[e] = n_gs<S, L0>(R, T, e);
+    }
+    __syncthreads();
+}
+
+// whether region cell (r, c) is red (the colour of the wrapped cell)
+template <typename S>
+__device__ __forceinline__ bool n_red(const NReg<S>& R, const NLevel& L, int r, int c)
+{
+    if (!L.seam) return ((r + c) & 1) == 0;
+    int I = R.I0 - R.h + c;
+    const int J = R.J0 - R.h + r;
+    return n_cell(L, J, I) && ((J + I) & 1) == 0;
+}
+
+template <typename S>
+__device__ __forceinline__ void n_region(NReg<S>& R, const NLevel& L, int tile, int h,
+                                         unsigned char* smem, bool l0)
+{
+    const int ty = tile / L.ntx, tx = tile - ty * L.ntx;
+    R.J0 = ty * L.th;
+    R.I0 = tx * L.tw;
+    R.h = h;
+    R.W = L.tw + 2 * h;
+    R.RH = L.th + 2 * h;
+    R.rW = 1.0f / (float)R.W;
+    const int n = R.W * R.RH;
+    S* p = (S*)smem;
+    R.x = p;
+    R.b = p + n;
+    if (l0) {
+        R.code = (uint8_t*)(p + 2 * n);
+        R.fx = R.fy = R.inv = nullptr;
+    } else {
+        R.fx = p + 2 * n;
+        R.fy = p + 3 * n;
+        R.inv = p + 4 * n;
+        R.code = nullptr;
+    }
+}
+
+// The cells of a region in batches of NB per thread: load(q, in, k, r, c) for
+// the NB cells (k: the element of cell (r, c) if it lies in the level; the
+// loads of a batch are in flight together), then use(q, e, in, k, r, c).
+constexpr int NB = 2;
+template <typename S, typename FL, typename FU>
+__device__ __forceinline__ void n_load(const NReg<S>& R, const NLevel& L, FL load, FU use)
+{
+    const int n = R.W * R.RH;
+    for (int e0 = threadIdx.x; e0 < n; e0 += NB * PS_NT) {
+        int rc[NB];
+        long long k[NB];
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            const int e = e0 + q * PS_NT;
+            const int r = fdiv(e, R.rW), c = e - r * R.W;
+            int I = R.I0 - R.h + c;
+            const int J = R.J0 - R.h + r;
+            const bool in = e < n && n_cell(L, J, I);
+            rc[q] = (r << 16) | c;
+            k[q] = in ? L.off + (long long)J * L.pitch + I : -1;
+            // (the wrapped cell's colour and column are needed below)
+            load(q, in, k[q], J, I);
+        }
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            const int e = e0 + q * PS_NT;
+            if (e < n) use(q, e, k[q] >= 0, k[q], rc[q] >> 16, rc[q] & 0xffff);
+        }
+    }
+}
+
+// coarse b of the agglomerates of the tile: the sum of the children's
+// residuals. After a black half sweep the black residuals are zero and only
+// the two red children contribute (all four next to a seam).
+template <typename S, bool L0>
+__device__ __forceinline__ void n_restrict(const NReg<S>& R, const NTab<S>& T, const NLevel& F,
+                                           const NLevel& C)
+{
+    const int wc = F.tw / 2, nc = wc * (F.th / 2);
+    const float rw = 1.0f / (float)wc;
+    for (int k = threadIdx.x; k < nc; k += PS_NT) {
+        const int a = fdiv(k, rw), c = k - a * wc;
+        const int J = R.J0 / 2 + a, I = R.I0 / 2 + c;
+        if (J >= C.nyn || I >= C.nxn) continue;
+        const int e = (R.h + 2 * a) * R.W + R.h + 2 * c;
+        S v = n_res<S, L0>(R, T, e);
+        if (!F.seam) v += n_res<S, L0>(R, T, e + R.W + 1);
+        else {
+            v += n_res<S, L0>(R, T, e + R.W);
+            // the last agglomerate of an odd count has one column (the next
+            // one of the region is the wrapped first)
+            if (2 * I + 1 < F.nxn)
+                v += n_res<S, L0>(R, T, e + 1) + n_res<S, L0>(R, T, e + R.W + 1);
+        }
+        ((S*)C.b)[C.off + (long long)J * C.pitch + I] = v;
+    }
+}
+
+// The tile's cells in batches, as n_load: load(q, in, k, e), use(q, k, e) with
+// k the element and e the region index of a cell of the level
+template <typename S, typename FL, typename FU>
+__device__ __forceinline__ void n_tile(const NReg<S>& R, const NLevel& L, FL load, FU use)
+{
+    const int n = L.tw * L.th;
+    const float rw = 1.0f / (float)L.tw;
+    for (int e0 = threadIdx.x; e0 < n; e0 += NB * PS_NT) {
+        int e[NB];
+        long long k[NB];
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            const int i = e0 + q * PS_NT;
+            const int a = fdiv(i, rw), c = i - a * L.tw;
+            const int J = R.J0 + a, I = R.I0 + c;
+            const bool in = i < n && J < L.nyn && I < L.nxn;
+            k[q] = in ? L.off + (long long)J * L.pitch + I : -1;
+            e[q] = (R.h + a) * R.W + R.h + c;
+            load(q, in, k[q], e[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < NB; ++q)
+            if (k[q] >= 0) use(q, k[q], e[q]);
+    }
+}
+
+// x of the tile's cells
+template <typename S>
+__device__ __forceinline__ void n_store(const NReg<S>& R, const NLevel& L, S* y)
+{
+    n_tile(R, L, [](int, bool, long long, int) {}, [&](int, long long k, int e) { y[k] = R.x[e]; });
+}
+
+// down leg of a coarse grid level
+template <typename S>
+__device__ __forceinline__ void n_down(const NSArgs& A, int l, unsigned char* smem,
+                                       const NTab<S>& T)
+{
+    const NLevel& L = A.lev[l];
+    for (int tile = blockIdx.x; tile < L.nt; tile += gridDim.x) {
+        NReg<S> R;
+        n_region<S>(R, L, tile, 4, smem, false);
+        const S* B = (const S*)L.b;
+        const S* FX = (const S*)L.fx;
+        const S* FY = (const S*)L.fy;
+        const S* IV = (const S*)L.inv;
+        S b[NB], fx[NB], fy[NB], iv[NB];
+        n_load(
+            R, L,
+            [&](int q, bool in, long long k, int, int) {
+                b[q] = in ? B[k] : S(0);
+                fx[q] = in ? FX[k] : S(0);
+                fy[q] = in ? FY[k] : S(0);
+                iv[q] = in ? IV[k] : S(0);
+            },
+            [&](int q, int e, bool, long long, int r, int c) {
+                R.b[e] = b[q];
+                R.fx[e] = fx[q];
+                R.fy[e] = fy[q];
+                R.inv[e] = iv[q];
+                R.x[e] = n_red(R, L, r, c) ? -b[q] * iv[q] : S(0);
+            });
+        __syncthreads();
+#pragma unroll 1
+        for (int rad = 3; rad >= 1; --rad) n_half<S, false>(R, T, L, rad & 1, rad);
+        n_restrict<S, false>(R, T, L, A.lev[l + 1]);
+        n_store<S>(R, L, (S*)L.xa);
+        __syncthreads();
+    }
+}
+
+// up leg of a coarse grid level: the black cells' own values do not enter
+// (the first half sweep overwrites them from the red ones), so only red
+// cells are prolongated (all next to a seam)
+template <typename S>
+__device__ __forceinline__ void n_up(const NSArgs& A, int l, unsigned char* smem,
+                                     const NTab<S>& T)
+{
+    const NLevel& L = A.lev[l];
+    const NLevel& C = A.lev[l + 1];
+    for (int tile = blockIdx.x; tile < L.nt; tile += gridDim.x) {
+        NReg<S> R;
+        n_region<S>(R, L, tile, 4, smem, false);
+        const S* B = (const S*)L.b;
+        const S* XA = (const S*)L.xa;
+        const S* XC = (const S*)C.x;
+        const S* FX = (const S*)L.fx;
+        const S* FY = (const S*)L.fy;
+        const S* IV = (const S*)L.inv;
+        S b[NB], fx[NB], fy[NB], iv[NB], xa[NB], xc[NB];
+        n_load(
+            R, L,
+            [&](int q, bool in, long long k, int J, int I) {
+                const bool use = in && (L.seam || ((J + I) & 1) == 0);
+                b[q] = in ? B[k] : S(0);
+                fx[q] = in ? FX[k] : S(0);
+                fy[q] = in ? FY[k] : S(0);
+                iv[q] = in ? IV[k] : S(0);
+                xa[q] = use ? XA[k] : S(0);
+                xc[q] = use ? XC[C.off + (long long)(J >> 1) * C.pitch + (I >> 1)] : S(0);
+            },
+            [&](int q, int e, bool, long long, int, int) {
+                R.b[e] = b[q];
+                R.fx[e] = fx[q];
+                R.fy[e] = fy[q];
+                R.inv[e] = iv[q];
+                R.x[e] = iv[q] != S(0) ? xa[q] + xc[q] : S(0);
+            });
+        __syncthreads();
+#pragma unroll 1
+        for (int rad = 3; rad >= 0; --rad) n_half<S, false>(R, T, L, rad & 1, rad);
+        n_store<S>(R, L, (S*)L.x);
+        __syncthreads();
+    }
+}
+
+// phase A: with it > 0 the CG update of the previous iteration (s, p, x of
+// the tile; r of the tile and its halo), the block's <r, r> and sum of x,
+// then the down leg of level 0 on the new residual
+template <typename S>
+__device__ __forceinline__ void n_phase_a(const NSArgs& A, int it, double alpha, double beta,
+                                          double (&tot)[2], unsigned char* smem,
+                                          const NTab<S>& T)
+{
+    const NLevel& L = A.lev[0];
+    const int par = it & 1;
+    const double* r0 = A.r[it > 0 ? 1 - par : 0];
+    const double* s0 = A.s[1 - par];
+    double* r1 = A.r[par];
+    double* s1 = A.s[par];
+    const S* z = (const S*)A.z;
+    for (int tile = blockIdx.x; tile < L.nt; tile += gridDim.x) {
+        NReg<S> R;
+        n_region<S>(R, L, tile, 4, smem, true);
+        uint8_t code[NB];
+        double rv[NB], sv[NB], wv[NB], xv[NB], pv[NB];
+        S zv[NB];
+        n_load(
+            R, L,
+            [&](int q, bool in, long long k, int, int) {
+                code[q] = in ? L.code[k] : 0;
+                rv[q] = in ? r0[k] : 0.0;
+                wv[q] = in && it > 0 ? A.w[k] : 0.0;
+                sv[q] = in && it > 1 ? s0[k] : 0.0;
+            },
+            [&](int q, int e, bool in, long long k, int r, int c) {
+                double rn = rv[q];
+                if (it > 0) {
+                    const double sn = wv[q] + beta * sv[q];
+                    rn -= alpha * sn;
+                    if (in && r >= 4 && r < 4 + L.th && c >= 4 && c < 4 + L.tw &&
+                        R.I0 - 4 + c < L.nxn) {
+                        s1[k] = sn;
+                        r1[k] = rn;
+                        tot[0] += rn * rn;  // (0 at dry cells)
+                    }
+                }
+                const S bi = conv<S>(rn) * T.inv[n_open(code[q])];
+                R.code[e] = code[q];
+                R.b[e] = bi;
+                R.x[e] = n_red(R, L, r, c) ? -bi : S(0);
+            });
+        __syncthreads();
+#pragma unroll 1
+        for (int rad = 3; rad >= 1; --rad) n_half<S, true>(R, T, L, rad & 1, rad);
+        n_restrict<S, true>(R, T, L, A.lev[1]);
+        // xa, and p and x of the tile
+        n_tile(
+            R, L,
+            [&](int q, bool in, long long k, int) {
+                xv[q] = in && it > 0 ? A.x[k] : 0.0;
+                pv[q] = in && it > 1 ? A.p[k] : 0.0;
+                zv[q] = in && it > 0 ? z[k] : S(0);
+            },
+            [&](int q, long long k, int e) {
+                ((S*)L.xa)[k] = R.x[e];
+                if (it == 0) return;
+                const double pn = conv<double>(zv[q]) + beta * pv[q];
+                A.p[k] = pn;
+                if (R.code[e]) {
+                    const double xn = xv[q] + alpha * pn;
+                    A.x[k] = xn;
+                    tot[1] += xn;
+                }
+            });
+        __syncthreads();
+    }
+}
+
+// phase B: up leg of level 0 (z), w = A z in FP64, <r, z> and <z, w>
+template <typename S>
+__device__ __forceinline__ void n_phase_b(const NSArgs& A, int it, double (&tot)[2],
+                                          unsigned char* smem, const NTab<S>& T)
+{
+    const NLevel& L = A.lev[0];
+    const NLevel& C = A.lev[1];
+    const double* rr = A.r[it & 1];
+    const S* XA = (const S*)L.xa;
+    const S* XC = (const S*)C.x;
+    const double cx = A.cx, cy = A.cy;
+    for (int tile = blockIdx.x; tile < L.nt; tile += gridDim.x) {
+        NReg<S> R;
+        n_region<S>(R, L, tile, NS_H, smem, true);
+        uint8_t code[NB];
+        double rv[NB];
+        S xa[NB], xc[NB];
+        n_load(
+            R, L,
+            [&](int q, bool in, long long k, int J, int I) {
+                const bool use = in && (L.seam || ((J + I) & 1) == 0);
+                code[q] = in ? L.code[k] : 0;
+                rv[q] = in ? rr[k] : 0.0;
+                xa[q] = use ? XA[k] : S(0);
+                xc[q] = use ? XC[C.off + (long long)(J >> 1) * C.pitch + (I >> 1)] : S(0);
+            },
+            [&](int q, int e, bool, long long, int, int) {
+                R.code[e] = code[q];
+                R.b[e] = conv<S>(rv[q]) * T.inv[n_open(code[q])];
+                R.x[e] = code[q] & 30 ? xa[q] + xc[q] : S(0);
+            });
+        __syncthreads();
+#pragma unroll 1
+        for (int rad = 4; rad >= 1; --rad) n_half<S, true>(R, T, L, 1 - (rad & 1), rad);
+        n_tile(
+            R, L, [&](int q, bool in, long long k, int) { rv[q] = in ? rr[k] : 0.0; },
+            [&](int q, long long k, int e) {
+                const uint8_t cd = R.code[e];
+                const double zc = conv<double>(R.x[e]);
+                // differences to the centre across open faces
+                const double dw = cd & 2 ? conv<double>(R.x[e - 1]) - zc : 0.0;
+                const double de = cd & 4 ? conv<double>(R.x[e + 1]) - zc : 0.0;
+                const double ds = cd & 8 ? conv<double>(R.x[e - R.W]) - zc : 0.0;
+                const double dn = cd & 16 ? conv<double>(R.x[e + R.W]) - zc : 0.0;
+                const double wv = cx * (dw + de) + cy * (ds + dn);
+                ((S*)A.z)[k] = R.x[e];
+                A.w[k] = wv;
+                tot[0] += rv[q] * zc;
+                tot[1] += zc * wv;
+            });
+        __syncthreads();
+    }
+}
+
+// cells of level 0, dealt to all threads of the grid by rows of 512 cells
+template <typename F>
+__device__ __forceinline__ void n_cells(const NLevel& L, F f)
+{
+    const int nseg = (L.nxn + PS_NT - 1) / PS_NT;
+    for (int q = blockIdx.x; q < L.nyn * nseg; q += gridDim.x) {
+        const int J = q / nseg, I = (q - J * nseg) * PS_NT + threadIdx.x;
+        if (I < L.nxn) f(J, I, L.off + (long long)J * L.pitch + I);
+    }
+}
+
+// Phases A and B when level 0 itself is the dense level (D: its x = z and
+// its b in the cycle's precision, without the halo)
+template <typename S>
+__device__ __forceinline__ void n_dense_a(const NSArgs& A, int it, double alpha, double beta,
+                                          double (&tot)[2])
+{
+    const NLevel& L = A.lev[0];
+    n_cells(L, [&](int J, int I, long long k) {
+        const int d = J * L.nxn + I;
+        double rv = A.r[0][k];
+        if (it > 0) {
+            double sv = A.w[k], pv = conv<double>(((const S*)L.x)[d]);
+            if (it > 1) {
+                sv += beta * A.s[0][k];
+                pv += beta * A.p[k];
             }
-            __syncthreads();
+            rv -= alpha * sv;
+            A.s[0][k] = sv;
+            A.r[0][k] = rv;
+            A.p[k] = pv;
+            if (L.code[k]) {
+                const double xn = A.x[k] + alpha * pv;
+                A.x[k] = xn;
+                tot[0] += rv * rv;
+                tot[1] += xn;
+            }
         }
+        ((S*)L.b)[d] = conv<S>(rv);
+    });
+}
+
+template <typename S>
+__device__ __forceinline__ void n_dense_b(const NSArgs& A, double (&tot)[2])
+{
+    const NLevel& L = A.lev[0];
+    const S* z = (const S*)L.x;
+    n_cells(L, [&](int J, int I, long long k) {
+        const int d = J * L.nxn + I;
+        const uint8_t c = L.code[k];
+        double wv = 0.0;
+        if (c) {
+            const double zc = conv<double>(z[d]);
+            const int dw_ = I > 0 ? d - 1 : d + L.nxn - 1, de_ = I + 1 < L.nxn ? d + 1 : d - I;
+            const double dw = c & 2 ? conv<double>(z[dw_]) - zc : 0.0;
+            const double de = c & 4 ? conv<double>(z[de_]) - zc : 0.0;
+            const double ds = c & 8 ? conv<double>(z[d - L.nxn]) - zc : 0.0;
+            const double dn = c & 16 ? conv<double>(z[d + L.nxn]) - zc : 0.0;
+            wv = A.cx * (dw + de) + A.cy * (ds + dn);
+            tot[0] += A.r[0][k] * zc;
+            tot[1] += zc * wv;
+        }
+        A.w[k] = wv;
+    });
+}
+
+template <typename S>
+__global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ NSArgs A)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ NTab<S> T;
+    if (threadIdx.x < 9) {
+        const int k = threadIdx.x;
+        T.inv[k] = conv<S>(A.inv[k]);
+        T.cs[k] = conv<S>(A.cs[k]);
+        T.cxi[k] = conv<S>(A.cx * A.inv[k]);
+        T.cyi[k] = conv<S>(A.cy * A.inv[k]);
     }
-}
-
-// FP32 cycle: its level-0 right-hand side from the FP64 Krylov residual, and
-// the preconditioned residual back in FP64
-__global__ void k_ns_to32(NLevel L, const double* __restrict__ r, float* __restrict__ r32)
-{
-    int J, I;
-    if (!cell(L, J, I)) return;
-    const long long k = cidx(L, J, I);
-    r32[k] = (float)r[k];
-}
-
-__global__ void k_ns_to64(NLevel L, const float* __restrict__ z32, double* __restrict__ z)
-{
-    int J, I;
-    if (!cell(L, J, I)) return;
-    const long long k = cidx(L, J, I);
-    z[k] = (double)z32[k];
-}
-
-// ---- Krylov ----------------------------------------------------------------
-__global__ void k_ns_sum(NLevel L, const double* __restrict__ a, DevScalars* sc,
-                         double* partials)
-{
-    int J, I;
-    double w[1] = {0.0};
-    if (cell(L, J, I)) {
-        const long long k = cidx(L, J, I);
-        if (L.m[k]) w[0] = a[k];
-    }
-    if (grid_reduce<1, false>(w, partials, &sc->counter[0])) sc->t = w[0];  // the sum
-}
-
-// b -= mean(b); r = b - A x; <b,b>, <r,r>; start state
-__global__ void k_ns_init(NLevel L, double* __restrict__ r, DevScalars* sc, double* partials,
-                          NGlobals* eg, long long nfluid, cudaGraphConditionalHandle cond)
-{
-    int J, I;
-    double w[2] = {0.0, 0.0};
-    const double mean = sc->t / (double)nfluid;
-    if (cell(L, J, I)) {
-        const long long k = cidx(L, J, I);
+    __shared__ struct {
+        double mean, bb, goal, rr, xsum, rz, irz, d, alpha, beta;
+        int done, status;
+    } c;
+    DevScalars* sc = (DevScalars*)A.sc;
+    PSGrid g = {(PSBar*)A.bar, &A.eg->status, 0u};
+    const NLevel& L = A.lev[0];
+    const unsigned G = gridDim.x;
+    // totals: <r, z>, <z, w> | <r, r>, sum x | sum b | <b, b>, <r, r>, sum x
+    double *pz = A.part, *pr = A.part + 2 * G, *pi = A.part + 4 * G, *pb = A.part + 5 * G;
+    // b -= mean(b)
+    double vb[1] = {0.0};
+    n_cells(L, [&](int, int, long long k) { if (L.code[k]) vb[0] += A.b[k]; });
+    ps_block_total<1>(vb, pi);
+    if (!ps_sync(g)) return;
+    ps_grid_total<1>(pi, [&](const double* t) { c.mean = t[0] / A.nfluid; });
+    // r = b - A x
+    double v[3] = {0.0, 0.0, 0.0};
+    n_cells(L, [&](int J, int I, long long k) {
+        const uint8_t cd = L.code[k];
         double rv = 0.0;
-        if (L.m[k]) {
-            double* b = (double*)L.b;
-            const double bv = b[k] - mean;
-            b[k] = bv;
-            rv = bv - n_apply<double>(L, (const double*)L.x, J, I, nullptr);
-            w[0] = bv * bv;
-            w[1] = rv * rv;
+        if (cd) {
+            const double bv = A.b[k] - c.mean, xc = A.x[k];
+            const long long kw = I > 0 ? k - 1 : k + L.nxn - 1;
+            const long long ke = I + 1 < L.nxn ? k + 1 : k - I;
+            const double dw = cd & 2 ? A.x[kw] - xc : 0.0, de = cd & 4 ? A.x[ke] - xc : 0.0;
+            const double ds = cd & 8 ? A.x[k - L.pitch] - xc : 0.0;
+            const double dn = cd & 16 ? A.x[k + L.pitch] - xc : 0.0;
+            rv = bv - (A.cx * (dw + de) + A.cy * (ds + dn));
+            A.b[k] = bv;
+            v[0] += bv * bv;
+            v[1] += rv * rv;
+            v[2] += xc;
         }
-        r[k] = rv;
-    }
-    if (grid_reduce<2, false>(w, partials, &sc->counter[1])) {
-        sc->bb = w[0];
-        sc->rr = w[1];
-        sc->iter = 0;
-        const int zero = w[0] == 0.0;
-        sc->converged = zero || w[1] <= sc->tol2 * w[0];
-        if (cond) cudaGraphSetConditional(cond, sc->converged ? 0u : 1u);
-    }
-}
-
-// rz = <r, z>, beta
-__global__ void k_ns_rz(NLevel L, const double* __restrict__ r, const double* __restrict__ z,
-                        DevScalars* sc, double* partials)
-{
-    int J, I;
-    double w[1] = {0.0};
-    if (cell(L, J, I)) {
-        const long long k = cidx(L, J, I);
-        if (L.m[k]) w[0] = r[k] * z[k];
-    }
-    if (grid_reduce<1, false>(w, partials, &sc->counter[2])) {
-        sc->beta = sc->iter == 0 ? 0.0 : w[0] / sc->rz;
-        sc->rz = w[0];
-    }
-}
-
-// p = z + beta p
-__global__ void k_ns_p(NLevel L, const double* __restrict__ z, double* __restrict__ p,
-                       const DevScalars* sc)
-{
-    int J, I;
-    if (!cell(L, J, I)) return;
-    const long long k = cidx(L, J, I);
-    const double beta = sc->beta;
-    p[k] = L.m[k] ? (sc->iter == 0 ? z[k] : z[k] + beta * p[k]) : 0.0;
-}
-
-// q = A p, <p, q>, alpha
-__global__ void k_ns_q(NLevel L, const double* __restrict__ p, double* __restrict__ q,
-                       DevScalars* sc, double* partials)
-{
-    int J, I;
-    double w[1] = {0.0};
-    if (cell(L, J, I)) {
-        const long long k = cidx(L, J, I);
-        double qv = 0.0;
-        if (L.m[k]) {
-            qv = n_apply<double>(L, p, J, I, nullptr);
-            w[0] = p[k] * qv;
+        A.r[0][k] = rv;
+    });
+    ps_block_total<3>(v, pb);
+    if (!ps_sync(g)) return;
+    ps_grid_total<3>(pb, [&](const double* t) {
+        c.bb = t[0];
+        c.rr = t[1];
+        c.xsum = t[2];
+        c.goal = sc->tol2 * t[0];
+        c.done = t[0] == 0.0 || t[1] <= c.goal;
+        c.status = 0;
+        c.alpha = c.beta = c.irz = c.d = 0.0;
+    });
+    const int maxit = sc->maxit;
+    int it = 0;
+    // the decision after the update of iteration it: warps 1 and 2, while
+    // thread 0 waits at the next barrier (the phase before it is lost when
+    // the solve is over, but its totals cost no time)
+    auto decide = [&] {
+        const int w = threadIdx.x >> 5;
+        if (it == 0 || w > 2) return;
+        const double a = ps_total(pr, w - 1);
+        if (threadIdx.x & 31) return;
+        if (w == 2) {
+            c.xsum = a;
+            return;
         }
-        q[k] = qv;
-    }
-    if (grid_reduce<1, false>(w, partials, &sc->counter[3])) {
-        sc->pq = w[0];
-        sc->alpha = sc->rz / w[0];
-    }
-}
-
-// x += alpha p, r -= alpha q, <r,r>, convergence, loop condition
-__global__ void k_ns_xr(NLevel L, const double* __restrict__ p, const double* __restrict__ q,
-                        double* __restrict__ r, DevScalars* sc, double* partials, NGlobals* eg,
-                        cudaGraphConditionalHandle cond)
-{
-    int J, I;
-    double w[1] = {0.0};
-    const double a = sc->alpha;
-    if (cell(L, J, I)) {
-        const long long k = cidx(L, J, I);
-        if (L.m[k]) {
-            ((double*)L.x)[k] += a * p[k];
-            const double rv = r[k] - a * q[k];
-            r[k] = rv;
-            w[0] = rv * rv;
+        c.rr = a;
+        if (!(a == a)) c.status = ST_NONFINITE;
+        else if (a > c.goal && it >= maxit) c.status = ST_PCG_MAXIT;
+        c.done = c.status || a <= c.goal;
+    };
+    while (!c.done) {
+        double t[2] = {0.0, 0.0};
+        if (A.ng > 0) n_phase_a<S>(A, it, c.alpha, c.beta, t, smem, T);
+        else n_dense_a<S>(A, it, c.alpha, c.beta, t);
+        if (it > 0) ps_block_total<2>(t, pr);
+        if (!ps_sync(g)) return;
+        for (int l = 1; l < A.ng; ++l) {
+            n_down<S>(A, l, smem, T);
+            if (!(l == 1 ? ps_sync(g, decide) : ps_sync(g))) return;
+            if (l == 1 && c.done) break;
         }
-    }
-    if (grid_reduce<1, false>(w, partials, &sc->counter[4])) {
-        sc->rr = w[0];
-        sc->iter += 1;
-        sc->total_iters += 1;
-        eg->iters += 1;
-        const bool bad = !(w[0] == w[0]);
-        bool conv = bad || w[0] <= sc->tol2 * sc->bb;
-        if (bad) eg->status |= ST_NONFINITE;
-        if (!conv && sc->iter >= sc->maxit) {
-            eg->status |= ST_PCG_MAXIT;
-            conv = true;
+        if (c.done) break;
+        const NLevel& D = A.lev[A.ng];
+        ps_dense<S>((const S*)A.minv, (const S*)D.b, (S*)D.x, A.nd, (S*)smem);
+        if (!(A.ng <= 1 ? ps_sync(g, decide) : ps_sync(g))) return;
+        if (c.done) break;
+        for (int l = A.ng - 1; l >= 1; --l) {
+            n_up<S>(A, l, smem, T);
+            if (!ps_sync(g)) return;
         }
-        sc->converged = conv;
-        if (cond) cudaGraphSetConditional(cond, conv ? 0u : 1u);
+        t[0] = t[1] = 0.0;
+        if (A.ng > 0) n_phase_b<S>(A, it, t, smem, T);
+        else n_dense_b<S>(A, t);
+        ps_block_total<2>(t, pz);
+        if (!ps_sync(g)) return;
+        ps_grid_total<2>(pz, [&](const double* u) {
+            // beta = rz / rz_old and <p, A p> = <z, w> - beta^2 <p, A p>_old,
+            // alpha = rz / <p, A p>
+            c.beta = u[0] * c.irz;
+            c.d = u[1] - c.beta * c.beta * c.d;
+            c.alpha = u[0] / c.d;
+            c.rz = u[0];
+        });
+        if (threadIdx.x == 0) c.irz = 1.0 / c.rz;  // for the next beta
+        ++it;
+    }
+    // zero-mean solution (its sum was formed with the last update)
+    const double xm = c.xsum / A.nfluid;
+    n_cells(L, [&](int, int, long long k) { if (L.code[k]) A.x[k] -= xm; });
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        sc->bb = c.bb;
+        sc->rr = c.rr;
+        sc->iter = it;
+        sc->converged = 1;
+        sc->total_iters += it;
+        A.eg->iters += it;
+        if (c.status) A.eg->status |= c.status;
     }
 }
 
-// x -= mean(x) over the fluid cells (mean = sc->t / nfluid)
-__global__ void k_ns_center(NLevel L, const DevScalars* sc, long long nfluid)
-{
-    int J, I;
-    if (!cell(L, J, I)) return;
-    const long long k = cidx(L, J, I);
-    if (L.m[k]) ((double*)L.x)[k] -= sc->t / (double)nfluid;
-}
-
-__global__ void k_ns_setup(DevScalars* sc, double tol2, int maxit)
+__global__ void k_ns_setup(DevScalars* sc, double tol2, int maxit, PSBar* bar)
 {
     sc->tol2 = tol2;
     sc->maxit = maxit;
     sc->converged = 0;
     sc->iter = 0;
+    bar->count = 0u;
+    bar->abort = 0;
 }
 
 // ---- host ----------------------------------------------------------------------
-static dim3 ngrid(const NLevel& L) { return dim3((L.nxn + 31) / 32, (L.nyn + 7) / 8); }
-// the cells of one colour: half the columns
-static dim3 ngrid_half(const NLevel& L)
+int ns_record(NSolver& s, cudaStream_t st, int* launches)
 {
-    return dim3(((L.nxn + 1) / 2 + 31) / 32, (L.nyn + 7) / 8);
+    k_ns_setup<<<1, 1, 0, st>>>(s.sc, s.tol * s.tol, s.maxit, (PSBar*)s.a.bar);
+    void* args[1] = {&s.a};
+    const void* kern = s.prec == 0 ? (const void*)k_ns_solve<double>
+                                   : (const void*)k_ns_solve<float>;
+    int e = (int)cudaGetLastError();
+    if (!e) e = ps_launch(kern, s.grid, s.smem, args, st);
+    if (launches) *launches = 2;
+    return e;
 }
 
-template <typename S>
-static int ns_vcycle_t(NSolver& s, cudaStream_t st)
+// Tiles of a level: of the partitions into even widths and heights that fit
+// the shared memory, the one with the smallest estimate of the busiest
+// block's time, (its tiles) x (a fixed cost + the FP64 or FP32 cycles of the
+// cells its leg visits, the halo among them). Up to about 1300^2 cells that
+// is one tile per block: its halo is small, and nothing is left over.
+constexpr size_t NS_SMEM = 200 * 1024;
+static void pick_tile(NLevel& L, int sms, int prec, int h, size_t cell_bytes)
 {
-    const dim3 blk(32, 8);
-    const int nl = (int)s.lev.size();
-    int cnt = 0;
-    // level 0 of the cycle: x = z (from zero), b = r
-    for (int l = 0; l < nl - 1; ++l) {
-        // x = 0 before the pre-smoothing (coarse levels: set by the restriction)
-        if (l == 0) k_ns_zero<S><<<ngrid(s.lev[l]), blk, 0, st>>>(s.dlev, l);
-        for (int k = 0; k < s.nu; ++k) {
-            k_ns_smooth<S><<<ngrid_half(s.lev[l]), blk, 0, st>>>(s.dlev, l, 0);
-            k_ns_smooth<S><<<ngrid_half(s.lev[l]), blk, 0, st>>>(s.dlev, l, 1);
-        }
-        k_ns_restrict<S><<<ngrid(s.lev[l + 1]), blk, 0, st>>>(s.dlev, l);
-        cnt += (l == 0 ? 2 : 1) + 2 * s.nu;
-    }
-    k_ns_coarse<S><<<1, 1024, 0, st>>>(s.dlev, nl - 1, s.ksweeps);
-    cnt += 1;
-    for (int l = nl - 2; l >= 0; --l) {
-        k_ns_prolong<S><<<ngrid(s.lev[l]), blk, 0, st>>>(s.dlev, l);
-        for (int k = 0; k < s.nu; ++k) {
-            k_ns_smooth<S><<<ngrid_half(s.lev[l]), blk, 0, st>>>(s.dlev, l, 1);
-            k_ns_smooth<S><<<ngrid_half(s.lev[l]), blk, 0, st>>>(s.dlev, l, 0);
-        }
-        cnt += 1 + 2 * s.nu;
-    }
-    return cnt;
-}
-
-// z = M r: the FP64 cycle works on z and r in place; the FP32 cycle on
-// FP32 copies (r -> r32, cycle, z32 -> z)
-static int ns_vcycle(NSolver& s, cudaStream_t st)
-{
-    if (s.prec == 0) return ns_vcycle_t<double>(s, st);
-    const dim3 blk(32, 8), gr = ngrid(s.prob);
-    k_ns_to32<<<gr, blk, 0, st>>>(s.prob, s.r, s.r32);
-    const int c = ns_vcycle_t<float>(s, st);
-    k_ns_to64<<<gr, blk, 0, st>>>(s.prob, s.z32, s.z);
-    return c + 2;
-}
-
-static int ns_body(NSolver& s, cudaStream_t st, cudaGraphConditionalHandle cond, int* cnt)
-{
-    const dim3 blk(32, 8);
-    const NLevel& P = s.prob;  // the Krylov level: FP64 couplings, level-0 layout
-    NLevel prob = P;           // the problem (x = the pressure)
-    prob.x = s.lev_x0;
-    const dim3 gr = ngrid(P);
-    int c = ns_vcycle(s, st);
-    k_ns_rz<<<gr, blk, 0, st>>>(P, s.r, s.z, s.sc, s.partials);
-    k_ns_p<<<gr, blk, 0, st>>>(P, s.z, s.p, s.sc);
-    k_ns_q<<<gr, blk, 0, st>>>(P, s.p, s.q, s.sc, s.partials);
-    k_ns_xr<<<gr, blk, 0, st>>>(prob, s.p, s.q, s.r, s.sc, s.partials, s.eg, cond);
-    c += 4;
-    if (cnt) *cnt = c;
-    return (int)cudaGetLastError();
-}
-
-int ns_record(NSolver& s, cudaStream_t st, cudaStream_t st2, bool eager, int* launches)
-{
-    const dim3 blk(32, 8);
-    NLevel prob = s.prob;
-    prob.x = s.lev_x0;
-    prob.b = s.lev_b0;
-    const dim3 gr = ngrid(prob);
-    int fixed = 0;
-    k_ns_setup<<<1, 1, 0, st>>>(s.sc, s.tol * s.tol, s.maxit);
-    k_ns_sum<<<gr, blk, 0, st>>>(prob, (const double*)prob.b, s.sc, s.partials);
-    fixed += 2;
-    cudaGraphConditionalHandle cond = 0;
-    if (!eager) {
-        cudaStreamCaptureStatus cs;
-        cudaGraph_t graph = nullptr;
-        cudaError_t e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &graph, nullptr, nullptr,
-                                                 nullptr);
-        if (e != cudaSuccess) return (int)e;
-        if (cs != cudaStreamCaptureStatusActive) return 1;
-        e = cudaGraphConditionalHandleCreate(&cond, graph, 1, cudaGraphCondAssignDefault);
-        if (e != cudaSuccess) return (int)e;
-    }
-    k_ns_init<<<gr, blk, 0, st>>>(prob, s.r, s.sc, s.partials, s.eg, s.nfluid, cond);
-    fixed += 1;
-    if (!eager) {
-        int r = add_while(st, st2, &cond, 1, [&](cudaStream_t sb) {
-            return ns_body(s, sb, cond, nullptr);
-        });
-        if (r) return r;
-    } else {
-        for (int it = 0; it <= s.maxit; ++it) {
-            DevScalars h;
-            if (cudaMemcpyAsync(&h, s.sc, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                cudaStreamSynchronize(st) != cudaSuccess)
-                return 2;
-            if (h.converged) break;
-            int r = ns_body(s, st, 0, nullptr);
-            if (r) return r;
+    const double per = prec == 0 ? 2.5 : 0.5;  // cycles of a visited cell
+    const int cap = L.seam ? NS_SEAM_T : 1 << 20;
+    double best = 0.0;
+    for (int ntx = 1; ntx <= (L.nxn + 7) / 8 || ntx == 1; ++ntx) {
+        const int tw = ((L.nxn + ntx - 1) / ntx + 1) / 2 * 2;
+        if (tw > cap || (L.nxn + tw - 1) / tw != ntx) continue;
+        for (int nty = 1; nty <= (L.nyn + 7) / 8 || nty == 1; ++nty) {
+            const int th = ((L.nyn + nty - 1) / nty + 1) / 2 * 2;
+            if (th > cap || (L.nyn + th - 1) / th != nty) continue;
+            const size_t n = (size_t)(tw + 2 * h) * (th + 2 * h);
+            if (n * cell_bytes > NS_SMEM) continue;
+            double cells = (double)n + (double)tw * th;
+            for (int q = 0; q < 4; ++q) cells += 0.5 * (tw + 2 * q) * (th + 2 * q);
+            const long long nt = (long long)ntx * nty;
+            const double cost = (double)((nt + sms - 1) / sms) * (1500.0 + per * cells);
+            if (best == 0.0 || cost < best) {
+                best = cost;
+                L.tw = tw;
+                L.th = th;
+                L.ntx = ntx;
+                L.nt = (int)nt;
+            }
         }
     }
-    // zero-mean solution
-    k_ns_sum<<<gr, blk, 0, st>>>(prob, (const double*)prob.x, s.sc, s.partials);
-    k_ns_center<<<gr, blk, 0, st>>>(prob, s.sc, s.nfluid);
-    fixed += 2;
-    if (launches) *launches = fixed;
-    return (int)cudaGetLastError();
+}
+
+// The dense level's inverse: of -A with one cell of every connected part
+// grounded, the parts' constants projected out of it (its pseudo-inverse);
+// dry cells and cells without couplings keep x = 0.
+static int dense_inverse(const std::vector<double>& fx, const std::vector<double>& fy, int nyn,
+                         int nxn, int per, double cx, double cy, int prec, void* out)
+{
+    const int n = nyn * nxn, bw = nxn, w1 = bw + 1;
+    std::vector<double> h((size_t)n * w1, 0.0);  // h[i w1 + k] = H(i, i - k)
+    std::vector<int> part(n);
+    std::iota(part.begin(), part.end(), 0);
+    auto root = [&](int k) {
+        while (part[k] != k) k = part[k] = part[part[k]];
+        return k;
+    };
+    auto link = [&](int a, int b, double c) {
+        if (c == 0.0) return;
+        h[(size_t)a * w1] += c;
+        h[(size_t)b * w1] += c;
+        h[(size_t)std::max(a, b) * w1 + std::abs(a - b)] -= c;
+        part[root(a)] = root(b);
+    };
+    for (int J = 0; J < nyn; ++J)
+        for (int I = 0; I < nxn; ++I) {
+            const int k = J * nxn + I;
+            if (I > 0) link(k, k - 1, fx[k]);
+            else if (per && nxn > 1) link(k, k + nxn - 1, fx[k]);
+            if (J > 0) link(k, k - nxn, fy[k]);
+        }
+    for (int k = 0; k < n; ++k) part[k] = root(k);
+    std::vector<int> size(n, 0);
+    for (int k = 0; k < n; ++k) size[part[k]] += 1;
+    for (int k = 0; k < n; ++k) {
+        if (size[part[k]] == 1) {
+            h[(size_t)k * w1] = 1.0;
+            part[k] = -1;
+        } else if (part[k] == k) {
+            h[(size_t)k * w1] += cx + cy;
+        }
+    }
+    return ps_invert(h, n, bw, part, -1.0, prec, out);
 }
 
 int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int per,
@@ -450,18 +820,6 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
     ns_free(s);
     s.prec = prec;
     const size_t es = prec == 0 ? 8 : 4;
-    // host couplings in the cycle's precision
-    auto conv = [&](const std::vector<double>& v) {
-        std::vector<unsigned char> out(v.size() * es);
-        for (size_t k = 0; k < v.size(); ++k) {
-            if (es == 8) memcpy(&out[k * 8], &v[k], 8);
-            else {
-                const float f = (float)v[k];
-                memcpy(&out[k * 4], &f, 4);
-            }
-        }
-        return out;
-    };
     auto dal = [&](size_t bytes) -> void* {
         void* p = nullptr;
         if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
@@ -469,7 +827,21 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
         s.owned.push_back(p);
         return p;
     };
-    // level 0 in the model layout; coarse levels dense with 32-element pitch
+    // a device array of n host values in the cycle's precision
+    auto up = [&](const std::vector<double>& v) -> void* {
+        void* p = dal(v.size() * es);
+        if (!p) return nullptr;
+        std::vector<float> f;
+        const void* src = v.data();
+        if (prec) {
+            f.assign(v.begin(), v.end());
+            src = f.data();
+        }
+        return cudaMemcpy(p, src, v.size() * es, cudaMemcpyHostToDevice) == cudaSuccess ? p
+                                                                                       : nullptr;
+    };
+    const int sms = ps_sms();
+    if (sms < 1) return 3;
     std::vector<uint8_t> m((size_t)nyn * nxn);
     long long nf = 0;
     for (int J = 0; J < nyn; ++J)
@@ -478,158 +850,149 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
             nf += m[(size_t)J * nxn + I];
         }
     if (nf == 0) return 6;
-    s.nfluid = nf;
     std::vector<double> fx((size_t)nyn * nxn, 0.0), fy((size_t)nyn * nxn, 0.0);
+    const size_t n0 = (size_t)(off + (long long)nyn * pitch);
+    std::vector<uint8_t> code(n0, 0);
     for (int J = 0; J < nyn; ++J)
         for (int I = 0; I < nxn; ++I) {
-            const bool c = m[(size_t)J * nxn + I];
-            if (!c) continue;
-            if (I > 0 && m[(size_t)J * nxn + I - 1]) fx[(size_t)J * nxn + I] = cx;
-            if (I == 0 && per && m[(size_t)J * nxn + nxn - 1]) fx[(size_t)J * nxn] = cx;
-            if (J > 0 && m[(size_t)(J - 1) * nxn + I]) fy[(size_t)J * nxn + I] = cy;
+            const size_t k = (size_t)J * nxn + I;
+            if (!m[k]) continue;
+            const bool w = I > 0 ? m[k - 1] : per && nxn > 1 && m[k + nxn - 1];
+            const bool e = I + 1 < nxn ? m[k + 1] : per && nxn > 1 && m[k - I];
+            const bool so = J > 0 && m[k - nxn];
+            const bool no = J + 1 < nyn && m[k + nxn];
+            if (w) fx[k] = cx;
+            if (so) fy[k] = cy;
+            code[off + (size_t)J * pitch + I] =
+                (uint8_t)(1 | (w ? 2 : 0) | (e ? 4 : 0) | (so ? 8 : 0) | (no ? 16 : 0));
         }
-    const size_t n0 = (size_t)(off + (long long)nyn * pitch);
-    s.r = (double*)dal(n0 * 8);
-    s.z = (double*)dal(n0 * 8);
-    s.p = (double*)dal(n0 * 8);
-    s.q = (double*)dal(n0 * 8);
-    double* fx0 = (double*)dal(n0 * 8);
-    double* fy0 = (double*)dal(n0 * 8);
-    uint8_t* m0 = (uint8_t*)dal(n0);
-    if (!s.r || !s.z || !s.p || !s.q || !fx0 || !fy0 || !m0) return 2;
-    {
-        std::vector<double> hx(n0, 0.0), hy(n0, 0.0);
-        std::vector<uint8_t> hm(n0, 0);
-        for (int J = 0; J < nyn; ++J)
-            for (int I = 0; I < nxn; ++I) {
-                const size_t k = (size_t)(off + (long long)J * pitch + I);
-                hx[k] = fx[(size_t)J * nxn + I];
-                hy[k] = fy[(size_t)J * nxn + I];
-                hm[k] = m[(size_t)J * nxn + I];
-            }
-        if (cudaMemcpy(fx0, hx.data(), n0 * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(fy0, hy.data(), n0 * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(m0, hm.data(), n0, cudaMemcpyHostToDevice) != cudaSuccess)
-            return 2;
+    NSArgs& a = s.a;
+    memset(&a, 0, sizeof(a));
+    a.cx = cx;
+    a.cy = cy;
+    a.nfluid = (double)nf;
+    for (int k = 0; k < 9; ++k) {
+        a.cs[k] = (k / 3) * cx + (k % 3) * cy;
+        a.inv[k] = a.cs[k] > 0.0 ? 1.0 / a.cs[k] : 0.0;
     }
-    NLevel L0;
-    memset(&L0, 0, sizeof(L0));
-    L0.fx = fx0;
-    L0.fy = fy0;
-    L0.m = m0;
-    L0.nyn = nyn;
-    L0.nxn = nxn;
+    a.x = x;
+    a.b = b;
+    double* vec[6];
+    for (auto& p : vec)
+        if (!(p = (double*)dal(n0 * 8))) return 2;
+    a.r[0] = vec[0];
+    a.r[1] = vec[1];
+    a.s[0] = vec[2];
+    a.s[1] = vec[3];
+    a.p = vec[4];
+    a.w = vec[5];
+    NLevel& L0 = a.lev[0];
+    uint8_t* dc = (uint8_t*)dal(n0);
+    if (!dc) return 2;
+    if (cudaMemcpy(dc, code.data(), n0, cudaMemcpyHostToDevice) != cudaSuccess) return 2;
+    L0.code = dc;
     L0.pitch = pitch;
     L0.off = off;
+    L0.nyn = nyn;
+    L0.nxn = nxn;
     L0.per = per;
-    s.prob = L0;  // the Krylov level (x, b set per record)
-    if (prec == 0) {
-        L0.x = s.z;  // the cycle's level 0: x = z, b = r
-        L0.b = s.r;
+    L0.seam = per && (nxn % 2);
+    // coarse levels (2x2 agglomerates) down to the dense one, which is level 0
+    // when that is small enough: then the preconditioner is the inverse and
+    // CG ends after one or two iterations (40^2: 1.6 instead of 9)
+    int ny = nyn, nx = nxn, l = 0;
+    if (ps_band_ok((long long)nyn * nxn, nxn)) {
+        L0.x = dal((size_t)nyn * nxn * es);
+        L0.b = dal((size_t)nyn * nxn * es);
+        if (!L0.x || !L0.b) return 2;
     } else {
-        // FP32 cycle: its own x, b and couplings in the level-0 layout
-        s.r32 = (float*)dal(n0 * 4);
-        s.z32 = (float*)dal(n0 * 4);
-        void* f32x = dal(n0 * 4);
-        void* f32y = dal(n0 * 4);
-        if (!s.r32 || !s.z32 || !f32x || !f32y) return 2;
-        std::vector<double> hx(n0, 0.0), hy(n0, 0.0);
-        for (int J = 0; J < nyn; ++J)
-            for (int I = 0; I < nxn; ++I) {
-                const size_t k = (size_t)(off + (long long)J * pitch + I);
-                hx[k] = fx[(size_t)J * nxn + I];
-                hy[k] = fy[(size_t)J * nxn + I];
-            }
-        const std::vector<unsigned char> cx4 = conv(hx), cy4 = conv(hy);
-        if (cudaMemcpy(f32x, cx4.data(), n0 * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(f32y, cy4.data(), n0 * 4, cudaMemcpyHostToDevice) != cudaSuccess)
-            return 2;
-        L0.x = s.z32;
-        L0.b = s.r32;
-        L0.fx = f32x;
-        L0.fy = f32y;
+        a.z = dal(n0 * es);
+        L0.xa = dal(n0 * es);
+        if (!a.z || !L0.xa) return 2;
+        pick_tile(L0, sms, prec, NS_H, 2 * es + 1);
     }
-    s.lev.push_back(L0);
-    s.lev_x0 = x;
-    s.lev_b0 = b;
-    // coarse levels (2x2 agglomerates; Galerkin couplings)
-    int ny = nyn, nxc = nxn;
-    while (ny > 8 && nxc > 8 && (!per || nxc % 2 == 0) && s.lev.size() < 16) {
-        const int cy_n = (ny + 1) / 2, cx_n = (nxc + 1) / 2;
-        std::vector<uint8_t> cm((size_t)cy_n * cx_n, 0);
-        std::vector<double> cfx((size_t)cy_n * cx_n, 0.0), cfy((size_t)cy_n * cx_n, 0.0);
-        for (int J = 0; J < cy_n; ++J)
-            for (int I = 0; I < cx_n; ++I) {
-                uint8_t v = 0;
+    while (!ps_band_ok((long long)ny * nx, nx)) {
+        if (l + 1 >= NS_LMAX) return 3;
+        const int cyn = (ny + 1) / 2, cxn = (nx + 1) / 2;
+        std::vector<double> cfx((size_t)cyn * cxn, 0.0), cfy((size_t)cyn * cxn, 0.0);
+        for (int J = 0; J < cyn; ++J)
+            for (int I = 0; I < cxn; ++I) {
                 double sx = 0.0, sy = 0.0;
-                for (int a = 0; a < 2; ++a)
-                    for (int c = 0; c < 2; ++c) {
-                        const int fj = 2 * J + a, fi = 2 * I + c;
-                        if (fj < ny && fi < nxc) v |= m[(size_t)fj * nxc + fi];
-                    }
-                // faces crossing the coarse west face: fine x-faces at column 2I
-                for (int a = 0; a < 2; ++a) {
-                    const int fj = 2 * J + a;
-                    if (fj < ny && 2 * I < nxc) sx += fx[(size_t)fj * nxc + 2 * I];
+                // fine x-faces at column 2I, y-faces at row 2J
+                for (int q = 0; q < 2; ++q) {
+                    if (2 * J + q < ny) sx += fx[(size_t)(2 * J + q) * nx + 2 * I];
+                    if (2 * I + q < nx) sy += fy[(size_t)(2 * J) * nx + 2 * I + q];
                 }
-                // faces crossing the coarse south face: fine y-faces at row 2J
-                for (int c = 0; c < 2; ++c) {
-                    const int fi = 2 * I + c;
-                    if (2 * J < ny && fi < nxc) sy += fy[(size_t)(2 * J) * nxc + fi];
-                }
-                cm[(size_t)J * cx_n + I] = v;
-                cfx[(size_t)J * cx_n + I] = 0.5 * sx;
-                cfy[(size_t)J * cx_n + I] = 0.5 * sy;
+                cfx[(size_t)J * cxn + I] = 0.5 * sx;
+                cfy[(size_t)J * cxn + I] = 0.5 * sy;
             }
-        NLevel C;
-        memset(&C, 0, sizeof(C));
-        C.nyn = cy_n;
-        C.nxn = cx_n;
-        C.pitch = (cx_n + 31) / 32 * 32;
+        // one coarse column: the wrap face joins the cell to itself
+        if (per && cxn == 1) std::fill(cfx.begin(), cfx.end(), 0.0);
+        ++l;
+        NLevel& C = a.lev[l];
+        const bool dense = ps_band_ok((long long)cyn * cxn, cxn);
+        C.nyn = cyn;
+        C.nxn = cxn;
+        C.pitch = dense ? cxn : (cxn + 31) / 32 * 32;
         C.off = 0;
         C.per = per;
-        const size_t n = (size_t)C.pitch * cy_n;
-        void* dx_ = dal(n * es);
-        void* db_ = dal(n * es);
-        void* dfx = dal(n * es);
-        void* dfy = dal(n * es);
-        uint8_t* dm = (uint8_t*)dal(n);
-        if (!dx_ || !db_ || !dfx || !dfy || !dm) return 2;
-        std::vector<double> hx(n, 0.0), hy(n, 0.0);
-        std::vector<uint8_t> hm(n, 0);
-        for (int J = 0; J < cy_n; ++J)
-            for (int I = 0; I < cx_n; ++I) {
-                hx[(size_t)J * C.pitch + I] = cfx[(size_t)J * cx_n + I];
-                hy[(size_t)J * C.pitch + I] = cfy[(size_t)J * cx_n + I];
-                hm[(size_t)J * C.pitch + I] = cm[(size_t)J * cx_n + I];
-            }
-        const std::vector<unsigned char> hxs = conv(hx), hys = conv(hy);
-        if (cudaMemcpy(dfx, hxs.data(), n * es, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(dfy, hys.data(), n * es, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(dm, hm.data(), n, cudaMemcpyHostToDevice) != cudaSuccess)
-            return 2;
-        C.x = dx_;
-        C.b = db_;
-        C.fx = dfx;
-        C.fy = dfy;
-        C.m = dm;
-        s.lev.push_back(C);
-        m.swap(cm);
+        C.seam = per && (cxn % 2);
+        const size_t n = (size_t)C.pitch * cyn;
+        C.x = dal(n * es);
+        C.b = dal(n * es);
+        if (!C.x || !C.b) return 2;
         fx.swap(cfx);
         fy.swap(cfy);
-        ny = cy_n;
-        nxc = cx_n;
+        ny = cyn;
+        nx = cxn;
+        if (dense) continue;  // (the last)
+        C.xa = dal(n * es);
+        std::vector<double> hx(n, 0.0), hy(n, 0.0), hi(n, 0.0);
+        for (int J = 0; J < cyn; ++J)
+            for (int I = 0; I < cxn; ++I) {
+                const size_t k = (size_t)J * cxn + I, g = (size_t)J * C.pitch + I;
+                const double fe = I + 1 < cxn ? fx[k + 1] : (per ? fx[k - I] : 0.0);
+                const double fn = J + 1 < cyn ? fy[k + cxn] : 0.0;
+                const double cs = (fx[k] + fe) + (fy[k] + fn);
+                hx[g] = fx[k];
+                hy[g] = fy[k];
+                hi[g] = cs > 0.0 ? 1.0 / cs : 0.0;
+            }
+        C.fx = up(hx);
+        C.fy = up(hy);
+        C.inv = up(hi);
+        if (!C.xa || !C.fx || !C.fy || !C.inv) return 2;
+        pick_tile(C, sms, prec, 4, 5 * es);
     }
-    s.ksweeps = std::min(64, std::max(4, std::max(ny, nxc)));
-    s.dlev = (NLevel*)dal(sizeof(NLevel) * s.lev.size());
+    a.ng = l;
+    a.nd = ny * nx;
+    void* minv = dal((size_t)a.nd * a.nd * es);
+    if (!minv) return 2;
+    int rc = dense_inverse(fx, fy, ny, nx, per, cx, cy, prec, minv);
+    if (rc) return rc;
+    a.minv = minv;
+    // every SM also for small problems: the rows of the dense level are dealt
+    // to all blocks, and a barrier of 152 blocks (1.36 us) costs hardly more
+    // than one of 25 (1.28 us)
+    s.grid = sms;
+    s.smem = (size_t)(a.nd + 4 * ((a.nd + sms - 1) / sms)) * es;
+    for (int q = 0; q < a.ng; ++q) {
+        const int h = q == 0 ? NS_H : 4;
+        const size_t n = (size_t)(a.lev[q].tw + 2 * h) * (a.lev[q].th + 2 * h);
+        s.smem = std::max(s.smem, q == 0 ? n * (2 * es + 1) : n * 5 * es);
+    }
+    const void* kern = prec == 0 ? (const void*)k_ns_solve<double> : (const void*)k_ns_solve<float>;
+    // (the attribute is per kernel: never lowered below another solver's need)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NS_SMEM) !=
+        cudaSuccess)
+        return 3;
     s.eg = (NGlobals*)dal(sizeof(NGlobals));
     s.sc = (DevScalars*)dal(sizeof(DevScalars));
-    const size_t nb = (size_t)((nxn + 31) / 32) * ((nyn + 7) / 8) + 64;
-    s.partials = (double*)dal(nb * 2 * sizeof(double));
-    if (!s.dlev || !s.eg || !s.sc || !s.partials) return 2;
-    if (cudaMemcpy(s.dlev, s.lev.data(), sizeof(NLevel) * s.lev.size(),
-                   cudaMemcpyHostToDevice) != cudaSuccess)
-        return 2;
+    a.part = (double*)dal((size_t)8 * sms * sizeof(double));
+    a.bar = dal(sizeof(PSBar));
+    if (!s.eg || !s.sc || !a.part || !a.bar) return 2;
+    a.eg = s.eg;
+    a.sc = s.sc;
     return 0;
 }
 
@@ -637,13 +1000,9 @@ void ns_free(NSolver& s)
 {
     for (void* p : s.owned) cudaFree(p);
     s.owned.clear();
-    s.lev.clear();
-    s.dlev = nullptr;
+    s.a = NSArgs{};
     s.eg = nullptr;
     s.sc = nullptr;
-    s.partials = nullptr;
-    s.r = s.z = s.p = s.q = nullptr;
-    s.r32 = s.z32 = nullptr;
 }
 
 }  // namespace f2d

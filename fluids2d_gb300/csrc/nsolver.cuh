@@ -8,41 +8,58 @@
 
 namespace f2d {
 
-// One level: cells (J, I) of nyn x nxn at off + J*pitch + I; face couplings
-// fx(J, I) between cells (J, I-1) and (J, I) (column 0: the periodic wrap
-// face, else 0), fy(J, I) between (J-1, I) and (J, I) (row 0: 0).
+constexpr int NS_LMAX = 16;  // levels, the dense one included
+
+// One grid level: cells (J, I) of nyn x nxn at off + J*pitch + I; face
+// couplings fx(J, I) between cells (J, I-1) and (J, I) (column 0: the
+// periodic wrap face, else 0), fy(J, I) between (J-1, I) and (J, I) (row 0:
+// 0), inv = 1 / (sum of a cell's four couplings), 0 where that sum is 0.
+// Level 0 has a code byte per cell instead (its couplings are cx, cy or 0).
 struct NLevel {
-    void* x;           // the level's precision (FP64; FP32 in the FP32 cycle)
+    void* x;           // the level's unknown (the cycle's precision)
+    void* xa;          // x after the pre-smoothing
     void* b;
     const void* fx;
     const void* fy;
-    const uint8_t* m;
-    int nyn, nxn;
+    const void* inv;
+    const uint8_t* code;  // level 0: bit 0 fluid, bits 1-4 open west, east, south, north
     long long pitch, off;
-    int per, pad;
+    int nyn, nxn, per;
+    int seam;          // x-periodic over an odd count: same-colour neighbours across the wrap
+    int tw, th, ntx, nt;  // tiles of tw x th cells (both even)
 };
 
 struct NGlobals {
-    unsigned int ticket[4];
     int status, pad;
     long long iters;
 };
 
+// everything the solve kernel reads, in its parameter bank
+struct NSArgs {
+    NLevel lev[NS_LMAX];
+    int ng;                // grid levels; level ng is the dense one
+    int nd;                // cells of the dense level
+    const void* minv;      // its inverse
+    double cx, cy;
+    double cs[9], inv[9];  // by 3 (open x-faces) + (open y-faces): coupling sum, its inverse
+    // FP64 vectors in the level-0 layout: solution, right-hand side, residual
+    // and s = A p (two buffers each, by the parity of the iteration), p, z, A z
+    double *x, *b, *r[2], *s[2], *p, *w;
+    void* z;               // the cycle's precision
+    double* part;          // block totals
+    void* bar;             // PSBar
+    void* sc;              // DevScalars
+    NGlobals* eg;
+    double nfluid;
+};
+
 struct NSolver {
-    std::vector<NLevel> lev;       // host copy
-    NLevel* dlev = nullptr;
+    NSArgs a = {};
     NGlobals* eg = nullptr;
     DevScalars* sc = nullptr;     // iteration state (own)
-    double* partials = nullptr;
-    double *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr;  // level-0 layout
-    float *r32 = nullptr, *z32 = nullptr;  // the FP32 cycle's level 0
-    NLevel prob;                  // the Krylov level: FP64 couplings, level-0 layout
     int prec = 0;                 // 0: FP64 cycle; 1: FP32 cycle
-    double* lev_x0 = nullptr;     // the problem: x (the pressure) and b
-    double* lev_b0 = nullptr;
-    long long nfluid = 0;
-    int ksweeps = 16;             // (R,B)^k (B,R)^k on the coarsest level
-    int nu = 2;                   // sweeps per leg
+    int grid = 0;                 // blocks of the solve kernel
+    size_t smem = 0;
     double tol = 1e-12;
     int maxit = 200;
     std::vector<void*> owned;
@@ -54,10 +71,10 @@ struct NSolver {
 int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int per,
              const uint8_t* hmask, double* x, double* b, double cx, double cy, int prec);
 void ns_free(NSolver& s);
-// Record a solve on `st` (conditional WHILE body on st2 under capture, or
-// host-driven loops otherwise): b is made zero-mean over the fluid cells (the
-// compatibility projection of the singular problem), x (warm start) is
-// iterated to |r| <= tol |b| and finally made zero-mean.
-int ns_record(NSolver& s, cudaStream_t st, cudaStream_t st2, bool eager, int* launches);
+// Record a solve on `st` (two launches, eager or captured): b is made
+// zero-mean over the fluid cells (the compatibility projection of the
+// singular problem), x (warm start) is iterated to |r| <= tol |b| and
+// finally made zero-mean.
+int ns_record(NSolver& s, cudaStream_t st, int* launches);
 
 }  // namespace f2d

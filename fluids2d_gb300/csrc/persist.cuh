@@ -1,0 +1,220 @@
+// Building blocks of the persistent solve kernels (nsolver.cu, psolver.cu): a
+// whole multigrid-preconditioned CG solve is one cooperative launch of one
+// block per SM, whose phases are separated by grid barriers instead of kernel
+// boundaries.
+//
+// Why: a CG iteration of a 256^2 .. 1024^2 model is a chain of 10 to 70 short
+// dependent steps. As kernels in a graph each costs its launch gap, the
+// dependent loads of its descriptors and the drain of its last blocks (5 to
+// 8 us for a few hundred ns of work); a grid barrier on GB300 costs about
+// 1.5 us and the descriptors stay in the kernel's parameters.
+#pragma once
+#include <vector>
+
+#include "common.cuh"
+
+namespace f2d {
+
+constexpr int PS_NT = 512;  // threads of a block (one block per SM)
+
+// ---- grid barrier ------------------------------------------------------------
+// One counter, zeroed before the launch, that every block increments once per
+// barrier; the k-th barrier is passed when it reaches k * gridDim.x. The wait
+// is bounded: after limit_ns without progress the block sets the abort word
+// and the kernel's status, and every block returns from the kernel.
+struct PSBar {
+    unsigned int count;  // arrivals
+    int abort;           // a wait ran out
+};
+
+struct PSGrid {
+    PSBar* bar;
+    int* status;
+    unsigned int target;
+};
+
+__device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p)
+{
+    unsigned int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Returns false when the kernel must return. Writes of all threads of all
+// blocks before the barrier are visible to all threads after it: the CTA
+// barrier orders them before thread 0's release, and its acquire before the
+// second CTA barrier. (Data written in the kernel is read with plain loads,
+// never through the read-only path.) While thread 0 waits, the other warps
+// run idle(): work that needs nothing of this phase and is over in less time
+// than the barrier takes.
+template <typename F>
+__device__ __forceinline__ bool ps_sync(PSGrid& g, F idle)
+{
+    __shared__ int s_dead;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        g.target += gridDim.x;
+        int dead = 0;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&g.bar->count) : "memory");
+        uint64_t t0 = 0;
+        for (unsigned spin = 0; (int)(ld_acquire(&g.bar->count) - g.target) < 0; ++spin) {
+            if ((spin & 255u) != 255u) continue;
+            const uint64_t t = globaltimer_ns();
+            if (t0 == 0) t0 = t;
+            if (t - t0 > 2000000000ull || *(volatile int*)&g.bar->abort) {
+                *(volatile int*)&g.bar->abort = 1;
+                atomicOr(g.status, ST_GRID_TIMEOUT);
+                dead = 1;
+                break;
+            }
+        }
+        s_dead = dead;
+    } else if (threadIdx.x >= 32) {
+        idle();
+    }
+    __syncthreads();
+    return s_dead == 0;
+}
+
+__device__ __forceinline__ bool ps_sync(PSGrid& g)
+{
+    return ps_sync(g, [] {});
+}
+
+// ---- deterministic sums over the blocks --------------------------------------
+// The block's totals of N <= 4 per-thread values into part[k * gridDim.x +
+// block]; after the next barrier every block adds all blocks' totals in one
+// fixed order, so all blocks hold the same bits and take the same decisions
+// without a broadcast. An FP64 instruction of a warp occupies its SM
+// partition's pipe for 64 cycles, so sums and scalar arithmetic are kept to
+// few warps: a shuffle tree in all 16 warps, or three divisions in all
+// threads, cost 1.3 us and 4.6 us of a phase of 5.
+template <int N>
+__device__ __forceinline__ void ps_block_total(const double (&v)[N], double* part)
+{
+    __shared__ double sh[N][PS_NT];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; ++k) sh[k][threadIdx.x] = v[k];
+    __syncthreads();
+    // value k: warps 4 k' .. (k' = k mod 4) hold a quarter each
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, k = w >> 2, q = w & 3;
+    if (k < N) {
+        const double* s = &sh[k][q * (PS_NT / 4) + lane];
+        double a = (s[0] + s[32]) + (s[64] + s[96]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        __syncwarp();
+        if (lane == 0) sh[k][q * (PS_NT / 4)] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x < N) {
+        const double* s = sh[threadIdx.x];
+        part[threadIdx.x * gridDim.x + blockIdx.x] =
+            (s[0] + s[PS_NT / 4]) + (s[PS_NT / 2] + s[3 * (PS_NT / 4)]);
+    }
+}
+
+// The grid's total of value k, by one whole warp (all lanes hold it)
+__device__ __forceinline__ double ps_total(const double* part, int k)
+{
+    const int lane = threadIdx.x & 31;
+    const double* p = part + (size_t)k * gridDim.x;
+    double a = 0.0, b = 0.0;
+    unsigned i = lane;
+    for (; i + 32 < gridDim.x; i += 64) {
+        a += __ldcg(&p[i]);
+        b += __ldcg(&p[i + 32]);
+    }
+    if (i < gridDim.x) a += __ldcg(&p[i]);
+    a += b;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+}
+
+// The grid's totals of N values, then f(totals) in thread 0, whose results
+// (shared variables) all threads may read on return.
+template <int N, typename F>
+__device__ __forceinline__ void ps_grid_total(const double* part, F f)
+{
+    __shared__ double tot[N];
+    const int w = threadIdx.x >> 5;
+    if (w < N) {
+        const double a = ps_total(part, w);
+        if ((threadIdx.x & 31) == 0) tot[w] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) f(tot);
+    __syncthreads();
+}
+
+// quotient of a non-negative index by a positive width through an FP32
+// reciprocal rw = 1/w: exact for indices below 2^20 (the fractional part of
+// (k + 0.5)/w is at least 0.5/w away from an integer)
+__device__ __forceinline__ int fdiv(int k, float rw) { return __float2int_rz((k + 0.5f) * rw); }
+
+// ---- dense coarsest level -----------------------------------------------------
+// x = M b for the n x n inverse M of the coarsest operator. The rows are dealt
+// to the blocks, a block's rows in quarters to its warps (its 16 warps stay
+// busy for any number of rows, and a warp's loads of a quarter are in flight
+// together); b is staged in shared memory. In FP64 n = 1024 costs 3.4k cycles
+// of the FP64 pipe and n = 2048 14k, the two legs and barriers of one more
+// grid level about 17k; and the coarse correction is exact.
+constexpr int PS_NDENSE = 2048;
+
+template <typename S>
+__device__ __forceinline__ void ps_dense(const S* __restrict__ M, const S* b, S* x, int n, S* sb)
+{
+    constexpr int NW = PS_NT / 32, U = 8;
+    S* part = sb + n;  // 4 per row of the block
+    for (int e = threadIdx.x; e < n; e += PS_NT) sb[e] = __ldcg(&b[e]);
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int rows = (n + gridDim.x - 1) / gridDim.x;  // of this block, at most
+    const int len = ((n + 3) / 4 + 31) & ~31;          // columns of a quarter
+    for (int t = threadIdx.x >> 5; t < 4 * rows; t += NW) {
+        const int row = (t >> 2) * gridDim.x + blockIdx.x;
+        S a = S(0);
+        if (row < n) {
+            const S* __restrict__ m = M + (size_t)row * n;
+            const int end = min(n, ((t & 3) + 1) * len);
+            for (int e = (t & 3) * len + lane; e < end; e += 32 * U) {
+                S v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = e + 32 * u < end ? m[e + 32 * u] : S(0);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (e + 32 * u < end) a += v[u] * sb[e + 32 * u];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        }
+        if (lane == 0) part[t] = a;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < rows; t += PS_NT) {
+        const int row = t * gridDim.x + blockIdx.x;
+        if (row < n) x[row] = (part[4 * t] + part[4 * t + 1]) + (part[4 * t + 2] + part[4 * t + 3]);
+    }
+}
+
+// Host: the inverse of a symmetric positive definite banded matrix H of n
+// rows, band[i (bw + 1) + k] = H(i, i - k), times `scale`, as an n x n array
+// of double (prec 0) or float on the device. Cholesky on the host (ps_band_ok
+// bounds its n bw^2 operations), the columns of the inverse on the GPU. part:
+// empty, or a part number per row: the constants of a part are projected out
+// of the result from both sides, and rows of part -1 become 0. 0 on success.
+int ps_invert(const std::vector<double>& band, int n, int bw, const std::vector<int>& part,
+              double scale, int prec, void* out);
+// whether a level of n cells in rows of bw may be the dense one
+inline bool ps_band_ok(long long n, long long bw)
+{
+    return n <= PS_NDENSE && n * bw * bw <= 50000000ll;
+}
+// Launch a cooperative kernel of PS_NT threads per block.
+int ps_launch(const void* kern, int grid, size_t smem, void** args, cudaStream_t st);
+// SMs of the current device.
+int ps_sms();
+
+}  // namespace f2d
