@@ -23,7 +23,8 @@
 // smooth errors, and the coarse correction comes out halved - half the sum is
 // the re-discretised coupling where the face is fully open and keeps the
 // partial openings of masked faces.) The first level of at most 2048 cells is
-// solved exactly with its precomputed dense pseudo-inverse. The FP32 form runs the cycle in FP32
+// solved exactly with its precomputed dense pseudo-inverse (the FP32 form:
+// replaced by the matrix of the V-cycle from it on, coarse_map). The FP32 form runs the cycle in FP32
 // (levels, couplings and smoothing in float; its right-hand side is the FP64
 // Krylov residual rounded, its result converted back), while the Krylov
 // vectors, the operator products, the dot products and the zero-mean
@@ -814,6 +815,152 @@ static int dense_inverse(const std::vector<double>& fx, const std::vector<double
     return ps_invert(h, n, bw, part, -1.0, prec, out);
 }
 
+// The FP32 form's dense level: not the inverse but the V-cycle on the levels
+// from it on (2 sweeps per leg, (R,B)^k (B,R)^k on the first level of at most
+// 8 cells in a direction), as the matrix of that linear map, column by column
+// in FP64. The euler models' FP32 velocities round differently wherever the
+// pressure moves by its tolerance, so this form keeps the cycle, and with it
+// the CG iterates, of the level-by-level form it replaced: the velocities and
+// the pressure stay the same to the last bits.
+constexpr int NC_LMAX = 12;
+struct NCoarse {
+    int nl, ksweeps;
+    int nyn[NC_LMAX], nxn[NC_LMAX], off[NC_LMAX], per;
+};
+
+__device__ __forceinline__ double nc_ax(const NCoarse& C, int l, const double* x,
+                                        const double* fx, const double* fy, int J, int I,
+                                        double& cs)
+{
+    const int nx = C.nxn[l], ny = C.nyn[l], o = C.off[l], k = o + J * nx + I;
+    const double cw = fx[k], so = fy[k];
+    const int ke = I + 1 < nx ? k + 1 : k - I;
+    const double ce = I + 1 < nx || C.per ? fx[ke] : 0.0;
+    const double cn = J + 1 < ny ? fy[k + nx] : 0.0;
+    double v = -((cw + ce) + (so + cn)) * x[k];
+    cs = (cw + ce) + (so + cn);
+    if (cw != 0.0) v += cw * x[I > 0 ? k - 1 : k + nx - 1];
+    if (ce != 0.0) v += ce * x[ke];
+    if (so != 0.0) v += so * x[k - nx];
+    if (cn != 0.0) v += cn * x[k + nx];
+    return v;
+}
+
+__device__ __forceinline__ void nc_half(const NCoarse& C, int l, double* x, const double* b,
+                                        const double* fx, const double* fy, int color)
+{
+    const int nx = C.nxn[l], n = nx * C.nyn[l], o = C.off[l];
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const int J = k / nx, I = k - J * nx;
+        if (((J + I) & 1) != color) continue;
+        double cs;
+        const double ax = nc_ax(C, l, x, fx, fy, J, I, cs);
+        if (cs > 0.0) x[o + k] += (ax - b[o + k]) / cs;
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(256)
+k_ns_coarse_map(const __grid_constant__ NCoarse C, const double* __restrict__ fx,
+                const double* __restrict__ fy, float* __restrict__ out)
+{
+    extern __shared__ double sm[];
+    const int nl = C.nl, tot = C.off[nl - 1] + C.nyn[nl - 1] * C.nxn[nl - 1];
+    double *x = sm, *b = sm + tot;
+    const int n = C.nyn[0] * C.nxn[0], col = blockIdx.x;
+    for (int k = threadIdx.x; k < tot; k += blockDim.x) {
+        x[k] = 0.0;
+        b[k] = k == col ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    for (int l = 0; l + 1 < nl; ++l) {
+        for (int s = 0; s < 4; ++s) nc_half(C, l, x, b, fx, fy, s & 1);
+        const int cx = C.nxn[l + 1];
+        for (int k = threadIdx.x; k < cx * C.nyn[l + 1]; k += blockDim.x) {
+            double v = 0.0, cs;
+            for (int q = 0; q < 4; ++q) {
+                const int J = 2 * (k / cx) + (q >> 1), I = 2 * (k % cx) + (q & 1);
+                if (J < C.nyn[l] && I < C.nxn[l])
+                    v += b[C.off[l] + J * C.nxn[l] + I] - nc_ax(C, l, x, fx, fy, J, I, cs);
+            }
+            b[C.off[l + 1] + k] = v;
+        }
+        __syncthreads();
+    }
+    for (int s = 0; s < 2 * C.ksweeps; ++s)
+        for (int h = 0; h < 2; ++h)
+            nc_half(C, nl - 1, x, b, fx, fy, s < C.ksweeps ? h : 1 - h);
+    for (int l = nl - 2; l >= 0; --l) {
+        const int nx = C.nxn[l], cx = C.nxn[l + 1];
+        for (int k = threadIdx.x; k < nx * C.nyn[l]; k += blockDim.x)
+            x[C.off[l] + k] += x[C.off[l + 1] + (k / nx / 2) * cx + k % nx / 2];
+        __syncthreads();
+        for (int s = 0; s < 4; ++s) nc_half(C, l, x, b, fx, fy, (s + 1) & 1);
+    }
+    // column col = row col (the cycle is symmetric)
+    for (int k = threadIdx.x; k < n; k += blockDim.x) out[(size_t)col * n + k] = (float)x[k];
+}
+
+static void coarsen(std::vector<double>& fx, std::vector<double>& fy, int& ny, int& nx, int per)
+{
+    const int cyn = (ny + 1) / 2, cxn = (nx + 1) / 2;
+    std::vector<double> cfx((size_t)cyn * cxn, 0.0), cfy((size_t)cyn * cxn, 0.0);
+    for (int J = 0; J < cyn; ++J)
+        for (int I = 0; I < cxn; ++I) {
+            double sx = 0.0, sy = 0.0;
+            // fine x-faces at column 2I, y-faces at row 2J
+            for (int q = 0; q < 2; ++q) {
+                if (2 * J + q < ny) sx += fx[(size_t)(2 * J + q) * nx + 2 * I];
+                if (2 * I + q < nx) sy += fy[(size_t)(2 * J) * nx + 2 * I + q];
+            }
+            cfx[(size_t)J * cxn + I] = 0.5 * sx;
+            cfy[(size_t)J * cxn + I] = 0.5 * sy;
+        }
+    // one coarse column: the wrap face joins the cell to itself
+    if (per && cxn == 1) std::fill(cfx.begin(), cfx.end(), 0.0);
+    fx.swap(cfx);
+    fy.swap(cfy);
+    ny = cyn;
+    nx = cxn;
+}
+
+static int coarse_map(std::vector<double> fx, std::vector<double> fy, int ny, int nx, int per,
+                      float* out)
+{
+    NCoarse C = {};
+    C.per = per;
+    const int n = ny * nx;
+    std::vector<double> ax, ay;
+    for (;;) {
+        C.nyn[C.nl] = ny;
+        C.nxn[C.nl] = nx;
+        C.off[C.nl] = (int)ax.size();
+        C.nl += 1;
+        ax.insert(ax.end(), fx.begin(), fx.end());
+        ay.insert(ay.end(), fy.begin(), fy.end());
+        if (!(ny > 8 && nx > 8 && (!per || nx % 2 == 0)) || C.nl == NC_LMAX) break;
+        coarsen(fx, fy, ny, nx, per);
+    }
+    C.ksweeps = std::min(64, std::max(4, std::max(ny, nx)));
+    double *dx = nullptr, *dy = nullptr;
+    const size_t bytes = ax.size() * 8;
+    int rc = 0;
+    if (cudaMalloc(&dx, bytes) != cudaSuccess || cudaMalloc(&dy, bytes) != cudaSuccess ||
+        cudaMemcpy(dx, ax.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(dy, ay.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess)
+        rc = 2;
+    if (!rc && cudaFuncSetAttribute(k_ns_coarse_map, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    96 * 1024) != cudaSuccess)
+        rc = 3;
+    if (!rc) {
+        k_ns_coarse_map<<<n, 256, 2 * bytes>>>(C, dx, dy, out);
+        if (cudaDeviceSynchronize() != cudaSuccess) rc = 3;
+    }
+    cudaFree(dx);
+    cudaFree(dy);
+    return rc;
+}
+
 int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int per,
              const uint8_t* hmask, double* x, double* b, double cx, double cy, int prec)
 {
@@ -913,21 +1060,8 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
     }
     while (!ps_band_ok((long long)ny * nx, nx)) {
         if (l + 1 >= NS_LMAX) return 3;
-        const int cyn = (ny + 1) / 2, cxn = (nx + 1) / 2;
-        std::vector<double> cfx((size_t)cyn * cxn, 0.0), cfy((size_t)cyn * cxn, 0.0);
-        for (int J = 0; J < cyn; ++J)
-            for (int I = 0; I < cxn; ++I) {
-                double sx = 0.0, sy = 0.0;
-                // fine x-faces at column 2I, y-faces at row 2J
-                for (int q = 0; q < 2; ++q) {
-                    if (2 * J + q < ny) sx += fx[(size_t)(2 * J + q) * nx + 2 * I];
-                    if (2 * I + q < nx) sy += fy[(size_t)(2 * J) * nx + 2 * I + q];
-                }
-                cfx[(size_t)J * cxn + I] = 0.5 * sx;
-                cfy[(size_t)J * cxn + I] = 0.5 * sy;
-            }
-        // one coarse column: the wrap face joins the cell to itself
-        if (per && cxn == 1) std::fill(cfx.begin(), cfx.end(), 0.0);
+        coarsen(fx, fy, ny, nx, per);
+        const int cyn = ny, cxn = nx;
         ++l;
         NLevel& C = a.lev[l];
         const bool dense = ps_band_ok((long long)cyn * cxn, cxn);
@@ -941,10 +1075,6 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
         C.x = dal(n * es);
         C.b = dal(n * es);
         if (!C.x || !C.b) return 2;
-        fx.swap(cfx);
-        fy.swap(cfy);
-        ny = cyn;
-        nx = cxn;
         if (dense) continue;  // (the last)
         C.xa = dal(n * es);
         std::vector<double> hx(n, 0.0), hy(n, 0.0), hi(n, 0.0);
@@ -968,7 +1098,8 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
     a.nd = ny * nx;
     void* minv = dal((size_t)a.nd * a.nd * es);
     if (!minv) return 2;
-    int rc = dense_inverse(fx, fy, ny, nx, per, cx, cy, prec, minv);
+    int rc = prec == 1 && a.ng > 0 ? coarse_map(fx, fy, ny, nx, per, (float*)minv)
+                                   : dense_inverse(fx, fy, ny, nx, per, cx, cy, prec, minv);
     if (rc) return rc;
     a.minv = minv;
     // every SM also for small problems: the rows of the dense level are dealt
