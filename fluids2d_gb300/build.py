@@ -21,7 +21,7 @@ INCLUDE = os.path.join(ROOT, "include")
 
 SOURCES = ["api.cu", "stage.cu", "mg.cu", "sweeps.cu", "mesh_host.cu",
            "noalloc.cu", "ensemble.cu", "solver.cu", "adjoint.cu", "nsolver.cu",
-           "persist.cu"]
+           "persist.cu", "psolver.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC",
          "-Xcompiler", "-O2", "--expt-relaxed-constexpr", "-I", INCLUDE]

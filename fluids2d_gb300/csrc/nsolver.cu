@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
     // b -= mean(b)
     double vb[1] = {0.0};
     n_cells(L, [&](int, int, long long k) { if (L.code[k]) vb[0] += A.b[k]; });
-    ps_block_total<1>(vb, pi);
+    ps_block_total<1>(vb, pi + blockIdx.x, G);
     if (!ps_sync(g)) return;
     ps_grid_total<1>(pi, [&](const double* t) { c.mean = t[0] / A.nfluid; });
     // r = b - A x
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
         }
         A.r[0][k] = rv;
     });
-    ps_block_total<3>(v, pb);
+    ps_block_total<3>(v, pb + blockIdx.x, G);
     if (!ps_sync(g)) return;
     ps_grid_total<3>(pb, [&](const double* t) {
         c.bb = t[0];
@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
     auto decide = [&] {
         const int w = threadIdx.x >> 5;
         if (it == 0 || w > 2) return;
-        const double a = ps_total(pr, w - 1);
+        const double a = ps_total(pr + (w - 1) * G, G);
         if (threadIdx.x & 31) return;
         if (w == 2) {
             c.xsum = a;
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
         double t[2] = {0.0, 0.0};
         if (A.ng > 0) n_phase_a<S>(A, it, c.alpha, c.beta, t, smem, T);
         else n_dense_a<S>(A, it, c.alpha, c.beta, t);
-        if (it > 0) ps_block_total<2>(t, pr);
+        if (it > 0) ps_block_total<2>(t, pr + blockIdx.x, G);
         if (!ps_sync(g)) return;
         for (int l = 1; l < A.ng; ++l) {
             n_down<S>(A, l, smem, T);
@@ -679,7 +679,8 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
         }
         if (c.done) break;
         const NLevel& D = A.lev[A.ng];
-        ps_dense<S>((const S*)A.minv, (const S*)D.b, (S*)D.x, A.nd, (S*)smem);
+        ps_dense<S>((const S*)A.minv, (const S*)D.b, (S*)D.x, A.nd, A.nd * blockIdx.x / G,
+                    A.nd * (blockIdx.x + 1) / G, (S*)smem);
         if (!(A.ng <= 1 ? ps_sync(g, decide) : ps_sync(g))) return;
         if (c.done) break;
         for (int l = A.ng - 1; l >= 1; --l) {
@@ -689,7 +690,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
         t[0] = t[1] = 0.0;
         if (A.ng > 0) n_phase_b<S>(A, it, t, smem, T);
         else n_dense_b<S>(A, t);
-        ps_block_total<2>(t, pz);
+        ps_block_total<2>(t, pz + blockIdx.x, G);
         if (!ps_sync(g)) return;
         ps_grid_total<2>(pz, [&](const double* u) {
             // beta = rz / rz_old and <p, A p> = <z, w> - beta^2 <p, A p>_old,

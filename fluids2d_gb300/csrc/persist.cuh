@@ -82,15 +82,14 @@ __device__ __forceinline__ bool ps_sync(PSGrid& g)
 }
 
 // ---- deterministic sums over the blocks --------------------------------------
-// The block's totals of N <= 4 per-thread values into part[k * gridDim.x +
-// block]; after the next barrier every block adds all blocks' totals in one
+// The block's totals of N <= 4 per-thread values into part[k * stride]; after the next barrier every block adds all blocks' totals in one
 // fixed order, so all blocks hold the same bits and take the same decisions
 // without a broadcast. An FP64 instruction of a warp occupies its SM
 // partition's pipe for 64 cycles, so sums and scalar arithmetic are kept to
 // few warps: a shuffle tree in all 16 warps, or three divisions in all
 // threads, cost 1.3 us and 4.6 us of a phase of 5.
 template <int N>
-__device__ __forceinline__ void ps_block_total(const double (&v)[N], double* part)
+__device__ __forceinline__ void ps_block_total(const double (&v)[N], double* part, int stride)
 {
     __shared__ double sh[N][PS_NT];
     __syncthreads();
@@ -110,23 +109,22 @@ __device__ __forceinline__ void ps_block_total(const double (&v)[N], double* par
     __syncthreads();
     if (threadIdx.x < N) {
         const double* s = sh[threadIdx.x];
-        part[threadIdx.x * gridDim.x + blockIdx.x] =
+        part[(size_t)threadIdx.x * stride] =
             (s[0] + s[PS_NT / 4]) + (s[PS_NT / 2] + s[3 * (PS_NT / 4)]);
     }
 }
 
-// The grid's total of value k, by one whole warp (all lanes hold it)
-__device__ __forceinline__ double ps_total(const double* part, int k)
+// The total of p[0 .. n) in a fixed order, by one whole warp (all lanes hold it)
+__device__ __forceinline__ double ps_total(const double* p, int n)
 {
     const int lane = threadIdx.x & 31;
-    const double* p = part + (size_t)k * gridDim.x;
     double a = 0.0, b = 0.0;
-    unsigned i = lane;
-    for (; i + 32 < gridDim.x; i += 64) {
+    int i = lane;
+    for (; i + 32 < n; i += 64) {
         a += __ldcg(&p[i]);
         b += __ldcg(&p[i + 32]);
     }
-    if (i < gridDim.x) a += __ldcg(&p[i]);
+    if (i < n) a += __ldcg(&p[i]);
     a += b;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
@@ -141,7 +139,7 @@ __device__ __forceinline__ void ps_grid_total(const double* part, F f)
     __shared__ double tot[N];
     const int w = threadIdx.x >> 5;
     if (w < N) {
-        const double a = ps_total(part, w);
+        const double a = ps_total(part + (size_t)w * gridDim.x, gridDim.x);
         if ((threadIdx.x & 31) == 0) tot[w] = a;
     }
     __syncthreads();
@@ -163,40 +161,37 @@ __device__ __forceinline__ int fdiv(int k, float rw) { return __float2int_rz((k 
 // grid level about 17k; and the coarse correction is exact.
 constexpr int PS_NDENSE = 2048;
 
+// rows r0 .. r1 - 1 of x = M b; sb: n + 4 (r1 - r0) elements of shared memory
 template <typename S>
-__device__ __forceinline__ void ps_dense(const S* __restrict__ M, const S* b, S* x, int n, S* sb)
+__device__ __forceinline__ void ps_dense(const S* __restrict__ M, const S* b, S* x, int n, int r0,
+                                         int r1, S* sb)
 {
     constexpr int NW = PS_NT / 32, U = 8;
-    S* part = sb + n;  // 4 per row of the block
+    S* part = sb + n;  // 4 per row
+    if (r1 <= r0) return;
     for (int e = threadIdx.x; e < n; e += PS_NT) sb[e] = __ldcg(&b[e]);
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int rows = (n + gridDim.x - 1) / gridDim.x;  // of this block, at most
-    const int len = ((n + 3) / 4 + 31) & ~31;          // columns of a quarter
-    for (int t = threadIdx.x >> 5; t < 4 * rows; t += NW) {
-        const int row = (t >> 2) * gridDim.x + blockIdx.x;
+    const int len = ((n + 3) / 4 + 31) & ~31;  // columns of a quarter
+    for (int t = threadIdx.x >> 5; t < 4 * (r1 - r0); t += NW) {
+        const S* __restrict__ m = M + (size_t)(r0 + (t >> 2)) * n;
         S a = S(0);
-        if (row < n) {
-            const S* __restrict__ m = M + (size_t)row * n;
-            const int end = min(n, ((t & 3) + 1) * len);
-            for (int e = (t & 3) * len + lane; e < end; e += 32 * U) {
-                S v[U];
+        const int end = min(n, ((t & 3) + 1) * len);
+        for (int e = (t & 3) * len + lane; e < end; e += 32 * U) {
+            S v[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) v[u] = e + 32 * u < end ? m[e + 32 * u] : S(0);
+            for (int u = 0; u < U; ++u) v[u] = e + 32 * u < end ? m[e + 32 * u] : S(0);
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (e + 32 * u < end) a += v[u] * sb[e + 32 * u];
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            for (int u = 0; u < U; ++u)
+                if (e + 32 * u < end) a += v[u] * sb[e + 32 * u];
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
         if (lane == 0) part[t] = a;
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < rows; t += PS_NT) {
-        const int row = t * gridDim.x + blockIdx.x;
-        if (row < n) x[row] = (part[4 * t] + part[4 * t + 1]) + (part[4 * t + 2] + part[4 * t + 3]);
-    }
+    for (int t = threadIdx.x; t < r1 - r0; t += PS_NT)
+        x[r0 + t] = (part[4 * t] + part[4 * t + 1]) + (part[4 * t + 2] + part[4 * t + 3]);
 }
 
 // Host: the inverse of a symmetric positive definite banded matrix H of n

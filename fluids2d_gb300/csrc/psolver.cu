@@ -1,0 +1,1004 @@
+// Persistent solve kernel of the masked vertex Poisson/Helmholtz operator
+// (the reference factorises it with SuperLU: elliptic.py:71-87, 114-195) for
+// a batch of one or many members: a whole multigrid-preconditioned CG solve
+// of every member in one cooperative launch of one block per SM
+// (persist.cuh), the CG iterations inside, its phases separated by grid
+// barriers.
+//
+// Operator, hierarchy and cycle are mg.cu's: red-black Gauss-Seidel with nu
+// sweeps per leg, bilinear prolongation and its transpose, coarse masks by
+// injection, re-discretised coarse operators. The first level with few enough
+// nodes is solved exactly with its dense inverse (a single model: up to 2048
+// nodes, level 0 itself if it is that small). S is the cycle's precision;
+// the CG vectors, the operator product and the inner products are FP64 in
+// both forms (FP32 form: the cycle's right-hand side is the FP64 residual
+// rounded).
+//
+// CG in the form of Chronopoulos and Gear (J. Comput. Appl. Math. 25, 1989):
+// w = A z and the two inner products <r, z>, <z, w> come from one pass, s =
+// A p by recurrence. Phases of an iteration, a barrier after each:
+//   A   update s, r, p, x (r on the tile and its halo, recomputed), <r, r>,
+//       pre-smoothing, residual and restriction of level 0
+//   D_l the same legs of the coarser grid levels;  the dense level
+//   U_l the up legs
+//   B   up leg of level 0 with z one node past the tile, w = A z, the two
+//       inner products
+// A leg works in shared memory on a tile and the halo its half sweeps reach
+// over (5 nodes at nu = 2); nodes within s of the region's edge are inexact
+// after half sweep s and only reach halo nodes. After the last black half
+// sweep the black residuals are zero and the black values do not enter the
+// up leg (its first half sweep overwrites them from the red ones), so only
+// red residuals are formed and only red nodes are prolongated.
+//
+// What it replaced, FP64: one launch per level and leg on 54 x 70-node tiles,
+// each bound by the FP64 pipe of the few SMs that had a tile (36 to 42 us a
+// launch for 40 to 400 ns of work on the whole chip).
+#include <algorithm>
+#include <cstring>
+
+#include "psolver.cuh"
+#include "solver.cuh"
+
+namespace f2d {
+
+template <typename S>
+struct PReg {
+    S *x, *b;  // b: right-hand side / diagonal, then the residual
+    uint8_t* m;
+    int J0, I0, h, W, RH, tw, th;
+    float rW;
+    S cxi, cyi, dg;
+};
+
+template <typename S>
+__device__ __forceinline__ PReg<S> p_region(const PTile& t, int h, unsigned char* smem)
+{
+    PReg<S> R;
+    R.J0 = t.J0;
+    R.I0 = t.I0;
+    R.tw = t.tw;
+    R.th = t.th;
+    R.h = h;
+    R.W = t.tw + 2 * h;
+    R.RH = t.th + 2 * h;
+    R.rW = 1.0f / (float)R.W;
+    const int n = R.W * R.RH;
+    R.x = (S*)smem;
+    R.b = R.x + n;
+    R.m = (uint8_t*)(R.b + n);
+    R.cxi = conv<S>(t.cxi);
+    R.cyi = conv<S>(t.cyi);
+    R.dg = conv<S>(t.dg);
+    return R;
+}
+
+__device__ __forceinline__ bool p_node(const PTile& t, int J, int& I)
+{
+    if (J < 0 || J >= t.nyn) return false;
+    if (t.per) {
+        while (I < 0) I += t.nxn;
+        while (I >= t.nxn) I -= t.nxn;
+        return true;
+    }
+    return I >= 0 && I < t.nxn;
+}
+
+// Gauss-Seidel value of region node e (non-fluid nodes hold x = 0)
+template <typename S>
+__device__ __forceinline__ S p_gs(const PReg<S>& R, int e)
+{
+    return R.b[e] - (R.cxi * (R.x[e - 1] + R.x[e + 1]) + R.cyi * (R.x[e - R.W] + R.x[e + R.W]));
+}
+
+// half sweep of a colour over the nodes within rad of the tile
+template <typename S>
+__device__ __forceinline__ void p_half(const PReg<S>& R, int color, int rad)
+{
+    const int o = R.h - rad, nr = R.th + 2 * rad, wc = R.tw / 2 + rad;
+    const float rw = 1.0f / (float)wc;
+    for (int k = threadIdx.x; k < nr * wc; k += PS_NT) {
+        const int a = fdiv(k, rw), r = o + a;
+        // J0 and I0 are even: the colour of region node (r, c) is r + c
+        const int c = o + 2 * (k - a * wc) + ((r + o + color) & 1);
+        const int e = r * R.W + c;
+        if (R.m[e]) R.x[e] = p_gs(R, e);
+    }
+    __syncthreads();
+}
+
+constexpr int PB = 2;  // nodes per thread and batch
+
+// The region's nodes in batches of PB per thread: load(q, in, k, J, I) for the
+// batch (its loads in flight together), then use(q, e, in, k, r, c)
+template <typename S, typename FL, typename FU>
+__device__ __forceinline__ void p_load(const PReg<S>& R, const PTile& t, FL load, FU use)
+{
+    const int n = R.W * R.RH;
+    for (int e0 = threadIdx.x; e0 < n; e0 += PB * PS_NT) {
+        int rc[PB];
+        long long k[PB];
+#pragma unroll
+        for (int q = 0; q < PB; ++q) {
+            const int e = e0 + q * PS_NT;
+            const int r = fdiv(e, R.rW), c = e - r * R.W;
+            int I = R.I0 - R.h + c;
+            const int J = R.J0 - R.h + r;
+            const bool in = e < n && p_node(t, J, I);
+            rc[q] = (r << 16) | c;
+            k[q] = in ? t.off + (long long)J * t.pitch + I : -1;
+            load(q, in, k[q], J, I);
+        }
+#pragma unroll
+        for (int q = 0; q < PB; ++q) {
+            const int e = e0 + q * PS_NT;
+            if (e < n) use(q, e, k[q] >= 0, k[q], rc[q] >> 16, rc[q] & 0xffff);
+        }
+    }
+}
+
+// the tile's nodes of the level, in batches: load(q, in, k), use(q, k, e)
+template <typename S, typename FL, typename FU>
+__device__ __forceinline__ void p_tile(const PReg<S>& R, const PTile& t, FL load, FU use)
+{
+    const int n = R.tw * R.th;
+    const float rw = 1.0f / (float)R.tw;
+    for (int e0 = threadIdx.x; e0 < n; e0 += PB * PS_NT) {
+        int e[PB];
+        long long k[PB];
+#pragma unroll
+        for (int q = 0; q < PB; ++q) {
+            const int i = e0 + q * PS_NT;
+            const int a = fdiv(i, rw), c = i - a * R.tw;
+            const int J = R.J0 + a, I = R.I0 + c;
+            const bool in = i < n && J < t.nyn && I < t.nxn;
+            k[q] = in ? t.off + (long long)J * t.pitch + I : -1;
+            e[q] = (R.h + a) * R.W + R.h + c;
+            load(q, in, k[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < PB; ++q)
+            if (k[q] >= 0) use(q, k[q], e[q]);
+    }
+}
+
+// From the region with b and the red x = b / diagonal: the rest of the
+// pre-smoothing, the red residuals, their restriction to the coarse nodes
+// whose centre lies in the tile (weight 1 at the centre, 1/4 at the corners).
+template <typename S>
+__device__ __forceinline__ void p_down_leg(const PReg<S>& R, const PTile& t, int nu)
+{
+#pragma unroll 1
+    for (int q = 1; q < 2 * nu; ++q) p_half(R, q & 1, 2 * nu + 1 - q);
+    {
+        // residual = diagonal (Gauss-Seidel value - x) of the red nodes within
+        // 1 of the tile, into b
+        const int o = R.h - 1, nr = R.th + 2, wc = R.tw / 2 + 1;
+        const float rw = 1.0f / (float)wc;
+        for (int k = threadIdx.x; k < nr * wc; k += PS_NT) {
+            const int a = fdiv(k, rw), r = o + a;
+            const int e = r * R.W + o + 2 * (k - a * wc) + ((r + o) & 1);
+            R.b[e] = R.m[e] ? R.dg * (p_gs(R, e) - R.x[e]) : S(0);
+        }
+        __syncthreads();
+    }
+    const int wc = R.tw / 2, nc = wc * (R.th / 2);
+    const float rw = 1.0f / (float)wc;
+    for (int k = threadIdx.x; k < nc; k += PS_NT) {
+        const int a = fdiv(k, rw), c = k - a * wc;
+        const int J = R.J0 / 2 + a, I = R.I0 / 2 + c;
+        if (J >= t.cyn || I >= t.cxn) continue;
+        const int e = (R.h + 2 * a) * R.W + R.h + 2 * c;
+        S v = S(0);
+        if (t.cm[t.cmoff + (long long)J * t.cmpitch + I])
+            v = R.b[e] + S(0.25) * ((R.b[e - R.W - 1] + R.b[e - R.W + 1]) +
+                                    (R.b[e + R.W - 1] + R.b[e + R.W + 1]));
+        ((S*)t.cb)[t.coff + (long long)J * t.cpitch + I] = v;
+    }
+}
+
+// P (coarse x) at the red node (J, I): the coarse node, or the mean of four
+template <typename S>
+__device__ __forceinline__ void p_coarse(const PTile& t, bool use, int J, int I, S (&v)[4])
+{
+    const S* X = (const S*)t.cx_;
+    const int cj = J >> 1, ci = I >> 1;
+    const bool odd = use && (J & 1);
+    const int c1 = ci + 1 < t.cxn ? ci + 1 : (t.per ? 0 : -1);
+    const long long k = t.coff + (long long)cj * t.cpitch;
+    const bool up = odd && cj + 1 < t.cyn;
+    v[0] = use ? X[k + ci] : S(0);
+    v[1] = odd && c1 >= 0 ? X[k + c1] : S(0);
+    v[2] = up ? X[k + t.cpitch + ci] : S(0);
+    v[3] = up && c1 >= 0 ? X[k + t.cpitch + c1] : S(0);
+}
+
+template <typename S>
+__device__ __forceinline__ void p_down(const PTile& t, int nu, unsigned char* smem)
+{
+    const PReg<S> R = p_region<S>(t, 2 * nu + 1, smem);
+    const S* B = (const S*)t.b;
+    const S id = conv<S>(t.id);
+    S b[PB];
+    uint8_t m[PB];
+    p_load(
+        R, t,
+        [&](int q, bool in, long long k, int, int) {
+            m[q] = in ? t.m[k] : 0;
+            b[q] = in ? B[k] : S(0);
+        },
+        [&](int q, int e, bool, long long, int r, int c) {
+            const S bi = m[q] ? b[q] * id : S(0);
+            R.m[e] = m[q];
+            R.b[e] = bi;
+            R.x[e] = (r + c) & 1 ? S(0) : bi;
+        });
+    __syncthreads();
+    p_down_leg(R, t, nu);
+    S* XA = (S*)t.xa;
+    p_tile(R, t, [](int, bool, long long) {}, [&](int, long long k, int e) { XA[k] = R.x[e]; });
+    __syncthreads();
+}
+
+template <typename S>
+__device__ __forceinline__ void p_up(const PTile& t, int nu, unsigned char* smem)
+{
+    const PReg<S> R = p_region<S>(t, 2 * nu, smem);
+    const S* B = (const S*)t.b;
+    const S* XA = (const S*)t.xa;
+    const S id = conv<S>(t.id);
+    S b[PB], xa[PB], cv[PB][4];
+    uint8_t m[PB];
+    p_load(
+        R, t,
+        [&](int q, bool in, long long k, int J, int I) {
+            const bool red = in && ((J + I) & 1) == 0;
+            m[q] = in ? t.m[k] : 0;
+            b[q] = in ? B[k] : S(0);
+            xa[q] = red ? XA[k] : S(0);
+            p_coarse<S>(t, red, J, I, cv[q]);
+        },
+        [&](int q, int e, bool, long long, int r, int c) {
+            // (a red node's parity is its row's: R.h and J0 are even)
+            const S pc = r & 1 ? S(0.25) * ((cv[q][0] + cv[q][1]) + (cv[q][2] + cv[q][3]))
+                               : cv[q][0];
+            R.m[e] = m[q];
+            R.b[e] = m[q] ? b[q] * id : S(0);
+            R.x[e] = m[q] && ((r + c) & 1) == 0 ? xa[q] + pc : S(0);
+        });
+    __syncthreads();
+#pragma unroll 1
+    for (int q = 1; q <= 2 * nu; ++q) p_half(R, q & 1, 2 * nu - q);
+    S* X = (S*)t.x;
+    p_tile(R, t, [](int, bool, long long) {}, [&](int, long long k, int e) { X[k] = R.x[e]; });
+    __syncthreads();
+}
+
+// phase A of a level-0 tile (it > 0: with the CG update of the previous
+// iteration): tot = <r, r>
+template <typename S>
+__device__ __forceinline__ void p_phase_a(const PSArgs& A, const PTile& t, int it, double alpha,
+                                          double beta, double (&tot)[1], unsigned char* smem)
+{
+    const int nu = A.nu, h = 2 * nu + 1, par = it & 1;
+    const PReg<S> R = p_region<S>(t, h, smem);
+    const double* r0 = A.r[it > 0 ? 1 - par : 0];
+    const double* s0 = A.s[1 - par];
+    double* r1 = A.r[par];
+    double* s1 = A.s[par];
+    const S* Z = (const S*)t.x;
+    const S id = conv<S>(t.id);
+    uint8_t m[PB];
+    double rv[PB], sv[PB], wv[PB], xv[PB], pv[PB];
+    S zv[PB];
+    p_load(
+        R, t,
+        [&](int q, bool in, long long k, int, int) {
+            m[q] = in ? t.m[k] : 0;
+            rv[q] = in ? r0[k] : 0.0;
+            wv[q] = in && it > 0 ? A.w[k] : 0.0;
+            sv[q] = in && it > 1 ? s0[k] : 0.0;
+        },
+        [&](int q, int e, bool in, long long k, int r, int c) {
+            double rn = rv[q];
+            if (it > 0) {
+                const double sn = wv[q] + beta * sv[q];
+                rn -= alpha * sn;
+                if (in && r >= h && r < h + R.th && c >= h && c < h + R.tw &&
+                    R.I0 - h + c < t.nxn) {
+                    s1[k] = sn;
+                    r1[k] = rn;
+                    tot[0] += rn * rn;  // (0 at non-fluid nodes)
+                }
+            }
+            const S bi = m[q] ? conv<S>(rn) * id : S(0);
+            R.m[e] = m[q];
+            R.b[e] = bi;
+            R.x[e] = (r + c) & 1 ? S(0) : bi;
+        });
+    __syncthreads();
+    p_down_leg(R, t, nu);
+    S* XA = (S*)t.xa;
+    p_tile(
+        R, t,
+        [&](int q, bool in, long long k) {
+            xv[q] = in && it > 0 ? A.x[k] : 0.0;
+            pv[q] = in && it > 1 ? A.p[k] : 0.0;
+            zv[q] = in && it > 0 ? Z[k] : S(0);
+        },
+        [&](int q, long long k, int e) {
+            XA[k] = R.x[e];
+            if (it == 0) return;
+            const double pn = conv<double>(zv[q]) + beta * pv[q];
+            A.p[k] = pn;
+            if (R.m[e]) A.x[k] = xv[q] + alpha * pn;
+        });
+    __syncthreads();
+}
+
+// phase B of a level-0 tile: tot = <r, z>, <z, A z>
+template <typename S>
+__device__ __forceinline__ void p_phase_b(const PSArgs& A, const PTile& t, int it,
+                                          double (&tot)[2], unsigned char* smem)
+{
+    const int nu = A.nu, h = 2 * nu + 1;
+    const PReg<S> R = p_region<S>(t, h, smem);
+    const double* rr = A.r[it & 1];
+    const S* XA = (const S*)t.xa;
+    const S id = conv<S>(t.id);
+    uint8_t m[PB];
+    double rv[PB];
+    S xa[PB], cv[PB][4];
+    p_load(
+        R, t,
+        [&](int q, bool in, long long k, int J, int I) {
+            const bool red = in && ((J + I) & 1) == 0;
+            m[q] = in ? t.m[k] : 0;
+            rv[q] = in ? rr[k] : 0.0;
+            xa[q] = red ? XA[k] : S(0);
+            p_coarse<S>(t, red, J, I, cv[q]);
+        },
+        [&](int q, int e, bool, long long, int r, int c) {
+            // (h is odd: even rows of the region are odd rows of the level)
+            const S pc = r & 1 ? cv[q][0]
+                               : S(0.25) * ((cv[q][0] + cv[q][1]) + (cv[q][2] + cv[q][3]));
+            R.m[e] = m[q];
+            R.b[e] = m[q] ? conv<S>(rv[q]) * id : S(0);
+            R.x[e] = m[q] && ((r + c) & 1) == 0 ? xa[q] + pc : S(0);
+        });
+    __syncthreads();
+#pragma unroll 1
+    for (int q = 1; q <= 2 * nu; ++q) p_half(R, q & 1, h - q);
+    S* Z = (S*)t.x;
+    const double cx = t.cx, cy = t.cy, md = t.md;
+    p_tile(
+        R, t, [&](int q, bool in, long long k) { rv[q] = in ? rr[k] : 0.0; },
+        [&](int q, long long k, int e) {
+            const double c = conv<double>(R.x[e]);
+            double wv = 0.0;
+            if (R.m[e]) {
+                // differences to the centre (apply_diff): the same operator,
+                // but far less cancellation for smooth z
+                const double sx = (conv<double>(R.x[e - 1]) - c) + (conv<double>(R.x[e + 1]) - c);
+                const double sy =
+                    (conv<double>(R.x[e - R.W]) - c) + (conv<double>(R.x[e + R.W]) - c);
+                wv = (cx * sx + cy * sy) - md * c;
+                tot[0] += rv[q] * c;
+                tot[1] += c * wv;
+            }
+            Z[k] = R.x[e];
+            A.w[k] = wv;
+        });
+    __syncthreads();
+}
+
+// Level 0 as the dense level (one member): phases A and B without smoothing;
+// z and the cycle's b in the compact layout of the dense level
+template <typename S>
+__device__ __forceinline__ void p_dense_a(const PSArgs& A, const PTile& t, const PDense& D, int it,
+                                          double alpha, double beta, double (&tot)[1],
+                                          unsigned char* smem)
+{
+    const PReg<S> R = p_region<S>(t, 0, smem);
+    p_tile(R, t, [](int, bool, long long) {}, [&](int, long long k, int e) {
+        const int a = fdiv(e, R.rW);
+        const int d = (t.J0 + a) * t.nxn + t.I0 + e - a * R.W;
+        double rv = A.r[0][k];
+        if (it > 0) {
+            double sv = A.w[k], pv = conv<double>(((const S*)D.x)[d]);
+            if (it > 1) {
+                sv += beta * A.s[0][k];
+                pv += beta * A.p[k];
+            }
+            rv -= alpha * sv;
+            A.s[0][k] = sv;
+            A.r[0][k] = rv;
+            A.p[k] = pv;
+            tot[0] += rv * rv;
+            if (t.m[k]) A.x[k] += alpha * pv;
+        }
+        ((S*)D.b)[d] = conv<S>(rv);
+    });
+}
+
+template <typename S>
+__device__ __forceinline__ void p_dense_b(const PSArgs& A, const PTile& t, const PDense& D,
+                                          double (&tot)[2], unsigned char* smem)
+{
+    const PReg<S> R = p_region<S>(t, 0, smem);
+    const S* z = (const S*)D.x;
+    p_tile(R, t, [](int, bool, long long) {}, [&](int, long long k, int e) {
+        const int a = fdiv(e, R.rW), J = t.J0 + a, I = t.I0 + e - a * R.W;
+        const int d = J * t.nxn + I;
+        double wv = 0.0;
+        if (t.m[k]) {
+            const int w = I > 0 ? d - 1 : t.per ? d + t.nxn - 1 : -1;
+            const int ea = I + 1 < t.nxn ? d + 1 : t.per ? d - I : -1;
+            const double c = conv<double>(z[d]);
+            // (non-fluid nodes hold z = 0)
+            const double zw = w >= 0 ? conv<double>(z[w]) : 0.0;
+            const double ze = ea >= 0 ? conv<double>(z[ea]) : 0.0;
+            const double zs = J > 0 ? conv<double>(z[d - t.nxn]) : 0.0;
+            const double zn = J + 1 < t.nyn ? conv<double>(z[d + t.nxn]) : 0.0;
+            wv = (t.cx * ((zw - c) + (ze - c)) + t.cy * ((zs - c) + (zn - c))) - t.md * c;
+            tot[0] += A.r[0][k] * c;
+            tot[1] += c * wv;
+        }
+        A.w[k] = wv;
+    });
+}
+
+// the dense level of every member: the rows of all members dealt to the blocks
+template <typename S>
+__device__ __forceinline__ void p_dense_rows(const PSArgs& A, unsigned char* smem)
+{
+    const int r0 = (int)((long long)A.nrows * blockIdx.x / gridDim.x);
+    const int r1 = (int)((long long)A.nrows * (blockIdx.x + 1) / gridDim.x);
+    for (int m = 0; m < A.nmem; ++m) {
+        const PDense D = A.dense[m];
+        const int a = max(r0 - D.row0, 0), b = min(r1 - D.row0, D.n);
+        if (a >= b) {
+            if (D.row0 >= r1) break;
+            continue;
+        }
+        ps_dense<S>((const S*)D.minv, (const S*)D.b, (S*)D.x, D.n, a, b, (S*)smem);
+        __syncthreads();
+    }
+}
+
+// r = b - A x of a tile; tot = <b, b>, <r, r>
+__device__ __forceinline__ void p_init(const PSArgs& A, const PTile& t, double (&tot)[2],
+                                       unsigned char* smem)
+{
+    const PReg<double> R = p_region<double>(t, 0, smem);
+    p_tile(R, t, [](int, bool, long long) {}, [&](int, long long k, int e) {
+        const int a = fdiv(e, R.rW), J = t.J0 + a, I = t.I0 + e - a * R.W;
+        double rv = 0.0;
+        if (t.m[k]) {
+            const long long kw = I > 0 ? k - 1 : t.per ? k + t.nxn - 1 : -1;
+            const long long ke = I + 1 < t.nxn ? k + 1 : t.per ? k - I : -1;
+            const bool s = J > 0 && t.m[k - t.pitch], n = J + 1 < t.nyn && t.m[k + t.pitch];
+            const double c = A.x[k], b = A.b[k];
+            const double xw = kw >= 0 && t.m[kw] ? A.x[kw] : 0.0;
+            const double xe = ke >= 0 && t.m[ke] ? A.x[ke] : 0.0;
+            const double xs = s ? A.x[k - t.pitch] : 0.0, xn = n ? A.x[k + t.pitch] : 0.0;
+            rv = b - ((t.cx * ((xw - c) + (xe - c)) + t.cy * ((xs - c) + (xn - c))) - t.md * c);
+            tot[0] += b * b;
+            tot[1] += rv * rv;
+        }
+        A.r[0][k] = rv;
+    });
+}
+
+// State of a level-0 tile's member, kept by every block that has one of its
+// tiles (a single member: one slot in every block), from the same totals in
+// the same order: the same bits.
+struct PSlot {
+    double alpha, beta, d, irz, goal, bb, rr;
+    int conv, zero, status;
+    int member, n0, nn, owner;  // owner: this block writes the member's state
+    int pad;
+};
+
+template <typename S>
+__global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ PSArgs A)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ PTile rec[PS_RECS];
+    __shared__ PSlot slot[PS_SLOTS];
+    __shared__ int rconv[PS_RECS];
+    __shared__ int lev0[PS_LMAX + 1];
+    const int nl = A.ng + 1;
+    if (threadIdx.x < nl) lev0[threadIdx.x] = A.rec0[blockIdx.x * nl + threadIdx.x];
+    __syncthreads();
+    const int base = lev0[0], nrec = lev0[A.ng] - base;
+    {
+        constexpr int W = sizeof(PTile) / 16;
+        const int4* src = (const int4*)(A.recs + base);
+        for (int k = threadIdx.x; k < nrec * W; k += PS_NT) ((int4*)rec)[k] = src[k];
+        for (int k = threadIdx.x; k < nrec; k += PS_NT) rconv[k] = 0;
+    }
+    __syncthreads();
+    const int ns = lev0[1] - base;  // level-0 tiles of the block
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool single = A.nmem == 1;
+    const int nt = A.ntiles;
+    // totals per tile: <r, z>, <z, w> | <r, r> | <b, b>, <r, r>
+    double *pz = A.part, *pr = A.part + 2 * nt, *pb = A.part + 3 * nt;
+    PSGrid g = {A.bar, A.status, 0u};
+    const double tol2 = A.scs[0].tol2;
+    const int maxit = A.scs[0].maxit;
+    // r = b - A x, <b, b>, <r, r>
+    for (int i = 0; i < ns; ++i) {
+        double v[2] = {0.0, 0.0};
+        p_init(A, rec[i], v, smem);
+        ps_block_total<2>(v, pb + rec[i].tile, nt);
+    }
+    const int nslot = single ? 1 : ns;
+    if (!ps_sync(g)) return;
+    for (int i = w; i < nslot; i += PS_NT / 32) {
+        const int n0 = single ? 0 : rec[i].n0, nn = single ? nt : rec[i].nn;
+        const double bb = ps_total(pb + n0, nn), rr = ps_total(pb + nt + n0, nn);
+        if (lane) continue;
+        PSlot& c = slot[i];
+        c.member = single ? 0 : rec[i].member;
+        c.n0 = n0;
+        c.nn = nn;
+        c.owner = single ? blockIdx.x == 0 : rec[i].tile == n0;
+        c.bb = bb;
+        c.rr = rr;
+        c.goal = tol2 * bb;
+        c.alpha = c.beta = c.d = c.irz = 0.0;
+        c.zero = bb == 0.0;
+        c.conv = c.zero || rr <= c.goal;
+        c.status = 0;
+        if (c.owner && !single) {
+            A.conv[c.member] = c.conv;
+            if (!c.conv) atomicAdd(A.active, 1);
+        }
+    }
+    __syncthreads();
+    for (int i = 0; i < ns; ++i)  // a zero right-hand side: x = 0
+        if (slot[single ? 0 : i].zero) {
+            const PTile& t = rec[i];
+            const PReg<double> R = p_region<double>(t, 0, smem);
+            p_tile(R, t, [](int, bool, long long) {}, [&](int, long long k, int) {
+                if (t.m[k]) A.x[k] = 0.0;
+            });
+        }
+    if (!ps_sync(g)) return;
+    int it = 0;
+    // The decision after the update of iteration `it`, by the idle warps of
+    // the next barrier: the tiles' <r, r> are complete, the phase before that
+    // barrier is lost when a solve is over, but the totals cost no time.
+    auto decide = [&] {
+        if (it == 0) return;
+        for (int i = w - 1; i < nslot; i += PS_NT / 32 - 1) {
+            PSlot& c = slot[i];
+            if (c.conv) continue;
+            const double rr = ps_total(pr + c.n0, c.nn);
+            if (lane) continue;
+            c.rr = rr;
+            if (!(rr == rr)) c.status = ST_NONFINITE;
+            else if (rr > c.goal && it >= maxit) c.status = ST_PCG_MAXIT;
+            c.conv = c.status || rr <= c.goal;
+            if (!c.owner) continue;
+            if (c.conv) {
+                if (!single) {
+                    A.conv[c.member] = 1;
+                    atomicSub(A.active, 1);
+                }
+                if (c.status) atomicOr(A.status, c.status);
+            }
+            DevScalars& sc = A.scs[c.member];
+            sc.iter = it;
+            sc.total_iters += 1;
+        }
+    };
+    // the converged members' flags for the tiles of the coarser levels (a
+    // flag seen early or late only skips or repeats work that is not used)
+    auto refresh = [&] {
+        if (single) return;
+        for (int k = threadIdx.x - 32; k < nrec; k += PS_NT - 32)
+            rconv[k] = *(volatile int*)&A.conv[rec[k].member];
+    };
+    // Members still iterating. Of a batch: the counter, which changes only
+    // while blocks wait at the barrier after phase A, so it reads the same in
+    // every block here.
+    __shared__ int s_go;
+    auto go_on = [&] {
+        if (single) return slot[0].conv == 0;
+        if (threadIdx.x == 0) s_go = *(volatile int*)A.active;
+        __syncthreads();
+        const int v = s_go;
+        __syncthreads();
+        return v > 0;
+    };
+    while (go_on()) {
+        for (int i = 0; i < ns; ++i) {
+            const PSlot& c = slot[single ? 0 : i];
+            if (c.conv) continue;
+            double t[1] = {0.0};
+            if (A.dense0) p_dense_a<S>(A, rec[i], A.dense[0], it, c.alpha, c.beta, t, smem);
+            else p_phase_a<S>(A, rec[i], it, c.alpha, c.beta, t, smem);
+            if (it > 0) ps_block_total<1>(t, pr + rec[i].tile, nt);
+        }
+        if (!ps_sync(g)) return;
+        bool told = false;
+        for (int l = 1; l < A.ng; ++l) {
+            for (int i = lev0[l] - base; i < lev0[l + 1] - base; ++i)
+                if (!rconv[i]) p_down<S>(rec[i], A.nu, smem);
+            if (!(told ? ps_sync(g, refresh) : ps_sync(g, decide))) return;
+            told = true;
+            if (single && slot[0].conv) break;
+        }
+        if (single && slot[0].conv) break;
+        p_dense_rows<S>(A, smem);
+        if (!(told ? ps_sync(g, refresh) : ps_sync(g, decide))) return;
+        if (single && slot[0].conv) break;
+        for (int l = A.ng - 1; l >= 1; --l) {
+            for (int i = lev0[l] - base; i < lev0[l + 1] - base; ++i)
+                if (!rconv[i]) p_up<S>(rec[i], A.nu, smem);
+            if (!ps_sync(g)) return;
+        }
+        for (int i = 0; i < ns; ++i) {
+            if (slot[single ? 0 : i].conv) continue;
+            double t[2] = {0.0, 0.0};
+            if (A.dense0) p_dense_b<S>(A, rec[i], A.dense[0], t, smem);
+            else p_phase_b<S>(A, rec[i], it, t, smem);
+            ps_block_total<2>(t, pz + rec[i].tile, nt);
+        }
+        if (!ps_sync(g)) return;
+        for (int i = w; i < nslot; i += PS_NT / 32) {
+            PSlot& c = slot[i];
+            if (c.conv) continue;
+            const double rz = ps_total(pz + c.n0, c.nn), zw = ps_total(pz + nt + c.n0, c.nn);
+            if (lane) continue;
+            // beta = rz / rz_old, <p, A p> = <z, w> - beta^2 <p, A p>_old,
+            // alpha = rz / <p, A p>
+            c.beta = rz * c.irz;
+            c.d = zw - c.beta * c.beta * c.d;
+            c.alpha = rz / c.d;
+            c.irz = 1.0 / rz;
+        }
+        __syncthreads();
+        ++it;
+    }
+    if (threadIdx.x == 0)
+        for (int i = 0; i < nslot; ++i)
+            if (slot[i].owner) {
+                DevScalars& sc = A.scs[slot[i].member];
+                sc.bb = slot[i].bb;
+                sc.rr = slot[i].rr;
+                sc.converged = 1;
+            }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        A.eg->loops_out += 1;
+        A.eg->loops_in += it;
+    }
+}
+
+// the level-0 down leg of every member by itself (a measurement)
+template <typename S>
+__global__ void __launch_bounds__(PS_NT, 1) k_ps_down0(const __grid_constant__ PSArgs A)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int* l0 = A.rec0 + blockIdx.x * (A.ng + 1);
+    double t[1] = {0.0};
+    for (int i = l0[0]; i < l0[1]; ++i) p_phase_a<S>(A, A.recs[i], 0, 0.0, 0.0, t, smem);
+}
+
+__global__ void k_ps_setup(const __grid_constant__ PSArgs A, double tol2, int maxit)
+{
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b == 0) {
+        A.bar->count = 0u;
+        A.bar->abort = 0;
+        *A.active = 0;
+    }
+    if (b < A.nmem) {
+        A.scs[b].tol2 = tol2;
+        A.scs[b].maxit = maxit;
+        A.scs[b].converged = 0;
+        A.scs[b].iter = 0;
+    }
+}
+
+// ---- host ----------------------------------------------------------------------
+constexpr size_t PS_SMEM = 180 * 1024;
+
+// estimated cycles of a block for one tile of tw x th nodes: a fixed cost and
+// the cells its legs visit (the FP64 pipe's rate, or the issue rate in FP32)
+static double tile_cost(int tw, int th, int prec)
+{
+    const double n = (double)(tw + 10) * (th + 10);
+    double cells = 2.0 * n + 3.0 * tw * th;
+    for (int q = 0; q < 5; ++q) cells += (double)(tw + 2 * q) * (th + 2 * q);
+    return 3000.0 + (prec == 0 ? 2.0 : 0.5) * cells;
+}
+
+struct TileDim {
+    int tw, th, ntx, nty;
+};
+
+// dimensions of a level's tiles: nx x ny nodes in ntx x nty tiles, even sizes
+static TileDim tile_dim(int nx, int ny, int ntx, int nty)
+{
+    TileDim d;
+    d.tw = std::max(2, ((nx + ntx - 1) / ntx + 1) / 2 * 2);
+    d.th = std::max(2, ((ny + nty - 1) / nty + 1) / 2 * 2);
+    d.ntx = (nx + d.tw - 1) / d.tw;
+    d.nty = (ny + d.th - 1) / d.th;
+    return d;
+}
+
+static size_t region_bytes(int tw, int th, int prec)
+{
+    return (size_t)(tw + 10) * (th + 10) * (prec == 0 ? 17 : 9);
+}
+
+// Tiles of one level of all members. One member: of all partitions the one
+// with the smallest estimate of the busiest block's time; up to about 1300^2
+// nodes that is one tile per block. A batch: all members get tiles of at most
+// T x T nodes, T the one with the smallest estimate of (tiles per block) x
+// (cost of a tile).
+static std::vector<TileDim> pick_tiles(const std::vector<std::pair<int, int>>& nxny, int sms,
+                                       int prec)
+{
+    std::vector<TileDim> best(nxny.size(), TileDim{0, 0, 0, 0}), cur(nxny.size());
+    double bc = 0.0;
+    if (nxny.size() == 1) {
+        const int nx = nxny[0].first, ny = nxny[0].second;
+        if (nx <= 0) return best;
+        for (int ntx = 1; ntx <= (nx + 7) / 8; ++ntx)
+            for (int nty = 1; nty <= (ny + 7) / 8; ++nty) {
+                const TileDim d = tile_dim(nx, ny, ntx, nty);
+                if (region_bytes(d.tw, d.th, prec) > PS_SMEM) continue;
+                const long long nt = (long long)d.ntx * d.nty;
+                const double c = (double)((nt + sms - 1) / sms) * tile_cost(d.tw, d.th, prec);
+                if (bc == 0.0 || c < bc) {
+                    bc = c;
+                    best[0] = d;
+                }
+            }
+        return best;
+    }
+    for (int T = 8; T <= 128; T += 4) {
+        if (region_bytes(T, T, prec) > PS_SMEM) break;
+        double total = 0.0, worst = 0.0;
+        for (size_t b = 0; b < nxny.size(); ++b) {
+            const int nx = nxny[b].first, ny = nxny[b].second;
+            cur[b] = TileDim{0, 0, 0, 0};
+            if (nx <= 0) continue;
+            cur[b] = tile_dim(nx, ny, (nx + T - 1) / T, (ny + T - 1) / T);
+            const double c = tile_cost(cur[b].tw, cur[b].th, prec);
+            total += c * cur[b].ntx * cur[b].nty;
+            worst = std::max(worst, c);
+        }
+        // list scheduling: at most the mean load and one more tile
+        const double c = total <= worst * sms ? std::max(worst, total / sms)
+                                              : total / sms + 0.5 * worst;
+        if (bc == 0.0 || c < bc) {
+            bc = c;
+            best = cur;
+        }
+    }
+    return best;
+}
+
+int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long nelem,
+             DevScalars* scs, BSGlobals* eg, int* status)
+{
+    ps_free(s);
+    const int n = (int)mem.size(), sms = ps_sms();
+    if (n < 1 || sms < 1 || nelem <= 0) return 0;
+    const size_t es = prec == 0 ? 8 : 4;
+    auto dal = [&](size_t bytes) -> void* {
+        void* p = nullptr;
+        if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
+        cudaMemset(p, 0, bytes);
+        s.owned.push_back(p);
+        return p;
+    };
+    // grid levels of every member: down to its dense level
+    std::vector<int> ng(n);
+    int maxg = 0, nrows = 0;
+    size_t minv_elems = 0;
+    for (int b = 0; b < n; ++b) {
+        const std::vector<MGLevel>& lev = mem[b].mg->lev;
+        int l = n == 1 ? 0 : 1;
+        for (; l < (int)lev.size(); ++l) {
+            const long long k = (long long)lev[l].nyn * lev[l].nxn;
+            if (k <= mem[b].ndense_cap && ps_band_ok(k, lev[l].nxn)) break;
+        }
+        if (l >= (int)lev.size() || l >= PS_LMAX) return 0;
+        for (int q = 0; q < l; ++q)  // colours and the coarse grid wrap only over an even count
+            if (lev[q].per && lev[q].nxn % 2) return 0;
+        ng[b] = l;
+        maxg = std::max(maxg, l);
+        nrows += lev[l].nyn * lev[l].nxn;
+        minv_elems += (size_t)lev[l].nyn * lev[l].nxn * lev[l].nyn * lev[l].nxn;
+    }
+    PSArgs& a = s.a;
+    memset(&a, 0, sizeof(a));
+    a.dense0 = maxg == 0;
+    a.ng = std::max(1, maxg);
+    a.nmem = n;
+    a.nrows = nrows;
+    // tiles, level by level; a level's tiles are dealt to the blocks in turn
+    std::vector<std::vector<PTile>> tl(a.ng);
+    std::vector<PDense> dense(n);
+    size_t smem = 0;
+    for (int b = 0; b < n; ++b) {
+        const MGLevel& D = mem[b].mg->lev[ng[b]];
+        const int nd = D.nyn * D.nxn;
+        dense[b].n = nd;
+        dense[b].row0 = b ? dense[b - 1].row0 + dense[b - 1].n : 0;
+        dense[b].b = dal((size_t)nd * es);
+        dense[b].x = dal((size_t)nd * es);
+        void* minv = dal((size_t)nd * nd * es);
+        dense[b].minv = minv;
+        if (!dense[b].b || !dense[b].x || !minv) return 2;
+        // -A of the dense level (identity rows at non-fluid nodes: their b is 0)
+        const std::vector<uint8_t>& hm = mem[b].mg->hmask[ng[b]];
+        const int w1 = D.nxn + 1;
+        std::vector<double> h((size_t)nd * w1, 0.0);
+        for (int J = 0; J < D.nyn; ++J)
+            for (int I = 0; I < D.nxn; ++I) {
+                const int k = J * D.nxn + I;
+                h[(size_t)k * w1] = hm[k] ? -D.diag : 1.0;
+                if (!hm[k]) continue;
+                if (I > 0 && hm[k - 1]) h[(size_t)k * w1 + 1] -= D.cx;
+                if (J > 0 && hm[k - D.nxn]) h[(size_t)k * w1 + D.nxn] -= D.cy;
+                if (D.per && I == D.nxn - 1 && D.nxn > 1 && hm[k - I])
+                    h[(size_t)k * w1 + I] -= D.cx;
+            }
+        const int rc = ps_invert(h, nd, D.nxn, {}, -1.0, prec, minv);
+        if (rc == 5) return 0;
+        if (rc) return rc;
+        smem = std::max(smem, (nd + 4 * (size_t)((nrows + sms - 1) / sms + 1)) * es);
+    }
+    for (int l = 0; l < a.ng; ++l) {
+        std::vector<std::pair<int, int>> dims(n);
+        for (int b = 0; b < n; ++b) {
+            const MGLevel& L = mem[b].mg->lev[l];
+            dims[b] = l < ng[b] || (l == 0 && a.dense0) ? std::make_pair(L.nxn, L.nyn)
+                                                        : std::make_pair(0, 0);
+        }
+        const std::vector<TileDim> td = pick_tiles(dims, sms, prec);
+        for (int b = 0; b < n; ++b) {
+            if (dims[b].first <= 0) continue;
+            if (td[b].tw <= 0) return 0;
+            const std::vector<MGLevel>& lev = mem[b].mg->lev;
+            const MGLevel& L = lev[l];
+            PTile t;
+            memset(&t, 0, sizeof(t));
+            t.m = L.m;
+            t.x = L.x;
+            t.xa = L.xa;
+            t.b = L.b;
+            t.off = L.off;
+            t.pitch = (int)L.pitch;
+            t.nyn = L.nyn;
+            t.nxn = L.nxn;
+            t.per = L.per;
+            t.member = b;
+            t.tw = td[b].tw;
+            t.th = td[b].th;
+            t.cx = L.cx;
+            t.cy = L.cy;
+            t.md = L.md;
+            t.id = L.idiag;
+            t.dg = L.diag;
+            t.cxi = L.cx * L.idiag;
+            t.cyi = L.cy * L.idiag;
+            if (l < ng[b]) {
+                const MGLevel& C = lev[l + 1];
+                const bool d = l + 1 == ng[b];
+                t.cx_ = d ? dense[b].x : C.x;
+                t.cb = d ? dense[b].b : C.b;
+                t.coff = d ? 0 : C.off;
+                t.cpitch = d ? C.nxn : (int)C.pitch;
+                t.cm = C.m;
+                t.cmoff = C.off;
+                t.cmpitch = (int)C.pitch;
+                t.cyn = C.nyn;
+                t.cxn = C.nxn;
+            }
+            t.n0 = (int)tl[l].size();
+            t.nn = td[b].ntx * td[b].nty;
+            for (int y = 0; y < td[b].nty; ++y)
+                for (int x = 0; x < td[b].ntx; ++x) {
+                    t.J0 = y * t.th;
+                    t.I0 = x * t.tw;
+                    t.tile = (int)tl[l].size();
+                    tl[l].push_back(t);
+                }
+            smem = std::max(smem, region_bytes(t.tw, t.th, prec));
+        }
+    }
+    a.ntiles = (int)tl[0].size();
+    std::vector<PTile> recs;
+    std::vector<int> rec0;
+    for (int g = 0; g < sms; ++g) {
+        const size_t first = recs.size();
+        for (int l = 0; l < a.ng; ++l) {
+            rec0.push_back((int)recs.size());
+            for (size_t t = g; t < tl[l].size(); t += sms) recs.push_back(tl[l][t]);
+            if (l == 0 && recs.size() - first > PS_SLOTS) return 0;
+        }
+        rec0.push_back((int)recs.size());
+        if (recs.size() - first > PS_RECS) return 0;
+    }
+    PTile* drec = (PTile*)dal(recs.size() * sizeof(PTile));
+    int* d0 = (int*)dal(rec0.size() * sizeof(int));
+    PDense* dd = (PDense*)dal(n * sizeof(PDense));
+    double* vec[6];
+    for (auto& p : vec)
+        if (!(p = (double*)dal((size_t)nelem * 8))) return 2;
+    a.part = (double*)dal((size_t)5 * a.ntiles * sizeof(double));
+    a.conv = (int*)dal(n * sizeof(int));
+    a.active = (int*)dal(sizeof(int));
+    a.bar = (PSBar*)dal(sizeof(PSBar));
+    if (!drec || !d0 || !dd || !a.part || !a.conv || !a.active || !a.bar) return 2;
+    if (cudaMemcpy(drec, recs.data(), recs.size() * sizeof(PTile), cudaMemcpyHostToDevice) !=
+            cudaSuccess ||
+        cudaMemcpy(d0, rec0.data(), rec0.size() * sizeof(int), cudaMemcpyHostToDevice) !=
+            cudaSuccess ||
+        cudaMemcpy(dd, dense.data(), n * sizeof(PDense), cudaMemcpyHostToDevice) != cudaSuccess)
+        return 2;
+    a.recs = drec;
+    a.rec0 = d0;
+    a.dense = dd;
+    a.r[0] = vec[0];
+    a.r[1] = vec[1];
+    a.s[0] = vec[2];
+    a.s[1] = vec[3];
+    a.p = vec[4];
+    a.w = vec[5];
+    a.scs = scs;
+    a.eg = eg;
+    a.status = status;
+    s.prec = prec;
+    s.grid = sms;
+    s.smem = smem;
+    for (const void* k : {(const void*)k_ps_solve<double>, (const void*)k_ps_solve<float>,
+                          (const void*)k_ps_down0<double>, (const void*)k_ps_down0<float>})
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS_SMEM) !=
+            cudaSuccess)
+            return 3;
+    if (smem > PS_SMEM) return 0;
+    s.on = true;
+    return 0;
+}
+
+void ps_free(PSolver& s)
+{
+    for (void* p : s.owned) cudaFree(p);
+    s.owned.clear();
+    s.on = false;
+    s.a = PSArgs{};
+}
+
+int ps_record(PSolver& s, double* x, double* b, int nu, double tol, int maxit, cudaStream_t st)
+{
+    s.a.x = x;
+    s.a.b = b;
+    s.a.nu = nu;
+    k_ps_setup<<<(s.a.nmem + 127) / 128, 128, 0, st>>>(s.a, tol * tol, maxit);
+    const int e = (int)cudaGetLastError();
+    if (e) return e;
+    void* args[1] = {&s.a};
+    return ps_launch(s.prec == 0 ? (const void*)k_ps_solve<double>
+                                 : (const void*)k_ps_solve<float>,
+                     s.grid, s.smem, args, st);
+}
+
+int ps_time_down(PSolver& s, int nu, cudaStream_t st)
+{
+    s.a.nu = nu;
+    if (s.prec == 0) k_ps_down0<double><<<s.grid, PS_NT, s.smem, st>>>(s.a);
+    else k_ps_down0<float><<<s.grid, PS_NT, s.smem, st>>>(s.a);
+    return (int)cudaGetLastError();
+}
+
+}  // namespace f2d

@@ -1,0 +1,83 @@
+// Persistent solve kernel for the masked vertex Poisson/Helmholtz operator of
+// one or many models: the FP64 form of the batched solver, and its FP32 form
+// for problems that do not fill the GPU. See psolver.cu.
+#pragma once
+#include <vector>
+
+#include "mg.cuh"
+#include "persist.cuh"
+
+namespace f2d {
+
+struct BSGlobals;
+
+// One tile of one level of one member: everything a block reads about it
+struct alignas(16) PTile {
+    const uint8_t* m;   // fluid mask of the level; node (J, I) at off + J pitch + I
+    void *x, *xa, *b;   // level arrays (level 0: z, xa, unused)
+    void *cx_, *cb;     // the next coarser level's x and b, node at coff + J cpitch + I
+    const uint8_t* cm;  // its mask, at cmoff + J cmpitch + I
+    long long off, coff, cmoff;
+    int pitch, cpitch, cmpitch;
+    int nyn, nxn, cyn, cxn, per;
+    int J0, I0, tw, th;
+    int member, tile;   // tile: index in the level's table
+    int n0, nn;         // the member's tiles in the level-0 table
+    int pad[2];
+    double cx, cy, md;              // the operator
+    double cxi, cyi, id, dg;        // couplings / diagonal, 1 / diagonal, diagonal
+};
+
+struct PDense {
+    const void* minv;  // n x n inverse of the member's dense level
+    void *b, *x;       // compact
+    int n, row0;       // rows of the members before it
+};
+
+constexpr int PS_LMAX = 14;
+constexpr int PS_RECS = 96;  // tile records of a block, all levels
+constexpr int PS_SLOTS = 64; // of these, on level 0
+
+struct PSArgs {
+    const PTile* recs;   // block b's records: rec0[b (ng + 1) + l] .. for level l
+    const int* rec0;
+    const PDense* dense;
+    int nmem, ng, nu;    // members, grid levels (of the deepest member)
+    int nrows;           // dense rows of all members
+    int dense0;          // one member whose level 0 is the dense level
+    int ntiles;          // level-0 tiles
+    double *x, *b, *r[2], *s[2], *p, *w;  // arenas, FP64
+    double* part;        // tile totals, 2 x 2 ntiles
+    int* conv;           // per member
+    int* active;         // members still iterating
+    DevScalars* scs;
+    BSGlobals* eg;
+    int* status;
+    PSBar* bar;
+};
+
+struct PSolver {
+    bool on = false;
+    PSArgs a = {};
+    int prec = 0, grid = 0;
+    size_t smem = 0;
+    std::vector<void*> owned;
+};
+
+struct PSMember {
+    const MGHost* mg;   // its hierarchy (mg_build)
+    int ndense_cap;     // nodes of its dense level, at most
+};
+
+// Build for the members' hierarchies: on = false (and no error) where the
+// kernel does not apply (no level small enough for the dense inverse, more
+// tiles than a block has records).
+int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long nelem,
+             DevScalars* scs, BSGlobals* eg, int* status);
+void ps_free(PSolver& s);
+// Record one solve of every member on `st`: x and b are the arenas (FP64).
+int ps_record(PSolver& s, double* x, double* b, int nu, double tol, int maxit, cudaStream_t st);
+// Measurement hook: one launch of the level-0 down leg of every member.
+int ps_time_down(PSolver& s, int nu, cudaStream_t st);
+
+}  // namespace f2d

@@ -22,6 +22,7 @@
 //    refinement round while the solution reaches FP64 accuracy.
 #include <cudaTypedefs.h>
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <type_traits>
@@ -1100,7 +1101,8 @@ int bs_time_down(BatchSolver& s, cudaStream_t st, int reps, int flush_l2, double
         if (fl) cudaMemsetAsync(fl, r & 0xff, flush_bytes, st);
         cudaEventRecord(a, st);
         const bool two = s.nu >= 2;
-        if (s.mode == 0) two ? launch_down0<double, 2>(s, st, ir) : launch_down0<double, 1>(s, st, ir);
+        if (s.mode == 0 && s.ps.on) err = ps_time_down(s.ps, s.nu, st);
+        else if (s.mode == 0) two ? launch_down0<double, 2>(s, st, ir) : launch_down0<double, 1>(s, st, ir);
         else two ? launch_down0<float, 2>(s, st, ir) : launch_down0<float, 1>(s, st, ir);
         cudaEventRecord(b, st);
         if (cudaEventSynchronize(b) != cudaSuccess) err = 3;
@@ -1119,6 +1121,11 @@ int bs_time_down(BatchSolver& s, cudaStream_t st, int reps, int flush_l2, double
 
 int bs_record(BatchSolver& s, cudaStream_t st, cudaStream_t st2, int* launches)
 {
+    if (s.ps.on) {
+        s.body_launches = 0;
+        if (launches) *launches = 2;
+        return ps_record(s.ps, (double*)s.v.x64, (double*)s.v.b64, s.nu, s.tol, s.maxit, st);
+    }
     return s.th == 64 ? bs_record_t<64>(s, st, st2, launches)
                       : bs_record_t<32>(s, st, st2, launches);
 }
@@ -1259,6 +1266,8 @@ static int bs_pipe_setup(BatchSolver& s, const std::vector<MGLevel>& levs,
     s.pipe = true;
     return 0;
 }
+
+constexpr long long PS_FP32_NODES = 1500000;
 
 int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uint8_t* dmask,
              int mode, const BSVecs& v, DevScalars* scs)
@@ -1420,7 +1429,26 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
         const int e = bs_pipe_setup(s, levs, info, dal);
         if (e) return e;
     }
-    if (mode == 1) {
+    // The persistent solve: every FP64 problem (its level kernels and loops
+    // cost more at every size), and FP32 problems of up to PS_FP32_NODES nodes:
+    // above that the refinement form's FP32 Krylov vectors and pipelined legs
+    // move less and are the faster ones.
+    {
+        long long n0 = 0;
+        std::vector<PSMember> pm(s.n);
+        for (int b = 0; b < s.n; ++b) {
+            const MGLevel& L = levs[(size_t)b * BS_LMAX];
+            n0 += (long long)L.nyn * L.nxn;
+            // the inverses of a batch: about 1.5M entries together
+            pm[b].mg = &s.mg[b];
+            pm[b].ndense_cap = s.n == 1 ? PS_NDENSE : (int)sqrt(1.5e6 / s.n);
+        }
+        if (mode == 0 || n0 <= PS_FP32_NODES) {
+            const int e = ps_build(s.ps, pm, mode, v.nelem, scs, s.eg, &s.eg->status);
+            if (e) return e;
+        }
+    }
+    if (mode == 1 && !s.ps.on) {
         if (v.nelem <= 0) return 1;
         s.pring = (float*)dal((size_t)BS_RING * v.nelem * sizeof(float));
         if (!s.pring) return 2;
@@ -1507,15 +1535,17 @@ int bs_autotune(BatchSolver& s, cudaStream_t st, cudaStream_t st2, void* x, cons
     cudaEventCreate(&eb);
     const bool eager = bs_eager();
     const double tin[5] = {1e-8, 1e-7, 1e-6, 1e-5, 1e-4};
-    const int ntin = s.mode == 1 ? 5 : 1;
+    const int ntin = s.mode == 1 && !s.ps.on ? 5 : 1;
     BSTune best{0, 0, 0.0, 1e300, 0};
     int err = 0;
     for (int th : {32, 64}) {
+        // (the persistent solve has the sweeps per leg as its only choice)
+        if (s.ps.on && th != s.th) continue;
         if (th != s.th && (err = bs_rebuild(s, th))) break;
         for (int nu : {1, 2}) {
             for (int k = 0; k < ntin && !err; ++k) {
                 s.nu = nu;
-                s.tol_in = s.mode == 1 ? tin[k] : s.tol_in;
+                s.tol_in = ntin > 1 ? tin[k] : s.tol_in;
                 s.v.x64 = x;
                 s.v.b64 = (void*)b;
                 cudaGraph_t g = nullptr;
@@ -1610,6 +1640,7 @@ int bs_set_schedule(BatchSolver& s, int th, int nu, double tol_in)
 
 void bs_free(BatchSolver& s)
 {
+    ps_free(s.ps);
     if (s.s3) {
         cudaStreamDestroy(s.s3);
         s.s3 = nullptr;

@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "mg.cuh"
+#include "psolver.cuh"
 
 namespace f2d {
 
@@ -59,6 +60,9 @@ struct BSMemberDesc {
 };
 
 struct BatchSolver {
+    // the whole solve in one persistent kernel (bs_build's rule); the kernels
+    // below where it does not apply
+    PSolver ps;
     int n = 0;
     int mode = 0;  // 0: FP64 multigrid-PCG; 1: FP32 inner PCG + FP64 refinement
     std::vector<MGHost> mg;
