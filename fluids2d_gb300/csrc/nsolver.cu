@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
     const int maxit = sc->maxit;
     int it = 0;
     // the decision after the update of iteration it: warps 1 and 2, while
-    // thread 0 waits at the next barrier (the phase before it is lost when
+    // warp 0 waits at the next barrier (the phase before it is lost when
     // the solve is over, but its totals cost no time)
     auto decide = [&] {
         const int w = threadIdx.x >> 5;
@@ -723,8 +723,7 @@ __global__ void k_ns_setup(DevScalars* sc, double tol2, int maxit, PSBar* bar)
     sc->maxit = maxit;
     sc->converged = 0;
     sc->iter = 0;
-    bar->count = 0u;
-    bar->abort = 0;
+    ps_reset(bar);
 }
 
 // ---- host ----------------------------------------------------------------------
@@ -1107,7 +1106,7 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
     // to all blocks, and a barrier of 152 blocks (1.36 us) costs hardly more
     // than one of 25 (1.28 us)
     s.grid = sms;
-    s.smem = (size_t)(a.nd + 4 * ((a.nd + sms - 1) / sms)) * es;
+    s.smem = (size_t)(a.nd + 128 * ((a.nd + sms - 1) / sms + 1)) * es;
     for (int q = 0; q < a.ng; ++q) {
         const int h = q == 0 ? NS_H : 4;
         const size_t n = (size_t)(a.lev[q].tw + 2 * h) * (a.lev[q].th + 2 * h);

@@ -18,20 +18,30 @@ namespace f2d {
 constexpr int PS_NT = 512;  // threads of a block (one block per SM)
 
 // ---- grid barrier ------------------------------------------------------------
-// One counter, zeroed before the launch, that every block increments once per
-// barrier; the k-th barrier is passed when it reaches k * gridDim.x. The wait
+// Four counters on lines of their own, zeroed before the launch; a block
+// increments one of them once per barrier, and the k-th barrier is passed when
+// each reaches k times its number of blocks. (One counter for all 152 blocks:
+// 2840 cycles with writes in flight, four: 2660. A flag per block that all
+// blocks poll: 5000 to 8500; clusters with one arrival each: 3500 and more.) The wait
 // is bounded: after limit_ns without progress the block sets the abort word
 // and the kernel's status, and every block returns from the kernel.
 struct PSBar {
-    unsigned int count;  // arrivals
-    int abort;           // a wait ran out
+    unsigned int count[4][32];  // arrivals
+    int abort;                  // a wait ran out
 };
 
 struct PSGrid {
     PSBar* bar;
     int* status;
-    unsigned int target;
+    unsigned int round;
 };
+
+// zero the counters (before the launch)
+__device__ __forceinline__ void ps_reset(PSBar* b)
+{
+    for (int k = 0; k < 4; ++k) b->count[k][0] = 0u;
+    b->abort = 0;
+}
 
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p)
 {
@@ -42,9 +52,9 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p)
 
 // Returns false when the kernel must return. Writes of all threads of all
 // blocks before the barrier are visible to all threads after it: the CTA
-// barrier orders them before thread 0's release, and its acquire before the
-// second CTA barrier. (Data written in the kernel is read with plain loads,
-// never through the read-only path.) While thread 0 waits, the other warps
+// barrier orders them before thread 0's release, and warp 0's acquires before
+// the second CTA barrier. (Data written in the kernel is read with plain loads,
+// never through the read-only path.) While warp 0 waits, the other warps
 // run idle(): work that needs nothing of this phase and is over in less time
 // than the barrier takes.
 template <typename F>
@@ -52,24 +62,33 @@ __device__ __forceinline__ bool ps_sync(PSGrid& g, F idle)
 {
     __shared__ int s_dead;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        g.target += gridDim.x;
+    if (threadIdx.x < 32) {
+        const unsigned lane = threadIdx.x;
         int dead = 0;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&g.bar->count) : "memory");
-        uint64_t t0 = 0;
-        for (unsigned spin = 0; (int)(ld_acquire(&g.bar->count) - g.target) < 0; ++spin) {
-            if ((spin & 255u) != 255u) continue;
-            const uint64_t t = globaltimer_ns();
-            if (t0 == 0) t0 = t;
-            if (t - t0 > 2000000000ull || *(volatile int*)&g.bar->abort) {
-                *(volatile int*)&g.bar->abort = 1;
-                atomicOr(g.status, ST_GRID_TIMEOUT);
-                dead = 1;
-                break;
+        g.round += 1;
+        if (lane == 0)
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(
+                             g.bar->count[blockIdx.x & 3])
+                         : "memory");
+        if (lane < 4) {
+            // blocks of counter `lane`
+            const unsigned target = g.round * ((gridDim.x + 3 - lane) / 4);
+            uint64_t t0 = 0;
+            for (unsigned spin = 0; (int)(ld_acquire(g.bar->count[lane]) - target) < 0; ++spin) {
+                if ((spin & 255u) != 255u) continue;
+                const uint64_t t = globaltimer_ns();
+                if (t0 == 0) t0 = t;
+                if (t - t0 > 2000000000ull || *(volatile int*)&g.bar->abort) {
+                    *(volatile int*)&g.bar->abort = 1;
+                    atomicOr(g.status, ST_GRID_TIMEOUT);
+                    dead = 1;
+                    break;
+                }
             }
         }
-        s_dead = dead;
-    } else if (threadIdx.x >= 32) {
+        dead = __any_sync(0xffffffffu, dead);
+        if (lane == 0) s_dead = dead;
+    } else {
         idle();
     }
     __syncthreads();
@@ -91,20 +110,39 @@ __device__ __forceinline__ bool ps_sync(PSGrid& g)
 template <int N>
 __device__ __forceinline__ void ps_block_total(const double (&v)[N], double* part, int stride)
 {
+    static_assert(N <= 4, "two values per half warp of four warps");
     __shared__ double sh[N][PS_NT];
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < N; ++k) sh[k][threadIdx.x] = v[k];
     __syncthreads();
-    // value k: warps 4 k' .. (k' = k mod 4) hold a quarter each
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, k = w >> 2, q = w & 3;
+    // warps 0 .. 3 values 0 and 1, warps 4 .. 7 values 2 and 3, each a quarter
+    // of the threads' values; the second value goes to the upper half warp at
+    // the first step, so the two share the rest of the tree
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, k = (w >> 2) * 2;
     if (k < N) {
-        const double* s = &sh[k][q * (PS_NT / 4) + lane];
-        double a = (s[0] + s[32]) + (s[64] + s[96]);
+        const int q = (w & 3) * (PS_NT / 4);
+        const double* s = &sh[k][q + lane];
+        double a = 0.0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        for (int i = 0; i < PS_NT / 4; i += 128)
+            a += (s[i] + s[i + 32]) + (s[i + 64] + s[i + 96]);
+        if (k + 1 < N) {
+            const double* u = &sh[k + 1 < N ? k + 1 : k][q + lane];
+            double b = 0.0;
+#pragma unroll
+            for (int i = 0; i < PS_NT / 4; i += 128)
+                b += (u[i] + u[i + 32]) + (u[i + 64] + u[i + 96]);
+            const double o = __shfl_xor_sync(0xffffffffu, lane < 16 ? b : a, 16);
+            a = (lane < 16 ? a : b) + o;
+        } else {
+            a += __shfl_xor_sync(0xffffffffu, a, 16);
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
         __syncwarp();
-        if (lane == 0) sh[k][q * (PS_NT / 4)] = a;
+        if (lane == 0) sh[k][q] = a;
+        if (lane == 16 && k + 1 < N) sh[k + 1 < N ? k + 1 : k][q] = a;
     }
     __syncthreads();
     if (threadIdx.x < N) {
@@ -129,6 +167,24 @@ __device__ __forceinline__ double ps_total(const double* p, int n)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     return a;
+}
+
+// Two of them at once
+__device__ __forceinline__ void ps_total2(const double* p, const double* q, int n, double& tp,
+                                          double& tq)
+{
+    const int lane = threadIdx.x & 31;
+    double a = 0.0, b = 0.0;
+    for (int i = lane; i < n; i += 32) {
+        a += __ldcg(&p[i]);
+        b += __ldcg(&q[i]);
+    }
+    const double o = __shfl_xor_sync(0xffffffffu, lane < 16 ? b : a, 16);
+    a = (lane < 16 ? a : b) + o;
+#pragma unroll
+    for (int s = 8; s > 0; s >>= 1) a += __shfl_xor_sync(0xffffffffu, a, s);
+    tp = __shfl_sync(0xffffffffu, a, 0);
+    tq = __shfl_sync(0xffffffffu, a, 16);
 }
 
 // The grid's totals of N values, then f(totals) in thread 0, whose results
@@ -161,13 +217,16 @@ __device__ __forceinline__ int fdiv(int k, float rw) { return __float2int_rz((k 
 // grid level about 17k; and the coarse correction is exact.
 constexpr int PS_NDENSE = 2048;
 
-// rows r0 .. r1 - 1 of x = M b; sb: n + 4 (r1 - r0) elements of shared memory
+// rows r0 .. r1 - 1 of x = M b; sb: n + 128 (r1 - r0) elements of shared
+// memory. The lanes' sums of a row's four quarters meet in shared memory (a
+// shuffle tree per quarter would cost as many FP64 instructions as the row's
+// products).
 template <typename S>
 __device__ __forceinline__ void ps_dense(const S* __restrict__ M, const S* b, S* x, int n, int r0,
                                          int r1, S* sb)
 {
     constexpr int NW = PS_NT / 32, U = 8;
-    S* part = sb + n;  // 4 per row
+    S* part = sb + n;  // 128 per row
     if (r1 <= r0) return;
     for (int e = threadIdx.x; e < n; e += PS_NT) sb[e] = __ldcg(&b[e]);
     __syncthreads();
@@ -185,13 +244,26 @@ __device__ __forceinline__ void ps_dense(const S* __restrict__ M, const S* b, S*
             for (int u = 0; u < U; ++u)
                 if (e + 32 * u < end) a += v[u] * sb[e + 32 * u];
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) part[t] = a;
+        part[32 * t + lane] = a;
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < r1 - r0; t += PS_NT)
-        x[r0 + t] = (part[4 * t] + part[4 * t + 1]) + (part[4 * t + 2] + part[4 * t + 3]);
+    // 8 lanes per row add 16 values each, then a tree over the 8
+    for (int t0 = 0; t0 < 8 * (r1 - r0); t0 += PS_NT) {
+        const int t = t0 + threadIdx.x;
+        const bool in = t < 8 * (r1 - r0);
+        S a = S(0);
+        if (in) {
+            // (stride 8: consecutive lanes read consecutive elements)
+            const S* p = part + 128 * (t >> 3) + (t & 7);
+#pragma unroll
+            for (int u = 0; u < 16; ++u) a += p[8 * u];
+        }
+        if (__any_sync(0xffffffffu, in)) {
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (in && (t & 7) == 0) x[r0 + (t >> 3)] = a;
+        }
+    }
 }
 
 // Host: the inverse of a symmetric positive definite banded matrix H of n

@@ -35,6 +35,8 @@
 // launch for 40 to 400 ns of work on the whole chip).
 #include <algorithm>
 #include <cstring>
+#include <functional>
+#include <queue>
 
 #include "psolver.cuh"
 #include "solver.cuh"
@@ -87,7 +89,8 @@ __device__ __forceinline__ bool p_node(const PTile& t, int J, int& I)
 template <typename S>
 __device__ __forceinline__ S p_gs(const PReg<S>& R, int e)
 {
-    return R.b[e] - (R.cxi * (R.x[e - 1] + R.x[e + 1]) + R.cyi * (R.x[e - R.W] + R.x[e + R.W]));
+    return fma(-R.cxi, R.x[e - 1] + R.x[e + 1],
+               fma(-R.cyi, R.x[e - R.W] + R.x[e + R.W], R.b[e]));
 }
 
 // half sweep of a colour over the nodes within rad of the tile
@@ -170,14 +173,14 @@ __device__ __forceinline__ void p_down_leg(const PReg<S>& R, const PTile& t, int
 #pragma unroll 1
     for (int q = 1; q < 2 * nu; ++q) p_half(R, q & 1, 2 * nu + 1 - q);
     {
-        // residual = diagonal (Gauss-Seidel value - x) of the red nodes within
+        // residual / diagonal = Gauss-Seidel value - x of the red nodes within
         // 1 of the tile, into b
         const int o = R.h - 1, nr = R.th + 2, wc = R.tw / 2 + 1;
         const float rw = 1.0f / (float)wc;
         for (int k = threadIdx.x; k < nr * wc; k += PS_NT) {
             const int a = fdiv(k, rw), r = o + a;
             const int e = r * R.W + o + 2 * (k - a * wc) + ((r + o) & 1);
-            R.b[e] = R.m[e] ? R.dg * (p_gs(R, e) - R.x[e]) : S(0);
+            R.b[e] = R.m[e] ? p_gs(R, e) - R.x[e] : S(0);
         }
         __syncthreads();
     }
@@ -190,26 +193,60 @@ __device__ __forceinline__ void p_down_leg(const PReg<S>& R, const PTile& t, int
         const int e = (R.h + 2 * a) * R.W + R.h + 2 * c;
         S v = S(0);
         if (t.cm[t.cmoff + (long long)J * t.cmpitch + I])
-            v = R.b[e] + S(0.25) * ((R.b[e - R.W - 1] + R.b[e - R.W + 1]) +
-                                    (R.b[e + R.W - 1] + R.b[e + R.W + 1]));
+            v = R.dg * fma(S(0.25), (R.b[e - R.W - 1] + R.b[e - R.W + 1]) +
+                                        (R.b[e + R.W - 1] + R.b[e + R.W + 1]),
+                           R.b[e]);
         ((S*)t.cb)[t.coff + (long long)J * t.cpitch + I] = v;
     }
 }
 
-// P (coarse x) at the red node (J, I): the coarse node, or the mean of four
+// P (coarse x) at the red node (J, I) is the coarse node v[0], or (odd rows)
+// the mean of the four v. use: whether to load at all. (The level has no fluid
+// node on a closed edge: those rows and columns of the coarse level are 0.)
 template <typename S>
 __device__ __forceinline__ void p_coarse(const PTile& t, bool use, int J, int I, S (&v)[4])
 {
-    const S* X = (const S*)t.cx_;
     const int cj = J >> 1, ci = I >> 1;
-    const bool odd = use && (J & 1);
+    const S* xc = (const S*)t.cx_ + t.coff + (long long)cj * t.cpitch;
+    const bool odd = use && (J & 1), up = odd && cj + 1 < t.cyn;
     const int c1 = ci + 1 < t.cxn ? ci + 1 : (t.per ? 0 : -1);
-    const long long k = t.coff + (long long)cj * t.cpitch;
-    const bool up = odd && cj + 1 < t.cyn;
-    v[0] = use ? X[k + ci] : S(0);
-    v[1] = odd && c1 >= 0 ? X[k + c1] : S(0);
-    v[2] = up ? X[k + t.cpitch + ci] : S(0);
-    v[3] = up && c1 >= 0 ? X[k + t.cpitch + c1] : S(0);
+    v[0] = use ? xc[ci] : S(0);
+    v[1] = odd && c1 >= 0 ? xc[c1] : S(0);
+    v[2] = up ? xc[t.cpitch + ci] : S(0);
+    v[3] = up && c1 >= 0 ? xc[t.cpitch + c1] : S(0);
+}
+
+// x = xa + P (coarse x) at the region's red nodes, 0 at its black ones. FP64:
+// the nodes of even rows of the level and those of odd rows are dealt to
+// different warps, so only the latter average and no lane idles on black
+// nodes (in the region's own order a warp spent five FP64 instructions on
+// every pair of rows, a sixth of phase B at 1024^2). FP32, where the indexing
+// costs more than the arithmetic: in the region's own order (p_load's use).
+template <typename S>
+__device__ __forceinline__ void p_prolong(const PReg<S>& R, const PTile& t)
+{
+    const S* XA = (const S*)t.xa;
+    const int wc = R.W / 2, n2 = wc * (R.RH / 2);
+    const float rw = 1.0f / (float)wc;
+    for (int i = threadIdx.x; i < 2 * n2; i += PS_NT) {
+        const bool odd = i >= n2;  // odd row of the level
+        const int a = fdiv(odd ? i - n2 : i, rw);
+        const int r = 2 * a + ((R.h & 1) != (int)odd);
+        const int c = 2 * ((odd ? i - n2 : i) - a * wc) + (r & 1);
+        const int J = R.J0 - R.h + r, e = r * R.W + c;
+        int I = R.I0 - R.h + c;
+        S x = S(0);
+        if (p_node(t, J, I)) {
+            const long long k = t.off + (long long)J * t.pitch + I;
+            const S xa = XA[k];
+            S v[4];
+            p_coarse<S>(t, true, J, I, v);
+            const S pc = odd ? S(0.25) * ((v[0] + v[1]) + (v[2] + v[3])) : v[0];
+            if (t.m[k]) x = xa + pc;
+        }
+        R.x[e] = x;
+        R.x[r * R.W + (c ^ 1)] = S(0);
+    }
 }
 
 template <typename S>
@@ -244,27 +281,34 @@ __device__ __forceinline__ void p_up(const PTile& t, int nu, unsigned char* smem
 {
     const PReg<S> R = p_region<S>(t, 2 * nu, smem);
     const S* B = (const S*)t.b;
-    const S* XA = (const S*)t.xa;
     const S id = conv<S>(t.id);
-    S b[PB], xa[PB], cv[PB][4];
+    S b[PB];
     uint8_t m[PB];
+    const S* XA = (const S*)t.xa;
+    S xr[PB], cv[PB][4];
+    int oj[PB];
     p_load(
         R, t,
         [&](int q, bool in, long long k, int J, int I) {
-            const bool red = in && ((J + I) & 1) == 0;
             m[q] = in ? t.m[k] : 0;
+            if constexpr (sizeof(S) == 4) {
+                const bool red = in && ((J + I) & 1) == 0;
+                xr[q] = red ? XA[k] : S(0);
+                p_coarse<S>(t, red, J, I, cv[q]);
+                oj[q] = J & 1;
+            }
             b[q] = in ? B[k] : S(0);
-            xa[q] = red ? XA[k] : S(0);
-            p_coarse<S>(t, red, J, I, cv[q]);
         },
-        [&](int q, int e, bool, long long, int r, int c) {
-            // (a red node's parity is its row's: R.h and J0 are even)
-            const S pc = r & 1 ? S(0.25) * ((cv[q][0] + cv[q][1]) + (cv[q][2] + cv[q][3]))
-                               : cv[q][0];
+        [&](int q, int e, bool, long long, int, int) {
             R.m[e] = m[q];
             R.b[e] = m[q] ? b[q] * id : S(0);
-            R.x[e] = m[q] && ((r + c) & 1) == 0 ? xa[q] + pc : S(0);
+            if constexpr (sizeof(S) == 4)
+                R.x[e] = m[q] ? xr[q] + (oj[q] ? S(0.25) * ((cv[q][0] + cv[q][1]) +
+                                                            (cv[q][2] + cv[q][3]))
+                                               : cv[q][0])
+                              : S(0);
         });
+    if constexpr (sizeof(S) == 8) p_prolong(R, t);
     __syncthreads();
 #pragma unroll 1
     for (int q = 1; q <= 2 * nu; ++q) p_half(R, q & 1, 2 * nu - q);
@@ -343,28 +387,34 @@ __device__ __forceinline__ void p_phase_b(const PSArgs& A, const PTile& t, int i
     const int nu = A.nu, h = 2 * nu + 1;
     const PReg<S> R = p_region<S>(t, h, smem);
     const double* rr = A.r[it & 1];
-    const S* XA = (const S*)t.xa;
     const S id = conv<S>(t.id);
     uint8_t m[PB];
     double rv[PB];
-    S xa[PB], cv[PB][4];
+    const S* XA = (const S*)t.xa;
+    S xr[PB], cv[PB][4];
+    int oj[PB];
     p_load(
         R, t,
         [&](int q, bool in, long long k, int J, int I) {
-            const bool red = in && ((J + I) & 1) == 0;
             m[q] = in ? t.m[k] : 0;
+            if constexpr (sizeof(S) == 4) {
+                const bool red = in && ((J + I) & 1) == 0;
+                xr[q] = red ? XA[k] : S(0);
+                p_coarse<S>(t, red, J, I, cv[q]);
+                oj[q] = J & 1;
+            }
             rv[q] = in ? rr[k] : 0.0;
-            xa[q] = red ? XA[k] : S(0);
-            p_coarse<S>(t, red, J, I, cv[q]);
         },
-        [&](int q, int e, bool, long long, int r, int c) {
-            // (h is odd: even rows of the region are odd rows of the level)
-            const S pc = r & 1 ? cv[q][0]
-                               : S(0.25) * ((cv[q][0] + cv[q][1]) + (cv[q][2] + cv[q][3]));
+        [&](int q, int e, bool, long long, int, int) {
             R.m[e] = m[q];
             R.b[e] = m[q] ? conv<S>(rv[q]) * id : S(0);
-            R.x[e] = m[q] && ((r + c) & 1) == 0 ? xa[q] + pc : S(0);
+            if constexpr (sizeof(S) == 4)
+                R.x[e] = m[q] ? xr[q] + (oj[q] ? S(0.25) * ((cv[q][0] + cv[q][1]) +
+                                                            (cv[q][2] + cv[q][3]))
+                                               : cv[q][0])
+                              : S(0);
         });
+    if constexpr (sizeof(S) == 8) p_prolong(R, t);
     __syncthreads();
 #pragma unroll 1
     for (int q = 1; q <= 2 * nu; ++q) p_half(R, q & 1, h - q);
@@ -493,7 +543,7 @@ __device__ __forceinline__ void p_init(const PSArgs& A, const PTile& t, double (
 // tiles (a single member: one slot in every block), from the same totals in
 // the same order: the same bits.
 struct PSlot {
-    double alpha, beta, d, irz, goal, bb, rr;
+    double alpha, beta, d, rz, irz, goal, bb, rr;
     int conv, zero, status;
     int member, n0, nn, owner;  // owner: this block writes the member's state
     int pad;
@@ -537,7 +587,8 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
     if (!ps_sync(g)) return;
     for (int i = w; i < nslot; i += PS_NT / 32) {
         const int n0 = single ? 0 : rec[i].n0, nn = single ? nt : rec[i].nn;
-        const double bb = ps_total(pb + n0, nn), rr = ps_total(pb + nt + n0, nn);
+        double bb, rr;
+        ps_total2(pb + n0, pb + nt + n0, nn, bb, rr);
         if (lane) continue;
         PSlot& c = slot[i];
         c.member = single ? 0 : rec[i].member;
@@ -547,7 +598,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
         c.bb = bb;
         c.rr = rr;
         c.goal = tol2 * bb;
-        c.alpha = c.beta = c.d = c.irz = 0.0;
+        c.alpha = c.beta = c.d = c.rz = c.irz = 0.0;
         c.zero = bb == 0.0;
         c.conv = c.zero || rr <= c.goal;
         c.status = 0;
@@ -578,6 +629,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
             const double rr = ps_total(pr + c.n0, c.nn);
             if (lane) continue;
             c.rr = rr;
+            c.irz = 1.0 / c.rz;  // for the next beta
             if (!(rr == rr)) c.status = ST_NONFINITE;
             else if (rr > c.goal && it >= maxit) c.status = ST_PCG_MAXIT;
             c.conv = c.status || rr <= c.goal;
@@ -651,14 +703,15 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
         for (int i = w; i < nslot; i += PS_NT / 32) {
             PSlot& c = slot[i];
             if (c.conv) continue;
-            const double rz = ps_total(pz + c.n0, c.nn), zw = ps_total(pz + nt + c.n0, c.nn);
+            double rz, zw;
+            ps_total2(pz + c.n0, pz + nt + c.n0, c.nn, rz, zw);
             if (lane) continue;
             // beta = rz / rz_old, <p, A p> = <z, w> - beta^2 <p, A p>_old,
             // alpha = rz / <p, A p>
             c.beta = rz * c.irz;
             c.d = zw - c.beta * c.beta * c.d;
             c.alpha = rz / c.d;
-            c.irz = 1.0 / rz;
+            c.rz = rz;
         }
         __syncthreads();
         ++it;
@@ -691,8 +744,7 @@ __global__ void k_ps_setup(const __grid_constant__ PSArgs A, double tol2, int ma
 {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b == 0) {
-        A.bar->count = 0u;
-        A.bar->abort = 0;
+        ps_reset(A.bar);
         *A.active = 0;
     }
     if (b < A.nmem) {
@@ -736,11 +788,33 @@ static size_t region_bytes(int tw, int th, int prec)
     return (size_t)(tw + 10) * (th + 10) * (prec == 0 ? 17 : 9);
 }
 
+// Longest tiles first, each to the block with the least work: the block of
+// every tile and the load of the busiest block
+static double deal(const std::vector<double>& cost, int blocks, std::vector<int>* where)
+{
+    std::vector<int> order(cost.size());
+    for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>,
+                        std::greater<std::pair<double, int>>> q;
+    for (int g = 0; g < blocks; ++g) q.push({0.0, g});
+    if (where) where->assign(cost.size(), 0);
+    double worst = 0.0;
+    for (int i : order) {
+        std::pair<double, int> t = q.top();
+        q.pop();
+        t.first += cost[i];
+        worst = std::max(worst, t.first);
+        if (where) (*where)[i] = t.second;
+        q.push(t);
+    }
+    return worst;
+}
+
 // Tiles of one level of all members. One member: of all partitions the one
 // with the smallest estimate of the busiest block's time; up to about 1300^2
 // nodes that is one tile per block. A batch: all members get tiles of at most
-// T x T nodes, T the one with the smallest estimate of (tiles per block) x
-// (cost of a tile).
+// T x T nodes, T the one with the smallest estimate for the busiest block.
 static std::vector<TileDim> pick_tiles(const std::vector<std::pair<int, int>>& nxny, int sms,
                                        int prec)
 {
@@ -764,19 +838,16 @@ static std::vector<TileDim> pick_tiles(const std::vector<std::pair<int, int>>& n
     }
     for (int T = 8; T <= 128; T += 4) {
         if (region_bytes(T, T, prec) > PS_SMEM) break;
-        double total = 0.0, worst = 0.0;
+        std::vector<double> cost;
         for (size_t b = 0; b < nxny.size(); ++b) {
             const int nx = nxny[b].first, ny = nxny[b].second;
             cur[b] = TileDim{0, 0, 0, 0};
             if (nx <= 0) continue;
             cur[b] = tile_dim(nx, ny, (nx + T - 1) / T, (ny + T - 1) / T);
-            const double c = tile_cost(cur[b].tw, cur[b].th, prec);
-            total += c * cur[b].ntx * cur[b].nty;
-            worst = std::max(worst, c);
+            cost.insert(cost.end(), (size_t)cur[b].ntx * cur[b].nty,
+                        tile_cost(cur[b].tw, cur[b].th, prec));
         }
-        // list scheduling: at most the mean load and one more tile
-        const double c = total <= worst * sms ? std::max(worst, total / sms)
-                                              : total / sms + 0.5 * worst;
+        const double c = deal(cost, sms, nullptr);
         if (bc == 0.0 || c < bc) {
             bc = c;
             best = cur;
@@ -824,7 +895,7 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     a.ng = std::max(1, maxg);
     a.nmem = n;
     a.nrows = nrows;
-    // tiles, level by level; a level's tiles are dealt to the blocks in turn
+    // tiles, level by level
     std::vector<std::vector<PTile>> tl(a.ng);
     std::vector<PDense> dense(n);
     size_t smem = 0;
@@ -855,7 +926,7 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
         const int rc = ps_invert(h, nd, D.nxn, {}, -1.0, prec, minv);
         if (rc == 5) return 0;
         if (rc) return rc;
-        smem = std::max(smem, (nd + 4 * (size_t)((nrows + sms - 1) / sms + 1)) * es);
+        smem = std::max(smem, (nd + 128 * (size_t)((nrows + sms - 1) / sms + 1)) * es);
     }
     for (int l = 0; l < a.ng; ++l) {
         std::vector<std::pair<int, int>> dims(n);
@@ -917,13 +988,21 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
         }
     }
     a.ntiles = (int)tl[0].size();
+    std::vector<std::vector<std::vector<int>>> of(sms, std::vector<std::vector<int>>(a.ng));
+    for (int l = 0; l < a.ng; ++l) {
+        std::vector<double> cost;
+        std::vector<int> where;
+        for (const PTile& t : tl[l]) cost.push_back(tile_cost(t.tw, t.th, prec));
+        deal(cost, sms, &where);
+        for (size_t t = 0; t < where.size(); ++t) of[where[t]][l].push_back((int)t);
+    }
     std::vector<PTile> recs;
     std::vector<int> rec0;
     for (int g = 0; g < sms; ++g) {
         const size_t first = recs.size();
         for (int l = 0; l < a.ng; ++l) {
             rec0.push_back((int)recs.size());
-            for (size_t t = g; t < tl[l].size(); t += sms) recs.push_back(tl[l][t]);
+            for (int t : of[g][l]) recs.push_back(tl[l][t]);
             if (l == 0 && recs.size() - first > PS_SLOTS) return 0;
         }
         rec0.push_back((int)recs.size());
