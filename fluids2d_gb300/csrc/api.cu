@@ -218,14 +218,15 @@ static int make_tmap(f2d_model_s* m, void* buf, bool flux_tile = false)
     CUtensorMap map;
     cuuint64_t dims[2] = {(cuuint64_t)m->g.NX, (cuuint64_t)m->g.NY};
     cuuint64_t strides[1] = {(cuuint64_t)(m->g.P * m->es)};
-    // tile + halo: SW x FSH for the flux-form stage (and the tracer of any
+    // tile + halo: SW x (8 R + 6) for the flux-form stage (and the tracer of any
     // model), SW x SH for the momentum kernel of rsw, euler and boussinesq
     cuuint32_t box[2] = {(cuuint32_t)SW,
                          (cuuint32_t)(!flux_tile && (m->p.model == F2D_MODEL_RSW ||
                                                      m->p.model == F2D_MODEL_QGRSW ||
                                                      projected(m->p.model))
                                           ? SH
-                                          : FSH)};
+                                          : 6 + 8 * (m->prec == 0 ? FluxRows<double>::R
+                                                                  : FluxRows<float>::R))};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(&map, m->prec == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
                                        : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,

@@ -83,8 +83,11 @@ k_ens_fluxform_stage(const int4* __restrict__ tiles, const Member* __restrict__ 
                      EnsArenas a, int par, int stage, DevScalars* scs, EnsGlobals* eg)
 {
     __shared__ FluxformSmem<T, M> sm;
-    const int4 tl = tiles[blockIdx.x];
+    // (a table tile of FTY rows is FRT / R stage tiles, blockIdx.y)
+    int4 tl = tiles[blockIdx.x];
+    tl.z += blockIdx.y * 8 * FluxRows<T>::R;
     const Member& mb = mem[tl.x];
+    if (tl.z >= mb.g.NY) return;
     const long long o = mb.off;
     const int k = stage & 15;  // stage = k | integrator << 4
     const DevScalars& sc = scs[tl.x];
@@ -437,7 +440,7 @@ static int ens_record_step(f2d_ensemble_s* e, int par, cudaStream_t s)
     for (int k = 1; k <= nst; ++k) {
         const int sk = k | (e->p.integrator << 4);
 #define ENS_FF(T, M)                                                                       \
-    k_ens_fluxform_stage<T, M><<<e->ncell, blk, 0, s>>>(e->cell_tiles, e->dmem, e->ar, par, \
+    k_ens_fluxform_stage<T, M><<<dim3(e->ncell, FRT / FluxRows<T>::R), blk, 0, s>>>(e->cell_tiles, e->dmem, e->ar, par, \
                                                         sk, e->scs, e->eg)
         const int M = e->p.compflux;
         if (e->prec == 0) {
@@ -645,7 +648,8 @@ int f2d_ensemble_create(const f2d_params* p, int count, const int* nxs, const in
         for (int k = 0; k < 2; ++k) {
             cuuint64_t dims[2] = {(cuuint64_t)g.NX, (cuuint64_t)g.NY};
             cuuint64_t strides[1] = {(cuuint64_t)(g.P * es)};
-            cuuint32_t box[2] = {(cuuint32_t)SW, (cuuint32_t)FSH};
+            const int rows = 8 * (e->prec == 0 ? FluxRows<double>::R : FluxRows<float>::R);
+            cuuint32_t box[2] = {(cuuint32_t)SW, (cuuint32_t)(rows + 6)};
             cuuint32_t estr[2] = {1, 1};
             CUresult r = enc(&mb.tq[k],
                              e->prec == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
@@ -1033,7 +1037,7 @@ int f2d_ensemble_time_stage(f2d_ensemble e, int stage, int reps, int flush_l2,
         if (fl) cudaMemsetAsync(fl, r & 0xff, flush_bytes, e->stream);
         cudaEventRecord(a, e->stream);
 #define ENS_FF(T, M)                                                                       \
-    k_ens_fluxform_stage<T, M><<<e->ncell, blk, 0, e->stream>>>(e->cell_tiles, e->dmem,   \
+    k_ens_fluxform_stage<T, M><<<dim3(e->ncell, FRT / FluxRows<T>::R), blk, 0, e->stream>>>(e->cell_tiles, e->dmem,   \
                                                                 e->ar, par,               \
                                                                 stage | (e->p.integrator << 4), \
                                                                 e->scs,                   \

@@ -41,7 +41,7 @@ k_fluxform_stage(const __grid_constant__ CUtensorMap tq, const T* __restrict__ q
     if (((stage >> 4) & 15) == 3 && sc->ite == 0) stage |= 256;  // first LFRA step
     fluxform_tile<T, M, true>(sm, &tq, qin, qout, Ux, Uy, code, ds_out, ds1, ds2, frc, stage,
                               g, sc->dt, sc->ragamma, &sc->status, blockIdx.x * TX,
-                              blockIdx.y * FTY);
+                              blockIdx.y * 8 * FluxRows<T>::R);
 }
 
 // ---------------------------------------------------------------------------
@@ -543,9 +543,9 @@ static dim3 tile_grid(const Geom& g)
     return dim3((g.NX + TX - 1) / TX, (g.NY + TY - 1) / TY);
 }
 
-static dim3 ftile_grid(const Geom& g)
+static dim3 ftile_grid(const Geom& g, int rows)
 {
-    return dim3((g.NX + TX - 1) / TX, (g.NY + FTY - 1) / FTY);
+    return dim3((g.NX + TX - 1) / TX, (g.NY + rows - 1) / rows);
 }
 
 int launch_fluxform_stage(int method, int prec, const CUtensorMap* tq,
@@ -554,7 +554,8 @@ int launch_fluxform_stage(int method, int prec, const CUtensorMap* tq,
                           const void* ds1, const void* ds2, const void* frc, int stage,
                           const Geom& g, DevScalars* sc, cudaStream_t s)
 {
-    dim3 grid = ftile_grid(g), block(TX, TY);
+    const int rows = 8 * (prec == 0 ? FluxRows<double>::R : FluxRows<float>::R);
+    dim3 grid = ftile_grid(g, rows), block(TX, TY);
 #define F2D_FF(T, M)                                                              \
     k_fluxform_stage<T, M><<<grid, block, 0, s>>>(                                \
         *tq, (const T*)qin, (T*)qout, (const T*)Ux, (const T*)Uy, code, (T*)ds_out, \

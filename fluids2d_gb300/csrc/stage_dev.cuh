@@ -13,6 +13,11 @@ constexpr int OX = 4, OY = 3;            // offset of cell (j0,i0) in the tile
 // of the blocks, each waiting once for its TMA tile, and 1.48x instead of
 // 2.19x staged cells per cell.
 constexpr int FRT = 4, FTY = 8 * FRT, FSH = FTY + 6;
+// In FP64 the stage is bound by the FP64 pipe of the SMs that have a tile, so
+// it takes 32 x 8R-cell tiles, R rows per thread: 256^2 gives 64 tiles of 32
+// rows for 152 SMs.
+template <typename T> struct FluxRows { static constexpr int R = FRT; };
+template <> struct FluxRows<double> { static constexpr int R = 1; };
 
 // Test hook of the failure detection (f2d_test_tma_wait). When enabled,
 // every stage kernel, once its TMA tile has landed, also waits for the next
@@ -187,9 +192,10 @@ __device__ __forceinline__ bool stage_tiles(T (*s0)[SW], const CUtensorMap* m0,
 // ---------------------------------------------------------------------------
 template <typename T, int M>
 struct FluxformSmem {
-    alignas(128) T sq[FSH][SW];
-    T sfx[FTY][TX + 1];
-    T sfy[FTY + 1][TX];
+    static constexpr int R = FluxRows<T>::R;
+    alignas(128) T sq[8 * R + 6][SW];
+    T sfx[8 * R][TX + 1];
+    T sfy[8 * R + 1][TX];
     T rk[3];
     uint64_t bar;
 };
@@ -211,6 +217,7 @@ __device__ __forceinline__ void fluxform_tile(
     const T* __restrict__ ds2, const T* __restrict__ frc, int stage, const Geom& g,
     double dt, double gamma, int* status, int i0, int j0)
 {
+    constexpr int R = FluxRows<T>::R, NR = 8 * R;  // rows per thread, of the tile
     auto& sq = sm.sq;
     auto& sfx = sm.sfx;
     auto& sfy = sm.sfy;
@@ -225,7 +232,7 @@ __device__ __forceinline__ void fluxform_tile(
     if (t == 0) mbar_init(&sm.bar, 1);
     __syncthreads();
     if (t == 0) {
-        mbar_expect_tx(&sm.bar, (uint32_t)(sizeof(T) * SW * FSH));
+        mbar_expect_tx(&sm.bar, (uint32_t)(sizeof(T) * SW * (NR + 6)));
         tma_load_2d(&sq[0][0], tq, i0 - OX, j0 - OY, &sm.bar);
     }
     // 2. ... overlapped with this thread's plain loads: the code word and
@@ -234,10 +241,10 @@ __device__ __forceinline__ void fluxform_tile(
     // x-faces / row of y-faces of the tile edge; all unconditional (clamped
     // index, then masked), so they are in flight together.
     const int i = i0 + tx;
-    uint32_t cd[FRT];
-    T ux[FRT], uy[FRT], d1[FRT], d2[FRT], fq[FRT];
+    uint32_t cd[R];
+    T ux[R], uy[R], d1[R], d2[R], fq[R];
 #pragma unroll
-    for (int q = 0; q < FRT; ++q) {
+    for (int q = 0; q < R; ++q) {
         const int j = j0 + ty + 8 * q;
         const bool in = j < g.NY && i < g.NX;
         const long long o = (long long)min(j, g.NY - 1) * g.P + min(i, g.NX - 1);
@@ -252,11 +259,12 @@ __device__ __forceinline__ void fluxform_tile(
     }
     uint32_t ce = 0u;
     T ue = T(0);
-    int er = 0, ec = 0, ex = 0;  // edge face: x (ex = 1) at (t, TX) or y (ex = 2) at (FTY, t-FTY)
-    if (t < FTY + TX) {
-        ex = t < FTY ? 1 : 2;
-        er = t < FTY ? t : FTY;
-        ec = t < FTY ? TX : t - FTY;
+    // edge face: x (ex = 1) at (t, TX) in warp 0, y (ex = 2) at (NR, t - 32) in warp 1
+    int er = 0, ec = 0, ex = 0;
+    if (t < NR || (t >= 32 && t < 64)) {
+        ex = t < NR ? 1 : 2;
+        er = t < NR ? t : NR;
+        ec = t < NR ? TX : t - 32;
         const int j = j0 + er, ii = i0 + ec;
         const bool in = j < g.NY && ii < g.NX;
         const long long o = (long long)min(j, g.NY - 1) * g.P + min(ii, g.NX - 1);
@@ -265,6 +273,7 @@ __device__ __forceinline__ void fluxform_tile(
         ce = in ? c : 0u;
         ue = u;
     }
+    if (t == 0) rk3_coefs<T>(sk, dt, sm.rk, gamma);  // (its divisions behind the copy)
     // 3. wait for the tile (bounded; uniform time-out exit)
     {
         const bool ok = mbar_wait(&sm.bar, 0) && tma_wait_test(&sm.bar);
@@ -296,19 +305,18 @@ __device__ __forceinline__ void fluxform_tile(
         sfy[r][c] = f;
     };
 #pragma unroll
-    for (int q = 0; q < FRT; ++q) {
+    for (int q = 0; q < R; ++q) {
         xflux(ty + 8 * q, tx, cd[q], ux[q]);
         yflux(ty + 8 * q, tx, cd[q], uy[q]);
     }
     if (ex == 1) xflux(er, ec, ce, ue);
     else if (ex == 2) yflux(er, ec, ce, ue);
-    if (t == 0) rk3_coefs<T>(sk, dt, sm.rk, gamma);
     __syncthreads();
 
     // 5. tendency, RK3 update and stores of this thread's cells
     if (i >= g.NX || !periodic_owner(g, i)) return;
 #pragma unroll
-    for (int q = 0; q < FRT; ++q) {
+    for (int q = 0; q < R; ++q) {
         const int r = ty + 8 * q, j = j0 + r;
         if (j >= g.NY) break;
         const T msk = (cd[q] & B_MSK) ? T(1) : T(0);

@@ -53,35 +53,37 @@ __device__ __forceinline__ T weno5z(T qmm, T qm, T q0, T qp, T qpp)
     return ((w1 * qi1 + w2 * qi2) + w3 * qi3) / ((w1 + w2) + w3);
 }
 
-// FP64 form of weno5z with one division instead of four: the weights
-// w_k = g_k (1 + tau/d_k), d_k = beta_k + eps, are scaled by d1 d2 d3, so
-// W_k = g_k (d_k + tau) prod_{m != k} d_m and the reconstruction is
-// sum W_k qi_k / sum W_k - the same value up to rounding. With d_k >= 1e-16
-// the products stay far inside the double range (>= 1e-48). On GB300 the
-// double divisions dominate the FP64 instruction count of the stencil.
+// FP64 form of weno5z. On GB300 an FP64 instruction of a warp occupies its SM
+// partition's pipe for 64 cycles and these kernels are bound by that pipe, so
+// the same reconstruction is written with few of them, from the differences
+// e0 = qm - qmm, e1 = q0 - qm, e2 = qp - q0, e3 = qpp - qp:
+//  * the smoothness indicators times 4: 4 beta_k = (13/3) a_k^2 + b_k^2 with
+//    a = e1 - e0, e2 - e1, e3 - e2 and b = 3 e1 - e0, e1 + e2, 3 e2 - e3; the
+//    weights 1 + tau/(beta + eps) do not see the common factor;
+//  * the candidates as q0 + c_k/6: c = 5 e1 - 2 e0, e1 + 2 e2, 4 e2 - e3;
+//  * one division instead of four: the weights scaled by d1 d2 d3, d_k =
+//    4 (beta_k + eps). With d_k >= 4e-16 the products stay far inside the
+//    double range (>= 6e-47).
+// 50 FP64 instructions, the division among them, instead of 64; equal up to
+// rounding (exact for constant q).
 template <>
 __device__ __forceinline__ double weno5z<double>(double qmm, double qm, double q0,
                                                  double qp, double qpp)
 {
-    const double eps = WenoConst<double>::eps5;
-    const double c13 = 1. / 3., c76 = 7. / 6., c116 = 11. / 6.;
-    const double c16 = 1. / 6., c56 = 5. / 6.;
-    const double qi1 = (c13 * qmm - c76 * qm) + c116 * q0;
-    const double qi2 = (-c16 * qm + c56 * q0) + c13 * qp;
-    const double qi3 = (c13 * q0 + c56 * qp) - c16 * qpp;
-    const double k1 = 13. / 12., k2 = 0.25;
-    const double a1 = (qmm - 2. * qm) + q0, b1 = (qmm - 4. * qm) + 3. * q0;
-    const double a2 = (qm - 2. * q0) + qp, b2 = qm - qp;
-    const double a3 = (q0 - 2. * qp) + qpp, b3 = (3. * q0 - 4. * qp) + qpp;
-    const double beta1 = k1 * (a1 * a1) + k2 * (b1 * b1);
-    const double beta2 = k1 * (a2 * a2) + k2 * (b2 * b2);
-    const double beta3 = k1 * (a3 * a3) + k2 * (b3 * b3);
-    const double tau5 = fabs(beta1 - beta3);
-    const double d1 = beta1 + eps, d2 = beta2 + eps, d3 = beta3 + eps;
-    const double W1 = (0.1 * (d1 + tau5)) * (d2 * d3);
-    const double W2 = (0.6 * (d2 + tau5)) * (d1 * d3);
-    const double W3 = (0.3 * (d3 + tau5)) * (d1 * d2);
-    return ((W1 * qi1 + W2 * qi2) + W3 * qi3) / ((W1 + W2) + W3);
+    const double eps4 = 4. * WenoConst<double>::eps5, k = 13. / 3.;
+    const double e0 = qm - qmm, e1 = q0 - qm, e2 = qp - q0, e3 = qpp - qp;
+    const double a1 = e1 - e0, a2 = e2 - e1, a3 = e3 - e2;
+    const double b1 = fma(3., e1, -e0), b2 = e1 + e2, b3 = fma(3., e2, -e3);
+    const double d1 = fma(k, a1 * a1, fma(b1, b1, eps4));
+    const double d2 = fma(k, a2 * a2, fma(b2, b2, eps4));
+    const double d3 = fma(k, a3 * a3, fma(b3, b3, eps4));
+    const double tau = fabs(d1 - d3);
+    const double W1 = (d1 + tau) * (d2 * d3);
+    const double W2 = (d2 + tau) * (6. * (d1 * d3));
+    const double W3 = (d3 + tau) * (3. * (d1 * d2));
+    const double c1 = fma(2., b1, -e1), c2 = fma(2., e2, e1), c3 = b3 + e2;
+    const double num = fma(W3, c3, fma(W2, c2, W1 * c1));
+    return q0 + num / (6. * ((W1 + W2) + W3));
 }
 
 // FP32 form of weno5z: the three weight quotients tau/d_k and the final
@@ -238,6 +240,14 @@ __device__ __forceinline__ T cweno5z(T qmmm, T qmm, T qm, T qp, T qpp, T qppp)
            (T(2) * ((w1 + w2) + w3));
 }
 
+// U > 0; in FP64 from the bits (sign 0, not +0, not NaN) on the integer pipe
+__device__ __forceinline__ bool positive(float U) { return U > 0.f; }
+__device__ __forceinline__ bool positive(double U)
+{
+    const long long b = __double_as_longlong(U);
+    return b > 0 && b <= 0x7ff0000000000000ll;
+}
+
 enum { METHOD_WENO = 0, METHOD_UPWIND = 1, METHOD_CENTERED = 2,
        METHOD_CWENO = 3,
        METHOD_CLASSIC = 4 /* innerproduct only: the 4-point kinetic energy */ };
@@ -252,7 +262,7 @@ __device__ __forceinline__ T flux6(T U, T q0, T q1, T q2, T q3, T q4, T q5)
     if (M == METHOD_CWENO) return cweno5z<T>(q0, q1, q2, q3, q4, q5);
     // upwind side chosen by the sign of U, mirrored stencil otherwise; the
     // operands are selected first so that one reconstruction is evaluated
-    const bool up = U > T(0);
+    const bool up = positive(U);
     const T a = up ? q0 : q5, b = up ? q1 : q4, c = up ? q2 : q3;
     const T d = up ? q3 : q2, e = up ? q4 : q1;
     if (M == METHOD_WENO) return weno5z<T>(a, b, c, d, e);
@@ -264,7 +274,7 @@ __device__ __forceinline__ T flux4(T U, T q1, T q2, T q3, T q4)
 {
     if (M == METHOD_CENTERED) return ce4<T>(q1, q2, q3, q4);
     if (M == METHOD_CWENO) return cweno3z<T>(U, q1, q2, q3, q4);
-    const bool up = U > T(0);
+    const bool up = positive(U);
     const T a = up ? q1 : q4, b = up ? q2 : q3, c = up ? q3 : q2;
     if (M == METHOD_WENO) return weno3z<T>(a, b, c);
     return up3<T>(a, b, c);
@@ -272,7 +282,7 @@ __device__ __forceinline__ T flux4(T U, T q1, T q2, T q3, T q4)
 
 template <int M, typename T> __device__ __forceinline__ T flux2(T U, T q2, T q3)
 {
-    if (M == METHOD_WENO || M == METHOD_UPWIND) return U > T(0) ? q2 : q3;
+    if (M == METHOD_WENO || M == METHOD_UPWIND) return positive(U) ? q2 : q3;
     return ce2<T>(q2, q3);
 }
 
