@@ -234,10 +234,13 @@ __device__ __forceinline__ To conv(From x)
 }
 
 // Maximum that propagates NaN, as numpy's max does (the reference's set_dt,
-// model.py:83-87, turns a NaN velocity into a NaN time step).
-__host__ __device__ __forceinline__ double nanmax(double a, double b)
+// model.py:83-87, turns a NaN velocity into a NaN time step), of values whose
+// sign bit is clear (|U|; NaN from fabs too) or -infinity (a reduction's
+// start): their order, NaN last, is that of their bits as integers. (As FP64
+// compares these maxima were a third of perpgrad's FP64 instructions.)
+__device__ __forceinline__ double nanmax(double a, double b)
 {
-    return (a > b || a != a) ? a : b;
+    return __double_as_longlong(a) > __double_as_longlong(b) ? a : b;
 }
 __host__ __device__ __forceinline__ float nanmaxf(float a, float b)
 {
