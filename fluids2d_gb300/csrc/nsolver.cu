@@ -23,7 +23,7 @@
 // smooth errors, and the coarse correction comes out halved - half the sum is
 // the re-discretised coupling where the face is fully open and keeps the
 // partial openings of masked faces.) The first level of at most 2048 cells is
-// solved exactly with its precomputed dense pseudo-inverse (the FP32 form:
+// solved exactly with its precomputed dense pseudo-inverse (the FP32 form: 4096,
 // replaced by the matrix of the V-cycle from it on, coarse_map). The FP32 form runs the cycle in FP32
 // (levels, couplings and smoothing in float; its right-hand side is the FP64
 // Krylov residual rounded, its result converted back), while the Krylov
@@ -608,6 +608,14 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
     PSGrid g = {(PSBar*)A.bar, &A.eg->status, 0u};
     const NLevel& L = A.lev[0];
     const unsigned G = gridDim.x;
+    // the block's rows of the dense level, kept in shared memory if they fit
+    const int d0 = A.nd * blockIdx.x / G, d1 = A.nd * (blockIdx.x + 1) / G;
+    const PSBox box = {A.nd, A.nd, 0, 1.0f / (float)A.nd};
+    const S* mrows = (const S*)A.minv + (size_t)d0 * ps_pitch<S>(A.nd);
+    if (A.mkeep) {
+        ps_copy16(smem + A.mkeep, mrows, (size_t)(d1 - d0) * ps_pitch<S>(A.nd) * sizeof(S));
+        mrows = (const S*)(smem + A.mkeep);
+    }
     // totals: <r, z>, <z, w> | <r, r>, sum x | sum b | <b, b>, <r, r>, sum x
     double *pz = A.part, *pr = A.part + 2 * G, *pi = A.part + 4 * G, *pb = A.part + 5 * G;
     // b -= mean(b)
@@ -679,8 +687,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
         }
         if (c.done) break;
         const NLevel& D = A.lev[A.ng];
-        ps_dense<S>((const S*)A.minv, (const S*)D.b, (S*)D.x, A.nd, A.nd * blockIdx.x / G,
-                    A.nd * (blockIdx.x + 1) / G, (S*)smem);
+        ps_dense<S>(mrows, (const S*)D.b, (S*)D.x, A.nd, d0, d1, (S*)smem, box);
         if (!(A.ng <= 1 ? ps_sync(g, decide) : ps_sync(g))) return;
         if (c.done) break;
         for (int l = A.ng - 1; l >= 1; --l) {
@@ -898,7 +905,9 @@ k_ns_coarse_map(const __grid_constant__ NCoarse C, const double* __restrict__ fx
         for (int s = 0; s < 4; ++s) nc_half(C, l, x, b, fx, fy, (s + 1) & 1);
     }
     // column col = row col (the cycle is symmetric)
-    for (int k = threadIdx.x; k < n; k += blockDim.x) out[(size_t)col * n + k] = (float)x[k];
+    const int np = ps_pitch<float>(n);
+    for (int k = threadIdx.x; k < np; k += blockDim.x)
+        out[(size_t)col * np + k] = k < n ? (float)x[k] : 0.f;
 }
 
 static void coarsen(std::vector<double>& fx, std::vector<double>& fy, int& ny, int& nx, int per)
@@ -949,8 +958,10 @@ static int coarse_map(std::vector<double> fx, std::vector<double> fy, int ny, in
         cudaMemcpy(dx, ax.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(dy, ay.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess)
         rc = 2;
-    if (!rc && cudaFuncSetAttribute(k_ns_coarse_map, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    96 * 1024) != cudaSuccess)
+    // (4096 cells and their coarser levels: 88 KB)
+    if (!rc && (2 * bytes > 128 * 1024 ||
+                cudaFuncSetAttribute(k_ns_coarse_map, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     128 * 1024) != cudaSuccess))
         rc = 3;
     if (!rc) {
         k_ns_coarse_map<<<n, 256, 2 * bytes>>>(C, dx, dy, out);
@@ -1048,7 +1059,8 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
     // when that is small enough: then the preconditioner is the inverse and
     // CG ends after one or two iterations (40^2: 1.6 instead of 9)
     int ny = nyn, nx = nxn, l = 0;
-    if (ps_band_ok((long long)nyn * nxn, nxn)) {
+    bool dense = ps_band_ok((long long)nyn * nxn, nxn, 0);
+    if (dense) {
         L0.x = dal((size_t)nyn * nxn * es);
         L0.b = dal((size_t)nyn * nxn * es);
         if (!L0.x || !L0.b) return 2;
@@ -1058,13 +1070,13 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
         if (!a.z || !L0.xa) return 2;
         pick_tile(L0, sms, prec, NS_H, 2 * es + 1);
     }
-    while (!ps_band_ok((long long)ny * nx, nx)) {
+    while (!dense) {
         if (l + 1 >= NS_LMAX) return 3;
         coarsen(fx, fy, ny, nx, per);
         const int cyn = ny, cxn = nx;
         ++l;
         NLevel& C = a.lev[l];
-        const bool dense = ps_band_ok((long long)cyn * cxn, cxn);
+        dense = ps_band_ok((long long)cyn * cxn, cxn, prec);
         C.nyn = cyn;
         C.nxn = cxn;
         C.pitch = dense ? cxn : (cxn + 31) / 32 * 32;
@@ -1096,7 +1108,8 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
     }
     a.ng = l;
     a.nd = ny * nx;
-    void* minv = dal((size_t)a.nd * a.nd * es);
+    const int np = prec == 0 ? ps_pitch<double>(a.nd) : ps_pitch<float>(a.nd);
+    void* minv = dal((size_t)a.nd * np * es);
     if (!minv) return 2;
     int rc = prec == 1 && a.ng > 0 ? coarse_map(fx, fy, ny, nx, per, (float*)minv)
                                    : dense_inverse(fx, fy, ny, nx, per, cx, cy, prec, minv);
@@ -1106,11 +1119,18 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
     // to all blocks, and a barrier of 152 blocks (1.36 us) costs hardly more
     // than one of 25 (1.28 us)
     s.grid = sms;
-    s.smem = (size_t)(a.nd + 128 * ((a.nd + sms - 1) / sms + 1)) * es;
+    const int rows = (a.nd + sms - 1) / sms;  // of a block, at most
+    s.smem = (prec == 0 ? ps_dense_elems<double>(a.nd, rows) : ps_dense_elems<float>(a.nd, rows)) *
+             es;
     for (int q = 0; q < a.ng; ++q) {
         const int h = q == 0 ? NS_H : 4;
         const size_t n = (size_t)(a.lev[q].tw + 2 * h) * (a.lev[q].th + 2 * h);
         s.smem = std::max(s.smem, q == 0 ? n * (2 * es + 1) : n * 5 * es);
+    }
+    s.smem = (s.smem + 15) / 16 * 16;
+    if (s.smem + (size_t)rows * np * es <= NS_SMEM) {
+        a.mkeep = (int)s.smem;
+        s.smem += (size_t)rows * np * es;
     }
     const void* kern = prec == 0 ? (const void*)k_ns_solve<double> : (const void*)k_ns_solve<float>;
     // (the attribute is per kernel: never lowered below another solver's need)

@@ -40,6 +40,7 @@ struct NSArgs {
     int ng;                // grid levels; level ng is the dense one
     int nd;                // cells of the dense level
     const void* minv;      // its inverse
+    int mkeep;             // offset in shared memory of the block's rows of it (0: not kept)
     double cx, cy;
     double cs[9], inv[9];  // by 3 (open x-faces) + (open y-faces): coupling sum, its inverse
     // FP64 vectors in the level-0 layout: solution, right-hand side, residual

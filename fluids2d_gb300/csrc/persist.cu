@@ -14,13 +14,13 @@ namespace f2d {
 // each), id: 1 / diagonal. Bound by the chain of 2 n dependent steps (about
 // 200 cycles each): 0.4 ms at n = 1600, bw = 40, where one launch per pivot
 // of a Gauss-Jordan elimination of the full matrix took 34 ms.
-constexpr int BI_W = 8;  // warps (columns) per block
+constexpr int BI_W = 8;  // warps (columns) per block, at most
 __global__ void __launch_bounds__(32 * BI_W)
 k_band_inverse(const double* __restrict__ lc, const double* __restrict__ lr,
                const double* __restrict__ id, int n, int bw, double* __restrict__ out)
 {
     extern __shared__ double cols[];
-    const int lane = threadIdx.x & 31, j = blockIdx.x * BI_W + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31, j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (j >= n) return;
     double* x = cols + (size_t)(threadIdx.x >> 5) * n;
     for (int i = lane; i < n; i += 32) x[i] = i == j ? 1.0 : 0.0;
@@ -65,14 +65,21 @@ __global__ void k_inverse_out(const double* __restrict__ X, const int* __restric
                               const double* __restrict__ r, const double* __restrict__ mean,
                               int n, double scale, S* __restrict__ out)
 {
+    const int np = ps_pitch<S>(n);
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (size_t)n * n) return;
-    const int i = (int)(e / n), j = (int)(e % n);
+    if (e >= (size_t)n * np) return;
+    const int i = (int)(e / np), j = (int)(e % np);
+    if (j >= n) {
+        out[e] = S(0);
+        return;
+    }
     // the mean of the two triangles: exactly symmetric
-    double v = 0.5 * (X[e] + X[(size_t)j * n + i]);
+    double v = 0.5 * (X[(size_t)i * n + j] + X[(size_t)j * n + i]);
     if (part) v = part[i] >= 0 && part[i] == part[j] ? v - (r[i] + r[j]) + mean[i] : 0.0;
     out[e] = (S)(scale * v);
 }
+
+static_assert(PS_NDENSE32 <= 2 * PS_NDENSE, "shared memory of k_band_inverse");
 
 int ps_invert(const std::vector<double>& band, int n, int bw, const std::vector<int>& part,
               double scale, int prec, void* out)
@@ -118,11 +125,12 @@ int ps_invert(const std::vector<double>& band, int n, int bw, const std::vector<
         double* did = (double*)dal(id.size() * 8, id.data());
         double* X = (double*)dal((size_t)n * n * 8, nullptr);
         if (!dlc || !dlr || !did || !X) return 2;
-        const size_t smem = (size_t)BI_W * n * sizeof(double);
+        const int w = n <= PS_NDENSE ? BI_W : BI_W / 2;
+        const size_t smem = (size_t)w * n * sizeof(double);
         if (cudaFuncSetAttribute(k_band_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  BI_W * PS_NDENSE * (int)sizeof(double)) != cudaSuccess)
             return 3;
-        k_band_inverse<<<(n + BI_W - 1) / BI_W, 32 * BI_W, smem>>>(dlc, dlr, did, n, bw, X);
+        k_band_inverse<<<(n + w - 1) / w, 32 * w, smem>>>(dlc, dlr, did, n, bw, X);
         int* dpart = nullptr;
         double *dr = nullptr, *dm = nullptr;
         if (!part.empty()) {
@@ -145,7 +153,7 @@ int ps_invert(const std::vector<double>& band, int n, int bw, const std::vector<
             dm = (double*)dal((size_t)n * 8, mean.data());
             if (!dm) return 2;
         }
-        const unsigned ng = (unsigned)(((size_t)n * n + 255) / 256);
+        const unsigned ng = (unsigned)(((size_t)n * (n + 4) + 255) / 256);
         if (prec == 0)
             k_inverse_out<double><<<ng, 256>>>(X, dpart, dr, dm, n, scale, (double*)out);
         else

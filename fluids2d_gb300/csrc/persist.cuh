@@ -209,40 +209,97 @@ __device__ __forceinline__ void ps_grid_total(const double* part, F f)
 __device__ __forceinline__ int fdiv(int k, float rw) { return __float2int_rz((k + 0.5f) * rw); }
 
 // ---- dense coarsest level -----------------------------------------------------
-// x = M b for the n x n inverse M of the coarsest operator. The rows are dealt
-// to the blocks, a block's rows in quarters to its warps (its 16 warps stay
-// busy for any number of rows, and a warp's loads of a quarter are in flight
-// together); b is staged in shared memory. In FP64 n = 1024 costs 3.4k cycles
-// of the FP64 pipe and n = 2048 14k, the two legs and barriers of one more
-// grid level about 17k; and the coarse correction is exact.
-constexpr int PS_NDENSE = 2048;
+// x = M b for the n x n inverse M of the coarsest operator, its rows dealt to
+// the blocks. The coarse correction is exact, and one more grid level would
+// cost two legs and barriers, about 17k cycles. M is stored with rows of
+// ps_pitch(n) elements and read 16 bytes per lane; a block whose rows fit
+// beside its tiles keeps them in shared memory for the whole solve. In FP64
+// n = 1024 costs 3.4k cycles of the FP64 pipe and n = 2048 14k; in FP32 the
+// reads of M from L2 count (n = 3000, 37 MB: 19k cycles with 4-byte loads,
+// too few bytes in flight).
+constexpr int PS_NDENSE = 2048, PS_NDENSE32 = 4096;
 
-// rows r0 .. r1 - 1 of x = M b; sb: n + 128 (r1 - r0) elements of shared
-// memory. The lanes' sums of a row's four quarters meet in shared memory (a
-// shuffle tree per quarter would cost as many FP64 instructions as the row's
-// products).
 template <typename S>
-__device__ __forceinline__ void ps_dense(const S* __restrict__ M, const S* b, S* x, int n, int r0,
-                                         int r1, S* sb)
+__host__ __device__ constexpr int ps_pitch(int n)
 {
-    constexpr int NW = PS_NT / 32, U = 8;
-    S* part = sb + n;  // 128 per row
+    constexpr int V = 16 / (int)sizeof(S);
+    return (n + V - 1) / V * V;
+}
+// shared memory of ps_dense for `rows` rows, in elements
+template <typename S>
+__host__ __device__ constexpr size_t ps_dense_elems(int n, int rows)
+{
+    return (size_t)ps_pitch<S>(n) + 128 * (size_t)rows;
+}
+
+template <typename S> struct Vec16;
+template <> struct Vec16<float> {
+    using T = float4;
+    static __device__ __forceinline__ float dot(float4 m, float4 b, float a)
+    {
+        a = fmaf(m.x, b.x, a);
+        a = fmaf(m.y, b.y, a);
+        a = fmaf(m.z, b.z, a);
+        return fmaf(m.w, b.w, a);
+    }
+};
+template <> struct Vec16<double> {
+    using T = double2;
+    static __device__ __forceinline__ double dot(double2 m, double2 b, double a)
+    {
+        return fma(m.y, b.y, fma(m.x, b.x, a));
+    }
+};
+
+// The unknowns of a dense level in its arrays (rows of ld elements): unknown e
+// is column e mod w of row e / w of the box that starts at element o.
+struct PSBox {
+    int w, ld, o;
+    float rw;  // 1 / w
+};
+
+// rows r0 .. r1 - 1 of x = M b, row r at M + (r - r0) pitch (global or shared
+// memory), the chunks of a row dealt to four warps; sb: ps_dense_elems. The
+// lanes' sums of a row's quarters meet in shared memory (a shuffle tree per
+// quarter would cost as many FP64 instructions as the row's products).
+template <typename S>
+__device__ __forceinline__ void ps_dense(const S* M, const S* b, S* x, int n, int r0, int r1,
+                                         S* sb, const PSBox& box)
+{
+    using V = typename Vec16<S>::T;
+    constexpr int NW = PS_NT / 32, U = 4, VN = 16 / (int)sizeof(S), CH = 32 * VN;
+    const int np = ps_pitch<S>(n);
+    S* part = sb + np;  // 128 per row
     if (r1 <= r0) return;
-    for (int e = threadIdx.x; e < n; e += PS_NT) sb[e] = __ldcg(&b[e]);
+    auto at = [&](int e) {
+        const int r = fdiv(e, box.rw);
+        return box.o + r * box.ld + e - r * box.w;
+    };
+    for (int e0 = threadIdx.x; e0 < np; e0 += 4 * PS_NT) {
+        S v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int e = e0 + u * PS_NT;
+            v[u] = e < n ? __ldcg(&b[at(e)]) : S(0);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (e0 + u * PS_NT < np) sb[e0 + u * PS_NT] = v[u];
+    }
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int len = ((n + 3) / 4 + 31) & ~31;  // columns of a quarter
     for (int t = threadIdx.x >> 5; t < 4 * (r1 - r0); t += NW) {
-        const S* __restrict__ m = M + (size_t)(r0 + (t >> 2)) * n;
+        const S* m = M + (size_t)(t >> 2) * np;
         S a = S(0);
-        const int end = min(n, ((t & 3) + 1) * len);
-        for (int e = (t & 3) * len + lane; e < end; e += 32 * U) {
-            S v[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) v[u] = e + 32 * u < end ? m[e + 32 * u] : S(0);
+        for (int e = (t & 3) * CH + lane * VN; e < np; e += 4 * CH * U) {
+            V v[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                if (e + 32 * u < end) a += v[u] * sb[e + 32 * u];
+                if (e + 4 * CH * u < np) v[u] = *(const V*)(m + e + 4 * CH * u);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (e + 4 * CH * u < np)
+                    a = Vec16<S>::dot(v[u], *(const V*)(sb + e + 4 * CH * u), a);
         }
         part[32 * t + lane] = a;
     }
@@ -261,23 +318,32 @@ __device__ __forceinline__ void ps_dense(const S* __restrict__ M, const S* b, S*
         if (__any_sync(0xffffffffu, in)) {
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-            if (in && (t & 7) == 0) x[r0 + (t >> 3)] = a;
+            if (in && (t & 7) == 0) x[at(r0 + (t >> 3))] = a;
         }
     }
 }
 
+// copy `bytes` (a multiple of 16) of global memory to shared memory
+__device__ __forceinline__ void ps_copy16(void* dst, const void* src, size_t bytes)
+{
+    const int4* g = (const int4*)src;
+    int4* d = (int4*)dst;
+    for (int k = threadIdx.x; k < (int)(bytes / 16); k += PS_NT) d[k] = __ldg(&g[k]);
+}
+
 // Host: the inverse of a symmetric positive definite banded matrix H of n
-// rows, band[i (bw + 1) + k] = H(i, i - k), times `scale`, as an n x n array
-// of double (prec 0) or float on the device. Cholesky on the host (ps_band_ok
+// rows, band[i (bw + 1) + k] = H(i, i - k), times `scale`, as n rows of
+// ps_pitch(n) doubles (prec 0) or floats on the device (zeros behind column
+// n). Cholesky on the host (ps_band_ok
 // bounds its n bw^2 operations), the columns of the inverse on the GPU. part:
 // empty, or a part number per row: the constants of a part are projected out
 // of the result from both sides, and rows of part -1 become 0. 0 on success.
 int ps_invert(const std::vector<double>& band, int n, int bw, const std::vector<int>& part,
               double scale, int prec, void* out);
 // whether a level of n cells in rows of bw may be the dense one
-inline bool ps_band_ok(long long n, long long bw)
+inline bool ps_band_ok(long long n, long long bw, int prec)
 {
-    return n <= PS_NDENSE && n * bw * bw <= 50000000ll;
+    return n <= (prec == 0 ? PS_NDENSE : PS_NDENSE32) && n * bw * bw <= 50000000ll;
 }
 // Launch a cooperative kernel of PS_NT threads per block.
 int ps_launch(const void* kern, int grid, size_t smem, void** args, cudaStream_t st);

@@ -330,6 +330,7 @@ __device__ __forceinline__ void p_phase_a(const PSArgs& A, const PTile& t, int i
     double* r1 = A.r[par];
     double* s1 = A.s[par];
     const S* Z = (const S*)t.x;
+    S* B32 = (S*)t.b;  // the FP32 form's copy of r for phase B
     const S id = conv<S>(t.id);
     uint8_t m[PB];
     double rv[PB], sv[PB], wv[PB], xv[PB], pv[PB];
@@ -344,17 +345,21 @@ __device__ __forceinline__ void p_phase_a(const PSArgs& A, const PTile& t, int i
         },
         [&](int q, int e, bool in, long long k, int r, int c) {
             double rn = rv[q];
+            const bool own = in && r >= h && r < h + R.th && c >= h && c < h + R.tw &&
+                             R.I0 - h + c < t.nxn;
             if (it > 0) {
                 const double sn = wv[q] + beta * sv[q];
                 rn -= alpha * sn;
-                if (in && r >= h && r < h + R.th && c >= h && c < h + R.tw &&
-                    R.I0 - h + c < t.nxn) {
+                if (own) {
                     s1[k] = sn;
                     r1[k] = rn;
                     tot[0] += rn * rn;  // (0 at non-fluid nodes)
                 }
             }
-            const S bi = m[q] ? conv<S>(rn) * id : S(0);
+            const S rs = m[q] ? conv<S>(rn) : S(0);
+            if constexpr (sizeof(S) == 4)
+                if (own) B32[k] = rs;
+            const S bi = rs * id;
             R.m[e] = m[q];
             R.b[e] = bi;
             R.x[e] = (r + c) & 1 ? S(0) : bi;
@@ -387,9 +392,12 @@ __device__ __forceinline__ void p_phase_b(const PSArgs& A, const PTile& t, int i
     const int nu = A.nu, h = 2 * nu + 1;
     const PReg<S> R = p_region<S>(t, h, smem);
     const double* rr = A.r[it & 1];
+    // the cycle's right-hand side: r, or the FP32 copy of it
+    const S* bb = sizeof(S) == 8 ? (const S*)rr : (const S*)t.b;
     const S id = conv<S>(t.id);
     uint8_t m[PB];
     double rv[PB];
+    S bv[PB];
     const S* XA = (const S*)t.xa;
     S xr[PB], cv[PB][4];
     int oj[PB];
@@ -403,11 +411,11 @@ __device__ __forceinline__ void p_phase_b(const PSArgs& A, const PTile& t, int i
                 p_coarse<S>(t, red, J, I, cv[q]);
                 oj[q] = J & 1;
             }
-            rv[q] = in ? rr[k] : 0.0;
+            bv[q] = in ? bb[k] : S(0);
         },
         [&](int q, int e, bool, long long, int, int) {
             R.m[e] = m[q];
-            R.b[e] = m[q] ? conv<S>(rv[q]) * id : S(0);
+            R.b[e] = m[q] ? bv[q] * id : S(0);
             if constexpr (sizeof(S) == 4)
                 R.x[e] = m[q] ? xr[q] + (oj[q] ? S(0.25) * ((cv[q][0] + cv[q][1]) +
                                                             (cv[q][2] + cv[q][3]))
@@ -419,19 +427,24 @@ __device__ __forceinline__ void p_phase_b(const PSArgs& A, const PTile& t, int i
 #pragma unroll 1
     for (int q = 1; q <= 2 * nu; ++q) p_half(R, q & 1, h - q);
     S* Z = (S*)t.x;
-    const double cx = t.cx, cy = t.cy, md = t.md;
+    const double cx = t.cx, cy = t.cy, md = t.md, dg = t.dg;
     p_tile(
         R, t, [&](int q, bool in, long long k) { rv[q] = in ? rr[k] : 0.0; },
         [&](int q, long long k, int e) {
             const double c = conv<double>(R.x[e]);
             double wv = 0.0;
             if (R.m[e]) {
-                // differences to the centre (apply_diff): the same operator,
-                // but far less cancellation for smooth z
-                const double sx = (conv<double>(R.x[e - 1]) - c) + (conv<double>(R.x[e + 1]) - c);
-                const double sy =
-                    (conv<double>(R.x[e - R.W]) - c) + (conv<double>(R.x[e + R.W]) - c);
-                wv = (cx * sx + cy * sy) - md * c;
+                const double w = conv<double>(R.x[e - 1]), ea = conv<double>(R.x[e + 1]);
+                const double so = conv<double>(R.x[e - R.W]), no = conv<double>(R.x[e + R.W]);
+                if constexpr (sizeof(S) == 4) {
+                    // sums of two floats are exact in FP64; the rest rounds
+                    // at 1e-16 |z|, 1e-11 of w and less than z's own rounding
+                    wv = cx * (w + ea) + (cy * (so + no) + dg * c);
+                } else {
+                    // differences to the centre (apply_diff): the same
+                    // operator, but far less cancellation for smooth z
+                    wv = (cx * ((w - c) + (ea - c)) + cy * ((so - c) + (no - c))) - md * c;
+                }
                 tot[0] += rv[q] * c;
                 tot[1] += c * wv;
             }
@@ -497,22 +510,32 @@ __device__ __forceinline__ void p_dense_b(const PSArgs& A, const PTile& t, const
     });
 }
 
-// the dense level of every member: the rows of all members dealt to the blocks
-template <typename S>
-__device__ __forceinline__ void p_dense_rows(const PSArgs& A, unsigned char* smem)
+// the dense level of every member: the rows of all members dealt to the
+// blocks; f(D, a, b) for this block's rows a .. b - 1 of a member
+template <typename F>
+__device__ __forceinline__ void p_dense_rows(const PSArgs& A, F f)
 {
     const int r0 = (int)((long long)A.nrows * blockIdx.x / gridDim.x);
     const int r1 = (int)((long long)A.nrows * (blockIdx.x + 1) / gridDim.x);
     for (int m = 0; m < A.nmem; ++m) {
         const PDense D = A.dense[m];
         const int a = max(r0 - D.row0, 0), b = min(r1 - D.row0, D.n);
-        if (a >= b) {
-            if (D.row0 >= r1) break;
-            continue;
-        }
-        ps_dense<S>((const S*)D.minv, (const S*)D.b, (S*)D.x, D.n, a, b, (S*)smem);
-        __syncthreads();
+        if (D.row0 >= r1) break;
+        if (a < b) f(D, a, b);
     }
+}
+
+template <typename S>
+__device__ __forceinline__ void p_dense(const PSArgs& A, unsigned char* smem)
+{
+    const S* kept = (const S*)(smem + A.mkeep);
+    p_dense_rows(A, [&](const PDense& D, int a, int b) {
+        const size_t np = ps_pitch<S>(D.n);
+        ps_dense<S>(A.mkeep ? kept : (const S*)D.minv + a * np, (const S*)D.b, (S*)D.x, D.n, a, b,
+                    (S*)smem, D.box);
+        kept += (b - a) * np;
+        __syncthreads();
+    });
 }
 
 // r = b - A x of a tile; tot = <b, b>, <r, r>
@@ -566,6 +589,14 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
         const int4* src = (const int4*)(A.recs + base);
         for (int k = threadIdx.x; k < nrec * W; k += PS_NT) ((int4*)rec)[k] = src[k];
         for (int k = threadIdx.x; k < nrec; k += PS_NT) rconv[k] = 0;
+    }
+    if (A.mkeep) {
+        unsigned char* kept = smem + A.mkeep;
+        p_dense_rows(A, [&](const PDense& D, int a, int b) {
+            const size_t np = ps_pitch<S>(D.n) * sizeof(S), bytes = (b - a) * np;
+            ps_copy16(kept, (const unsigned char*)D.minv + a * np, bytes);
+            kept += bytes;
+        });
     }
     __syncthreads();
     const int ns = lev0[1] - base;  // level-0 tiles of the block
@@ -684,7 +715,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
             if (single && slot[0].conv) break;
         }
         if (single && slot[0].conv) break;
-        p_dense_rows<S>(A, smem);
+        p_dense<S>(A, smem);
         if (!(told ? ps_sync(g, refresh) : ps_sync(g, decide))) return;
         if (single && slot[0].conv) break;
         for (int l = A.ng - 1; l >= 1; --l) {
@@ -758,14 +789,16 @@ __global__ void k_ps_setup(const __grid_constant__ PSArgs A, double tol2, int ma
 // ---- host ----------------------------------------------------------------------
 constexpr size_t PS_SMEM = 180 * 1024;
 
-// estimated cycles of a block for one tile of tw x th nodes: a fixed cost and
-// the cells its legs visit (the FP64 pipe's rate, or the issue rate in FP32)
+// Cycles of phases A and B for a tile of tw x th nodes: a fixed cost (the
+// chain of loads, half sweeps and sums) and one per cell that the legs visit.
+// Fitted to FP64 tiles of 26 x 18 (28.5k) and 52 x 52 (57k) and FP32 tiles of
+// 34 x 40 (37k).
 static double tile_cost(int tw, int th, int prec)
 {
     const double n = (double)(tw + 10) * (th + 10);
     double cells = 2.0 * n + 3.0 * tw * th;
     for (int q = 0; q < 5; ++q) cells += (double)(tw + 2 * q) * (th + 2 * q);
-    return 3000.0 + (prec == 0 ? 2.0 : 0.5) * cells;
+    return prec == 0 ? 20700.0 + 1.15 * cells : 15000.0 + 1.3 * cells;
 }
 
 struct TileDim {
@@ -873,21 +906,30 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     // grid levels of every member: down to its dense level
     std::vector<int> ng(n);
     int maxg = 0, nrows = 0;
-    size_t minv_elems = 0;
+    auto unknowns = [](const MGLevel& L) {
+        return (long long)(L.per ? L.nxn : std::max(0, L.nxn - 2)) * std::max(0, L.nyn - 2);
+    };
     for (int b = 0; b < n; ++b) {
         const std::vector<MGLevel>& lev = mem[b].mg->lev;
         int l = n == 1 ? 0 : 1;
         for (; l < (int)lev.size(); ++l) {
-            const long long k = (long long)lev[l].nyn * lev[l].nxn;
-            if (k <= mem[b].ndense_cap && ps_band_ok(k, lev[l].nxn)) break;
+            const long long k = unknowns(lev[l]);
+            if (k <= mem[b].ndense_cap && ps_band_ok(k, lev[l].nxn, prec)) break;
         }
-        if (l >= (int)lev.size() || l >= PS_LMAX) return 0;
+        if (l >= (int)lev.size() || l >= PS_LMAX || unknowns(lev[l]) < 1) return 0;
         for (int q = 0; q < l; ++q)  // colours and the coarse grid wrap only over an even count
             if (lev[q].per && lev[q].nxn % 2) return 0;
+        // the unknowns leave the closed edges out: they must be dry
+        const std::vector<uint8_t>& hm = mem[b].mg->hmask[l];
+        for (int J = 0; J < lev[l].nyn; ++J)
+            for (int I = 0; I < lev[l].nxn; ++I)
+                if ((J == 0 || J == lev[l].nyn - 1 ||
+                     (!lev[l].per && (I == 0 || I == lev[l].nxn - 1))) &&
+                    hm[(size_t)J * lev[l].nxn + I])
+                    return 0;
         ng[b] = l;
         maxg = std::max(maxg, l);
-        nrows += lev[l].nyn * lev[l].nxn;
-        minv_elems += (size_t)lev[l].nyn * lev[l].nxn * lev[l].nyn * lev[l].nxn;
+        nrows += (int)unknowns(lev[l]);
     }
     PSArgs& a = s.a;
     memset(&a, 0, sizeof(a));
@@ -898,35 +940,44 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     // tiles, level by level
     std::vector<std::vector<PTile>> tl(a.ng);
     std::vector<PDense> dense(n);
-    size_t smem = 0;
+    size_t smem = 0, maxrow = 0;
     for (int b = 0; b < n; ++b) {
         const MGLevel& D = mem[b].mg->lev[ng[b]];
-        const int nd = D.nyn * D.nxn;
+        // the unknowns: all nodes but the closed edges' (no fluid node there)
+        const int e0 = D.per ? 0 : 1, w = D.nxn - 2 * e0, nd = w * (D.nyn - 2);
+        const size_t nodes = (size_t)D.nyn * D.nxn;
         dense[b].n = nd;
         dense[b].row0 = b ? dense[b - 1].row0 + dense[b - 1].n : 0;
-        dense[b].b = dal((size_t)nd * es);
-        dense[b].x = dal((size_t)nd * es);
-        void* minv = dal((size_t)nd * nd * es);
+        dense[b].box = PSBox{w, D.nxn, D.nxn + e0, 1.0f / (float)w};
+        dense[b].b = dal(nodes * es);
+        dense[b].x = dal(nodes * es);
+        const int np = prec == 0 ? ps_pitch<double>(nd) : ps_pitch<float>(nd);
+        void* minv = dal((size_t)nd * np * es);
+        maxrow = std::max(maxrow, np * es);
         dense[b].minv = minv;
         if (!dense[b].b || !dense[b].x || !minv) return 2;
         // -A of the dense level (identity rows at non-fluid nodes: their b is 0)
         const std::vector<uint8_t>& hm = mem[b].mg->hmask[ng[b]];
-        const int w1 = D.nxn + 1;
+        const int w1 = w + 1;
         std::vector<double> h((size_t)nd * w1, 0.0);
-        for (int J = 0; J < D.nyn; ++J)
-            for (int I = 0; I < D.nxn; ++I) {
-                const int k = J * D.nxn + I;
-                h[(size_t)k * w1] = hm[k] ? -D.diag : 1.0;
-                if (!hm[k]) continue;
-                if (I > 0 && hm[k - 1]) h[(size_t)k * w1 + 1] -= D.cx;
-                if (J > 0 && hm[k - D.nxn]) h[(size_t)k * w1 + D.nxn] -= D.cy;
-                if (D.per && I == D.nxn - 1 && D.nxn > 1 && hm[k - I])
-                    h[(size_t)k * w1 + I] -= D.cx;
-            }
-        const int rc = ps_invert(h, nd, D.nxn, {}, -1.0, prec, minv);
+        auto fluid = [&](int J, int I) {
+            return J >= 0 && J < D.nyn && I >= 0 && I < D.nxn && hm[(size_t)J * D.nxn + I] != 0;
+        };
+        for (int k = 0; k < nd; ++k) {
+            const int J = 1 + k / w, I = e0 + k % w;
+            double* r = &h[(size_t)k * w1];
+            r[0] = fluid(J, I) ? -D.diag : 1.0;
+            if (!fluid(J, I)) continue;
+            if (k % w > 0 && fluid(J, I - 1)) r[1] -= D.cx;
+            if (J > 1 && fluid(J - 1, I)) r[w] -= D.cy;
+            if (D.per && I == D.nxn - 1 && D.nxn > 1 && fluid(J, 0)) r[I] -= D.cx;
+        }
+        const int rc = ps_invert(h, nd, w, {}, -1.0, prec, minv);
         if (rc == 5) return 0;
         if (rc) return rc;
-        smem = std::max(smem, (nd + 128 * (size_t)((nrows + sms - 1) / sms + 1)) * es);
+        const int rows = (nrows + sms - 1) / sms;  // of a block, at most
+        smem = std::max(smem, es * (prec == 0 ? ps_dense_elems<double>(nd, rows)
+                                              : ps_dense_elems<float>(nd, rows)));
     }
     for (int l = 0; l < a.ng; ++l) {
         std::vector<std::pair<int, int>> dims(n);
@@ -988,6 +1039,12 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
         }
     }
     a.ntiles = (int)tl[0].size();
+    smem = (smem + 15) / 16 * 16;
+    const size_t keep = maxrow * ((nrows + sms - 1) / sms);
+    if (smem + keep <= PS_SMEM) {
+        a.mkeep = (int)smem;
+        smem += keep;
+    }
     std::vector<std::vector<std::vector<int>>> of(sms, std::vector<std::vector<int>>(a.ng));
     for (int l = 0; l < a.ng; ++l) {
         std::vector<double> cost;

@@ -14,7 +14,7 @@ struct BSGlobals;
 // One tile of one level of one member: everything a block reads about it
 struct alignas(16) PTile {
     const uint8_t* m;   // fluid mask of the level; node (J, I) at off + J pitch + I
-    void *x, *xa, *b;   // level arrays (level 0: z, xa, unused)
+    void *x, *xa, *b;   // level arrays (level 0: z, xa, the FP32 copy of r)
     void *cx_, *cb;     // the next coarser level's x and b, node at coff + J cpitch + I
     const uint8_t* cm;  // its mask, at cmoff + J cmpitch + I
     long long off, coff, cmoff;
@@ -29,9 +29,10 @@ struct alignas(16) PTile {
 };
 
 struct PDense {
-    const void* minv;  // n x n inverse of the member's dense level
-    void *b, *x;       // compact
-    int n, row0;       // rows of the members before it
+    const void* minv;  // inverse of the member's dense level (n unknowns)
+    void *b, *x;       // compact: rows of nxn nodes
+    int n, row0;       // unknowns; those of the members before it
+    PSBox box;         // the unknowns: the nodes off the closed edges
 };
 
 constexpr int PS_LMAX = 14;
@@ -46,6 +47,7 @@ struct PSArgs {
     int nrows;           // dense rows of all members
     int dense0;          // one member whose level 0 is the dense level
     int ntiles;          // level-0 tiles
+    int mkeep;           // offset in shared memory of the block's dense rows (0: not kept)
     double *x, *b, *r[2], *s[2], *p, *w;  // arenas, FP64
     double* part;        // tile totals, 2 x 2 ntiles
     int* conv;           // per member

@@ -1439,9 +1439,9 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
         for (int b = 0; b < s.n; ++b) {
             const MGLevel& L = levs[(size_t)b * BS_LMAX];
             n0 += (long long)L.nyn * L.nxn;
-            // the inverses of a batch: about 1.5M entries together
+            // the inverses of a batch: about 1.5M entries together (FP32: 6M)
             pm[b].mg = &s.mg[b];
-            pm[b].ndense_cap = s.n == 1 ? PS_NDENSE : (int)sqrt(1.5e6 / s.n);
+            pm[b].ndense_cap = s.n == 1 ? PS_NDENSE32 : (int)sqrt((mode == 0 ? 1.5e6 : 6e6) / s.n);
         }
         if (mode == 0 || n0 <= PS_FP32_NODES) {
             const int e = ps_build(s.ps, pm, mode, v.nelem, scs, s.eg, &s.eg->status);
