@@ -791,14 +791,14 @@ constexpr size_t PS_SMEM = 180 * 1024;
 
 // Cycles of phases A and B for a tile of tw x th nodes: a fixed cost (the
 // chain of loads, half sweeps and sums) and one per cell that the legs visit.
-// Fitted to FP64 tiles of 26 x 18 (28.5k) and 52 x 52 (57k) and FP32 tiles of
+// Fitted to FP64 tiles of 26 x 18 (28.5k) and 52 x 52 (84k) and FP32 tiles of
 // 34 x 40 (37k).
 static double tile_cost(int tw, int th, int prec)
 {
     const double n = (double)(tw + 10) * (th + 10);
     double cells = 2.0 * n + 3.0 * tw * th;
     for (int q = 0; q < 5; ++q) cells += (double)(tw + 2 * q) * (th + 2 * q);
-    return prec == 0 ? 20700.0 + 1.15 * cells : 15000.0 + 1.3 * cells;
+    return 13400.0 + (prec == 0 ? 2.24 : 1.45) * cells;
 }
 
 struct TileDim {
@@ -846,8 +846,9 @@ static double deal(const std::vector<double>& cost, int blocks, std::vector<int>
 
 // Tiles of one level of all members. One member: of all partitions the one
 // with the smallest estimate of the busiest block's time; up to about 1300^2
-// nodes that is one tile per block. A batch: all members get tiles of at most
-// T x T nodes, T the one with the smallest estimate for the busiest block.
+// nodes that is one tile per block. A batch: one tile per block, the members
+// cut in turn, or tiles of at most T x T nodes for all members, whichever has
+// the smallest estimate for the busiest block.
 static std::vector<TileDim> pick_tiles(const std::vector<std::pair<int, int>>& nxny, int sms,
                                        int prec)
 {
@@ -868,6 +869,44 @@ static std::vector<TileDim> pick_tiles(const std::vector<std::pair<int, int>>& n
                 }
             }
         return best;
+    }
+    // one tile per block at most: the member with the costliest tiles is cut
+    // once more, in the direction that helps it more, while blocks are left
+    {
+        std::vector<std::pair<int, int>> cut(nxny.size(), {1, 1});
+        std::vector<double> cost(nxny.size(), 0.0);
+        auto dim = [&](size_t b, int x, int y) {
+            return tile_dim(nxny[b].first, nxny[b].second, x, y);
+        };
+        auto price = [&](const TileDim& d) {
+            return region_bytes(d.tw, d.th, prec) > PS_SMEM ? 1e12 * d.tw * d.th
+                                                            : tile_cost(d.tw, d.th, prec);
+        };
+        int total = 0;
+        for (size_t b = 0; b < nxny.size(); ++b) {
+            if (nxny[b].first <= 0) continue;
+            cur[b] = dim(b, 1, 1);
+            cost[b] = price(cur[b]);
+            ++total;
+        }
+        while (total <= sms) {
+            const size_t b = std::max_element(cost.begin(), cost.end()) - cost.begin();
+            const TileDim x = dim(b, cut[b].first + 1, cut[b].second);
+            const TileDim y = dim(b, cut[b].first, cut[b].second + 1);
+            const bool wide = price(x) <= price(y);
+            const TileDim& d = wide ? x : y;
+            const int more = d.ntx * d.nty - cur[b].ntx * cur[b].nty;
+            if (total + more > sms || price(d) >= cost[b]) break;
+            total += more;
+            cur[b] = d;
+            cost[b] = price(d);
+            (wide ? cut[b].first : cut[b].second) += 1;
+        }
+        const double worst = *std::max_element(cost.begin(), cost.end());
+        if (total <= sms && worst < 1e9) {
+            bc = worst;
+            best = cur;
+        }
     }
     for (int T = 8; T <= 128; T += 4) {
         if (region_bytes(T, T, prec) > PS_SMEM) break;
