@@ -150,7 +150,7 @@ __device__ __forceinline__ void set_rz(DevScalars& sc, int ir, double rz)
 // up leg writes one total per tile and no more, so its blocks never wait on
 // a fence or a ticket; members whose level 0 is in the tail (mnn = 0) get
 // theirs from k_bs_tail.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 k_bs_rz(const BSInfo* __restrict__ info, DevScalars* scs, const double* __restrict__ tpart,
         int ir)
 {
@@ -320,7 +320,7 @@ k_bs_pq(const int4* __restrict__ tiles, int ntiles, const MGLevel* __restrict__ 
 // <p, q> of every member from k_bs_pq's tile totals (fixed order), alpha =
 // rz / <p, q>. The tile kernels write their totals and no more (no fence or
 // ticket per block); one block per member sums them here.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 k_bs_alpha(const BSInfo* __restrict__ info, DevScalars* scs, const double* __restrict__ tpart,
            int ir)
 {
@@ -421,7 +421,7 @@ k_bs_xr(const int4* __restrict__ tiles, int ntiles, const MGLevel* __restrict__ 
 // <r, r> of every member from k_bs_xr's tile totals (fixed order), the
 // member's convergence, and the loop condition (the block that completes
 // the count over all members sets it).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 k_bs_conv(const BSInfo* __restrict__ info, DevScalars* scs, const double* __restrict__ tpart,
           BSGlobals* eg, cudaGraphConditionalHandle cond, int ir, int nmem)
 {
@@ -476,10 +476,18 @@ k_bs_conv(const BSInfo* __restrict__ info, DevScalars* scs, const double* __rest
 // FP64 residual r = b - A x of the tile (x staged with a one-node halo);
 // the per-thread sums of b*b (BB) and r*r; r and its FP32 copy rin where
 // given. GB300 runs FP64 at 1/64 of its FP32 rate and this is the FP64
-// kernel of the FP32 form, so the variants are compile-time (a runtime
-// select would issue both sides): HELM, an operator with a main-diagonal
-// term (maindiag != 0; exact for members without one too); UNIT, square
-// cells (cx = cy = 1: the same sums without the multiplies).
+// kernel of the FP32 form, bound by that pipe, so:
+//  * the variants are compile-time (a runtime select would issue both sides):
+//    HELM, an operator with a main-diagonal term (maindiag != 0; exact for
+//    members without one too); UNIT, square cells (cx = cy = 1: the same sums
+//    without the multiplies);
+//  * a difference of two neighbours is formed once for both: a thread marches
+//    down TH/8 consecutive rows of its column, keeping the north difference
+//    as the next row's south one, and takes the west difference from the
+//    neighbouring lane's east one (lane 0's, for all rows, from one
+//    instruction whose lane k forms row k's). (w - c) + (e - c) =
+//    (e - c) - (c - w) to the last bit, so the result does not change; 7
+//    FP64 instructions a node instead of 9 (Poisson, square cells).
 template <int TH, bool HELM, bool UNIT, bool BB>
 __device__ __forceinline__ void residual64(const int4& tl, const MGLevel& L,
                                            const double* __restrict__ x,
@@ -487,43 +495,54 @@ __device__ __forceinline__ void residual64(const int4& tl, const MGLevel& L,
                                            float* __restrict__ rin, double (&w)[2])
 {
     constexpr int H = 1, W = Reg<H, TH>::WX, N = Reg<H, TH>::N, TQ = TH / 8;
+    static_assert(TQ <= 32, "a lane per row for the west differences");
     __shared__ double sx[N];
     __shared__ uint8_t sm[N];
     stage_region<H, TH, double, double>(L, tl.z, tl.y, x, sx, (const double*)nullptr,
                                         (double*)nullptr, sm);
+    const int c = threadIdx.x, r0 = threadIdx.y * TQ;  // the thread's first tile row
     double bv[TQ];
     long long k[TQ];
     bool ok[TQ];
 #pragma unroll
-    for (int qr = 0; qr < TQ; ++qr) {
-        const int J = tl.z + threadIdx.y + 8 * qr, I = tl.y + threadIdx.x;
-        ok[qr] = J < L.nyn && I < L.nxn;
-        k[qr] = nidx(L, min(J, L.nyn - 1), min(I, L.nxn - 1));
-        bv[qr] = b[k[qr]];
+    for (int q = 0; q < TQ; ++q) {
+        const int J = tl.z + r0 + q, I = tl.y + c;
+        ok[q] = J < L.nyn && I < L.nxn;
+        k[q] = nidx(L, min(J, L.nyn - 1), min(I, L.nxn - 1));
+        bv[q] = b[k[q]];
     }
     __syncthreads();
     const double cx = L.cx, cy = L.cy, md = L.md;
+    // west edge of the tile: x(row, 0) - x(row, -1), lane q for row r0 + q
+    const int er = (r0 + min(c, TQ - 1) + H) * W;
+    const double wedge = sx[er + H] - sx[er + H - 1];
+    double xc = sx[(r0 + H) * W + c + H];
+    double south = xc - sx[(r0 + H - 1) * W + c + H];
 #pragma unroll
-    for (int qr = 0; qr < TQ; ++qr) {
-        const int rr = threadIdx.y + 8 * qr, c = threadIdx.x;
-        const int e = (rr + H) * W + c + H;
+    for (int q = 0; q < TQ; ++q) {
+        const int e = (r0 + q + H) * W + c + H;
+        const double xn = sx[e + W];
+        const double east = sx[e + 1] - xc, north = xn - xc;
+        const double we = __shfl_sync(0xffffffffu, wedge, q);
+        const double wl = __shfl_up_sync(0xffffffffu, east, 1);
+        const double west = c > 0 ? wl : we;
+        const double sxw = east - west, syw = north - south;
+        double ax;
+        if constexpr (UNIT) ax = sxw + syw;
+        else ax = cx * sxw + cy * syw;
+        if constexpr (HELM) ax = ax - md * xc;
         double rv = 0.0;
-        if (sm[e] && ok[qr]) {
-            const double c = sx[e];
-            const double sxw = (sx[e - 1] - c) + (sx[e + 1] - c);
-            const double syw = (sx[e - W] - c) + (sx[e + W] - c);
-            double ax;
-            if constexpr (UNIT) ax = sxw + syw;
-            else ax = cx * sxw + cy * syw;
-            if constexpr (HELM) ax = ax - md * c;
-            rv = bv[qr] - ax;
-            if constexpr (BB) w[0] += bv[qr] * bv[qr];
+        if (sm[e] && ok[q]) {
+            rv = bv[q] - ax;
+            if constexpr (BB) w[0] += bv[q] * bv[q];
             w[1] += rv * rv;
         }
-        if (ok[qr]) {
-            if (r) r[k[qr]] = rv;
-            if (rin) rin[k[qr]] = f64_to_f32_rn(rv);
+        if (ok[q]) {
+            if (r) r[k[q]] = rv;
+            if (rin) rin[k[q]] = f64_to_f32_rn(rv);
         }
+        xc = xn;
+        south = north;
     }
 }
 
@@ -548,7 +567,7 @@ k_bs_init(const int4* __restrict__ tiles, const MGLevel* __restrict__ levs,
 
 // FP64 form, per member from k_bs_init's tile sums: <b,b>, <r,r>, the start
 // state of the solve; the loop condition (the block completing the count)
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 k_bs_init_fin(const BSInfo* __restrict__ info, DevScalars* scs,
               const double* __restrict__ tpart, BSGlobals* eg,
               cudaGraphConditionalHandle cond, int nmem)
@@ -601,7 +620,7 @@ k_bs_refine(const int4* __restrict__ tiles, const MGLevel* __restrict__ levs,
 
 // Refinement form, per member from k_bs_refine's tile sums: converged, or
 // start a new round; the outer loop condition.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 k_bs_refine_fin(const BSInfo* __restrict__ info, DevScalars* scs,
                 const double* __restrict__ tpart, BSGlobals* eg, int first,
                 cudaGraphConditionalHandle cond, int nmem)
@@ -878,7 +897,7 @@ static int cg_body(BatchSolver& s, cudaStream_t st, cudaGraphConditionalHandle c
     V* x = ir ? (V*)nullptr : (V*)s.v.x64;  // the refinement form's x is the ring
     int cnt = vcycle<S, TH>(s, st, ir);
     if (s.maxl > 0) {
-        launch_pdl(k_bs_rz, dim3(s.n), dim3(256), 0, st, (const BSInfo*)s.dinfo, s.scs,
+        launch_pdl(k_bs_rz, dim3(s.n), dim3(s.fin_threads), 0, st, (const BSInfo*)s.dinfo, s.scs,
                    (const double*)s.mpartials, ir);
         cnt += 1;
     }
@@ -887,12 +906,12 @@ static int cg_body(BatchSolver& s, cudaStream_t st, cudaGraphConditionalHandle c
                (const int4*)s.rtiles, nt, (const MGLevel*)s.dlevs, (const S*)s.v.z, (V*)s.v.p,
                (V*)s.v.p2, (V*)s.v.q, (const DevScalars*)s.scs, s.partials, ir, ring,
                (long long)s.v.nelem);
-    launch_pdl(k_bs_alpha, dim3(s.n), dim3(256), 0, st, (const BSInfo*)s.dinfo, s.scs,
+    launch_pdl(k_bs_alpha, dim3(s.n), dim3(s.fin_threads), 0, st, (const BSInfo*)s.dinfo, s.scs,
                (const double*)s.partials, ir);
     launch_pdl(k_bs_xr<V, TH>, dim3(resident_grid<k_bs_xr<V, TH>>(nt)), blk, 0, st,
                (const int4*)s.rtiles, nt, (const MGLevel*)s.dlevs, x, r, (const V*)s.v.p,
                (const V*)s.v.p2, (const V*)s.v.q, (const DevScalars*)s.scs, s.partials, ir);
-    launch_pdl(k_bs_conv, dim3(s.n), dim3(256), 0, st, (const BSInfo*)s.dinfo, s.scs,
+    launch_pdl(k_bs_conv, dim3(s.n), dim3(s.fin_threads), 0, st, (const BSInfo*)s.dinfo, s.scs,
                (const double*)s.partials, s.eg, cond, ir, s.n);
     cnt += 4;
     s.body_launches = cnt;
@@ -969,7 +988,7 @@ static int bs_record_t(BatchSolver& s, cudaStream_t st, cudaStream_t st2, int* l
             if (e != cudaSuccess) return (int)e;
         }
         launch_init<TH>(s, st);
-        k_bs_init_fin<<<s.n, 256, 0, st>>>(s.dinfo, s.scs, s.partials, s.eg, cond, s.n);
+        k_bs_init_fin<<<s.n, s.fin_threads, 0, st>>>(s.dinfo, s.scs, s.partials, s.eg, cond, s.n);
         fixed += 2;
         if (capturing) {
             int r = add_while(st, st2, &cond, 1, [&](cudaStream_t sb) {
@@ -1000,7 +1019,7 @@ static int bs_record_t(BatchSolver& s, cudaStream_t st, cudaStream_t st2, int* l
     }
     k_bs_reset<<<1, 1, 0, st>>>(s.eg);
     launch_refine<TH, true>(s, st);
-    k_bs_refine_fin<<<s.n, 256, 0, st>>>(s.dinfo, s.scs, s.partials, s.eg, 1, cond_o, s.n);
+    k_bs_refine_fin<<<s.n, s.fin_threads, 0, st>>>(s.dinfo, s.scs, s.partials, s.eg, 1, cond_o, s.n);
     fixed += 3;
     auto round_tail = [&](cudaStream_t sb) {
         k_bs_correct<TH><<<nt, blk, 0, sb>>>(s.rtiles, s.dlevs, (double*)s.v.x64,
@@ -1008,7 +1027,7 @@ static int bs_record_t(BatchSolver& s, cudaStream_t st, cudaStream_t st2, int* l
                                              s.scs);
         k_bs_reset<<<1, 1, 0, sb>>>(s.eg);
         launch_refine<TH, false>(s, sb);
-        k_bs_refine_fin<<<s.n, 256, 0, sb>>>(s.dinfo, s.scs, s.partials, s.eg, 0, cond_o, s.n);
+        k_bs_refine_fin<<<s.n, s.fin_threads, 0, sb>>>(s.dinfo, s.scs, s.partials, s.eg, 0, cond_o, s.n);
     };
     if (capturing) {
         int r = add_while(st, st2, &cond_o, 1, [&](cudaStream_t sb) {
@@ -1267,7 +1286,7 @@ static int bs_pipe_setup(BatchSolver& s, const std::vector<MGLevel>& levs,
     return 0;
 }
 
-constexpr long long PS_FP32_NODES = 1500000;
+constexpr long long PS_FP32_NODES = 2000000;
 
 int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uint8_t* dmask,
              int mode, const BSVecs& v, DevScalars* scs)
@@ -1424,13 +1443,19 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         s.tail_threads = s.n > nsm ? 512 : 1024;
+        // the member-sum kernels: one block per member; 1024 threads where a
+        // member has thousands of tiles (qg 4096^2: 17 us with 256)
+        int nn = 0;
+        for (const BSInfo& in : info) nn = std::max(nn, in.nn);
+        s.fin_threads = nn > 2048 ? 1024 : 256;
     }
     {
         const int e = bs_pipe_setup(s, levs, info, dal);
         if (e) return e;
     }
     // The persistent solve: every FP64 problem (its level kernels and loops
-    // cost more at every size), and FP32 problems of up to PS_FP32_NODES nodes:
+    // cost more at every size), and FP32 problems of up to PS_FP32_NODES nodes
+    // (batches half of that):
     // above that the refinement form's FP32 Krylov vectors and pipelined legs
     // move less and are the faster ones.
     {
@@ -1443,7 +1468,7 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
             pm[b].mg = &s.mg[b];
             pm[b].ndense_cap = s.n == 1 ? PS_NDENSE32 : (int)sqrt((mode == 0 ? 1.5e6 : 6e6) / s.n);
         }
-        if (mode == 0 || n0 <= PS_FP32_NODES) {
+        if (mode == 0 || n0 <= (s.n == 1 ? PS_FP32_NODES : PS_FP32_NODES / 2)) {
             const int e = ps_build(s.ps, pm, mode, v.nelem, scs, s.eg, &s.eg->status);
             if (e) return e;
         }
