@@ -345,6 +345,9 @@ static int rec_warm(f2d_model_s* m, int warm, cudaStream_t s)
     w.p1 = (double*)fb(m, "psi.p1");
     w.d1 = (double*)fb(m, "psi.d1");
     w.d2 = (double*)fb(m, "psi.d2");
+    w.e1 = (double*)fb(m, "psi.e1");
+    w.e2 = (double*)fb(m, "psi.e2");
+    w.e3 = (double*)fb(m, "psi.e3");
     CKI(launch_psi_warm(warm, w, (long long)m->g.P * m->g.NY, m->sc, s));
     m->rec_launches += 1;
     return 0;
@@ -1196,8 +1199,11 @@ int f2d_model_create(const f2d_params* p, const int8_t* msk, f2d_model* out)
     // previous step's stage increments (the warm start of the stage solves,
     // rec_warm)
     if (p->model == F2D_MODEL_EULERPSI || p->model == F2D_MODEL_QG)
-        for (const char* f : {"psi.s0", "psi.p1", "psi.d1", "psi.d2"})
-            if ((e = add_field(m, f, false, 8))) return bail(e);
+        for (const char* f :
+             {"psi.s0", "psi.p1", "psi.d1", "psi.d2", "psi.e1", "psi.e2", "psi.e3"})
+            if ((f[4] != 'e' || psi_warm_brackets(m->prec, (long long)m->g.P * m->g.NY)) &&
+                (e = add_field(m, f, false, 8)))
+                return bail(e);
     // qgrsw keeps the third stage's (or LFRA's) tendency too: it is
     // projected between the tendency kernel and the update
     for (const char* f : prog) m->prog.push_back(f);

@@ -41,7 +41,7 @@ struct Member {
     int t0, nt;         // range in the cell-tile table
     int n0, nn;         // range in the level-0 node-tile table
     int nl, ltail, ksweeps;
-    int pad;
+    int ext;            // the warm start keeps its brackets (psi_warm_brackets)
     long long poff;     // offset of the member's packed (NY, NX) array in the
                         // all-members host layout of f2d_ensemble_fields_*
 };
@@ -73,7 +73,7 @@ struct EnsArenas {
     void *q[2], *ds1, *ds2, *Ux, *Uy, *rhs, *psi, *fv;
     // the warm start of the stage solves (WarmArrays, stage.cuh): psi at the
     // step start and of stage 1, the previous step's stage increments
-    double *psi_s0, *psi_p1, *psi_d1, *psi_d2;
+    double *psi_s0, *psi_p1, *psi_d1, *psi_d2, *psi_e1, *psi_e2, *psi_e3;
     const uint32_t* code;
 };
 
@@ -104,15 +104,16 @@ k_ens_fluxform_stage(const int4* __restrict__ tiles, const Member* __restrict__ 
                         tl.y, tl.z);
 }
 
-// Warm start of the solve of RK3 stage mode+1 (psi_warm_point, stage.cuh) on
+// Warm start of the solve of RK3 stage mode+1 (psi_warm_pairs, stage.cuh) on
 // every member's array (all P x NY elements: the pads are 0 and stay 0),
 // with the member's own step-size ratio: blockIdx.y is the member, the
 // blocks of a member stride over its elements in 16-byte pairs, two pairs
 // per thread and pass (the member arrays start 32-element aligned, P is
 // even). Mode 2 also records the
 // member's dt_warm (block 0 of the member; mode 2 reads no dt_warm).
+template <int MODE>
 __global__ void __launch_bounds__(256) k_ens_psi_warm(const Member* __restrict__ mem,
-                                                       EnsArenas a, int mode, DevScalars* scs)
+                                                       EnsArenas a, DevScalars* scs)
 {
     const Member& mb = mem[blockIdx.y];
     const Geom g = mb.g;
@@ -125,6 +126,10 @@ __global__ void __launch_bounds__(256) k_ens_psi_warm(const Member* __restrict__
     w.p1 = a.psi_p1 + mb.off;
     w.d1 = a.psi_d1 + mb.off;
     w.d2 = a.psi_d2 + mb.off;
+    w.e1 = a.psi_e1 + mb.off;
+    w.e2 = a.psi_e2 + mb.off;
+    w.e3 = a.psi_e3 + mb.off;
+    const bool ext = mb.ext;
     const long long n = g.P * (long long)g.NY;
     // pairs of elements, two pairs per thread and pass (see psi_warm_pairs)
     constexpr int U = 2;
@@ -138,9 +143,10 @@ __global__ void __launch_bounds__(256) k_ens_psi_warm(const Member* __restrict__
             k[u] = k0 + u * step;
             ok[u] = k[u] < n;
         }
-        psi_warm_pairs<U>(mode, w, k, ok, hist, rho);
+        if (ext) psi_warm_pairs<MODE, true, U>(w, k, ok, hist, rho);
+        else psi_warm_pairs<MODE, false, U>(w, k, ok, hist, rho);
     }
-    if (mode == 2 && blockIdx.x == 0 && threadIdx.x == 0) sc.dt_warm = sc.dt;
+    if (MODE == 2 && blockIdx.x == 0 && threadIdx.x == 0) sc.dt_warm = sc.dt;
 }
 
 // centerstovertices (+ beta-plane term) into the FP64 right-hand side
@@ -412,7 +418,10 @@ static int ens_record_diag(f2d_ensemble_s* e, int par, cudaStream_t s, int warm 
         k_ens_c2v<float><<<e->ncell, blk, 0, s>>>(e->cell_tiles, e->dmem, e->ar, par, use_fv);
     e->rec += 1;
     if (warm >= 0) {
-        k_ens_psi_warm<<<dim3(48, e->n), 256, 0, s>>>(e->dmem, e->ar, warm, e->scs);
+        const dim3 gr(48, e->n);
+        if (warm == 0) k_ens_psi_warm<0><<<gr, 256, 0, s>>>(e->dmem, e->ar, e->scs);
+        else if (warm == 1) k_ens_psi_warm<1><<<gr, 256, 0, s>>>(e->dmem, e->ar, e->scs);
+        else k_ens_psi_warm<2><<<gr, 256, 0, s>>>(e->dmem, e->ar, e->scs);
         e->rec += 1;
     }
     int r = ens_record_solve(e, s);
@@ -572,6 +581,7 @@ int f2d_ensemble_create(const f2d_params* p, int count, const int* nxs, const in
         g.P = (g.NX + 15) / 16 * 16;
         g.xper = q.xperiodic ? 1 : 0;
         mb.off = (long long)off;
+        mb.ext = psi_warm_brackets(e->prec, (long long)mb.g.P * mb.g.NY);
         mb.poff = (long long)poff;
         poff += (size_t)g.NX * g.NY;
         const double dx = q.Lx / q.nx, dy = q.Ly / q.ny;
@@ -597,6 +607,12 @@ int f2d_ensemble_create(const f2d_params* p, int count, const int* nxs, const in
     e->ar.psi_p1 = (double*)A(8);
     e->ar.psi_d1 = (double*)A(8);
     e->ar.psi_d2 = (double*)A(8);
+    bool ext = false;  // the brackets' arenas: where a member keeps them
+    for (int b = 0; b < count; ++b) ext = ext || e->hmem[b].ext;
+    for (double** q : {&e->ar.psi_e1, &e->ar.psi_e2, &e->ar.psi_e3}) {
+        *q = ext ? (double*)A(8) : nullptr;
+        if (ext && !*q) return bail(f2d_internal_fail(2, "out of device memory for the ensemble"));
+    }
     e->ar.fv = A(8);
     e->code = A(4);
     e->gmask = A(1);

@@ -687,22 +687,40 @@ int launch_fill_periodic(int prec, void* a, const Geom& g, cudaStream_t s)
     return (int)cudaGetLastError();
 }
 
-// Warm start of the Poisson solve of SSP-RK3 stage mode+1 (psi_warm_point,
-// stage.cuh): a grid-stride loop over every element.
-__global__ void k_psi_warm(int mode, WarmArrays w, long long n, DevScalars* sc)
+// Warm start of the Poisson solve of SSP-RK3 stage mode+1 (psi_warm_pairs,
+// stage.cuh): a grid-stride loop over the pairs of elements.
+template <int MODE, bool EXT>
+__global__ void __launch_bounds__(256) k_psi_warm(WarmArrays w, long long n, DevScalars* sc)
 {
     const bool hist = sc->dt_warm > 0.0;
     const double rho = hist ? sc->dt / sc->dt_warm : 0.0;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-         k += (long long)gridDim.x * blockDim.x)
-        psi_warm_point(mode, w, k, hist, rho);
-    if (mode == 2 && blockIdx.x == 0 && threadIdx.x == 0) sc->dt_warm = sc->dt;
+    const long long step = 2ll * gridDim.x * blockDim.x;
+    for (long long k0 = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x); k0 < n;
+         k0 += U * step) {
+        long long k[U];
+        bool ok[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            k[u] = k0 + u * step;
+            ok[u] = k[u] < n;
+        }
+        psi_warm_pairs<MODE, EXT, U>(w, k, ok, hist, rho);
+    }
+    if (MODE == 2 && blockIdx.x == 0 && threadIdx.x == 0) sc->dt_warm = sc->dt;
 }
 
 int launch_psi_warm(int mode, const WarmArrays& w, long long n, DevScalars* sc, cudaStream_t s)
 {
-    const int nb = (int)std::min<long long>((n + 255) / 256, 152 * 8);
-    k_psi_warm<<<nb, 256, 0, s>>>(mode, w, n, sc);
+    const int nb = (int)std::min<long long>((n / 2 + 255) / 256, 152 * 8);
+    if (w.e1) {
+        if (mode == 0) k_psi_warm<0, true><<<nb, 256, 0, s>>>(w, n, sc);
+        else if (mode == 1) k_psi_warm<1, true><<<nb, 256, 0, s>>>(w, n, sc);
+        else k_psi_warm<2, true><<<nb, 256, 0, s>>>(w, n, sc);
+    } else {
+        if (mode == 0) k_psi_warm<0, false><<<nb, 256, 0, s>>>(w, n, sc);
+        else if (mode == 1) k_psi_warm<1, false><<<nb, 256, 0, s>>>(w, n, sc);
+        else k_psi_warm<2, false><<<nb, 256, 0, s>>>(w, n, sc);
+    }
     return (int)cudaGetLastError();
 }
 
@@ -746,6 +764,7 @@ __global__ void k_euler_div(const T* __restrict__ ux, const T* __restrict__ uy, 
     if (j >= g.NY || i >= g.NX) return;
     const long long o = (long long)j * g.P + i;
     T d = i <= g.NX - 2 ? -(ux[o + 1] * rdx2 - ux[o] * rdx2) : dv[o];
+    constexpr int U = 2;
     if (j <= g.NY - 2) d -= uy[o + g.P] * rdy2 - uy[o] * rdy2;
     d *= (code[o] & B_MSK) ? T(1) : T(0);
     dv[o] = d;
