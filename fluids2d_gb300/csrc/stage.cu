@@ -44,6 +44,12 @@ k_fluxform_stage(const __grid_constant__ CUtensorMap tq, const T* __restrict__ q
                               blockIdx.y * 8 * FluxRows<T>::R);
 }
 
+// a constant in the kernel's precision: the conversions of three doubles per
+// thread kept k_rsw_diag<float>'s FP64 pipe 40 % busy
+template <typename T> __device__ __forceinline__ T of(double d, float f);
+template <> __device__ __forceinline__ double of<double>(double d, float) { return d; }
+template <> __device__ __forceinline__ float of<float>(double, float f) { return f; }
+
 // ---------------------------------------------------------------------------
 // Rotating shallow water right-hand side (equations.py:139-148) + RK3 update
 // of (u.x, u.y, h): vortex force (weno.vortexforce), Coriolis, gradients of
@@ -53,7 +59,7 @@ k_fluxform_stage(const __grid_constant__ CUtensorMap tq, const T* __restrict__ q
 // equations.py:29-35).
 // ---------------------------------------------------------------------------
 template <typename T, int M>
-__global__ void __launch_bounds__(TX * TY)
+__global__ void __launch_bounds__(TX * TY, sizeof(T) == 4 ? 4 : 2)
 k_rsw_stage(const __grid_constant__ CUtensorMap th,
             const __grid_constant__ CUtensorMap tw, RswIn a,
             const uint32_t* __restrict__ code, int stage, Geom g, DevScalars* sc)
@@ -71,13 +77,93 @@ k_rsw_stage(const __grid_constant__ CUtensorMap th,
     const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
     const T* __restrict__ Ux = (const T*)a.Ux;
     const T* __restrict__ Uy = (const T*)a.Uy;
+    const T* __restrict__ ke = (const T*)a.ke;
+    const T* __restrict__ p = (const T*)a.p;
+    const bool wrap = a.euler == 3 && g.xper;
 
-    if (!stage_tiles<T>(sh, &th, sw, &tw, i0, j0, &bar, &sc->status)) return;
+    // 1. the TMA copy of the tiles of h and omega ...
+    if (t == 0) {
+        mbar_init(&bar, 1);
+        mbar_expect_tx(&bar, (uint32_t)(sizeof(T) * SW * SH * 2));
+        tma_load_2d(&sh[0][0], &th, i0 - OX, j0 - OY, &bar);
+        tma_load_2d(&sw[0][0], &tw, i0 - OX, j0 - OY, &bar);
+    }
+    // 2. ... and behind it all of this thread's plain loads, in flight
+    // together: where they were used, one after the other, the kernel waited
+    // for memory half of its time (1500 x 1030 FP32: 69 us).
+    const int j = j0 + ty, i = i0 + tx;
+    const bool in = j < g.NY && i < g.NX;
+    // qgrsw's raw tendency is consumed before any halo fill (the reference
+    // forms the PV from it, operators.py:179-180): every point, halo columns
+    // included, is evaluated locally with the numpy-slice semantics
+    const bool live = in && (a.euler == 3 || periodic_owner(g, i));
+    const long long o = (long long)j * g.P + i;
+    const uint32_t cf = in ? code[o] : 0u;  // of the cell's faces
+    const uint32_t cd = live ? cf : 0u;
+    const T ux = in ? Ux[o] : T(0), uy = in ? Uy[o] : T(0);
+    auto nb = [&](const T* __restrict__ f, int jj, int ii) {
+        return !live ? T(0) : wrap ? ldw(f, jj, ii, g) : ldz(f, jj, ii, g);
+    };
+    const T uxe = nb(Ux, j, i + 1), uxs = nb(Ux, j - 1, i), uxse = nb(Ux, j - 1, i + 1);
+    const T uyn = nb(Uy, j + 1, i), uyw = nb(Uy, j, i - 1), uynw = nb(Uy, j + 1, i - 1);
+    T kc = T(0), kw = T(0), ks = T(0), pc = T(0), pw = T(0), ps = T(0);
+    if (live && a.euler != 3) {
+        kc = ke[o];
+        if (i >= 1) kw = ke[o - 1];
+        if (j >= 1) ks = ke[o - g.P];
+        if (a.euler == 0) {
+            pc = p[o];
+            if (i >= 1) pw = p[o - 1];
+            if (j >= 1) ps = p[o - g.P];
+        }
+    }
+    const bool hm = a.euler != 1;  // mass (rsw) or buoyancy (boussinesq) equation
+    const bool tend = ((sk >> 4) & 15) == INTEG_TENDENCY;
+    T qx = T(0), qy = T(0), x1 = T(0), y1 = T(0), h1 = T(0), x2 = T(0), y2 = T(0), h2 = T(0);
+    if (live && a.euler != 3 && !tend) {
+        qx = ((const T*)a.ux)[o];
+        qy = ((const T*)a.uy)[o];
+        if (stage >= 2 || lf) {
+            x1 = ((const T*)a.dux1)[o];
+            y1 = ((const T*)a.duy1)[o];
+            if (hm) h1 = ((const T*)a.dh1)[o];
+        }
+        if (stage == 3) {
+            x2 = ((const T*)a.dux2)[o];
+            y2 = ((const T*)a.duy2)[o];
+            if (hm) h2 = ((const T*)a.dh2)[o];
+        }
+    }
+    // edge face: x at (t, TX) in warp 0, y at (TY, t - 32) in warp 1
+    uint32_t ce = 0u;
+    T ue = T(0);
+    const int ex = t < TY ? 1 : (t >= 32 && t < 32 + TX) ? 2 : 0;
+    const int er = ex == 1 ? t : TY, ec = ex == 1 ? TX : t - 32;
+    if (ex && hm) {
+        const int je = j0 + er, ie = i0 + ec;
+        if (je < g.NY && ie < g.NX) {
+            const long long oe = (long long)je * g.P + ie;
+            ce = code[oe];
+            ue = ex == 1 ? Ux[oe] : Uy[oe];
+        }
+    }
+    if (t == 0) {
+        rk3_coefs<T>(sk, sc->dt, srk, sc->ragamma);
+        srk[3] = T(a.fc);
+    }
+    __syncthreads();  // the barrier's initialisation
+    {
+        const bool ok = mbar_wait(&bar, 0) && tma_wait_test(&bar);
+        const int all = __syncthreads_and(ok ? 1 : 0);
+        if (!all) {
+            if (t == 0) atomicOr(&sc->status, ST_TMA_TIMEOUT);
+            return;
+        }
+    }
     // qgrsw consumes the raw tendency of the x-periodic halo columns (its PV
     // is formed before the halo fill, operators.py:179-180), where the
     // reference's stencils over the raveled array run into the neighbouring
     // row: the edge tiles take those values in place of the out-of-array 0
-    const bool wrap = a.euler == 3 && g.xper;
     if (wrap && (i0 < OX || i0 - OX + SW > g.NX)) {
         const T* __restrict__ hg = (const T*)a.h;
         const T* __restrict__ wg = (const T*)a.w;
@@ -92,67 +178,42 @@ k_rsw_stage(const __grid_constant__ CUtensorMap th,
     }
 
     // mass fluxes U*h at the faces (compflux, weno.py:349-363)
-    auto xface = [&](int r, int c) {
-        const int j = j0 + r, i = i0 + c;
+    auto xface = [&](int r, int c, uint32_t cw, T U) {
         T f = T(0);
-        if (j < g.NY && i < g.NX) {
-            const long long o = (long long)j * g.P + i;
-            const int L = lev(code[o], SH_OCX);
-            if (L) {
-                const T U = Ux[o];
-                const T* w = &sh[r + OY][c + OX - 3];
-                f = face_value<M, T>(L, U, w[0], w[1], w[2], w[3], w[4], w[5]) * U;
-            }
+        const int L = lev(cw, SH_OCX);
+        if (L) {
+            const T* w = &sh[r + OY][c + OX - 3];
+            f = face_value<M, T>(L, U, w[0], w[1], w[2], w[3], w[4], w[5]) * U;
         }
         sfx[r][c] = f;
     };
-    auto yface = [&](int r, int c) {
-        const int j = j0 + r, i = i0 + c;
+    auto yface = [&](int r, int c, uint32_t cw, T U) {
         T f = T(0);
-        if (j < g.NY && i < g.NX) {
-            const long long o = (long long)j * g.P + i;
-            const int L = lev(code[o], SH_OCY);
-            if (L) {
-                const T U = Uy[o];
-                const int cc = c + OX;
-                f = face_value<M, T>(L, U, sh[r][cc], sh[r + 1][cc], sh[r + 2][cc],
-                                     sh[r + 3][cc], sh[r + 4][cc], sh[r + 5][cc]) *
-                    U;
-            }
+        const int L = lev(cw, SH_OCY);
+        if (L) {
+            const int cc = c + OX;
+            f = face_value<M, T>(L, U, sh[r][cc], sh[r + 1][cc], sh[r + 2][cc], sh[r + 3][cc],
+                                 sh[r + 4][cc], sh[r + 5][cc]) *
+                U;
         }
         sfy[r][c] = f;
     };
-    if (a.euler != 1) {
-        xface(ty, tx);
-        yface(ty, tx);
-        if (t < TY) xface(t, TX);
-        else if (t < TY + TX) yface(TY, t - TY);
+    if (hm) {
+        xface(ty, tx, cf, ux);
+        yface(ty, tx, cf, uy);
+        if (ex == 1) xface(er, ec, ce, ue);
+        else if (ex == 2) yface(er, ec, ce, ue);
     }
 
     // The vortex force needs no shared fluxes: it is evaluated before the
     // barrier, so warps with fewer faces above do not idle at it.
-    const int j = j0 + ty, i = i0 + tx;
-    // qgrsw's raw tendency is consumed before any halo fill (the reference
-    // forms the PV from it, operators.py:179-180): every point, halo columns
-    // included, is evaluated locally with the numpy-slice semantics
-    const bool live = j < g.NY && i < g.NX && (a.euler == 3 || periodic_owner(g, i));
-    const long long o = (long long)j * g.P + i;
-    const uint32_t cd = live ? code[o] : 0u;
-    const T* __restrict__ ke = (const T*)a.ke;
-    const T* __restrict__ p = (const T*)a.p;
-
     // du.x: vortex force along y (sign +1), weno.py:370-384 with s = row
     // length, s2 = 1: omega window rows j-2..j+3 at column i.
     T dux = T(0);
     {
         const int L = lev(cd, SH_OVY);
         if (L) {
-            const T Vm = wrap ? T(0.25) * (((Uy[o] + ldw(Uy, j + 1, i, g)) +
-                                            ldw(Uy, j, i - 1, g)) +
-                                           ldw(Uy, j + 1, i - 1, g))
-                              : T(0.25) * (((Uy[o] + ldz(Uy, j + 1, i, g)) +
-                                            ldz(Uy, j, i - 1, g)) +
-                                           ldz(Uy, j + 1, i - 1, g));
+            const T Vm = T(0.25) * (((uy + uyn) + uyw) + uynw);
             const int c = tx + OX, r = ty + OY;
             dux = face_value<M, T>(L, Vm, sw[r - 2][c], sw[r - 1][c], sw[r][c],
                                    sw[r + 1][c], sw[r + 2][c], sw[r + 3][c]) *
@@ -164,19 +225,10 @@ k_rsw_stage(const __grid_constant__ CUtensorMap th,
     {
         const int L = lev(cd, SH_OVX);
         if (L) {
-            const T Vm = wrap ? T(0.25) * (((Ux[o] + ldw(Ux, j, i + 1, g)) +
-                                            ldw(Ux, j - 1, i, g)) +
-                                           ldw(Ux, j - 1, i + 1, g))
-                              : T(0.25) * (((Ux[o] + ldz(Ux, j, i + 1, g)) +
-                                            ldz(Ux, j - 1, i, g)) +
-                                           ldz(Ux, j - 1, i + 1, g));
+            const T Vm = T(0.25) * (((ux + uxe) + uxs) + uxse);
             const T* w = &sw[ty + OY][tx + OX - 2];
             duy = -face_value<M, T>(L, Vm, w[0], w[1], w[2], w[3], w[4], w[5]) * Vm;
         }
-    }
-    if (tx == 0 && ty == 0) {
-        rk3_coefs<T>(sk, sc->dt, srk, sc->ragamma);
-        srk[3] = T(a.fc);
     }
     __syncthreads();
     if (!live) return;
@@ -187,36 +239,33 @@ k_rsw_stage(const __grid_constant__ CUtensorMap th,
     const T fc = srk[3];
     const bool cor = a.euler == 0 || a.euler == 3;
     if (cor && j <= g.NY - 2 && i >= 1 && i <= g.NX - 2)
-        dux += fc * (((ldz(Uy, j, i - 1, g) + ldz(Uy, j + 1, i - 1, g)) + Uy[o]) +
-                     ldz(Uy, j + 1, i, g));
+        dux += fc * (((uyw + uynw) + uy) + uyn);
     if (cor && j >= 1 && j <= g.NY - 2 && i <= g.NX - 2)
-        duy -= fc * (((ldz(Ux, j - 1, i, g) + ldz(Ux, j - 1, i + 1, g)) + Ux[o]) +
-                     ldz(Ux, j, i + 1, g));
+        duy -= fc * (((uxs + uxse) + ux) + uxe);
     // gradients of ke then p (addgrad, operators.py:49-56)
     if (i >= 1 && a.euler != 3) {
         const T mx = (cd & B_MSKX) ? T(1) : T(0);
-        dux -= (ke[o] - ke[o - 1]) * mx;
-        if (a.euler == 0) dux -= (p[o] - p[o - 1]) * mx;
+        dux -= (kc - kw) * mx;
+        if (a.euler == 0) dux -= (pc - pw) * mx;
     }
     if (j >= 1 && a.euler != 3) {
         const T my = (cd & B_MSKY) ? T(1) : T(0);
-        duy -= (ke[o] - ke[o - g.P]) * my;
-        if (a.euler == 0) duy -= (p[o] - p[o - g.P]) * my;
+        duy -= (kc - ks) * my;
+        if (a.euler == 0) duy -= (pc - ps) * my;
         // boussinesq buoyancy (operators.py:152-153), after the gradients
         if (a.euler == 2)
-            duy += (T(a.bdy) * (sh[ty + OY][tx + OX] + sh[ty + OY - 1][tx + OX])) * my;
+            duy += (of<T>(a.bdy, a.fbdy) * (sh[ty + OY][tx + OX] + sh[ty + OY - 1][tx + OX])) * my;
     }
     // mass: dh = -div(flux) * msk
     const T msk = (cd & B_MSK) ? T(1) : T(0);
     T dh = (-(sfx[ty][tx + 1] - sfx[ty][tx]) - (sfy[ty + 1][tx] - sfy[ty][tx])) * msk;
-    const bool hm = a.euler != 1;  // mass (rsw) or buoyancy (boussinesq) equation
     if (a.fx && a.euler != 3) {
         // the forcing term after the right-hand side (equations.py:229-238)
         dux += ((const T*)a.fx)[o];
         duy += ((const T*)a.fy)[o];
         if (hm) dh += ((const T*)a.fh)[o];
     }
-    if (((sk >> 4) & 15) == INTEG_TENDENCY && a.euler != 3) {
+    if (tend && a.euler != 3) {
         // the tendency alone, with the halo fill of the reference's rhs
         store_filled((T*)a.dux, g, j, i, dux);
         store_filled((T*)a.duy, g, j, i, duy);
@@ -239,14 +288,14 @@ k_rsw_stage(const __grid_constant__ CUtensorMap th,
         // dux.. = out (buffers alternating with the parity)
         const bool first = sc->ite == 0;
         T qn, pn;
-        lfra_update<T>(first, srk, ((const T*)a.ux)[o], ((const T*)a.dux1)[o], dux, qn, pn);
+        lfra_update<T>(first, srk, qx, x1, dux, qn, pn);
         store_filled((T*)a.uxo, g, j, i, qn);
         store_filled((T*)a.dux, g, j, i, pn);
-        lfra_update<T>(first, srk, ((const T*)a.uy)[o], ((const T*)a.duy1)[o], duy, qn, pn);
+        lfra_update<T>(first, srk, qy, y1, duy, qn, pn);
         store_filled((T*)a.uyo, g, j, i, qn);
         store_filled((T*)a.duy, g, j, i, pn);
         if (hm) {
-            lfra_update<T>(first, srk, sh[ty + OY][tx + OX], ((const T*)a.dh1)[o], dh, qn, pn);
+            lfra_update<T>(first, srk, sh[ty + OY][tx + OX], h1, dh, qn, pn);
             store_filled((T*)a.ho, g, j, i, qn);
             store_filled((T*)a.dh, g, j, i, pn);
         }
@@ -257,16 +306,16 @@ k_rsw_stage(const __grid_constant__ CUtensorMap th,
         iy = rk3_increment<T>(1, dt, duy, T(0), T(0));
         if (hm) ih = rk3_increment<T>(1, dt, dh, T(0), T(0));
     } else if (stage == 2) {
-        ix = rk3_increment<T>(2, dt, ((const T*)a.dux1)[o], dux, T(0));
-        iy = rk3_increment<T>(2, dt, ((const T*)a.duy1)[o], duy, T(0));
-        if (hm) ih = rk3_increment<T>(2, dt, ((const T*)a.dh1)[o], dh, T(0));
+        ix = rk3_increment<T>(2, dt, x1, dux, T(0));
+        iy = rk3_increment<T>(2, dt, y1, duy, T(0));
+        if (hm) ih = rk3_increment<T>(2, dt, h1, dh, T(0));
     } else {
-        ix = rk3_increment<T>(3, dt, ((const T*)a.dux1)[o], ((const T*)a.dux2)[o], dux);
-        iy = rk3_increment<T>(3, dt, ((const T*)a.duy1)[o], ((const T*)a.duy2)[o], duy);
-        if (hm) ih = rk3_increment<T>(3, dt, ((const T*)a.dh1)[o], ((const T*)a.dh2)[o], dh);
+        ix = rk3_increment<T>(3, dt, x1, x2, dux);
+        iy = rk3_increment<T>(3, dt, y1, y2, duy);
+        if (hm) ih = rk3_increment<T>(3, dt, h1, h2, dh);
     }
-    store_filled((T*)a.uxo, g, j, i, ((const T*)a.ux)[o] + ix);
-    store_filled((T*)a.uyo, g, j, i, ((const T*)a.uy)[o] + iy);
+    store_filled((T*)a.uxo, g, j, i, qx + ix);
+    store_filled((T*)a.uyo, g, j, i, qy + iy);
     if (hm) store_filled((T*)a.ho, g, j, i, sh[ty + OY][tx + OX] + ih);
     if (a.dux) {
         store_filled((T*)a.dux, g, j, i, dux);
@@ -297,12 +346,12 @@ k_rsw_diag(const __grid_constant__ CUtensorMap tux,
     if (j >= g.NY || i >= g.NX) return;
     const long long o = (long long)j * g.P + i;
     const int r = ty + OY, c = tx + OX;
-    const T rdx2 = T(a.rdx2), rdy2 = T(a.rdy2);
+    const T rdx2 = of<T>(a.rdx2, a.frdx2), rdy2 = of<T>(a.rdy2, a.frdy2);
     const T ux = sx[r][c], uy = sy[r][c];
     // sharp: U = u / dx^2 everywhere (no fill in the reference; u is filled)
     ((T*)a.Ux)[o] = ux * rdx2;
     ((T*)a.Uy)[o] = uy * rdy2;
-    if (!a.euler) ((T*)a.p)[o] = T(a.goa) * ((const T*)a.h)[o];
+    if (!a.euler) ((T*)a.p)[o] = of<T>(a.goa, a.fgoa) * ((const T*)a.h)[o];
     if (!periodic_owner(g, i)) return;  // omega and ke: halo fill copies
     const uint32_t cd = code[o];
     // vorticity: omega[1:,:] = -diff(u.x, 0); omega[:,1:] += diff(u.y, 1)
@@ -574,9 +623,11 @@ int launch_fluxform_stage(int method, int prec, const CUtensorMap* tq,
 }
 
 int launch_rsw_stage(int method, int prec, const CUtensorMap* th,
-                     const CUtensorMap* tw, const RswIn& a, const uint32_t* code,
+                     const CUtensorMap* tw, const RswIn& args, const uint32_t* code,
                      int stage, const Geom& g, DevScalars* sc, cudaStream_t s)
 {
+    RswIn a = args;
+    a.fbdy = (float)a.bdy;
     dim3 grid = tile_grid(g), block(TX, TY);
 #define F2D_RS(T, M) k_rsw_stage<T, M><<<grid, block, 0, s>>>(*th, *tw, a, code, stage, g, sc)
 #define F2D_DISPATCH(T)                                      \
@@ -593,9 +644,13 @@ int launch_rsw_stage(int method, int prec, const CUtensorMap* th,
 }
 
 int launch_rsw_diag(int method, int prec, const CUtensorMap* tux,
-                    const CUtensorMap* tuy, const RswDiag& a, const uint32_t* code,
+                    const CUtensorMap* tuy, const RswDiag& args, const uint32_t* code,
                     const Geom& g, DevScalars* sc, cudaStream_t s)
 {
+    RswDiag a = args;
+    a.frdx2 = (float)a.rdx2;
+    a.frdy2 = (float)a.rdy2;
+    a.fgoa = (float)a.goa;
     dim3 grid = tile_grid(g), block(TX, TY);
 #define F2D_RD(T, M) k_rsw_diag<T, M><<<grid, block, 0, s>>>(*tux, *tuy, a, code, g, sc)
 #define F2D_DISPATCH(T)                                      \
@@ -692,6 +747,7 @@ int launch_fill_periodic(int prec, void* a, const Geom& g, cudaStream_t s)
 template <int MODE, bool EXT>
 __global__ void __launch_bounds__(256) k_psi_warm(WarmArrays w, long long n, DevScalars* sc)
 {
+    constexpr int U = 2;
     const bool hist = sc->dt_warm > 0.0;
     const double rho = hist ? sc->dt / sc->dt_warm : 0.0;
     const long long step = 2ll * gridDim.x * blockDim.x;
@@ -764,7 +820,6 @@ __global__ void k_euler_div(const T* __restrict__ ux, const T* __restrict__ uy, 
     if (j >= g.NY || i >= g.NX) return;
     const long long o = (long long)j * g.P + i;
     T d = i <= g.NX - 2 ? -(ux[o + 1] * rdx2 - ux[o] * rdx2) : dv[o];
-    constexpr int U = 2;
     if (j <= g.NY - 2) d -= uy[o + g.P] * rdy2 - uy[o] * rdy2;
     d *= (code[o] & B_MSK) ? T(1) : T(0);
     dv[o] = d;

@@ -15,6 +15,7 @@ struct RswIn {
     const void *fx, *fy, *fh;       // forcing terms added to the tendencies (or null)
     double fc;                      // f0 * area * 0.25 (operators.py:33)
     double bdy;                     // 0.5 * dy (addbuoyancy, operators.py:152-153)
+    float fbdy;                     // the same in FP32 (set by the launcher)
     // 0 rsw; 1 euler (vortex force + grad ke only); 2 boussinesq (euler +
     // buoyancy, with the buoyancy b advected in place of h); 3 qgrsw (the
     // raw tendency of vortex force, Coriolis and mass flux into dux/duy/dh,
@@ -27,6 +28,7 @@ struct RswDiag {
     void *Ux, *Uy, *omega, *ke, *p;
     double rdx2, rdy2;  // 1/dx**2, 1/dy**2 (operators.py:62-63)
     double goa;         // g/area (operators.py:111)
+    float frdx2, frdy2, fgoa;  // the same in FP32 (set by the launcher)
     int euler;          // euler model: no pressure from h
     int noke;           // qgrsw: no kinetic energy (equations.py:127-133)
 };
@@ -58,93 +60,122 @@ int launch_set_dt(DevScalars* sc, cudaStream_t s);
 // 2dt/3 L3 (integrators.py:92-107, L_k the tendency at the stage's input),
 // and psi solves a linear problem in y, so with S_k = dt A^-1 B(L_k):
 // psi1 = psi0 + S1, psi2 = psi0 + (S1 + S2)/4. The guesses extrapolate the
-// S_k, not psi: S1 (the tendency at t) ~ the previous step's S2 (taken at
-// y1 ~ y(t)); S2 (at y1 ~ t+dt) ~ S1 + the previous step's S2 - S1; S3 (at
-// y2 ~ t+dt/2) ~ (S1 + S2)/2. The previous step's increments are kept as
-// d1 = 4 psi2 - 3 psi0 - psi1 = S2 and d2 = 4 psi2 - 2 psi0 - 2 psi1 = S2 - S1,
-// scaled by dt / dt_warm when the step size changed. On eulerpsi 128^2
-// (the oracle's operator) the starting relative residuals of stages 1 and
-// 2 fall from 3.8e-4 and 1.9e-4 (linear extrapolation of psi itself) to
-// 3.2e-5 and 2.0e-5; stage 3's guess, 2 psi2 - psi0, is the same in both
-// (1.3e-5). A guess only moves the solve's starting point.
+// S_k, not psi, from the relations of the previous step (primes: its values,
+// scaled by dt / dt_warm when the step size changed):
+//   S1 (the tendency at t)       ~ S2' + (S1' - S2'')          (S2' at y1' ~ y(t))
+//   S2 (at y1 ~ t + dt)          ~ S1 + D' + (D' - D''), D = S2 - S1
+//   S3 (at y2 ~ t + dt/2)        ~ (S1 + S2)/2 + (S3' - (S1' + S2')/2)
+// with S3 = 1.5 (psi3 - psi0) - (S1 + S2)/4. The terms in brackets, kept as
+// e1, e2, e3 (0 until the steps they need are there), change slowly: on
+// eulerpsi 128^2 they cut the starting relative residuals from 1.3e-5, 7e-6
+// and 4.4e-6 to 1.7e-6, 9e-7 and 5.5e-7, on qg 128^2 turbulence from 1.3e-3,
+// 7.5e-4 and 4.7e-4 to 5.6e-4, 5.6e-4 and 3.2e-4. Where the increments of a
+// step come down to the FP32 rounding of the state (psi_warm_brackets) the
+// brackets are noise and left out. A guess only moves the solve's starting
+// point.
 struct WarmArrays {
     double* psi;  // in: the last solution; out: the guess
     double* s0;   // psi at the step start
     double* p1;   // psi of stage 1
-    double* d1;   // the previous step's increments (see above)
-    double* d2;
+    double* d1;   // the previous step's S2
+    double* d2;   // the previous step's D = S2 - S1
+    double *e1, *e2, *e3;  // the brackets, or null
 };
-
-// The arrays do not overlap; every load of a point is issued before its
-// stores (a store ahead of a load through another pointer would hold the
-// load back until the store's address is known not to alias it).
-__device__ __forceinline__ void psi_warm_point(int mode, const WarmArrays& w, long long k,
-                                               bool hist, double rho)
+// whether a model keeps the brackets: FP64 states always, FP32 ones up to 3M
+// points. (A CFL step's change shrinks with the grid spacing, its rounding
+// does not. FP32 CG iterations per solve without and with them: 9.67 and 8.36
+// on the 256-member ensemble of 64^2 .. 512^2, 8.33 and 8.64 on qg 4096^2;
+// 2048^2 gains what the extra arrays cost.)
+inline bool psi_warm_brackets(int prec, long long points)
 {
-    const double a = w.psi[k];
-    if (mode == 0) {  // a = psi0
-        const double d1 = hist ? w.d1[k] : 0.0;
-        w.s0[k] = a;
-        if (hist) w.psi[k] = a + rho * d1;
-    } else if (mode == 1) {  // a = psi1
-        const double s0 = w.s0[k];
-        const double d2 = hist ? w.d2[k] : 0.0;
-        w.p1[k] = a;
-        double g = s0 + 0.5 * (a - s0);
-        if (hist) g += 0.25 * rho * d2;
-        w.psi[k] = g;
-    } else {  // a = psi2
-        const double s0 = w.s0[k], p1 = w.p1[k];
-        w.d1[k] = (4.0 * a - 3.0 * s0) - p1;
-        w.d2[k] = (4.0 * a - 2.0 * s0) - 2.0 * p1;
-        w.psi[k] = 2.0 * a - s0;
-    }
+    return prec == 0 || points <= 3000000ll;
 }
 
-// psi_warm_point on U pairs of elements (k, k+1), k even and every array
-// 16-byte aligned there: 16-byte loads and stores, all the loads of the U
-// pairs before any store. ok[u] false skips pair u.
-template <int U>
-__device__ __forceinline__ void psi_warm_pairs(int mode, const WarmArrays& w,
-                                               const long long (&k)[U], const bool (&ok)[U],
-                                               bool hist, double rho)
+// U pairs of elements (k, k + 1), k even and every array 16-byte aligned
+// there: 16-byte loads and stores, all the loads of the U pairs before any
+// store (the arrays do not overlap, but a store ahead of a load through
+// another pointer would hold the load back). ok[u] false skips pair u. hist:
+// there is a previous step, of dt / rho. The large grids are bound by the FP64
+// pipe here too, so the mode and the brackets (EXT) are compile-time.
+// e3 holds t3 = 1.5 psi0 + 0.75 (S1 + S2) of the step between its stages 2
+// and 3 (S3 - (S1 + S2)/2 = 1.5 psi3 - t3).
+template <int MODE, bool EXT, int U>
+__device__ __forceinline__ void psi_warm_pairs(const WarmArrays& w, const long long (&k)[U],
+                                               const bool (&ok)[U], bool hist, double rho)
 {
-    double2 a[U], s0[U], p1[U], d[U];
+    double2 a[U], s0[U], p1[U], d1[U], d2[U], e[U], t3[U];
+    const double* ein = MODE == 0 ? w.e1 : MODE == 1 ? w.e2 : w.e3;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const double2 z = make_double2(0.0, 0.0);
+        const bool h = ok[u] && hist;
         a[u] = ok[u] ? *(const double2*)(w.psi + k[u]) : z;
-        s0[u] = ok[u] && mode >= 1 ? *(const double2*)(w.s0 + k[u]) : z;
-        p1[u] = ok[u] && mode == 2 ? *(const double2*)(w.p1 + k[u]) : z;
-        d[u] = ok[u] && mode == 0 && hist ? *(const double2*)(w.d1 + k[u])
-             : (ok[u] && mode == 1 && hist ? *(const double2*)(w.d2 + k[u]) : z);
+        s0[u] = MODE >= 1 && ok[u] ? *(const double2*)(w.s0 + k[u]) : z;
+        p1[u] = MODE == 2 && ok[u] ? *(const double2*)(w.p1 + k[u]) : z;
+        d1[u] = (MODE == 0 || (MODE == 1 && EXT)) && h ? *(const double2*)(w.d1 + k[u]) : z;
+        d2[u] = (MODE == 1 || (MODE == 2 && EXT)) && h ? *(const double2*)(w.d2 + k[u]) : z;
+        e[u] = EXT && h ? *(const double2*)(ein + k[u]) : z;
+        t3[u] = EXT && MODE == 0 && h ? *(const double2*)(w.e3 + k[u]) : z;
     }
+    const double rq = 0.25 * rho, r23 = rho * (2.0 / 3.0);
+    // one element: the guess g, the bracket en, mode 2: S2, D and t3
+    auto one = [&](double A, double S, double P, double D1, double D2, double E, double T3,
+                   double& g, double& en, double& n1, double& n2, double& n3) {
+        if constexpr (MODE == 0) {  // A = psi0, psi3 of the previous step
+            if constexpr (EXT) {
+                en = fma(1.5, A, -T3);
+                D1 += E;
+            }
+            g = fma(rho, D1, A);
+        } else if constexpr (MODE == 1) {  // A = psi1
+            const double S1 = A - S;
+            if constexpr (EXT) {
+                en = fma(-rho, D1, S1);
+                D2 += E;
+            }
+            g = S + fma(rq, D2, 0.5 * S1);
+        } else {  // A = psi2
+            const double t = A - S, S1 = P - S;
+            n1 = fma(4.0, t, -S1);
+            n2 = n1 - S1;
+            g = A + t;
+            if constexpr (EXT) {
+                en = fma(-rho, D2, n2);
+                g = fma(r23, E, g);
+                n3 = fma(1.5, S, 0.75 * (S1 + n1));
+            }
+        }
+    };
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         if (!ok[u]) continue;
-        const double2 A = a[u], S = s0[u], P = p1[u], D = d[u];
-        if (mode == 0) {
-            *(double2*)(w.s0 + k[u]) = A;
-            if (hist) *(double2*)(w.psi + k[u]) = make_double2(A.x + rho * D.x, A.y + rho * D.y);
-        } else if (mode == 1) {
-            *(double2*)(w.p1 + k[u]) = A;
-            double gx = S.x + 0.5 * (A.x - S.x), gy = S.y + 0.5 * (A.y - S.y);
-            if (hist) {
-                gx += 0.25 * rho * D.x;
-                gy += 0.25 * rho * D.y;
-            }
-            *(double2*)(w.psi + k[u]) = make_double2(gx, gy);
+        double2 g, en, n1, n2, n3;
+        one(a[u].x, s0[u].x, p1[u].x, d1[u].x, d2[u].x, e[u].x, t3[u].x, g.x, en.x, n1.x, n2.x,
+            n3.x);
+        one(a[u].y, s0[u].y, p1[u].y, d1[u].y, d2[u].y, e[u].y, t3[u].y, g.y, en.y, n1.y, n2.y,
+            n3.y);
+        if (!hist) en = make_double2(0.0, 0.0);
+        if constexpr (MODE == 0) {
+            *(double2*)(w.s0 + k[u]) = a[u];
+            if (hist) *(double2*)(w.psi + k[u]) = g;
+            if constexpr (EXT) *(double2*)(w.e3 + k[u]) = en;
+        } else if constexpr (MODE == 1) {
+            *(double2*)(w.p1 + k[u]) = a[u];
+            *(double2*)(w.psi + k[u]) = g;
+            if constexpr (EXT) *(double2*)(w.e1 + k[u]) = en;
         } else {
-            *(double2*)(w.d1 + k[u]) = make_double2((4.0 * A.x - 3.0 * S.x) - P.x,
-                                                    (4.0 * A.y - 3.0 * S.y) - P.y);
-            *(double2*)(w.d2 + k[u]) = make_double2((4.0 * A.x - 2.0 * S.x) - 2.0 * P.x,
-                                                    (4.0 * A.y - 2.0 * S.y) - 2.0 * P.y);
-            *(double2*)(w.psi + k[u]) = make_double2(2.0 * A.x - S.x, 2.0 * A.y - S.y);
+            *(double2*)(w.d1 + k[u]) = n1;
+            *(double2*)(w.d2 + k[u]) = n2;
+            *(double2*)(w.psi + k[u]) = g;
+            if constexpr (EXT) {
+                *(double2*)(w.e2 + k[u]) = en;
+                *(double2*)(w.e3 + k[u]) = n3;
+            }
         }
     }
 }
 
-// the single-model form over n elements (every point; non-fluid points
+// the single-model form over n elements, n even (every point; non-fluid points
 // stay 0); mode 2 records dt_warm
 int launch_psi_warm(int mode, const WarmArrays& w, long long n, DevScalars* sc,
                     cudaStream_t s);
