@@ -10,6 +10,8 @@ namespace f2d {
 // fsz elements per slot, the forward precision)
 int launch_adj_snap(int prec, const void* w, const void* ux, const void* uy, void* arena,
                     long long fsz, const int* slot, cudaStream_t s);
+int launch_adj_guess(double* x, double* p, double* q, long long n, const int* hist,
+                     cudaStream_t s);
 int launch_adj_slot(int* slot, int delta, cudaStream_t s);
 // the per-stage streamfunction cache: store (store != 0) cache[*slot] = psi
 // or restore psi = cache[*slot]

@@ -93,10 +93,12 @@ struct AdjState {
     int* slot = nullptr;
     double *yb = nullptr, *d1 = nullptr, *d2 = nullptr, *d3 = nullptr;
     double *gx = nullptr, *gy = nullptr, *ubx = nullptr, *uby = nullptr;
-    // psib: the adjoint Poisson right-hand side; rbs[k]: the adjoint solve's
-    // solution for RK3 stage k+1, kept per stage so that each adjoint solve
-    // starts from the same stage's solution of the step after it
-    double *psib = nullptr, *rbs[3] = {nullptr, nullptr, nullptr};
+    // psib: the adjoint Poisson right-hand side; rbs[k][0]: the adjoint solve's
+    // solution for RK3 stage k+1; [1], [2]: those of the two steps solved
+    // before it, from which the next solve's starting point is extrapolated;
+    // hist: how many steps are solved
+    double *psib = nullptr, *rbs[3][3] = {};
+    int* hist = nullptr;
     // the forward's streamfunction after every stage (slot 3n + k after
     // stage k of step n, slot 0 after the initial diagnostics), so that the
     // recompute of a segment needs no Poisson solve; used when it fits
@@ -838,10 +840,12 @@ static int rec_adj_vjp(f2d_model_s* m, int soff, const double* db, cudaStream_t 
     CKI(launch_adj_vjp_pre(m->p.compflux, m->prec, g, m->d_code, a.arena, fsz, a.slot, soff, db,
                            a.gx, a.gy, a.ubx, a.uby, m->rdx2, m->rdy2, a.psib, s));
     m->rec_launches += 2;
-    int e = rec_solve(m, 0, a.psib, a.rbs[soff], s);
+    double** x = a.rbs[soff];
+    CKI(launch_adj_guess(x[0], x[1], x[2], fsz, a.hist, s));
+    int e = rec_solve(m, 0, a.psib, x[0], s);
     if (e) return e;
-    CKI(launch_adj_vjp_post(g, m->d_code, a.gx, a.gy, fsz, a.rbs[soff], a.yb, s));
-    m->rec_launches += 1;
+    CKI(launch_adj_vjp_post(g, m->d_code, a.gx, a.gy, fsz, x[0], a.yb, s));
+    m->rec_launches += 2;
     return 0;
 }
 
@@ -863,7 +867,10 @@ static int rec_adj_step(f2d_model_s* m, cudaStream_t s)
     if (e) return e;
     CKI(launch_adj_comb(g, a.yb, a.d1, a.d2, a.d3, 2, dt, 0, 0, s));
     m->rec_launches += 1;
-    return rec_adj_vjp(m, 0, a.d1, s);
+    if ((e = rec_adj_vjp(m, 0, a.d1, s))) return e;
+    CKI(launch_adj_slot(a.hist, 1, s));
+    m->rec_launches += 1;
+    return 0;
 }
 
 // F2D_EAGER=1 runs every recorded sequence directly on the stream (the
@@ -1941,10 +1948,13 @@ int f2d_adjoint_forward(f2d_model m, const double* w0, double* wT, int nsteps, d
     const Geom& g = m->g;
     const size_t fb64 = field_bytes(m, 8), fbs = field_bytes(m, m->es);
     if (!a.yb) {
-        double** v[] = {&a.yb, &a.d1, &a.d2, &a.d3, &a.ubx, &a.uby, &a.psib,
-                        &a.rbs[0], &a.rbs[1], &a.rbs[2]};
+        double** v[] = {&a.yb, &a.d1, &a.d2, &a.d3, &a.ubx, &a.uby, &a.psib};
         for (double** p : v)
             if (!(*p = (double*)dalloc(m, fb64))) return fail(2, "out of device memory");
+        for (auto& r : a.rbs)
+            for (double*& p : r)
+                if (!(p = (double*)dalloc(m, fb64))) return fail(2, "out of device memory");
+        if (!(a.hist = (int*)dalloc(m, 256))) return fail(2, "out of device memory");
         a.gx = (double*)dalloc(m, 6 * fb64);
         a.gy = (double*)dalloc(m, 6 * fb64);
         a.slot = (int*)dalloc(m, 256);
@@ -2038,7 +2048,9 @@ int f2d_adjoint_backward(f2d_model m, const double* lamT, double* lam0)
     const size_t fbs = field_bytes(m, m->es);
     CK(cudaMemcpy2DAsync(a.yb, g.P * 8, lamT, g.NX * 8, g.NX * 8, g.NY,
                          cudaMemcpyDeviceToDevice, m->stream));
-    for (double* r : a.rbs) CK(cudaMemsetAsync(r, 0, field_bytes(m, 8), m->stream));
+    for (auto& r : a.rbs)
+        for (double* x : r) CK(cudaMemsetAsync(x, 0, field_bytes(m, 8), m->stream));
+    CK(cudaMemsetAsync(a.hist, 0, sizeof(int), m->stream));
     // the time step of the forward run (the model's dt may have changed)
     m->dt_const = a.dt;
     CK(cudaMemcpyAsync(&m->sc->dt, &m->dt_const, 8, cudaMemcpyHostToDevice, m->stream));
