@@ -680,6 +680,13 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
         else n_dense_a<S>(A, it, c.alpha, c.beta, t);
         if (it > 0) ps_block_total<2>(t, pr + blockIdx.x, G);
         if (!ps_sync(g)) return;
+        if (A.ng == 0 && it > 0) {
+            // no level leg to hide the decision behind, and the phase that
+            // would be lost is the whole solve: decide first
+            if (threadIdx.x >= 32) decide();
+            __syncthreads();
+            if (c.done) break;
+        }
         for (int l = 1; l < A.ng; ++l) {
             n_down<S>(A, l, smem, T);
             if (!(l == 1 ? ps_sync(g, decide) : ps_sync(g))) return;
@@ -688,7 +695,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
         if (c.done) break;
         const NLevel& D = A.lev[A.ng];
         ps_dense<S>(mrows, (const S*)D.b, (S*)D.x, A.nd, d0, d1, (S*)smem, box);
-        if (!(A.ng <= 1 ? ps_sync(g, decide) : ps_sync(g))) return;
+        if (!(A.ng == 1 ? ps_sync(g, decide) : ps_sync(g))) return;
         if (c.done) break;
         for (int l = A.ng - 1; l >= 1; --l) {
             n_up<S>(A, l, smem, T);

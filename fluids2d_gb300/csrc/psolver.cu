@@ -715,6 +715,14 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
             if (single && slot[0].conv) break;
         }
         if (single && slot[0].conv) break;
+        if (A.dense0 && single && it > 0) {
+            // no level leg to hide the decision behind, and the phase that
+            // would be lost is the whole solve: decide first
+            if (w > 0) decide();
+            __syncthreads();
+            if (slot[0].conv) break;
+            told = true;
+        }
         p_dense<S>(A, smem);
         if (!(told ? ps_sync(g, refresh) : ps_sync(g, decide))) return;
         if (single && slot[0].conv) break;
