@@ -341,16 +341,20 @@ static int rec_solve(f2d_model_s* m, int which, const void* b, void* x, cudaStre
 static int rec_warm(f2d_model_s* m, int warm, cudaStream_t s)
 {
     if (warm < 0) return 0;
+    const std::string x = projected(m->p.model) ? "p" : "psi";
+    auto f = [&](const char* n) { return (double*)fb(m, (x + n).c_str()); };
     WarmArrays w;
-    w.psi = (double*)fb(m, "psi");
-    w.s0 = (double*)fb(m, "psi.s0");
-    w.p1 = (double*)fb(m, "psi.p1");
-    w.d1 = (double*)fb(m, "psi.d1");
-    w.d2 = (double*)fb(m, "psi.d2");
-    w.e1 = (double*)fb(m, "psi.e1");
-    w.e2 = (double*)fb(m, "psi.e2");
-    w.e3 = (double*)fb(m, "psi.e3");
-    CKI(launch_psi_warm(warm, w, (long long)m->g.P * m->g.NY, m->sc, s));
+    w.psi = f("");
+    w.s0 = f(".s0");
+    w.p1 = f(".p1");
+    w.d1 = f(".d1");
+    w.d2 = f(".d2");
+    w.e1 = f(".e1");
+    w.e2 = f(".e2");
+    w.e3 = f(".e3");
+    const long long n = (long long)m->g.P * m->g.NY;
+    if (projected(m->p.model)) CKI(launch_p_warm(warm, w, m->d_code, n, m->sc, s));
+    else CKI(launch_psi_warm(warm, w, n, m->sc, s));
     m->rec_launches += 1;
     return 0;
 }
@@ -394,6 +398,7 @@ static int rec_diag(f2d_model_s* m, int par, cudaStream_t s, int warm = -1)
                              m->nrhs, m->d_code, m->rdx2, m->rdy2, m->area, g, s));
         int e = ensure_ns(m);
         if (e) return e;
+        if ((e = rec_warm(m, warm, s))) return e;
         int fixed = 0;
         CKI(ns_record(m->ns, s, &fixed));
         if (g.xper) CKI(launch_fill_periodic(0, fb(m, "p"), g, s));
@@ -724,7 +729,8 @@ static int rec_stage(f2d_model_s* m, int k, int par, cudaStream_t s)
     int e = launch_stage_kernel(m, k, par, s);
     if (e) return e;
     const bool warm = m->p.integrator == F2D_INTEG_RK3 &&
-                      (m->p.model == F2D_MODEL_EULERPSI || m->p.model == F2D_MODEL_QG);
+                      (m->p.model == F2D_MODEL_EULERPSI || m->p.model == F2D_MODEL_QG ||
+                       (projected(m->p.model) && m->prec == 0));
     return rec_diag(m, 1 - par, s, warm ? k - 1 : -1);
 }
 
@@ -1211,6 +1217,9 @@ int f2d_model_create(const f2d_params* p, const int8_t* msk, f2d_model* out)
             if ((f[4] != 'e' || psi_warm_brackets(m->prec, (long long)m->g.P * m->g.NY)) &&
                 (e = add_field(m, f, false, 8)))
                 return bail(e);
+    if (projected(p->model) && m->prec == 0)
+        for (const char* f : {"p.s0", "p.d1", "p.d2", "p.e1", "p.e2", "p.e3"})
+            if ((e = add_field(m, f, false, 8))) return bail(e);
     // qgrsw keeps the third stage's (or LFRA's) tendency too: it is
     // projected between the tendency kernel and the update
     for (const char* f : prog) m->prog.push_back(f);

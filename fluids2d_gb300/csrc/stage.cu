@@ -780,6 +780,51 @@ int launch_psi_warm(int mode, const WarmArrays& w, long long n, DevScalars* sc, 
     return (int)cudaGetLastError();
 }
 
+// Warm start of the pressure solves (launch_p_warm) at the fluid cells: the
+// others are never solved for.
+template <int MODE>
+__global__ void __launch_bounds__(256) k_p_warm(WarmArrays w, const uint32_t* __restrict__ code,
+                                                long long n, DevScalars* sc)
+{
+    const bool hist = sc->dt_warm > 0.0;
+    const double rho = hist ? sc->dt / sc->dt_warm : 0.0;
+    const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (k < n && (code[k] & B_MSK)) {
+        const double p = w.psi[k];
+        if constexpr (MODE == 0) {
+            if (hist) {
+                const double S2 = w.d1[k];
+                const double e3 = fma(1.5, p, -0.375 * (w.s0[k] + S2));
+                w.psi[k] = rho * (S2 + w.e1[k]);
+                w.e3[k] = e3;
+            }
+        } else if constexpr (MODE == 1) {
+            const double d1 = w.d1[k], d2 = w.d2[k], e2 = w.e2[k];
+            w.s0[k] = p;
+            w.e1[k] = hist ? fma(-rho, d1, p) : 0.0;
+            w.psi[k] = fma(0.25 * rho, d2 + e2, -0.5 * p);
+        } else {
+            const double S1 = w.s0[k], d2 = w.d2[k], e3 = w.e3[k];
+            const double S2 = fma(4.0, p, 3.0 * S1), D = S2 - S1;
+            w.d1[k] = S2;
+            w.d2[k] = D;
+            w.e2[k] = hist ? fma(-rho, d2, D) : 0.0;
+            w.psi[k] = fma(rho * (2.0 / 3.0), e3, 0.25 * (S1 + S2));
+        }
+    }
+    if (MODE == 2 && k == 0) sc->dt_warm = sc->dt;
+}
+
+int launch_p_warm(int mode, const WarmArrays& w, const uint32_t* code, long long n,
+                  DevScalars* sc, cudaStream_t s)
+{
+    const unsigned nb = (unsigned)((n + 255) / 256);
+    if (mode == 0) k_p_warm<0><<<nb, 256, 0, s>>>(w, code, n, sc);
+    else if (mode == 1) k_p_warm<1><<<nb, 256, 0, s>>>(w, code, n, sc);
+    else k_p_warm<2><<<nb, 256, 0, s>>>(w, code, n, sc);
+    return (int)cudaGetLastError();
+}
+
 // the TMA wait test switch of this translation unit's stage kernels
 int tma_wait_test_set_stage(int enabled, unsigned long long limit_ns)
 {

@@ -179,6 +179,19 @@ __device__ __forceinline__ void psi_warm_pairs(const WarmArrays& w, const long l
 // stay 0); mode 2 records dt_warm
 int launch_psi_warm(int mode, const WarmArrays& w, long long n, DevScalars* sc,
                     cudaStream_t s);
+
+// Warm start of the pressure solve of RK3 stage mode+1 (euler and boussinesq,
+// FP64 states). The stages add -3/4 L1 + 1/4 L2 and so on of the unprojected
+// tendencies, so with Q_k the pressure of L_k and S_k = dt Q_k the three solves
+// give p1 = S1, p2 = (S2 - 3 S1)/4 and p3 = 2/3 S3 - (S1 + S2)/12, whose signs
+// alternate: the previous solution is no better a start than zero. The S_k are
+// extrapolated like those of psi above (s0 holds S1, d1 S2, d2 S2 - S1, e1 to
+// e3 the brackets, p1 is not used). CG iterations per solve, euler 512^2 with
+// the previous solution and with this: 9.0 and 6.9. FP32 states keep the
+// former: their velocities round differently wherever the pressure moves by
+// the solve's tolerance.
+int launch_p_warm(int mode, const WarmArrays& w, const uint32_t* code, long long n,
+                  DevScalars* sc, cudaStream_t s);
 // the failure-detection test switch of the stage kernels' TMA waits, one per
 // translation unit (stage.cu, ensemble.cu)
 int tma_wait_test_set_stage(int enabled, unsigned long long limit_ns);
