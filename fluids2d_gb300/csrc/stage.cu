@@ -20,6 +20,7 @@
 // [3,6) and [nx,nx+3) also write the copies, so no separate fill pass runs.
 #include <algorithm>
 
+#include "persist.cuh"
 #include "stage.cuh"
 #include "stage_dev.cuh"
 
@@ -28,8 +29,8 @@ namespace f2d {
 // ---------------------------------------------------------------------------
 // Flux-form stage kernel of one model (tile = block index).
 // ---------------------------------------------------------------------------
-template <typename T, int M>
-__global__ void __launch_bounds__(TX * TY, sizeof(T) == 4 ? 5 : 3)
+template <typename T, int M, int TYK>
+__global__ void __launch_bounds__(TX * TYK, sizeof(T) == 4 ? 5 : 3)
 k_fluxform_stage(const __grid_constant__ CUtensorMap tq, const T* __restrict__ qin,
                  T* __restrict__ qout, const T* __restrict__ Ux,
                  const T* __restrict__ Uy, const uint32_t* __restrict__ code,
@@ -37,11 +38,11 @@ k_fluxform_stage(const __grid_constant__ CUtensorMap tq, const T* __restrict__ q
                  const T* __restrict__ ds2, const T* __restrict__ frc, int stage, Geom g,
                  DevScalars* sc)
 {
-    __shared__ FluxformSmem<T, M> sm;
+    __shared__ FluxformSmem<T, M, TYK> sm;
     if (((stage >> 4) & 15) == 3 && sc->ite == 0) stage |= 256;  // first LFRA step
-    fluxform_tile<T, M, true>(sm, &tq, qin, qout, Ux, Uy, code, ds_out, ds1, ds2, frc, stage,
+    fluxform_tile<T, M, true, TYK>(sm, &tq, qin, qout, Ux, Uy, code, ds_out, ds1, ds2, frc, stage,
                               g, sc->dt, sc->ragamma, &sc->status, blockIdx.x * TX,
-                              blockIdx.y * 8 * FluxRows<T>::R);
+                              blockIdx.y * TYK * FluxRows<T>::R);
 }
 
 // a constant in the kernel's precision: the conversions of three doubles per
@@ -58,23 +59,23 @@ template <> __device__ __forceinline__ float of<float>(double, float f) { return
 // (euler + buoyancy, with the flux divergence of b in place of h,
 // equations.py:29-35).
 // ---------------------------------------------------------------------------
-template <typename T, int M>
-__global__ void __launch_bounds__(TX * TY, sizeof(T) == 4 ? 4 : 2)
+template <typename T, int M, int TYK>
+__global__ void __launch_bounds__(TX * TYK, sizeof(T) == 4 ? 4 : 2)
 k_rsw_stage(const __grid_constant__ CUtensorMap th,
             const __grid_constant__ CUtensorMap tw, RswIn a,
             const uint32_t* __restrict__ code, int stage, Geom g, DevScalars* sc)
 {
     __shared__ alignas(128) T sh[SH][SW];
     __shared__ alignas(128) T sw[SH][SW];
-    __shared__ T sfx[TY][TX + 1];
-    __shared__ T sfy[TY + 1][TX];
+    __shared__ T sfx[TYK][TX + 1];
+    __shared__ T sfy[TYK + 1][TX];
     __shared__ T srk[4];  // RK3 coefficients, Coriolis parameter
     __shared__ uint64_t bar;
     const int sk = stage;  // stage | integrator << 4
     const bool lf = ((sk >> 4) & 15) == 3;
     stage &= 15;
     const int tx = threadIdx.x, ty = threadIdx.y, t = ty * TX + tx;
-    const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
+    const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TYK;
     const T* __restrict__ Ux = (const T*)a.Ux;
     const T* __restrict__ Uy = (const T*)a.Uy;
     const T* __restrict__ ke = (const T*)a.ke;
@@ -134,11 +135,11 @@ k_rsw_stage(const __grid_constant__ CUtensorMap th,
             if (hm) h2 = ((const T*)a.dh2)[o];
         }
     }
-    // edge face: x at (t, TX) in warp 0, y at (TY, t - 32) in warp 1
+    // edge face: x at (t, TX) in warp 0, y at (TYK, t - 32) in warp 1
     uint32_t ce = 0u;
     T ue = T(0);
-    const int ex = t < TY ? 1 : (t >= 32 && t < 32 + TX) ? 2 : 0;
-    const int er = ex == 1 ? t : TY, ec = ex == 1 ? TX : t - 32;
+    const int ex = t < TYK ? 1 : (t >= 32 && t < 32 + TX) ? 2 : 0;
+    const int er = ex == 1 ? t : TYK, ec = ex == 1 ? TX : t - 32;
     if (ex && hm) {
         const int je = j0 + er, ie = i0 + ec;
         if (je < g.NY && ie < g.NX) {
@@ -167,7 +168,7 @@ k_rsw_stage(const __grid_constant__ CUtensorMap th,
     if (wrap && (i0 < OX || i0 - OX + SW > g.NX)) {
         const T* __restrict__ hg = (const T*)a.h;
         const T* __restrict__ wg = (const T*)a.w;
-        for (int e = t; e < SH * SW; e += TX * TY) {
+        for (int e = t; e < SH * SW; e += TX * TYK) {
             const int r = e / SW, c = e % SW;
             const int gj = j0 - OY + r, gi = i0 - OX + c;
             if (gi >= 0 && gi < g.NX) continue;
@@ -329,8 +330,8 @@ k_rsw_stage(const __grid_constant__ CUtensorMap th,
 // (times slip coefficient), WENO kinetic energy, pressure; omega and ke get
 // the halo fill.
 // ---------------------------------------------------------------------------
-template <typename T, int M>
-__global__ void __launch_bounds__(TX * TY)
+template <typename T, int M, int TYK>
+__global__ void __launch_bounds__(TX * TYK)
 k_rsw_diag(const __grid_constant__ CUtensorMap tux,
            const __grid_constant__ CUtensorMap tuy, RswDiag a,
            const uint32_t* __restrict__ code, Geom g, DevScalars* sc)
@@ -339,7 +340,7 @@ k_rsw_diag(const __grid_constant__ CUtensorMap tux,
     __shared__ alignas(128) T sy[SH][SW];
     __shared__ uint64_t bar;
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
+    const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TYK;
     if (!stage_tiles<T>(sx, &tux, sy, &tuy, i0, j0, &bar, &sc->status)) return;
 
     const int j = j0 + ty, i = i0 + tx;
@@ -587,14 +588,16 @@ __global__ void k_pushforward(DevScalars* sc)
 // ---------------------------------------------------------------------------
 // Host-side launchers
 // ---------------------------------------------------------------------------
-static dim3 tile_grid(const Geom& g)
-{
-    return dim3((g.NX + TX - 1) / TX, (g.NY + TY - 1) / TY);
-}
-
-static dim3 ftile_grid(const Geom& g, int rows)
+static dim3 tile_grid(const Geom& g, int rows)
 {
     return dim3((g.NX + TX - 1) / TX, (g.NY + rows - 1) / rows);
+}
+
+// rows of threads of the stage kernels (TYS, stage_dev.cuh)
+static int stage_rows(int prec, const Geom& g)
+{
+    const dim3 n = tile_grid(g, TY);
+    return prec == 0 && (int)(n.x * n.y) <= ps_sms() ? TYS : TY;
 }
 
 int launch_fluxform_stage(int method, int prec, const CUtensorMap* tq,
@@ -603,20 +606,23 @@ int launch_fluxform_stage(int method, int prec, const CUtensorMap* tq,
                           const void* ds1, const void* ds2, const void* frc, int stage,
                           const Geom& g, DevScalars* sc, cudaStream_t s)
 {
-    const int rows = 8 * (prec == 0 ? FluxRows<double>::R : FluxRows<float>::R);
-    dim3 grid = ftile_grid(g, rows), block(TX, TY);
-#define F2D_FF(T, M)                                                              \
-    k_fluxform_stage<T, M><<<grid, block, 0, s>>>(                                \
+    const int ty = stage_rows(prec, g);
+    dim3 grid = tile_grid(g, ty * (prec == 0 ? FluxRows<double>::R : FluxRows<float>::R));
+    dim3 block(TX, ty);
+#define F2D_FF(T, M, TYK)                                                         \
+    k_fluxform_stage<T, M, TYK><<<grid, block, 0, s>>>(                           \
         *tq, (const T*)qin, (T*)qout, (const T*)Ux, (const T*)Uy, code, (T*)ds_out, \
         (const T*)ds1, (const T*)ds2, (const T*)frc, stage, g, sc)
-#define F2D_DISPATCH(T)                                                  \
-    switch (method) {                                                    \
-    case METHOD_WENO: F2D_FF(T, METHOD_WENO); break;                     \
-    case METHOD_UPWIND: F2D_FF(T, METHOD_UPWIND); break;                 \
-    case METHOD_CENTERED: F2D_FF(T, METHOD_CENTERED); break;             \
-    default: F2D_FF(T, METHOD_CWENO); break;                             \
+#define F2D_DISPATCH(T, TYK)                                      \
+    switch (method) {                                             \
+    case METHOD_WENO: F2D_FF(T, METHOD_WENO, TYK); break;         \
+    case METHOD_UPWIND: F2D_FF(T, METHOD_UPWIND, TYK); break;     \
+    case METHOD_CENTERED: F2D_FF(T, METHOD_CENTERED, TYK); break; \
+    default: F2D_FF(T, METHOD_CWENO, TYK); break;                 \
     }
-    if (prec == 0) { F2D_DISPATCH(double) } else { F2D_DISPATCH(float) }
+    if (prec != 0) { F2D_DISPATCH(float, TY) }
+    else if (ty == TY) { F2D_DISPATCH(double, TY) }
+    else { F2D_DISPATCH(double, TYS) }
 #undef F2D_DISPATCH
 #undef F2D_FF
     return (int)cudaGetLastError();
@@ -628,16 +634,20 @@ int launch_rsw_stage(int method, int prec, const CUtensorMap* th,
 {
     RswIn a = args;
     a.fbdy = (float)a.bdy;
-    dim3 grid = tile_grid(g), block(TX, TY);
-#define F2D_RS(T, M) k_rsw_stage<T, M><<<grid, block, 0, s>>>(*th, *tw, a, code, stage, g, sc)
-#define F2D_DISPATCH(T)                                      \
-    switch (method) {                                        \
-    case METHOD_WENO: F2D_RS(T, METHOD_WENO); break;         \
-    case METHOD_UPWIND: F2D_RS(T, METHOD_UPWIND); break;     \
-    case METHOD_CENTERED: F2D_RS(T, METHOD_CENTERED); break; \
-    default: F2D_RS(T, METHOD_CWENO); break;                 \
+    const int ty = stage_rows(prec, g);
+    dim3 grid = tile_grid(g, ty), block(TX, ty);
+#define F2D_RS(T, M, TYK) \
+    k_rsw_stage<T, M, TYK><<<grid, block, 0, s>>>(*th, *tw, a, code, stage, g, sc)
+#define F2D_DISPATCH(T, TYK)                                      \
+    switch (method) {                                             \
+    case METHOD_WENO: F2D_RS(T, METHOD_WENO, TYK); break;         \
+    case METHOD_UPWIND: F2D_RS(T, METHOD_UPWIND, TYK); break;     \
+    case METHOD_CENTERED: F2D_RS(T, METHOD_CENTERED, TYK); break; \
+    default: F2D_RS(T, METHOD_CWENO, TYK); break;                 \
     }
-    if (prec == 0) { F2D_DISPATCH(double) } else { F2D_DISPATCH(float) }
+    if (prec != 0) { F2D_DISPATCH(float, TY) }
+    else if (ty == TY) { F2D_DISPATCH(double, TY) }
+    else { F2D_DISPATCH(double, TYS) }
 #undef F2D_DISPATCH
 #undef F2D_RS
     return (int)cudaGetLastError();
@@ -651,17 +661,20 @@ int launch_rsw_diag(int method, int prec, const CUtensorMap* tux,
     a.frdx2 = (float)a.rdx2;
     a.frdy2 = (float)a.rdy2;
     a.fgoa = (float)a.goa;
-    dim3 grid = tile_grid(g), block(TX, TY);
-#define F2D_RD(T, M) k_rsw_diag<T, M><<<grid, block, 0, s>>>(*tux, *tuy, a, code, g, sc)
-#define F2D_DISPATCH(T)                                      \
-    switch (method) {                                        \
-    case METHOD_WENO: F2D_RD(T, METHOD_WENO); break;         \
-    case METHOD_UPWIND: F2D_RD(T, METHOD_UPWIND); break;     \
-    case METHOD_CENTERED: F2D_RD(T, METHOD_CENTERED); break; \
-    case METHOD_CLASSIC: F2D_RD(T, METHOD_CLASSIC); break;   \
-    default: F2D_RD(T, METHOD_CWENO); break;                 \
+    const int ty = stage_rows(prec, g);
+    dim3 grid = tile_grid(g, ty), block(TX, ty);
+#define F2D_RD(T, M, TYK) k_rsw_diag<T, M, TYK><<<grid, block, 0, s>>>(*tux, *tuy, a, code, g, sc)
+#define F2D_DISPATCH(T, TYK)                                      \
+    switch (method) {                                             \
+    case METHOD_WENO: F2D_RD(T, METHOD_WENO, TYK); break;         \
+    case METHOD_UPWIND: F2D_RD(T, METHOD_UPWIND, TYK); break;     \
+    case METHOD_CENTERED: F2D_RD(T, METHOD_CENTERED, TYK); break; \
+    case METHOD_CLASSIC: F2D_RD(T, METHOD_CLASSIC, TYK); break;   \
+    default: F2D_RD(T, METHOD_CWENO, TYK); break;                 \
     }
-    if (prec == 0) { F2D_DISPATCH(double) } else { F2D_DISPATCH(float) }
+    if (prec != 0) { F2D_DISPATCH(float, TY) }
+    else if (ty == TY) { F2D_DISPATCH(double, TY) }
+    else { F2D_DISPATCH(double, TYS) }
 #undef F2D_DISPATCH
 #undef F2D_RD
     return (int)cudaGetLastError();

@@ -12,12 +12,18 @@ constexpr int OX = 4, OY = 3;            // offset of cell (j0,i0) in the tile
 // The flux-form stage runs 32 x 32-cell tiles (4 rows per thread): a quarter
 // of the blocks, each waiting once for its TMA tile, and 1.48x instead of
 // 2.19x staged cells per cell.
-constexpr int FRT = 4, FTY = 8 * FRT, FSH = FTY + 6;
+constexpr int FRT = 4, FTY = 8 * FRT;
 // In FP64 the stage is bound by the FP64 pipe of the SMs that have a tile, so
 // it takes 32 x 8R-cell tiles, R rows per thread: 256^2 gives 64 tiles of 32
 // rows for 152 SMs.
 template <typename T> struct FluxRows { static constexpr int R = FRT; };
 template <> struct FluxRows<double> { static constexpr int R = 1; };
+// The FP64 stage kernels of a grid with no more 32 x 8 tiles than the device
+// has SMs run half-height tiles: four warps, one per FP64 pipe of the SM,
+// instead of two on each. euler 40^2 (12 tiles of 8 rows): k_rsw_stage 17.4 ->
+// 12.3 us, k_rsw_diag 13.8 -> 9.7 us; above that number the tiles only pay
+// for their extra edge faces. The staged (TMA) box keeps its height.
+constexpr int TYS = 4;
 
 // Test hook of the failure detection (f2d_test_tma_wait). When enabled,
 // every stage kernel, once its TMA tile has landed, also waits for the next
@@ -190,12 +196,13 @@ __device__ __forceinline__ bool stage_tiles(T (*s0)[SW], const CUtensorMap* m0,
 // the RK3 update. `tq` is the TMA map of qin (param or global memory).
 // Returns after the (uniform) TMA timeout check; all threads must call it.
 // ---------------------------------------------------------------------------
-template <typename T, int M>
+// TYK: rows of threads (a thread has the tile rows ty + TYK q).
+template <typename T, int M, int TYK = TY>
 struct FluxformSmem {
     static constexpr int R = FluxRows<T>::R;
-    alignas(128) T sq[8 * R + 6][SW];
-    T sfx[8 * R][TX + 1];
-    T sfy[8 * R + 1][TX];
+    alignas(128) T sq[TY * R + 6][SW];
+    T sfx[TYK * R][TX + 1];
+    T sfy[TYK * R + 1][TX];
     T rk[3];
     uint64_t bar;
 };
@@ -209,15 +216,15 @@ constexpr int INTEG_TENDENCY = 15;
 // FRC: the kernel takes a forcing field `frc` (may be null at run time),
 // added to the tendency after the right-hand side (addforcingterm,
 // equations.py:229-238).
-template <typename T, int M, bool FRC = false>
+template <typename T, int M, bool FRC = false, int TYK = TY>
 __device__ __forceinline__ void fluxform_tile(
-    FluxformSmem<T, M>& sm, const CUtensorMap* tq, const T* __restrict__ qin,
+    FluxformSmem<T, M, TYK>& sm, const CUtensorMap* tq, const T* __restrict__ qin,
     T* __restrict__ qout, const T* __restrict__ Ux, const T* __restrict__ Uy,
     const uint32_t* __restrict__ code, T* __restrict__ ds_out, const T* __restrict__ ds1,
     const T* __restrict__ ds2, const T* __restrict__ frc, int stage, const Geom& g,
     double dt, double gamma, int* status, int i0, int j0)
 {
-    constexpr int R = FluxRows<T>::R, NR = 8 * R;  // rows per thread, of the tile
+    constexpr int R = FluxRows<T>::R, NR = TYK * R;  // rows per thread, of the tile
     auto& sq = sm.sq;
     auto& sfx = sm.sfx;
     auto& sfy = sm.sfy;
@@ -232,7 +239,7 @@ __device__ __forceinline__ void fluxform_tile(
     if (t == 0) mbar_init(&sm.bar, 1);
     __syncthreads();
     if (t == 0) {
-        mbar_expect_tx(&sm.bar, (uint32_t)(sizeof(T) * SW * (NR + 6)));
+        mbar_expect_tx(&sm.bar, (uint32_t)(sizeof(T) * SW * (TY * R + 6)));
         tma_load_2d(&sq[0][0], tq, i0 - OX, j0 - OY, &sm.bar);
     }
     // 2. ... overlapped with this thread's plain loads: the code word and
@@ -245,7 +252,7 @@ __device__ __forceinline__ void fluxform_tile(
     T ux[R], uy[R], d1[R], d2[R], fq[R];
 #pragma unroll
     for (int q = 0; q < R; ++q) {
-        const int j = j0 + ty + 8 * q;
+        const int j = j0 + ty + TYK * q;
         const bool in = j < g.NY && i < g.NX;
         const long long o = (long long)min(j, g.NY - 1) * g.P + min(i, g.NX - 1);
         const uint32_t c = code[o];
@@ -306,8 +313,8 @@ __device__ __forceinline__ void fluxform_tile(
     };
 #pragma unroll
     for (int q = 0; q < R; ++q) {
-        xflux(ty + 8 * q, tx, cd[q], ux[q]);
-        yflux(ty + 8 * q, tx, cd[q], uy[q]);
+        xflux(ty + TYK * q, tx, cd[q], ux[q]);
+        yflux(ty + TYK * q, tx, cd[q], uy[q]);
     }
     if (ex == 1) xflux(er, ec, ce, ue);
     else if (ex == 2) yflux(er, ec, ce, ue);
@@ -317,7 +324,7 @@ __device__ __forceinline__ void fluxform_tile(
     if (i >= g.NX || !periodic_owner(g, i)) return;
 #pragma unroll
     for (int q = 0; q < R; ++q) {
-        const int r = ty + 8 * q, j = j0 + r;
+        const int r = ty + TYK * q, j = j0 + r;
         if (j >= g.NY) break;
         const T msk = (cd[q] & B_MSK) ? T(1) : T(0);
         T ds = (-(sfx[r][tx + 1] - sfx[r][tx]) - (sfy[r + 1][tx] - sfy[r][tx])) * msk;
