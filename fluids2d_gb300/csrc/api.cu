@@ -1461,10 +1461,17 @@ int f2d_set_coriolis(f2d_model m, const double* f)
     return 0;
 }
 
+// diag of what may be a new state: no second-order warm start of the next step
+static int diag_state(f2d_model_s* m)
+{
+    CK(cudaMemsetAsync(&m->sc->warm_ext, 0, sizeof(int), m->stream));
+    return run_graph(m, 0);
+}
+
 int f2d_diag(f2d_model m)
 {
     if (!m) return fail(1, "null model");
-    return run_graph(m, 0);
+    return diag_state(m);
 }
 
 int f2d_qg_projection(f2d_model m)
@@ -2029,7 +2036,7 @@ int f2d_adjoint_forward(f2d_model m, const double* w0, double* wT, int nsteps, d
         a.use_psic = a.psic && a.psic_slots >= slots;
     }
     if ((e = adj_put(m, fb(m, "omega", m->cur), w0))) return e;
-    if ((e = run_graph(m, 0))) return e;
+    if ((e = diag_state(m))) return e;
     if (a.use_psic) {
         CK(cudaMemsetAsync(a.pslot, 0, sizeof(int), m->stream));
         if ((e = rec_psi_store(m, m->stream))) return e;
@@ -2075,7 +2082,7 @@ int f2d_adjoint_backward(f2d_model m, const double* lamT, double* lam0)
             const int p0 = 3 * n0;
             CK(cudaMemcpyAsync(a.pslot, &p0, sizeof(int), cudaMemcpyHostToDevice, m->stream));
             if ((e = rec_diag_cached(m, m->stream))) return e;
-        } else if ((e = run_graph(m, 0))) {
+        } else if ((e = diag_state(m))) {
             return e;
         }
         CK(cudaMemsetAsync(a.slot, 0, sizeof(int), m->stream));

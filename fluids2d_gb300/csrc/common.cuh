@@ -73,12 +73,35 @@ struct DevScalars {
     // (param.py:50 RAgamma, integrators.py:39-55)
     double ragamma;
     // time step of the step whose stage increments the warm start keeps
-    // (0: none yet); the next step scales them by dt / dt_warm
-    double dt_warm;
+    // (0: none yet), by which the next step scales them, and whether they may
+    // be extrapolated to second order (not right after a diag: the state may
+    // be a new one). Written at stage 3; *0: copies of the step under way
+    double dt_warm, dt_warm0;
+    int warm_ext, warm_ext0;
     // step lengths (FP32) of the inner iterations of the current refinement
     // round: the round's correction is sum alpha_i p_i (solver.cu)
     float ahist[32];
 };
+
+// The warm start's state as stage MODE + 1 of a step reads it, and its update
+// by one thread of the grid: a grid never reads what it writes.
+struct WarmState {
+    bool hist, ext;
+    double rho;
+};
+template <int MODE> __device__ __forceinline__ WarmState warm_state(DevScalars* sc, bool owner)
+{
+    const double last = MODE == 0 ? sc->dt_warm : sc->dt_warm0;
+    const int ext = MODE == 0 ? sc->warm_ext : sc->warm_ext0;
+    if (MODE == 0 && owner) {
+        sc->dt_warm0 = last;
+        sc->warm_ext0 = ext;
+    } else if (MODE == 2 && owner) {
+        sc->dt_warm = sc->dt;
+        sc->warm_ext = 1;
+    }
+    return {last > 0.0, last > 0.0 && ext, last > 0.0 ? sc->dt / last : 0.0};
+}
 
 // ---------------------------------------------------------------------------
 // Small PTX helpers: TMA tile loads through an mbarrier, with a time-bounded

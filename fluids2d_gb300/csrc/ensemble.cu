@@ -109,8 +109,7 @@ k_ens_fluxform_stage(const int4* __restrict__ tiles, const Member* __restrict__ 
 // with the member's own step-size ratio: blockIdx.y is the member, the
 // blocks of a member stride over its elements in 16-byte pairs, two pairs
 // per thread and pass (the member arrays start 32-element aligned, P is
-// even). Mode 2 also records the
-// member's dt_warm (block 0 of the member; mode 2 reads no dt_warm).
+// even).
 template <int MODE>
 __global__ void __launch_bounds__(256) k_ens_psi_warm(const Member* __restrict__ mem,
                                                        EnsArenas a, DevScalars* scs)
@@ -118,8 +117,7 @@ __global__ void __launch_bounds__(256) k_ens_psi_warm(const Member* __restrict__
     const Member& mb = mem[blockIdx.y];
     const Geom g = mb.g;
     DevScalars& sc = scs[blockIdx.y];
-    const bool hist = sc.dt_warm > 0.0;
-    const double rho = hist ? sc.dt / sc.dt_warm : 0.0;
+    const WarmState ws = warm_state<MODE>(&sc, blockIdx.x == 0 && threadIdx.x == 0);
     WarmArrays w;
     w.psi = at<double>(a.psi, mb.off);
     w.s0 = a.psi_s0 + mb.off;
@@ -143,10 +141,9 @@ __global__ void __launch_bounds__(256) k_ens_psi_warm(const Member* __restrict__
             k[u] = k0 + u * step;
             ok[u] = k[u] < n;
         }
-        if (ext) psi_warm_pairs<MODE, true, U>(w, k, ok, hist, rho);
-        else psi_warm_pairs<MODE, false, U>(w, k, ok, hist, rho);
+        if (ext) psi_warm_pairs<MODE, true, U>(w, k, ok, ws);
+        else psi_warm_pairs<MODE, false, U>(w, k, ok, ws);
     }
-    if (MODE == 2 && blockIdx.x == 0 && threadIdx.x == 0) sc.dt_warm = sc.dt;
 }
 
 // centerstovertices (+ beta-plane term) into the FP64 right-hand side
@@ -881,6 +878,10 @@ int64_t f2d_ensemble_packed_size(f2d_ensemble e)
 int f2d_ensemble_diag(f2d_ensemble e)
 {
     if (!e) return f2d_internal_fail(1, "null ensemble");
+    // the states may be new ones: no second-order warm start of the next step
+    if (cudaMemset2DAsync(&e->scs->warm_ext, sizeof(DevScalars), 0, sizeof(int), e->n,
+                          e->stream) != cudaSuccess)
+        return f2d_internal_fail(3, "cudaMemset2DAsync");
     return ens_run_graph(e, 0);
 }
 

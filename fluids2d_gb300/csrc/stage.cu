@@ -761,8 +761,7 @@ template <int MODE, bool EXT>
 __global__ void __launch_bounds__(256) k_psi_warm(WarmArrays w, long long n, DevScalars* sc)
 {
     constexpr int U = 2;
-    const bool hist = sc->dt_warm > 0.0;
-    const double rho = hist ? sc->dt / sc->dt_warm : 0.0;
+    const WarmState ws = warm_state<MODE>(sc, blockIdx.x == 0 && threadIdx.x == 0);
     const long long step = 2ll * gridDim.x * blockDim.x;
     for (long long k0 = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x); k0 < n;
          k0 += U * step) {
@@ -773,9 +772,8 @@ __global__ void __launch_bounds__(256) k_psi_warm(WarmArrays w, long long n, Dev
             k[u] = k0 + u * step;
             ok[u] = k[u] < n;
         }
-        psi_warm_pairs<MODE, EXT, U>(w, k, ok, hist, rho);
+        psi_warm_pairs<MODE, EXT, U>(w, k, ok, ws);
     }
-    if (MODE == 2 && blockIdx.x == 0 && threadIdx.x == 0) sc->dt_warm = sc->dt;
 }
 
 int launch_psi_warm(int mode, const WarmArrays& w, long long n, DevScalars* sc, cudaStream_t s)
@@ -799,33 +797,31 @@ template <int MODE>
 __global__ void __launch_bounds__(256) k_p_warm(WarmArrays w, const uint32_t* __restrict__ code,
                                                 long long n, DevScalars* sc)
 {
-    const bool hist = sc->dt_warm > 0.0;
-    const double rho = hist ? sc->dt / sc->dt_warm : 0.0;
     const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const WarmState ws = warm_state<MODE>(sc, k == 0);
+    const double rho = ws.rho;
     if (k < n && (code[k] & B_MSK)) {
         const double p = w.psi[k];
         if constexpr (MODE == 0) {
-            if (hist) {
-                const double S2 = w.d1[k];
-                const double e3 = fma(1.5, p, -0.375 * (w.s0[k] + S2));
-                w.psi[k] = rho * (S2 + w.e1[k]);
-                w.e3[k] = e3;
+            if (ws.hist) {
+                const double S2 = w.d1[k], e1 = ws.ext ? w.e1[k] : 0.0;
+                w.e3[k] = ws.ext ? fma(1.5, p, -0.375 * (w.s0[k] + S2)) : 0.0;
+                w.psi[k] = rho * (S2 + e1);
             }
         } else if constexpr (MODE == 1) {
-            const double d1 = w.d1[k], d2 = w.d2[k], e2 = w.e2[k];
+            const double d1 = w.d1[k], d2 = w.d2[k], e2 = ws.ext ? w.e2[k] : 0.0;
             w.s0[k] = p;
-            w.e1[k] = hist ? fma(-rho, d1, p) : 0.0;
+            w.e1[k] = ws.ext ? fma(-rho, d1, p) : 0.0;
             w.psi[k] = fma(0.25 * rho, d2 + e2, -0.5 * p);
         } else {
             const double S1 = w.s0[k], d2 = w.d2[k], e3 = w.e3[k];
             const double S2 = fma(4.0, p, 3.0 * S1), D = S2 - S1;
             w.d1[k] = S2;
             w.d2[k] = D;
-            w.e2[k] = hist ? fma(-rho, d2, D) : 0.0;
+            w.e2[k] = ws.ext ? fma(-rho, d2, D) : 0.0;
             w.psi[k] = fma(rho * (2.0 / 3.0), e3, 0.25 * (S1 + S2));
         }
     }
-    if (MODE == 2 && k == 0) sc->dt_warm = sc->dt;
 }
 
 int launch_p_warm(int mode, const WarmArrays& w, const uint32_t* code, long long n,

@@ -94,28 +94,30 @@ inline bool psi_warm_brackets(int prec, long long points)
 // U pairs of elements (k, k + 1), k even and every array 16-byte aligned
 // there: 16-byte loads and stores, all the loads of the U pairs before any
 // store (the arrays do not overlap, but a store ahead of a load through
-// another pointer would hold the load back). ok[u] false skips pair u. hist:
-// there is a previous step, of dt / rho. The large grids are bound by the FP64
+// another pointer would hold the load back). ok[u] false skips pair u. The
+// brackets are 0 without ws.ext. The large grids are bound by the FP64
 // pipe here too, so the mode and the brackets (EXT) are compile-time.
 // e3 holds t3 = 1.5 psi0 + 0.75 (S1 + S2) of the step between its stages 2
 // and 3 (S3 - (S1 + S2)/2 = 1.5 psi3 - t3).
 template <int MODE, bool EXT, int U>
 __device__ __forceinline__ void psi_warm_pairs(const WarmArrays& w, const long long (&k)[U],
-                                               const bool (&ok)[U], bool hist, double rho)
+                                               const bool (&ok)[U], const WarmState& ws)
 {
+    const bool hist = ws.hist;
+    const double rho = ws.rho;
     double2 a[U], s0[U], p1[U], d1[U], d2[U], e[U], t3[U];
     const double* ein = MODE == 0 ? w.e1 : MODE == 1 ? w.e2 : w.e3;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const double2 z = make_double2(0.0, 0.0);
-        const bool h = ok[u] && hist;
+        const bool h = ok[u] && hist, hb = ok[u] && ws.ext;
         a[u] = ok[u] ? *(const double2*)(w.psi + k[u]) : z;
         s0[u] = MODE >= 1 && ok[u] ? *(const double2*)(w.s0 + k[u]) : z;
         p1[u] = MODE == 2 && ok[u] ? *(const double2*)(w.p1 + k[u]) : z;
         d1[u] = (MODE == 0 || (MODE == 1 && EXT)) && h ? *(const double2*)(w.d1 + k[u]) : z;
         d2[u] = (MODE == 1 || (MODE == 2 && EXT)) && h ? *(const double2*)(w.d2 + k[u]) : z;
-        e[u] = EXT && h ? *(const double2*)(ein + k[u]) : z;
-        t3[u] = EXT && MODE == 0 && h ? *(const double2*)(w.e3 + k[u]) : z;
+        e[u] = EXT && hb ? *(const double2*)(ein + k[u]) : z;
+        t3[u] = EXT && MODE == 0 && hb ? *(const double2*)(w.e3 + k[u]) : z;
     }
     const double rq = 0.25 * rho, r23 = rho * (2.0 / 3.0);
     // one element: the guess g, the bracket en, mode 2: S2, D and t3
@@ -154,7 +156,7 @@ __device__ __forceinline__ void psi_warm_pairs(const WarmArrays& w, const long l
             n3.x);
         one(a[u].y, s0[u].y, p1[u].y, d1[u].y, d2[u].y, e[u].y, t3[u].y, g.y, en.y, n1.y, n2.y,
             n3.y);
-        if (!hist) en = make_double2(0.0, 0.0);
+        if (!ws.ext) en = make_double2(0.0, 0.0);
         if constexpr (MODE == 0) {
             *(double2*)(w.s0 + k[u]) = a[u];
             if (hist) *(double2*)(w.psi + k[u]) = g;
@@ -176,7 +178,7 @@ __device__ __forceinline__ void psi_warm_pairs(const WarmArrays& w, const long l
 }
 
 // the single-model form over n elements, n even (every point; non-fluid points
-// stay 0); mode 2 records dt_warm
+// stay 0)
 int launch_psi_warm(int mode, const WarmArrays& w, long long n, DevScalars* sc,
                     cudaStream_t s);
 
