@@ -1,0 +1,169 @@
+"""The elliptic solves and the small-grid stage kernels at the sizes where
+their rules change: a grid that is one dense level or just more, odd coarse
+widths, one tile or just more, the sizes on both sides of the FP32 forms'
+limits, and batches of uneven members.
+
+Tolerances. Solves stop at a recurrence residual of 1e-12 |b|; the true one
+drifts from it by rounding, iterations x eps x |A||x|/|b| <= 20 x 1.1e-16 x 4e4
+(a 300-point basin) = 1e-10. A projected FP64 velocity has that divergence;
+an FP32 one is rounded three times, 2^-24 each, and a divergence sums four of
+them: 16 x 2^-24 |u|. Whole steps: 1e-10 per step as in the parity tests.
+
+The FP32 divergence of two unconnected basins sums to 1e-7 in each instead of
+0, and only the mean of both is taken off, so that system has no solution: the
+solve reports its iteration limit.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+from fluids2d_gb300 import workloads as wl  # noqa: E402
+from fluids2d_gb300._lib import F2DError  # noqa: E402
+from test_gpu_parity import (_ensemble, _model, _oracle_like, compare,  # noqa: E402
+                             rel_l2)
+
+
+def _mask(nx, ny, xper=False, islands=0, wall=False):
+    msk = wl.default_mask(nx, ny, xperiodic=xper)
+    rng = np.random.default_rng(nx * 1000 + ny)
+    for _ in range(islands):
+        j, i = int(rng.integers(4, ny)), int(rng.integers(6, nx))
+        msk[j:j + max(2, ny // 9), i:i + max(2, nx // 11)] = 0
+    if wall:  # two basins
+        msk[3 + ny // 2] = 0
+    if xper:
+        msk[:, :3], msk[:, -3:] = msk[:, -6:-3], msk[:, 3:6]
+    return msk
+
+
+@pytest.mark.parametrize("model,nx,ny,precision,xper", [
+    ("eulerpsi", 9, 7, "fp64", False),     # one dense level
+    ("eulerpsi", 47, 45, "fp64", False),   # 46 x 44 nodes: the largest dense level
+    ("eulerpsi", 48, 45, "fp64", False),   # just above it
+    ("qg", 65, 64, "fp32", False),         # the same of the FP32 form: 4032 nodes
+    ("qg", 67, 64, "fp32", False),
+    ("qg", 48, 40, "fp64", True),
+    ("qg", 45, 40, "fp64", True),          # odd periodic widths
+    ("qg", 90, 61, "fp32", True),
+    ("eulerpsi", 257, 33, "fp64", False),
+    ("qg", 131, 97, "fp64", False),
+    ("eulerpsi", 301, 287, "fp32", False),
+    ("qg", 1450, 1400, "fp32", False),     # above 2M nodes: the level kernels
+])
+def test_vertex_solve(model, nx, ny, precision, xper):
+    kw = dict(xperiodic=xper, f0=30.0 if model == "qg" else 0.0, g=1.0, H=1.0)
+    msk = _mask(nx, ny, xper, islands=2 if min(nx, ny) > 30 else 0)
+    m = _model(model, nx, ny, msk, precision=precision, **kw)
+    solver = m.mesh.qg_helmholtz if model == "qg" else m.mesh.poisson_vertices
+    b = np.random.default_rng(3).standard_normal(m.mesh.shape) * (m.mesh.G_vertices >= 0)
+    x = np.zeros(m.mesh.shape)
+    solver.solve(b, x)
+    om = O.Mesh(O.Param(model=model, nx=nx, ny=ny, **kw))
+    om.msk[:] = msk
+    om.finalize()
+    A, G = O.laplacian(om, om.maindiag if model == "qg" else 0.0)[:2]
+    sel = G >= 0
+    r = b[sel] - A @ x[sel]
+    assert np.linalg.norm(r) <= 1e-10 * np.linalg.norm(b[sel])
+
+
+@pytest.mark.parametrize("nx,ny,precision,xper,wall", [
+    (8, 9, "fp64", False, False),
+    (45, 45, "fp64", False, False),   # one dense level
+    (46, 45, "fp64", False, True),    # just above it, two basins
+    (41, 37, "fp64", True, False),    # odd periodic widths on every level
+    (44, 61, "fp64", True, True),
+    (131, 97, "fp64", False, True),
+    (257, 160, "fp64", True, False),
+    (45, 64, "fp32", False, False),   # between the FP32 form's two limits
+    (64, 64, "fp32", True, False),
+    (65, 64, "fp32", False, False),
+    (65, 64, "fp32", False, True),
+    (161, 300, "fp32", False, False),
+])
+def test_pressure_solve(nx, ny, precision, xper, wall):
+    msk = _mask(nx, ny, xper, islands=1 if min(nx, ny) > 30 else 0, wall=wall)
+    m = _model("euler", nx, ny, msk, precision=precision, xperiodic=xper, Lx=nx, Ly=ny)
+    rng = np.random.default_rng(4)
+    s = m.state
+    for a, k in ((s.u.x, m.mesh.mskx), (s.u.y, m.mesh.msky)):
+        v = rng.standard_normal(a.shape) * k
+        if xper:
+            v[:, :3], v[:, -3:] = v[:, -6:-3], v[:, 3:6]
+        a[:] = v.astype(np.float32)
+    fl = m.mesh.msk > 0
+    if xper:
+        fl[:, :3] = fl[:, -3:] = False
+
+    def div():
+        d = np.zeros(m.mesh.shape)
+        d[:, :-1] = np.diff(s.u.x.astype(np.float64), axis=1)
+        d[:-1] += np.diff(s.u.y.astype(np.float64), axis=0)
+        return np.linalg.norm(d[fl])
+
+    u0 = np.hypot(np.linalg.norm(s.u.x), np.linalg.norm(s.u.y))
+    d0 = div()
+    assert d0 > 0.1 * u0
+    m.integrator.diag(s)
+    if wall and precision == "fp32":
+        with pytest.raises(F2DError, match="max iterations"):
+            m.sync()
+        return
+    m.sync()
+    s = m.state
+    assert div() <= (1e-10 * d0 if precision == "fp64" else 16 * 2.0 ** -24 * u0)
+
+
+@pytest.mark.parametrize("kind", ["eulerpsi", "rsw", "boussinesq"])
+@pytest.mark.parametrize("nx,ny", [(26, 26), (27, 29), (90, 59),
+                                   # 8 x 19 = 152 tiles of 32 x 8, and one row more
+                                   (250, 146), (250, 147)])
+def test_small_grid_stages(kind, nx, ny):
+    make = {"eulerpsi": wl.eulerpsi_case, "rsw": wl.rsw_case,
+            "boussinesq": wl.boussinesq_case}[kind]
+    case = make(n=nx, ny=ny, seed=9, nislands=1)
+    om = _oracle_like(case, kind, cfl=0.5)
+    kw = dict(xperiodic=case.get("xperiodic", False), Lx=case["Lx"], Ly=case["Ly"],
+              tend=1e300, maxite=10 ** 9, cfl=0.5)
+    for k in ("f0", "g", "H", "beta"):
+        if k in case:
+            kw[k] = case[k]
+    m = _model(kind, nx, ny, case["msk"], **kw)
+    s = m.state
+    for k, v in case["fields"].items():
+        if "." in k:
+            getattr(getattr(s, k.split(".")[0]), k.split(".")[1])[:] = v
+        else:
+            getattr(s, k)[:] = v
+    m.integrator.diag(s)
+    om.run_steps(2)
+    m.advance(2)
+    m.sync()
+    compare(m, lambda k: om.s.get(k), 1e-10)
+
+
+@pytest.mark.parametrize("sizes,precision,tol", [
+    ([(20, 17), (47, 45), (48, 45), (129, 65), (250, 131)], "fp64", 1e-10),
+    # above 1M nodes: the level kernels, against single models' persistent
+    # solves (FP32: as for the members of the parity tests)
+    ([(512, 512)] * 4 + [(33, 47)], "fp32", 1e-6),
+])
+def test_uneven_ensemble(sizes, precision, tol):
+    cs = [wl.eulerpsi_case(n=nx, ny=ny, seed=20 + k, nislands=k % 3)
+          for k, (nx, ny) in enumerate(sizes)]
+    e = _ensemble(cs, precision)
+    e.run(4)
+    e.sync()
+    for b, c in enumerate(cs):
+        m = _model("eulerpsi", c["nx"], c["ny"], c["msk"], cfl=0.8, tend=1e300,
+                   maxite=10 ** 9, precision=precision)
+        m.state.omega[:] = c["fields"]["omega"]
+        m.integrator.diag(m.state)
+        m.advance(4)
+        m.sync()
+        assert rel_l2(e.get_field(b, "omega"), m.state.omega) <= tol, b
+        assert rel_l2(e.get_field(b, "psi"), m.state.psi) <= tol, b
