@@ -28,6 +28,7 @@ constexpr int PS_NT = 512;  // threads of a block (one block per SM)
 struct PSBar {
     unsigned int count[4][32];  // arrivals
     int abort;                  // a wait ran out
+    unsigned int base;          // barriers passed by the launches before (k_ps_cycle)
 };
 
 struct PSGrid {
@@ -41,6 +42,7 @@ __device__ __forceinline__ void ps_reset(PSBar* b)
 {
     for (int k = 0; k < 4; ++k) b->count[k][0] = 0u;
     b->abort = 0;
+    b->base = 0u;
 }
 
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p)

@@ -779,6 +779,47 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_down0(const __grid_constant__ P
     for (int i = l0[0]; i < l0[1]; ++i) p_phase_a<S>(A, A.recs[i], 0, 0.0, 0.0, t, smem);
 }
 
+// The V-cycle of one member on the levels from A.l0 on, for the FP32 form's
+// level kernels of the grids that do not take the whole solve: a launch per
+// level and leg took 8 to 9 us, whatever the level's size (its chain of
+// dependent loads, tile record, flags, tensor map, tile, starts over with
+// each), and the one-block kernel of the coarsest levels 23 us. Here a leg is
+// a barrier and a tile, and the coarsest level is the dense one.
+// qg 4096^2, the five levels from 512^2 on: 45 us; its step 14.28 -> 13.41 ms.
+template <typename S>
+__global__ void __launch_bounds__(PS_NT, 1) k_ps_cycle(const __grid_constant__ PSArgs A, int ir)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ PTile rec[PS_RECS];
+    __shared__ int lev0[PS_LMAX + 1];
+    const DevScalars& sc = A.scs[0];
+    const int skip = sc.converged | (ir ? sc.conv_in : 0);
+    PSGrid g = {A.bar, A.status, A.bar->base};
+    const int nl = A.ng + 1;
+    if (threadIdx.x < nl) lev0[threadIdx.x] = A.rec0[blockIdx.x * nl + threadIdx.x];
+    if (skip) return;  // (the same in every block: no barrier is left waiting)
+    __syncthreads();
+    const int base = lev0[0], nrec = lev0[A.ng] - base;
+    {
+        constexpr int W = sizeof(PTile) / 16;
+        const int4* src = (const int4*)(A.recs + base);
+        for (int k = threadIdx.x; k < nrec * W; k += PS_NT) ((int4*)rec)[k] = src[k];
+    }
+    __syncthreads();
+    for (int l = A.l0; l < A.ng; ++l) {
+        for (int i = lev0[l] - base; i < lev0[l + 1] - base; ++i) p_down<S>(rec[i], A.nu, smem);
+        if (!ps_sync(g)) return;
+    }
+    p_dense<S>(A, smem);
+    for (int l = A.ng - 1; l >= A.l0; --l) {
+        if (!ps_sync(g)) return;
+        for (int i = lev0[l] - base; i < lev0[l + 1] - base; ++i) p_up<S>(rec[i], A.nu, smem);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.bar->base = g.round;
+}
+
+__global__ void k_ps_cycle_reset(PSBar* bar) { ps_reset(bar); }
+
 __global__ void k_ps_setup(const __grid_constant__ PSArgs A, double tol2, int maxit)
 {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -937,11 +978,11 @@ static std::vector<TileDim> pick_tiles(const std::vector<std::pair<int, int>>& n
 }
 
 int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long nelem,
-             DevScalars* scs, BSGlobals* eg, int* status)
+             DevScalars* scs, BSGlobals* eg, int* status, int l0)
 {
     ps_free(s);
     const int n = (int)mem.size(), sms = ps_sms();
-    if (n < 1 || sms < 1 || nelem <= 0) return 0;
+    if (n < 1 || sms < 1 || (l0 == 0 && nelem <= 0) || (l0 > 0 && n > 1)) return 0;
     const size_t es = prec == 0 ? 8 : 4;
     auto dal = [&](size_t bytes) -> void* {
         void* p = nullptr;
@@ -958,13 +999,13 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     };
     for (int b = 0; b < n; ++b) {
         const std::vector<MGLevel>& lev = mem[b].mg->lev;
-        int l = n == 1 ? 0 : 1;
+        int l = l0 > 0 ? l0 + 1 : n == 1 ? 0 : 1;  // (a cycle: one grid level at least)
         for (; l < (int)lev.size(); ++l) {
             const long long k = unknowns(lev[l]);
             if (k <= mem[b].ndense_cap && ps_band_ok(k, lev[l].nxn, prec)) break;
         }
         if (l >= (int)lev.size() || l >= PS_LMAX || unknowns(lev[l]) < 1) return 0;
-        for (int q = 0; q < l; ++q)  // colours and the coarse grid wrap only over an even count
+        for (int q = l0; q < l; ++q)  // colours and the coarse grid wrap only over an even count
             if (lev[q].per && lev[q].nxn % 2) return 0;
         // the unknowns leave the closed edges out: they must be dry
         const std::vector<uint8_t>& hm = mem[b].mg->hmask[l];
@@ -981,6 +1022,7 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     PSArgs& a = s.a;
     memset(&a, 0, sizeof(a));
     a.dense0 = maxg == 0;
+    a.l0 = l0;
     a.ng = std::max(1, maxg);
     a.nmem = n;
     a.nrows = nrows;
@@ -1026,7 +1068,7 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
         smem = std::max(smem, es * (prec == 0 ? ps_dense_elems<double>(nd, rows)
                                               : ps_dense_elems<float>(nd, rows)));
     }
-    for (int l = 0; l < a.ng; ++l) {
+    for (int l = l0; l < a.ng; ++l) {
         std::vector<std::pair<int, int>> dims(n);
         for (int b = 0; b < n; ++b) {
             const MGLevel& L = mem[b].mg->lev[l];
@@ -1088,7 +1130,7 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     a.ntiles = (int)tl[0].size();
     smem = (smem + 15) / 16 * 16;
     const size_t keep = maxrow * ((nrows + sms - 1) / sms);
-    if (smem + keep <= PS_SMEM) {
+    if (l0 == 0 && smem + keep <= PS_SMEM) {  // (a cycle reads them once)
         a.mkeep = (int)smem;
         smem += keep;
     }
@@ -1115,10 +1157,10 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     PTile* drec = (PTile*)dal(recs.size() * sizeof(PTile));
     int* d0 = (int*)dal(rec0.size() * sizeof(int));
     PDense* dd = (PDense*)dal(n * sizeof(PDense));
-    double* vec[6];
+    double* vec[6] = {};
     for (auto& p : vec)
-        if (!(p = (double*)dal((size_t)nelem * 8))) return 2;
-    a.part = (double*)dal((size_t)5 * a.ntiles * sizeof(double));
+        if (l0 == 0 && !(p = (double*)dal((size_t)nelem * 8))) return 2;
+    a.part = (double*)dal((size_t)5 * std::max(1, a.ntiles) * sizeof(double));
     a.conv = (int*)dal(n * sizeof(int));
     a.active = (int*)dal(sizeof(int));
     a.bar = (PSBar*)dal(sizeof(PSBar));
@@ -1145,7 +1187,8 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     s.grid = sms;
     s.smem = smem;
     for (const void* k : {(const void*)k_ps_solve<double>, (const void*)k_ps_solve<float>,
-                          (const void*)k_ps_down0<double>, (const void*)k_ps_down0<float>})
+                          (const void*)k_ps_down0<double>, (const void*)k_ps_down0<float>,
+                          (const void*)k_ps_cycle<float>})
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS_SMEM) !=
             cudaSuccess)
             return 3;
@@ -1174,6 +1217,19 @@ int ps_record(PSolver& s, double* x, double* b, int nu, double tol, int maxit, c
     return ps_launch(s.prec == 0 ? (const void*)k_ps_solve<double>
                                  : (const void*)k_ps_solve<float>,
                      s.grid, s.smem, args, st);
+}
+
+int ps_record_cycle_reset(PSolver& s, cudaStream_t st)
+{
+    k_ps_cycle_reset<<<1, 1, 0, st>>>(s.a.bar);
+    return (int)cudaGetLastError();
+}
+
+int ps_record_cycle(PSolver& s, int nu, int ir, cudaStream_t st)
+{
+    s.a.nu = nu;
+    void* args[2] = {&s.a, &ir};
+    return ps_launch((const void*)k_ps_cycle<float>, s.grid, s.smem, args, st);
 }
 
 int ps_time_down(PSolver& s, int nu, cudaStream_t st)

@@ -44,6 +44,7 @@ struct PSArgs {
     const int* rec0;
     const PDense* dense;
     int nmem, ng, nu;    // members, grid levels (of the deepest member)
+    int l0;              // first level: 0, or that of the cycle alone
     int nrows;           // dense rows of all members
     int dense0;          // one member whose level 0 is the dense level
     int ntiles;          // level-0 tiles
@@ -73,12 +74,18 @@ struct PSMember {
 
 // Build for the members' hierarchies: on = false (and no error) where the
 // kernel does not apply (no level small enough for the dense inverse, more
-// tiles than a block has records).
+// tiles than a block has records). l0 > 0: one member, for ps_record_cycle
+// alone, on the levels from l0 on (nelem is not used).
 int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long nelem,
-             DevScalars* scs, BSGlobals* eg, int* status);
+             DevScalars* scs, BSGlobals* eg, int* status, int l0 = 0);
 void ps_free(PSolver& s);
 // Record one solve of every member on `st`: x and b are the arenas (FP64).
 int ps_record(PSolver& s, double* x, double* b, int nu, double tol, int maxit, cudaStream_t st);
+// Record the V-cycle on the levels from l0 on (from its b to its x), skipped
+// when the member is not iterating (ir: its inner loop); ps_record_cycle_reset
+// before the first of a solve.
+int ps_record_cycle(PSolver& s, int nu, int ir, cudaStream_t st);
+int ps_record_cycle_reset(PSolver& s, cudaStream_t st);
 // Measurement hook: one launch of the level-0 down leg of every member.
 int ps_time_down(PSolver& s, int nu, cudaStream_t st);
 

@@ -827,7 +827,8 @@ static int vcycle_pipe(BatchSolver& s, cudaStream_t st, int ir)
     const CUtensorMap* maps = (const CUtensorMap*)s.mmaps;
     int* status = &s.eg->status;
     int cnt = 0;
-    for (int l = 0; l < s.maxl; ++l) {
+    const int lt = s.pc.on ? s.lc : s.maxl;
+    for (int l = 0; l < lt; ++l) {
         const int n = s.nmtiles[l];
         if (n == 0) continue;
         launch_pdl(k_mgp_down<NU>, dim3(std::min(n, s.pipe_gdown)), blk, sizeof(MPDown), st,
@@ -835,10 +836,13 @@ static int vcycle_pipe(BatchSolver& s, cudaStream_t st, int ir)
                    (const DevScalars*)s.scs, ir, status);
         cnt += 1;
     }
-    launch_pdl(k_bs_tail<float>, dim3(s.n), dim3(s.tail_threads), s.tail_smem, st,
-               (const BSInfo*)s.dinfo, (const MGLevel*)s.dlevs, s.scs, ir, NU);
+    if (s.pc.on)
+        ps_record_cycle(s.pc, NU, ir, st);
+    else
+        launch_pdl(k_bs_tail<float>, dim3(s.n), dim3(s.tail_threads), s.tail_smem, st,
+                   (const BSInfo*)s.dinfo, (const MGLevel*)s.dlevs, s.scs, ir, NU);
     cnt += 1;
-    for (int l = s.maxl - 1; l >= 0; --l) {
+    for (int l = lt - 1; l >= 0; --l) {
         const int n = s.nmtiles[l];
         if (n == 0) continue;
         if (l > 0)
@@ -1018,6 +1022,11 @@ static int bs_record_t(BatchSolver& s, cudaStream_t st, cudaStream_t st2, int* l
         if (e != cudaSuccess) return (int)e;
     }
     k_bs_reset<<<1, 1, 0, st>>>(s.eg);
+    if (s.pc.on) {
+        const int r = ps_record_cycle_reset(s.pc, st);
+        if (r) return r;
+        fixed += 1;
+    }
     launch_refine<TH, true>(s, st);
     k_bs_refine_fin<<<s.n, s.fin_threads, 0, st>>>(s.dinfo, s.scs, s.partials, s.eg, 1, cond_o, s.n);
     fixed += 3;
@@ -1287,6 +1296,9 @@ static int bs_pipe_setup(BatchSolver& s, const std::vector<MGLevel>& levs,
 }
 
 constexpr long long PS_FP32_NODES = 2000000;
+// largest level of the coarse levels' launch: on larger ones its tiles are slower
+// than the pipelined legs with their launches (1024^2: 16 us a leg, against 9)
+constexpr long long PC_NODES = 300000;
 
 int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uint8_t* dmask,
              int mode, const BSVecs& v, DevScalars* scs)
@@ -1470,6 +1482,17 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
         }
         if (mode == 0 || n0 <= (s.n == 1 ? PS_FP32_NODES : PS_FP32_NODES / 2)) {
             const int e = ps_build(s.ps, pm, mode, v.nelem, scs, s.eg, &s.eg->status);
+            if (e) return e;
+        }
+    }
+    // The level kernels of one FP32 member: its coarser levels in one launch.
+    if (mode == 1 && !s.ps.on && s.pipe && s.n == 1) {
+        const std::vector<MGLevel>& lev = s.mg[0].lev;
+        s.lc = 1;
+        while (s.lc < s.maxl && (long long)lev[s.lc].nyn * lev[s.lc].nxn > PC_NODES) ++s.lc;
+        if (s.lc < s.maxl) {
+            const std::vector<PSMember> pm = {{&s.mg[0], PS_NDENSE}};
+            const int e = ps_build(s.pc, pm, mode, 0, scs, s.eg, &s.eg->status, s.lc);
             if (e) return e;
         }
     }
@@ -1666,6 +1689,7 @@ int bs_set_schedule(BatchSolver& s, int th, int nu, double tol_in)
 void bs_free(BatchSolver& s)
 {
     ps_free(s.ps);
+    ps_free(s.pc);
     if (s.s3) {
         cudaStreamDestroy(s.s3);
         s.s3 = nullptr;

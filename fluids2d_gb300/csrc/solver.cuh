@@ -86,6 +86,9 @@ struct BatchSolver {
     int maxl = 0;
     size_t tail_smem = 0;
     int tail_threads = 1024;  // block size of k_bs_tail (bs_build)
+    // FP32 form of one member: the levels from lc on in one launch (k_ps_cycle)
+    PSolver pc;
+    int lc = 0;
     int fin_threads = 256;    // of the member-sum kernels
     bool helm = false, unit = false;  // FP64 residual variant (bs_build)
     // refinement form: the inner iterations' directions p_0 .. p_{k-1}, one
