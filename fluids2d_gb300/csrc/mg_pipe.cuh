@@ -438,12 +438,14 @@ k_mgp_down(const int4* __restrict__ tiles, int ntiles, const MGLevel* __restrict
 // Up leg of level l: x = xa + P (coarse x) at the fluid nodes, then NU
 // (black, red) sweeps; x of the tile to level l's x. RZ (level 0): the
 // tile's part of <r, z> (r = b, z = x) into tpart[k] (k_bs_rz sums a
-// member's tiles: no fence or ticket holds the block up here).
+// member's tiles: no fence or ticket holds the block up here); with one member
+// (ticket) the block's part, and the last block sets the member's rz in place
+// of k_bs_rz (9 us at 4096^2).
 template <int NU, bool RZ>
 __global__ void __launch_bounds__(256, 3)
 k_mgp_up(const int4* __restrict__ tiles, int ntiles, const MGLevel* __restrict__ levs,
-         const CUtensorMap* __restrict__ maps, int l, const DevScalars* __restrict__ scs,
-         int ir, double* tpart, int* status)
+         const CUtensorMap* __restrict__ maps, int l, DevScalars* __restrict__ scs, int ir,
+         double* tpart, unsigned int* ticket, int* status)
 {
     pdl_wait();
     extern __shared__ __align__(128) unsigned char mp_dyn[];
@@ -476,6 +478,8 @@ k_mgp_up(const int4* __restrict__ tiles, int ntiles, const MGLevel* __restrict__
     }
     __syncthreads();
     uint32_t ph = 0;
+    double blk = 0.0;   // thread 0: the block's <r, z>
+    bool any = false;
     for (int k = blockIdx.x, it = 0; k < ntiles; k += G, ++it) {
         const int slot = it & 1;
         const int4 tl = st.rec[slot];
@@ -554,7 +558,11 @@ k_mgp_up(const int4* __restrict__ tiles, int ntiles, const MGLevel* __restrict__
             if (RZ) {
                 // b x = diag bid x, summed per warp in FP32, combined in FP64
                 const double tot = block_sum<float>(acc);
-                if (t == 0) tpart[k] = (double)F.fdiag * tot;
+                any = true;
+                if (t == 0) {
+                    if (ticket) blk += (double)F.fdiag * tot;
+                    else tpart[k] = (double)F.fdiag * tot;
+                }
             }
         } else {
             __syncthreads();
@@ -563,6 +571,12 @@ k_mgp_up(const int4* __restrict__ tiles, int ntiles, const MGLevel* __restrict__
             ncv = scs[nrec.x].converged;
             nci = scs[nrec.x].conv_in;
         }
+    }
+    if (RZ && ticket && any) {
+        if (t == 0) tpart[blockIdx.x] = blk;
+        if (!last_block(ticket, gridDim.x)) return;
+        const double rz = grid_sum(tpart, gridDim.x);
+        if (t == 0) set_rz(scs[0], ir, rz);
     }
 }
 

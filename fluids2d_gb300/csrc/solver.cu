@@ -120,6 +120,44 @@ __device__ __forceinline__ double block_sum(V acc)
     return w[0];
 }
 
+// True in the last of the grid's n blocks to get here; its block sees the
+// writes of the others
+__device__ __forceinline__ bool last_block(unsigned int* ticket, unsigned n)
+{
+    __shared__ int s_last;
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == n - 1;
+        if (s_last) {
+            *ticket = 0;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    return s_last != 0;
+}
+
+// the grid's total of part[0 .. n) in thread 0
+__device__ __forceinline__ double grid_sum(const double* part, int n)
+{
+    __shared__ double sh[32];
+    double w[1];
+    final_sum<1, false>(w, part, 0, n, tid256(), 256);
+    __syncthreads();
+    block_reduce<1, false>(w, sh);
+    return w[0];
+}
+
+// rz = <r, z> of a member, beta = rz / rz_old (0 on the first iteration of
+// a loop); run by the thread that holds the member's total
+__device__ __forceinline__ void set_rz(DevScalars& sc, int ir, double rz)
+{
+    const int first = ir ? sc.iter_in == 0 : sc.iter == 0;
+    sc.beta = first ? 0.0 : rz / sc.rz;
+    sc.rz = rz;
+}
+
 // Completion of a kernel over all members, counted per member: the kernels
 // that call it run one block per member, whose thread 0 calls it with
 // mine = true, so the global ticket sees n increments. True in the thread
@@ -134,15 +172,6 @@ __device__ __forceinline__ bool members_done(bool mine, unsigned int* ticket, in
         return true;
     }
     return false;
-}
-
-// rz = <r, z> of a member, beta = rz / rz_old (0 on the first iteration of
-// a loop); run by the thread that holds the member's total
-__device__ __forceinline__ void set_rz(DevScalars& sc, int ir, double rz)
-{
-    const int first = ir ? sc.iter_in == 0 : sc.iter == 0;
-    sc.beta = first ? 0.0 : rz / sc.rz;
-    sc.rz = rz;
 }
 
 // <r, z> of every member from the tile totals of the level-0 up leg
@@ -203,6 +232,14 @@ k_bs_tail(const BSInfo* __restrict__ info, const MGLevel* __restrict__ levs, Dev
         block_reduce<1, false>(w, sh);
     }
     if (threadIdx.x == 0) set_rz(sc, ir, w[0]);
+}
+
+// <p, q> of a member: alpha = rz / <p, q>; run by the thread with the total
+__device__ __forceinline__ void set_alpha(DevScalars& sc, int ir, double pq)
+{
+    sc.pq = pq;
+    sc.alpha = sc.rz / pq;
+    if (ir) sc.ahist[sc.iter_in] = f64_to_f32_rn(sc.alpha);
 }
 
 // ---- Krylov kernels on level 0 ------------------------------------------------
@@ -322,21 +359,18 @@ k_bs_pq(const int4* __restrict__ tiles, int ntiles, const MGLevel* __restrict__ 
 // ticket per block); one block per member sums them here.
 __global__ void __launch_bounds__(1024)
 k_bs_alpha(const BSInfo* __restrict__ info, DevScalars* scs, const double* __restrict__ tpart,
-           int ir)
+           int ir, int wide)
 {
     pdl_wait();
     const BSInfo in = info[blockIdx.x];
     DevScalars& sc = scs[blockIdx.x];
     if (bs_skip(sc, ir)) return;
     double acc[1] = {0.0};
-    final_sum<1, false>(acc, tpart, in.n0, in.nn, threadIdx.x, blockDim.x);
+    final_sum<1, false>(acc, tpart, wide ? in.q0 : in.n0, wide ? in.qn : in.nn, threadIdx.x,
+                        blockDim.x);
     __shared__ double sh[32];
     block_reduce<1, false>(acc, sh);
-    if (threadIdx.x == 0) {
-        sc.pq = acc[0];
-        sc.alpha = sc.rz / acc[0];
-        if (ir) sc.ahist[sc.iter_in] = f64_to_f32_rn(sc.alpha);
-    }
+    if (threadIdx.x == 0) set_alpha(sc, ir, acc[0]);
 }
 
 // x += alpha p (FP64 form, x the solution; x == nullptr in the refinement
@@ -418,12 +452,45 @@ k_bs_xr(const int4* __restrict__ tiles, int ntiles, const MGLevel* __restrict__ 
     }
 }
 
+// <r, r> of a member: its convergence; run by the thread with the total
+__device__ __forceinline__ void set_conv(DevScalars& sc, BSGlobals* eg, int ir, double rr)
+{
+    const int zero = ir ? 0 : sc.pad1;
+    sc.total_iters += 1;
+    const bool bad = !(rr == rr);
+    if (bad) atomicOr(&eg->status, ST_NONFINITE);
+    if (ir) {
+        sc.iter_in += 1;
+        // a round stops at its relative tolerance, or as soon as its
+        // residual is a tenth of what the whole solve must reach (the
+        // last round of a solve needs only the digits missing, not
+        // tol_in more)
+        const double goal = fmax(sc.tol_in2 * sc.rr0, 0.01 * sc.tol2 * sc.bb);
+        const int done = bad || rr <= goal || sc.iter_in >= sc.maxit_in;
+        if (done) {
+            sc.conv_in = 1;
+            atomicSub(&eg->active_in, 1);
+        }
+    } else {
+        sc.rr = rr;
+        sc.iter += 1;
+        const int conv = bad || zero || (rr <= sc.tol2 * sc.bb);
+        sc.pad1 = 0;
+        const int more = !conv && sc.iter < sc.maxit;
+        if (!conv && !more) atomicOr(&eg->status, ST_PCG_MAXIT);
+        if (!more) {
+            sc.converged = 1;
+            atomicSub(&eg->active_out, 1);
+        }
+    }
+}
+
 // <r, r> of every member from k_bs_xr's tile totals (fixed order), the
 // member's convergence, and the loop condition (the block that completes
 // the count over all members sets it).
 __global__ void __launch_bounds__(1024)
 k_bs_conv(const BSInfo* __restrict__ info, DevScalars* scs, const double* __restrict__ tpart,
-          BSGlobals* eg, cudaGraphConditionalHandle cond, int ir, int nmem)
+          BSGlobals* eg, cudaGraphConditionalHandle cond, int ir, int nmem, int wide)
 {
     pdl_wait();
     const BSInfo in = info[blockIdx.x];
@@ -431,45 +498,197 @@ k_bs_conv(const BSInfo* __restrict__ info, DevScalars* scs, const double* __rest
     const bool skip = bs_skip(sc, ir);
     double w[1] = {0.0};
     if (!skip) {
-        final_sum<1, false>(w, tpart, in.n0, in.nn, threadIdx.x, blockDim.x);
+        final_sum<1, false>(w, tpart, wide ? in.q0 : in.n0, wide ? in.qn : in.nn, threadIdx.x,
+                            blockDim.x);
         __shared__ double sh[32];
         block_reduce<1, false>(w, sh);
     }
     const bool mine = threadIdx.x == 0;
-    if (mine && !skip) {
-        const int zero = ir ? 0 : sc.pad1;
-        sc.total_iters += 1;
-        const bool bad = !(w[0] == w[0]);
-        if (bad) atomicOr(&eg->status, ST_NONFINITE);
-        if (ir) {
-            sc.iter_in += 1;
-            // a round stops at its relative tolerance, or as soon as its
-            // residual is a tenth of what the whole solve must reach (the
-            // last round of a solve needs only the digits missing, not
-            // tol_in more)
-            const double goal = fmax(sc.tol_in2 * sc.rr0, 0.01 * sc.tol2 * sc.bb);
-            const int done = bad || w[0] <= goal || sc.iter_in >= sc.maxit_in;
-            if (done) {
-                sc.conv_in = 1;
-                atomicSub(&eg->active_in, 1);
-            }
-        } else {
-            sc.rr = w[0];
-            sc.iter += 1;
-            const int conv = bad || zero || (w[0] <= sc.tol2 * sc.bb);
-            sc.pad1 = 0;
-            const int more = !conv && sc.iter < sc.maxit;
-            if (!conv && !more) atomicOr(&eg->status, ST_PCG_MAXIT);
-            if (!more) {
-                sc.converged = 1;
-                atomicSub(&eg->active_out, 1);
-            }
-        }
-    }
+    if (mine && !skip) set_conv(sc, eg, ir, w[0]);
     if (members_done(mine, &eg->ticket[1], nmem)) {
         eg->loops_in += 1;
         const int act = ir ? *(volatile int*)&eg->active_in : *(volatile int*)&eg->active_out;
         if (cond) cudaGraphSetConditional(cond, act > 0 ? 1u : 0u);
+    }
+}
+
+// ---- the FP32 form's Krylov kernels with 16-byte accesses ----------------------
+// k_bs_pq and k_bs_xr for members that are not x-periodic, whose rows start a
+// multiple of 16 bytes apart and whose mask is 0 beside the node columns
+// (bs_pipe_layout_ok): a lane has four adjacent columns of its row, aligned in
+// memory, a warp marches down WQ_R rows. Neighbours are registers, the lanes
+// beside (a warp's first and last lane only serve as such: 120 of its 128
+// columns are its own) and the rows before and after; nothing is staged, no
+// barrier waits, and the loads of WQ_G rows are in flight together. Bound by
+// DRAM: qg 4096^2: k_bs_pq 71 us and k_bs_alpha 11 us, this 52 us (4.25 arrays:
+// 42 us at the copy rate); k_bs_xr 41 us and k_bs_conv 13 us, this 40 us (3.25
+// arrays: 32 us). 256 members: 87 -> 54 us, 54 -> 38 us.
+// Sums: four products of a row pairwise, four rows pairwise, the rest FP64.
+// SINGLE (one member): the last block sums the blocks' totals and sets alpha or
+// the convergence in place of k_bs_alpha, k_bs_conv.
+constexpr int WQ_R = 16, WQ_G = 4, WQ_C = 120, WQ_H = 8 * WQ_R;  // a block: WQ_H x WQ_C nodes
+
+struct WRow {
+    float4 v;
+    uint32_t m;  // fluid mask bytes
+};
+
+__device__ __forceinline__ float4 w_mask(float4 v, uint32_t m)
+{
+    return make_float4(m & 0xffu ? v.x : 0.f, m & 0xff00u ? v.y : 0.f, m & 0xff0000u ? v.z : 0.f,
+                       m & 0xff000000u ? v.w : 0.f);
+}
+
+__device__ __forceinline__ float w_dot(float4 a, float4 b)
+{
+    return fmaf(a.x, b.x, a.y * b.y) + fmaf(a.z, b.z, a.w * b.w);
+}
+
+template <bool SINGLE>
+__global__ void __launch_bounds__(256, 3)
+k_bs_pq4(const int4* __restrict__ tiles, const MGLevel* __restrict__ levs,
+         const float* __restrict__ z, float* __restrict__ q, DevScalars* __restrict__ scs,
+         double* partials, float* ring, long long rstride, BSGlobals* eg)
+{
+    pdl_wait();
+    const int4 tl = tiles[blockIdx.x];
+    DevScalars& sc = scs[tl.x];
+    if (bs_skip(sc, 1)) return;
+    const MGLevel& L = levs[tl.x * BS_LMAX];
+    const int it = sc.iter_in, lane = threadIdx.x;
+    const bool first = it == 0;
+    const float* __restrict__ po = ring + (long long)max(it - 1, 0) * rstride;
+    float* __restrict__ pn = ring + (long long)it * rstride;
+    const uint8_t* __restrict__ gm = L.m;
+    const float beta = (float)sc.beta, cx = L.fcx, cy = L.fcy, md = L.fmd;
+    const int nyn = L.nyn, nxn = L.nxn, I = tl.y + 4 * (lane - 1);
+    const int J0 = tl.z + (int)threadIdx.y * WQ_R;
+    const long long pitch = L.pitch, k0 = L.off + I;
+    const bool col = I + 3 >= 0 && I < nxn, own = col && lane > 0 && lane < 31;
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    double acc = 0.0;
+    // rows j .. j + n - 1 of p
+    auto rows = [&](int j, auto& out) {
+        constexpr int n = sizeof(out) / sizeof(WRow);
+        float4 zv[n], pv[n];
+#pragma unroll
+        for (int u = 0; u < n; ++u) {
+            const bool in = col && j + u >= 0 && j + u < nyn;
+            const long long k = k0 + (j + u) * pitch;
+            out[u].m = in ? *(const uint32_t*)(gm + k) : 0u;
+            zv[u] = in ? *(const float4*)(z + k) : zero4;
+            pv[u] = in && !first ? *(const float4*)(po + k) : zero4;
+        }
+#pragma unroll
+        for (int u = 0; u < n; ++u) {
+            float4 v = zv[u];
+            if (!first)
+                v = make_float4(v.x + beta * pv[u].x, v.y + beta * pv[u].y, v.z + beta * pv[u].z,
+                                v.w + beta * pv[u].w);
+            out[u].v = w_mask(v, out[u].m);
+        }
+    };
+    if (J0 < nyn) {
+        WRow e[2];
+        rows(J0 - 1, e);
+        WRow a = e[0], c = e[1];  // the rows above and at j
+#pragma unroll 1
+        for (int j = J0; j < J0 + WQ_R && j < nyn; j += WQ_G) {
+            WRow b[WQ_G];
+            rows(j + 1, b);
+            float s[WQ_G];
+#pragma unroll
+            for (int u = 0; u < WQ_G; ++u) {
+                const float4 v = c.v, n = b[u].v;
+                const float we = __shfl_up_sync(0xffffffffu, v.w, 1);
+                const float ea = __shfl_down_sync(0xffffffffu, v.x, 1);
+                const float4 qv = w_mask(
+                    make_float4(apply_diff<float>(cx, cy, md, v.x, we, v.y, a.v.x, n.x),
+                                apply_diff<float>(cx, cy, md, v.y, v.x, v.z, a.v.y, n.y),
+                                apply_diff<float>(cx, cy, md, v.z, v.y, v.w, a.v.z, n.z),
+                                apply_diff<float>(cx, cy, md, v.w, v.z, ea, a.v.w, n.w)),
+                    c.m);
+                const bool st = own && j + u < nyn;
+                if (st) {
+                    const long long k = k0 + (j + u) * pitch;
+                    *(float4*)(pn + k) = v;
+                    *(float4*)(q + k) = qv;
+                }
+                s[u] = st ? w_dot(v, qv) : 0.f;
+                a = c;
+                c = b[u];
+            }
+            acc += (double)((s[0] + s[1]) + (s[2] + s[3]));
+        }
+    }
+    __shared__ double sh[32];
+    double w[1] = {acc};
+    block_reduce<1, false>(w, sh);
+    if (tid256() == 0) partials[blockIdx.x] = w[0];
+    if constexpr (SINGLE) {
+        if (!last_block(&eg->ticket[2], gridDim.x)) return;
+        const double tot = grid_sum(partials, gridDim.x);
+        if (tid256() == 0) set_alpha(sc, 1, tot);
+    }
+}
+
+template <bool SINGLE>
+__global__ void __launch_bounds__(256, 3)
+k_bs_xr4(const int4* __restrict__ tiles, const MGLevel* __restrict__ levs,
+         float* __restrict__ r, const float* __restrict__ q, DevScalars* __restrict__ scs,
+         double* partials, BSGlobals* eg, cudaGraphConditionalHandle cond)
+{
+    pdl_wait();
+    const int4 tl = tiles[blockIdx.x];
+    DevScalars& sc = scs[tl.x];
+    if (bs_skip(sc, 1)) return;
+    const MGLevel& L = levs[tl.x * BS_LMAX];
+    const int lane = threadIdx.x;
+    const uint8_t* __restrict__ gm = L.m;
+    const float al = (float)sc.alpha;
+    const int nyn = L.nyn, I = tl.y + 4 * (lane - 1);
+    const int J0 = tl.z + (int)threadIdx.y * WQ_R;
+    const long long pitch = L.pitch, k0 = L.off + I;
+    const bool own = I + 3 >= 0 && I < L.nxn && lane > 0 && lane < 31;
+    double acc = 0.0;
+    if (own) {
+#pragma unroll 1
+        for (int j = J0; j < J0 + WQ_R && j < nyn; j += WQ_G) {
+            float4 rv[WQ_G], qv[WQ_G];
+            uint32_t m[WQ_G];
+            float s[WQ_G];
+#pragma unroll
+            for (int u = 0; u < WQ_G; ++u) {
+                const long long k = k0 + min(j + u, nyn - 1) * pitch;
+                m[u] = *(const uint32_t*)(gm + k);
+                rv[u] = *(const float4*)(r + k);
+                qv[u] = *(const float4*)(q + k);
+            }
+#pragma unroll
+            for (int u = 0; u < WQ_G; ++u) {
+                const float4 d = w_mask(qv[u], m[u]);
+                const float4 v = make_float4(rv[u].x - al * d.x, rv[u].y - al * d.y,
+                                             rv[u].z - al * d.z, rv[u].w - al * d.w);
+                const bool st = j + u < nyn;
+                if (st) *(float4*)(r + k0 + (j + u) * pitch) = v;
+                const float4 f = w_mask(v, m[u]);
+                s[u] = st ? w_dot(f, f) : 0.f;
+            }
+            acc += (double)((s[0] + s[1]) + (s[2] + s[3]));
+        }
+    }
+    __shared__ double sh[32];
+    double w[1] = {acc};
+    block_reduce<1, false>(w, sh);
+    if (tid256() == 0) partials[blockIdx.x] = w[0];
+    if constexpr (SINGLE) {
+        if (!last_block(&eg->ticket[3], gridDim.x)) return;
+        const double tot = grid_sum(partials, gridDim.x);
+        if (tid256() == 0) {
+            set_conv(sc, eg, 1, tot);
+            eg->loops_in += 1;
+            if (cond) cudaGraphSetConditional(cond, *(volatile int*)&eg->active_in > 0 ? 1u : 0u);
+        }
     }
 }
 
@@ -738,7 +957,7 @@ __global__ void k_bs_setup(DevScalars* scs, int n, double tol2, int maxit, doubl
     if (b == 0) {
         eg->active_out = 0;
         eg->active_in = 0;
-        for (int k = 0; k < 4; ++k) eg->ticket[k] = 0;
+        for (int k = 0; k < 8; ++k) eg->ticket[k] = 0;
     }
     if (b < n) {
         DevScalars& s = scs[b];
@@ -847,12 +1066,12 @@ static int vcycle_pipe(BatchSolver& s, cudaStream_t st, int ir)
         if (n == 0) continue;
         if (l > 0)
             launch_pdl(k_mgp_up<NU, false>, dim3(std::min(n, s.pipe_gup)), blk, sizeof(MPUp), st,
-                       (const int4*)s.mtiles[l], n, (const MGLevel*)s.dlevs, maps, l,
-                       (const DevScalars*)s.scs, ir, (double*)nullptr, status);
+                       (const int4*)s.mtiles[l], n, (const MGLevel*)s.dlevs, maps, l, s.scs, ir,
+                       (double*)nullptr, (unsigned*)nullptr, status);
         else
             launch_pdl(k_mgp_up<NU, true>, dim3(std::min(n, s.pipe_gup)), blk, sizeof(MPUp), st,
-                       (const int4*)s.mtiles[0], n, (const MGLevel*)s.dlevs, maps, 0,
-                       (const DevScalars*)s.scs, ir, s.mpartials, status);
+                       (const int4*)s.mtiles[0], n, (const MGLevel*)s.dlevs, maps, 0, s.scs, ir,
+                       s.mpartials, s.n == 1 ? &s.eg->ticket[4] : (unsigned*)nullptr, status);
         cnt += 1;
     }
     return cnt;
@@ -891,6 +1110,33 @@ static int vcycle(BatchSolver& s, cudaStream_t st, int ir)
     return s.nu >= 2 ? vcycle_nu<S, 2, TH>(s, st, ir) : vcycle_nu<S, 1, TH>(s, st, ir);
 }
 
+// the Krylov part of the inner FP32 loop's body with the wide kernels
+static int wide_krylov(BatchSolver& s, cudaStream_t st, cudaGraphConditionalHandle cond)
+{
+    const dim3 blk(32, 8), gr(s.nqtiles);
+    const int4* qt = s.qtiles;
+    const MGLevel* lv = s.dlevs;
+    const float* z = (const float*)s.v.z;
+    float *q = (float*)s.v.q, *r = (float*)s.v.rin;
+    const long long ne = s.v.nelem;
+    if (s.n == 1) {
+        launch_pdl(k_bs_pq4<true>, gr, blk, 0, st, qt, lv, z, q, s.scs, s.partials, s.pring, ne,
+                   s.eg);
+        launch_pdl(k_bs_xr4<true>, gr, blk, 0, st, qt, lv, r, (const float*)q, s.scs, s.partials,
+                   s.eg, cond);
+        return 2;
+    }
+    launch_pdl(k_bs_pq4<false>, gr, blk, 0, st, qt, lv, z, q, s.scs, s.partials, s.pring, ne,
+               s.eg);
+    launch_pdl(k_bs_alpha, dim3(s.n), dim3(s.fin_threads), 0, st, (const BSInfo*)s.dinfo, s.scs,
+               (const double*)s.partials, 1, 1);
+    launch_pdl(k_bs_xr4<false>, gr, blk, 0, st, qt, lv, r, (const float*)q, s.scs, s.partials,
+               s.eg, cond);
+    launch_pdl(k_bs_conv, dim3(s.n), dim3(s.fin_threads), 0, st, (const BSInfo*)s.dinfo, s.scs,
+               (const double*)s.partials, s.eg, cond, 1, s.n, 1);
+    return 4;
+}
+
 // the CG loop body; FP64 form (S = V = double) or the inner FP32 loop
 template <typename S, typename V, int TH>
 static int cg_body(BatchSolver& s, cudaStream_t st, cudaGraphConditionalHandle cond, int ir)
@@ -900,23 +1146,29 @@ static int cg_body(BatchSolver& s, cudaStream_t st, cudaGraphConditionalHandle c
     V* r = (V*)(ir ? s.v.rin : s.v.r64);
     V* x = ir ? (V*)nullptr : (V*)s.v.x64;  // the refinement form's x is the ring
     int cnt = vcycle<S, TH>(s, st, ir);
-    if (s.maxl > 0) {
+    constexpr bool F = std::is_same<S, float>::value;
+    if (s.maxl > 0 && !(F && s.pipe && s.n == 1)) {  // (one member: in the up leg)
         launch_pdl(k_bs_rz, dim3(s.n), dim3(s.fin_threads), 0, st, (const BSInfo*)s.dinfo, s.scs,
                    (const double*)s.mpartials, ir);
         cnt += 1;
     }
+    if constexpr (F)
+        if (s.wide) {
+            s.body_launches = cnt + wide_krylov(s, st, cond);
+            return (int)cudaGetLastError();
+        }
     V* ring = ir ? (V*)s.pring : (V*)nullptr;
     launch_pdl(k_bs_pq<S, V, TH>, dim3(resident_grid<k_bs_pq<S, V, TH>>(nt)), blk, 0, st,
                (const int4*)s.rtiles, nt, (const MGLevel*)s.dlevs, (const S*)s.v.z, (V*)s.v.p,
                (V*)s.v.p2, (V*)s.v.q, (const DevScalars*)s.scs, s.partials, ir, ring,
                (long long)s.v.nelem);
     launch_pdl(k_bs_alpha, dim3(s.n), dim3(s.fin_threads), 0, st, (const BSInfo*)s.dinfo, s.scs,
-               (const double*)s.partials, ir);
+               (const double*)s.partials, ir, 0);
     launch_pdl(k_bs_xr<V, TH>, dim3(resident_grid<k_bs_xr<V, TH>>(nt)), blk, 0, st,
                (const int4*)s.rtiles, nt, (const MGLevel*)s.dlevs, x, r, (const V*)s.v.p,
                (const V*)s.v.p2, (const V*)s.v.q, (const DevScalars*)s.scs, s.partials, ir);
     launch_pdl(k_bs_conv, dim3(s.n), dim3(s.fin_threads), 0, st, (const BSInfo*)s.dinfo, s.scs,
-               (const double*)s.partials, s.eg, cond, ir, s.n);
+               (const double*)s.partials, s.eg, cond, ir, s.n, 0);
     cnt += 4;
     s.body_launches = cnt;
     return (int)cudaGetLastError();
@@ -1433,10 +1685,26 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
     }
     s.nrtiles = s.ntiles[0];
     s.rtiles = s.tiles[0];
+    // tiles of the wide kernels: every node (theirs differ from the tiles
+    // above, whose nodes all need their p), lane 1's first column
+    std::vector<int4> qt;
+    for (int b = 0; b < s.n; ++b) {
+        const MGLevel& L = levs[(size_t)b * BS_LMAX];
+        info[b].q0 = (int)qt.size();
+        for (int J0 = 0; J0 < L.nyn; J0 += WQ_H)
+            for (int I0 = -(int)(L.off & 3); I0 < L.nxn; I0 += WQ_C)
+                qt.push_back(make_int4(b, I0, J0, 0));
+        info[b].qn = (int)qt.size() - info[b].q0;
+    }
+    s.nqtiles = (int)qt.size();
+    s.qtiles = (int4*)dal(qt.size() * sizeof(int4));
+    if (!s.qtiles || cudaMemcpy(s.qtiles, qt.data(), qt.size() * sizeof(int4),
+                                cudaMemcpyHostToDevice) != cudaSuccess)
+        return 2;
     s.dlevs = (MGLevel*)dal(levs.size() * sizeof(MGLevel));
     s.dinfo = (BSInfo*)dal(info.size() * sizeof(BSInfo));
     s.eg = (BSGlobals*)dal(sizeof(BSGlobals));
-    s.partials = (double*)dal((rt.size() * 2 + 64) * sizeof(double));
+    s.partials = (double*)dal((std::max(rt.size() * 2, qt.size()) + 64) * sizeof(double));
     s.mpartials = (double*)dal((mt[0].size() + 64) * sizeof(double));
     if (!s.mpartials) return 2;
     if (!s.dlevs || !s.dinfo || !s.eg || !s.partials) return 2;
@@ -1465,6 +1733,15 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
         const int e = bs_pipe_setup(s, levs, info, dal);
         if (e) return e;
     }
+    // the wide Krylov kernels: where the pipelined level kernels run (aligned
+    // rows, no mask byte beside the node columns) and no member wraps around
+    s.wide = s.pipe && v.nelem % 4 == 0;
+    for (int b = 0; b < s.n; ++b) {
+        const MGLevel& L = levs[(size_t)b * BS_LMAX];
+        s.wide = s.wide && !L.per && L.pitch % 4 == 0 && (uintptr_t)L.m % 4 == 0;
+    }
+    for (const void* p : {(const void*)v.z, (const void*)v.q, (const void*)v.rin})
+        s.wide = s.wide && (uintptr_t)p % 16 == 0;
     // The persistent solve: every FP64 problem (its level kernels and loops
     // cost more at every size), and FP32 problems of up to PS_FP32_NODES nodes
     // (batches half of that):

@@ -20,11 +20,12 @@ struct BSInfo {
     // the member's range in the level-0 table of the multigrid level kernels
     // (the tile totals of <r, z> written by the level-0 up leg); mnn = 0 when
     // level 0 is in the member's tail
-    int mn0, mnn, pad0, pad1;
+    int mn0, mnn;
+    int q0, qn;              // in the table of the wide Krylov kernels
 };
 
 struct BSGlobals {
-    unsigned int ticket[4];
+    unsigned int ticket[8];
     int active_out, active_in;  // members still iterating (outer / inner)
     int status, pad;
     long long loops_out, loops_in;  // loop iterations (all members together)
@@ -83,6 +84,10 @@ struct BatchSolver {
     int pipe_gdown = 0, pipe_gup = 0;
     int4* rtiles = nullptr;    // level-0 tiles of the Krylov kernels
     int nrtiles = 0;
+    // FP32 form: the wide Krylov kernels (k_bs_pq4, k_bs_xr4) and their tiles
+    bool wide = false;
+    int4* qtiles = nullptr;
+    int nqtiles = 0;
     int maxl = 0;
     size_t tail_smem = 0;
     int tail_threads = 1024;  // block size of k_bs_tail (bs_build)
