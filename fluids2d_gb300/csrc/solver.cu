@@ -950,6 +950,72 @@ k_bs_correct(const int4* __restrict__ tiles, const MGLevel* __restrict__ levs,
     }
 }
 
+// k_bs_correct in the same layout: qg 4096^2, eight directions: 236 -> 187 us.
+// (The FP64 residual gains nothing from it, 293 -> 309 us: its pipe is busy
+// either way, and the side lanes cost it a fifteenth of its instructions.)
+__global__ void __launch_bounds__(256, 2)
+k_bs_correct4(const int4* __restrict__ tiles, const MGLevel* __restrict__ levs,
+              double* __restrict__ x, const float* __restrict__ ring, long long rstride,
+              const DevScalars* __restrict__ scs)
+{
+    const int4 tl = tiles[blockIdx.x];
+    const DevScalars& sc = scs[tl.x];
+    if (sc.converged) return;
+    const MGLevel& L = levs[tl.x * BS_LMAX];
+    const uint8_t* __restrict__ gm = L.m;
+    const int zero = sc.zero, kit = sc.iter_in;
+    const int nyn = L.nyn, lane = threadIdx.x, I = tl.y + 4 * (lane - 1);
+    const int J0 = tl.z + (int)threadIdx.y * WQ_R;
+    if (!(I + 3 >= 0 && I < L.nxn && lane > 0 && lane < 31)) return;
+    const long long pitch = L.pitch, k0 = L.off + I;
+    constexpr int G = 2, CH = 4;  // rows and directions in flight
+#pragma unroll 1
+    for (int j = J0; j < J0 + WQ_R && j < nyn; j += G) {
+        long long k[G];
+        float4 e[G];
+        uint32_t m[G];
+        double2 xa[G], xb[G];
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+            k[u] = k0 + min(j + u, nyn - 1) * pitch;
+            e[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            m[u] = *(const uint32_t*)(gm + k[u]);
+            xa[u] = *(const double2*)(x + k[u]);
+            xb[u] = *(const double2*)(x + k[u] + 2);
+        }
+        // e = sum alpha_i p_i in the order of the iterations, as k_bs_correct
+        for (int i0 = 0; i0 < kit; i0 += CH) {
+            float4 pv[CH][G];
+#pragma unroll
+            for (int c = 0; c < CH; ++c)
+#pragma unroll
+                for (int u = 0; u < G; ++u)
+                    pv[c][u] = *(const float4*)(ring + (long long)min(i0 + c, kit - 1) * rstride +
+                                                k[u]);
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                if (i0 + c >= kit) break;
+                const float a = sc.ahist[i0 + c];
+#pragma unroll
+                for (int u = 0; u < G; ++u)
+                    e[u] = make_float4(fmaf(a, pv[c][u].x, e[u].x), fmaf(a, pv[c][u].y, e[u].y),
+                                       fmaf(a, pv[c][u].z, e[u].z), fmaf(a, pv[c][u].w, e[u].w));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+            if (j + u >= nyn) break;
+            auto at = [&](double xv, float ev, uint32_t mv) {
+                return !mv ? xv : zero ? 0.0 : xv + f32_to_f64(ev);
+            };
+            *(double2*)(x + k[u]) = make_double2(at(xa[u].x, e[u].x, m[u] & 0xffu),
+                                                 at(xa[u].y, e[u].y, m[u] & 0xff00u));
+            *(double2*)(x + k[u] + 2) = make_double2(at(xb[u].x, e[u].z, m[u] & 0xff0000u),
+                                                     at(xb[u].y, e[u].w, m[u] & 0xff000000u));
+        }
+    }
+}
+
 __global__ void k_bs_setup(DevScalars* scs, int n, double tol2, int maxit, double tol_in2,
                            int maxit_in, int maxouter, BSGlobals* eg)
 {
@@ -1283,9 +1349,14 @@ static int bs_record_t(BatchSolver& s, cudaStream_t st, cudaStream_t st2, int* l
     k_bs_refine_fin<<<s.n, s.fin_threads, 0, st>>>(s.dinfo, s.scs, s.partials, s.eg, 1, cond_o, s.n);
     fixed += 3;
     auto round_tail = [&](cudaStream_t sb) {
-        k_bs_correct<TH><<<nt, blk, 0, sb>>>(s.rtiles, s.dlevs, (double*)s.v.x64,
-                                             (const float*)s.pring, (long long)s.v.nelem,
-                                             s.scs);
+        if (s.wide && (uintptr_t)s.v.x64 % 16 == 0)  // (x is given per solve)
+            k_bs_correct4<<<s.nqtiles, blk, 0, sb>>>(s.qtiles, s.dlevs, (double*)s.v.x64,
+                                                     (const float*)s.pring,
+                                                     (long long)s.v.nelem, s.scs);
+        else
+            k_bs_correct<TH><<<nt, blk, 0, sb>>>(s.rtiles, s.dlevs, (double*)s.v.x64,
+                                                 (const float*)s.pring, (long long)s.v.nelem,
+                                                 s.scs);
         k_bs_reset<<<1, 1, 0, sb>>>(s.eg);
         launch_refine<TH, false>(s, sb);
         k_bs_refine_fin<<<s.n, s.fin_threads, 0, sb>>>(s.dinfo, s.scs, s.partials, s.eg, 0, cond_o, s.n);
