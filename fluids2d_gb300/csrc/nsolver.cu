@@ -863,10 +863,11 @@ __device__ __forceinline__ double nc_ax(const NCoarse& C, int l, const double* x
 __device__ __forceinline__ void nc_half(const NCoarse& C, int l, double* x, const double* b,
                                         const double* fx, const double* fy, int color)
 {
-    const int nx = C.nxn[l], n = nx * C.nyn[l], o = C.off[l];
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const int J = k / nx, I = k - J * nx;
-        if (((J + I) & 1) != color) continue;
+    // (the colour's cells only: an FP64 instruction takes as long for half a warp)
+    const int nx = C.nxn[l], wc = (nx + 1) / 2, n = wc * C.nyn[l], o = C.off[l];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int J = i / wc, I = 2 * (i - J * wc) + ((J + color) & 1), k = J * nx + I;
+        if (I >= nx) continue;
         double cs;
         const double ax = nc_ax(C, l, x, fx, fy, J, I, cs);
         if (cs > 0.0) x[o + k] += (ax - b[o + k]) / cs;
