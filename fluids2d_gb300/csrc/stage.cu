@@ -60,7 +60,7 @@ template <> __device__ __forceinline__ float of<float>(double, float f) { return
 // equations.py:29-35).
 // ---------------------------------------------------------------------------
 template <typename T, int M, int TYK>
-__global__ void __launch_bounds__(TX * TYK, sizeof(T) == 4 ? 4 : 2)
+__global__ void __launch_bounds__(TX * TYK, sizeof(T) == 4 ? 4 : 3)
 k_rsw_stage(const __grid_constant__ CUtensorMap th,
             const __grid_constant__ CUtensorMap tw, RswIn a,
             const uint32_t* __restrict__ code, int stage, Geom g, DevScalars* sc)
