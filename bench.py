@@ -102,9 +102,9 @@ ENSEMBLE_DESC = ("ensemble of 256 eulerpsi closed basins, sizes uniform in "
 
 
 def solver_roofline(timer, pipelined, handle, workload, peak, peak_src):
-    """Roofline of the solver's largest kernel (the level-0 down leg of the
-    V-cycle, k_mgp_down when the solver runs the pipelined FP32 kernels, else
-    k_mg_down: b and mask read, the pre-smoothed x written, the restricted
+    """Roofline of the solver's level-0 down leg of the V-cycle (k_mgp_down when
+    the FP32 level arrays fit the pipelined kernels, else the leg of the FP64
+    persistent solve, k_ps_down0: b and mask read, the pre-smoothed x written, the restricted
     right-hand side written at a quarter of the nodes = (2.25 es + 1) bytes
     per level-0 node), timed alone with CUDA events, L2 flushed."""
     import ctypes
@@ -119,7 +119,7 @@ def solver_roofline(timer, pipelined, handle, workload, peak, peak_src):
         return None
     alg = nodes.value * (2.25 * es.value + 1)
     achieved = alg / (avg.value * 1e-3) / 1e9
-    kname = "k_mgp_down" if pipe.value else "k_mg_down"
+    kname = "k_mgp_down" if pipe.value else "k_ps_down0"
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak,
             "traffic": read_profile_traffic(f"{kname}_{workload}"),

@@ -1,7 +1,9 @@
 // Pipelined FP32 multigrid level kernels: the down and up legs of the
 // V-cycle on the grid levels finer than a member's tail, in the FP32 refinement
 // form (solver.cu launches them when the level arrays pass the layout checks
-// of bs_build; the FP64 form and the other cases keep mg_reg.cuh's kernels).
+// of bs_build; the other cases keep mg_reg.cuh's kernels). They run the FP32
+// problems that are too large for the persistent solve (psolver.cu); of a
+// single model only the finest levels, the coarser ones in k_ps_cycle.
 //
 // Same smoothing arithmetic and region geometry as mg_reg.cuh (a block
 // smooths a tile of MR_TH x MR_TW nodes from a region of MR_WY x MR_W nodes

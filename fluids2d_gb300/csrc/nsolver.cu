@@ -23,12 +23,12 @@
 // smooth errors, and the coarse correction comes out halved - half the sum is
 // the re-discretised coupling where the face is fully open and keeps the
 // partial openings of masked faces.) The first level of at most 2048 cells is
-// solved exactly with its precomputed dense pseudo-inverse (the FP32 form: 4096,
-// replaced by the matrix of the V-cycle from it on, coarse_map). The FP32 form runs the cycle in FP32
-// (levels, couplings and smoothing in float; its right-hand side is the FP64
-// Krylov residual rounded, its result converted back), while the Krylov
-// vectors, the operator products, the dot products and the zero-mean
-// projections stay FP64.
+// solved exactly with its precomputed dense pseudo-inverse (the FP32 form: 4096
+// cells and the matrix of the V-cycle from it on, coarse_map). The FP32 form
+// runs the cycle in FP32 (levels, couplings and smoothing in float; its
+// right-hand side is the FP64 Krylov residual rounded, its result converted
+// back), while the Krylov vectors, the operator products, the dot products and
+// the zero-mean projections stay FP64.
 //
 // The solve is one cooperative kernel (persist.cuh), one block per SM. CG in
 // the form of Chronopoulos and Gear (s-step methods for symmetric linear
@@ -45,7 +45,11 @@
 // A leg works on a tile and a halo of the 4 (B: 5) cells its half sweeps
 // reach over, in shared memory, so a leg needs one barrier; tile sizes are
 // chosen per level so that the chip is filled (pick_tile).
-// What bounds it: at 40^2 and 64^2 the barriers, at 512^2 the FP64 pipe.
+// What bounds it: at 40^2 (one iteration on the dense level, 48 us) the latency
+// of its phases and barriers; at 512^2 FP64 (75 us an iteration) the FP64 pipe,
+// 40 % busy, and between its bursts the loads of a phase and the barriers (2.6k
+// cycles each). One launch per sweep and level before it: 11.4 ms a step of
+// euler 512^2, now 2.1 ms with the warm start.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>

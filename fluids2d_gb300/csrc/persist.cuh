@@ -103,8 +103,9 @@ __device__ __forceinline__ bool ps_sync(PSGrid& g)
 }
 
 // ---- deterministic sums over the blocks --------------------------------------
-// The block's totals of N <= 4 per-thread values into part[k * stride]; after the next barrier every block adds all blocks' totals in one
-// fixed order, so all blocks hold the same bits and take the same decisions
+// The block's totals of N <= 4 per-thread values into part[k * stride]; after
+// the next barrier every block adds all blocks' totals in one fixed order, so
+// all blocks hold the same bits and take the same decisions
 // without a broadcast. An FP64 instruction of a warp occupies its SM
 // partition's pipe for 64 cycles, so sums and scalar arithmetic are kept to
 // few warps: a shuffle tree in all 16 warps, or three divisions in all

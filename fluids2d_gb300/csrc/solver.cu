@@ -12,6 +12,12 @@
 // WHILE nodes that run until every member has converged (converged members'
 // tiles are skipped).
 //
+// Most problems do not use these kernels: the FP64 form, and the FP32 form of
+// up to PS_FP32_NODES nodes, run the whole solve in one persistent kernel
+// (psolver.cu). What is here is the FP32 form of larger problems, and the FP64
+// form where that kernel does not apply (x-periodic levels of odd width, no
+// level small enough for the dense inverse).
+//
 // Two forms:
 //  * mode 0 (FP64): preconditioned CG in FP64 with an FP64 V-cycle.
 //  * mode 1 (FP32 + FP64 refinement): the outer loop forms the FP64 residual

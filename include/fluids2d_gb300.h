@@ -215,7 +215,9 @@ int f2d_time_stage(f2d_model m, int stage, int reps, int flush_l2,
  * timed over `reps` solves from the warm start 0.999 psi; the fastest that
  * reaches the tolerance is kept (the step graphs are re-captured). The state
  * is unchanged. Outputs may be NULL. Models with a vertex Poisson/Helmholtz
- * solve (eulerpsi, qg, qgrsw) and ensembles. */
+ * solve (eulerpsi, qg, qgrsw) and ensembles. Where the whole solve is one
+ * persistent kernel (FP64; FP32 up to 2M nodes, ensembles 1M) only the sweeps
+ * matter and only they are tried. */
 int f2d_autotune(f2d_model m, int reps, int *tile_rows, int *sweeps, double *tol_in,
                  double *ms_per_solve);
 /* Set the multigrid schedule directly (what f2d_autotune would pick):
@@ -223,17 +225,16 @@ int f2d_autotune(f2d_model m, int reps, int *tile_rows, int *sweeps, double *tol
  * tolerance of the FP32 form's refinement rounds (0 < tol_in < 1; unused in
  * the FP64 form). Recorded graphs are dropped. No reference counterpart. */
 int f2d_set_schedule(f2d_model m, int tile_rows, int sweeps, double tol_in);
-/* Time `reps` launches of the Poisson solver's level-0 down kernel
- * (pre-smoothing + residual + restriction of the V-cycle, the solver's largest
- * share) on the current right-hand side, L2 flushed between launches when
- * flush_l2 != 0; *avg_ms = mean ms, *nodes = level-0 nodes, *elem_bytes = 4
+/* Time `reps` launches of the Poisson solver's level-0 down leg
+ * (pre-smoothing + residual + restriction of the V-cycle; FP64: the same leg of
+ * the persistent solve kernel, launched by itself) on the current right-hand
+ * side, L2 flushed between launches when flush_l2 != 0; *avg_ms = mean ms, *nodes = level-0 nodes, *elem_bytes = 4
  * or 8 (multigrid precision). Measurement hook of the benchmark; no
  * reference counterpart. The model must have solved once. */
 int f2d_time_solver(f2d_model m, int reps, int flush_l2, double *avg_ms,
                     int64_t *nodes, int *elem_bytes);
-/* Which level kernels the solver timed by f2d_time_solver runs: *pipelined =
- * 1 for the persistent TMA-staged FP32 kernels (k_mgp_down / k_mgp_up), 0
- * for the one-tile-per-block kernels (k_mg_down / k_mg_up: the FP64 form,
+/* Which level kernels f2d_time_solver times: *pipelined = 1 for the persistent
+ * TMA-staged FP32 kernels (k_mgp_down / k_mgp_up), 0 otherwise (the FP64 form,
  * or level arrays outside the pipelined kernels' layout). Instrumentation,
  * no reference counterpart. The model must have solved once. */
 int f2d_solver_pipelined(f2d_model m, int *pipelined);
@@ -252,7 +253,7 @@ int f2d_test_tma_wait(int enabled, double limit_ms);
 int f2d_test_conversions(const double *x64, int64_t n64, float *sw32, float *hw32,
                          const float *x32, int64_t n32, double *sw64, double *hw64);
 /* Refinement rounds of the FP32 form's solves summed since creation (see
- * f2d_ensemble_refine_rounds). Instrumentation. */
+ * f2d_ensemble_refine_rounds; a persistent solve has none). Instrumentation. */
 int f2d_refine_rounds(f2d_model m, int64_t *rounds);
 /* Counters: Poisson iterations summed over all solves since creation; the
  * kernels one time step launches outside the Poisson loops; the kernels one
