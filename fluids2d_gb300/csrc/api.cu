@@ -403,7 +403,7 @@ static int rec_diag(f2d_model_s* m, int par, cudaStream_t s, int warm = -1)
         CKI(ns_record(m->ns, s, &fixed));
         if (g.xper) CKI(launch_fill_periodic(0, fb(m, "p"), g, s));
         CKI(launch_euler_project(m->prec, fb(m, "u.x", par), fb(m, "u.y", par),
-                                 (const double*)fb(m, "p"), m->d_code, g, s));
+                                 (const double*)fb(m, "p"), m->d_code, g, m->sc, s));
         m->rec_launches += 3 + fixed + (g.xper ? 1 : 0);
         RswDiag a;
         memset(&a, 0, sizeof(a));
@@ -416,13 +416,12 @@ static int rec_diag(f2d_model_s* m, int par, cudaStream_t s, int warm = -1)
         a.rdx2 = m->rdx2;
         a.rdy2 = m->rdy2;
         a.euler = 1;
+        a.maxu = 1;  // for set_dt (model.py:83-85)
         CKI(make_tmap(m, (void*)a.ux));
         CKI(make_tmap(m, (void*)a.uy));
         CKI(launch_rsw_diag(m->p.innerproduct, m->prec, tmap(m, (void*)a.ux),
                             tmap(m, (void*)a.uy), a, m->d_code, g, m->sc, s));
-        // max|U.x|, max|U.y| for set_dt (model.py:83-85)
-        CKI(launch_maxabs2(m->prec, a.Ux, a.Uy, g, m->sc, m->partials, s));
-        m->rec_launches += 2;
+        m->rec_launches += 1;
         return 0;
     }
     case F2D_MODEL_QGRSW: {

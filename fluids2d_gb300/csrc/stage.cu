@@ -325,12 +325,27 @@ k_rsw_stage(const __grid_constant__ CUtensorMap th,
     }
 }
 
+// bits of the warp's largest |v|, as a double's (NaN above all)
+__device__ __forceinline__ unsigned long long warp_max_abs(float v)
+{
+    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(v)));
+    return (unsigned long long)__double_as_longlong(f32_to_f64(__uint_as_float(m)));
+}
+__device__ __forceinline__ unsigned long long warp_max_abs(double v)
+{
+    const unsigned long long b = __double_as_longlong(v) & 0x7fffffffffffffffull;
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(b >> 32));
+    const unsigned lo =
+        __reduce_max_sync(0xffffffffu, (unsigned)(b >> 32) == hi ? (unsigned)b : 0u);
+    return (unsigned long long)hi << 32 | lo;
+}
+
 // ---------------------------------------------------------------------------
 // Rotating shallow water diagnostics (equations.py:150-155): sharp, vorticity
 // (times slip coefficient), WENO kinetic energy, pressure; omega and ke get
 // the halo fill.
 // ---------------------------------------------------------------------------
-template <typename T, int M, int TYK>
+template <typename T, int M, int TYK, bool MAXU>
 __global__ void __launch_bounds__(TX * TYK)
 k_rsw_diag(const __grid_constant__ CUtensorMap tux,
            const __grid_constant__ CUtensorMap tuy, RswDiag a,
@@ -344,14 +359,36 @@ k_rsw_diag(const __grid_constant__ CUtensorMap tux,
     if (!stage_tiles<T>(sx, &tux, sy, &tuy, i0, j0, &bar, &sc->status)) return;
 
     const int j = j0 + ty, i = i0 + tx;
-    if (j >= g.NY || i >= g.NX) return;
+    const bool in = j < g.NY && i < g.NX;
+    if (!MAXU && !in) return;
     const long long o = (long long)j * g.P + i;
     const int r = ty + OY, c = tx + OX;
     const T rdx2 = of<T>(a.rdx2, a.frdx2), rdy2 = of<T>(a.rdy2, a.frdy2);
     const T ux = sx[r][c], uy = sy[r][c];
     // sharp: U = u / dx^2 everywhere (no fill in the reference; u is filled)
-    ((T*)a.Ux)[o] = ux * rdx2;
-    ((T*)a.Uy)[o] = uy * rdy2;
+    if (in) {
+        ((T*)a.Ux)[o] = ux * rdx2;
+        ((T*)a.Uy)[o] = uy * rdy2;
+    }
+    // max |U| (set_dt, model.py:83-85) of euler and boussinesq here, where U is
+    // at hand, on the integer pipe: bits of |U| order as the values, NaN last. A
+    // kernel of its own was 5 to 9 us a stage.
+    if constexpr (MAXU) {
+        __shared__ unsigned long long smax[2];
+        if (tx == 0 && ty < 2) smax[ty] = 0ull;
+        __syncthreads();
+        const unsigned long long mx = warp_max_abs(in ? ux * rdx2 : T(0));
+        const unsigned long long my = warp_max_abs(in ? uy * rdy2 : T(0));
+        if (tx == 0) {
+            atomicMax(&smax[0], mx);
+            atomicMax(&smax[1], my);
+        }
+        __syncthreads();
+        unsigned long long* m = (unsigned long long*)(ty ? &sc->maxUy : &sc->maxUx);
+        if (tx == 0 && ty < 2 && smax[ty] > *(volatile unsigned long long*)m)
+            atomicMax(m, smax[ty]);
+        if (!in) return;
+    }
     if (!a.euler) ((T*)a.p)[o] = of<T>(a.goa, a.fgoa) * ((const T*)a.h)[o];
     if (!periodic_owner(g, i)) return;  // omega and ke: halo fill copies
     const uint32_t cd = code[o];
@@ -663,7 +700,9 @@ int launch_rsw_diag(int method, int prec, const CUtensorMap* tux,
     a.fgoa = (float)a.goa;
     const int ty = stage_rows(prec, g);
     dim3 grid = tile_grid(g, ty), block(TX, ty);
-#define F2D_RD(T, M, TYK) k_rsw_diag<T, M, TYK><<<grid, block, 0, s>>>(*tux, *tuy, a, code, g, sc)
+#define F2D_RD(T, M, TYK)                                                                       \
+    if (a.maxu) k_rsw_diag<T, M, TYK, true><<<grid, block, 0, s>>>(*tux, *tuy, a, code, g, sc); \
+    else k_rsw_diag<T, M, TYK, false><<<grid, block, 0, s>>>(*tux, *tuy, a, code, g, sc)
 #define F2D_DISPATCH(T, TYK)                                      \
     switch (method) {                                             \
     case METHOD_WENO: F2D_RD(T, METHOD_WENO, TYK); break;         \
@@ -880,13 +919,15 @@ __global__ void k_euler_div(const T* __restrict__ ux, const T* __restrict__ uy, 
     rhs[o] = -(double)d * area;
 }
 
-// u -= grad p (addgrad, operators.py:49-53), then the halo fill of u
+// u -= grad p (addgrad, operators.py:49-53), then the halo fill of u; the maxima
+// of |U| that k_rsw_diag forms next start at 0
 template <typename T>
 __global__ void k_euler_project(T* ux, T* uy, const double* __restrict__ p,
-                                const uint32_t* __restrict__ code, Geom g)
+                                const uint32_t* __restrict__ code, Geom g, DevScalars* sc)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    if (i == 0 && j == 0) sc->maxUx = sc->maxUy = 0.0;
     if (j >= g.NY || i >= g.NX || !periodic_owner(g, i)) return;
     const long long o = (long long)j * g.P + i;
     const uint32_t cd = code[o];
@@ -912,13 +953,13 @@ int launch_euler_div(int prec, const void* ux, const void* uy, void* dv, double*
 }
 
 int launch_euler_project(int prec, void* ux, void* uy, const double* p, const uint32_t* code,
-                         const Geom& g, cudaStream_t s)
+                         const Geom& g, DevScalars* sc, cudaStream_t s)
 {
     const dim3 gr = pt_grid(g), bl(32, 8);
     if (prec == 0)
-        k_euler_project<double><<<gr, bl, 0, s>>>((double*)ux, (double*)uy, p, code, g);
+        k_euler_project<double><<<gr, bl, 0, s>>>((double*)ux, (double*)uy, p, code, g, sc);
     else
-        k_euler_project<float><<<gr, bl, 0, s>>>((float*)ux, (float*)uy, p, code, g);
+        k_euler_project<float><<<gr, bl, 0, s>>>((float*)ux, (float*)uy, p, code, g, sc);
     return (int)cudaGetLastError();
 }
 

@@ -31,6 +31,7 @@ struct RswDiag {
     float frdx2, frdy2, fgoa;  // the same in FP32 (set by the launcher)
     int euler;          // euler model: no pressure from h
     int noke;           // qgrsw: no kinetic energy (equations.py:127-133)
+    int maxu;           // max |U.x|, |U.y| into the scalars (zeroed before)
 };
 
 int launch_fluxform_stage(int method, int prec, const CUtensorMap* tq,
@@ -240,6 +241,6 @@ int launch_bulk(int prec, const BulkArgs& a, const Geom& g, DevScalars* sc, doub
 // a field as packed (NY, NX) float32 (the history's dtype "f", io.py:71)
 int launch_to_f32(int prec, const void* in, float* out, const Geom& g, cudaStream_t s);
 int launch_euler_project(int prec, void* ux, void* uy, const double* p, const uint32_t* code,
-                         const Geom& g, cudaStream_t s);
+                         const Geom& g, DevScalars* sc, cudaStream_t s);
 
 }  // namespace f2d
