@@ -721,9 +721,13 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
         if (threadIdx.x == 0) c.irz = 1.0 / c.rz;  // for the next beta
         ++it;
     }
-    // zero-mean solution (its sum was formed with the last update)
+    // zero-mean solution (its sum was formed with the last update); 0 for a zero
+    // right-hand side, whatever x was on entry
     const double xm = c.xsum / A.nfluid;
-    n_cells(L, [&](int, int, long long k) { if (L.code[k]) A.x[k] -= xm; });
+    const bool zero = c.bb == 0.0;
+    n_cells(L, [&](int, int, long long k) {
+        if (L.code[k]) A.x[k] = zero ? 0.0 : A.x[k] - xm;
+    });
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sc->bb = c.bb;
         sc->rr = c.rr;

@@ -167,3 +167,30 @@ def test_uneven_ensemble(sizes, precision, tol):
         m.sync()
         assert rel_l2(e.get_field(b, "omega"), m.state.omega) <= tol, b
         assert rel_l2(e.get_field(b, "psi"), m.state.psi) <= tol, b
+
+
+@pytest.mark.parametrize("nx,ny,precision,xper", [
+    (32, 24, "fp64", False),   # one dense level
+    (128, 96, "fp64", True),
+    (32, 24, "fp32", True),
+    (128, 96, "fp32", False),
+])
+def test_fluid_at_rest_stays_at_rest(nx, ny, precision, xper):
+    """A zero right-hand side has the pressure 0, whatever was there before:
+    a flow that is stopped does not start again."""
+    case = wl.euler_case(n=nx, ny=ny, seed=8, nislands=1, xperiodic=xper)
+    m = _model("euler", nx, ny, case["msk"], precision=precision, xperiodic=xper,
+               Lx=case["Lx"], Ly=case["Ly"], cfl=0.5, tend=1e300, maxite=10 ** 9)
+    s = m.state
+    s.u.x[:], s.u.y[:] = case["fields"]["u.x"], case["fields"]["u.y"]
+    m.integrator.diag(s)
+    m.advance(3)
+    s = m.state
+    s.u.x[:] = 0.0
+    s.u.y[:] = 0.0
+    m.integrator.diag(s)
+    m.advance(2)
+    m.sync()
+    s = m.state
+    for a in (s.u.x, s.u.y, s.p):
+        assert np.all(a == 0)
