@@ -1460,10 +1460,10 @@ int f2d_set_coriolis(f2d_model m, const double* f)
     return 0;
 }
 
-// diag of what may be a new state: no second-order warm start of the next step
+// diag of what may be a new state: the next step has no history to start from
 static int diag_state(f2d_model_s* m)
 {
-    CK(cudaMemsetAsync(&m->sc->warm_ext, 0, sizeof(int), m->stream));
+    CK(cudaMemsetAsync(&m->sc->dt_warm, 0, WARM_BYTES, m->stream));
     return run_graph(m, 0);
 }
 
@@ -1837,7 +1837,7 @@ int f2d_autotune(f2d_model m, int reps, int* th, int* nu, double* tol_in, double
         return fail(1, "the autotuner tunes the multigrid of eulerpsi, qg and qgrsw");
     const int which = m->p.model == F2D_MODEL_EULERPSI ? 0 : 1;
     // the right-hand side and solution of the current state's diagnostics
-    int e = run_graph(m, 0);
+    int e = diag_state(m);
     if (e) return e;
     const void* b = fb(m, which == 0 ? "vomega" : "work");
     if (m->p.model == F2D_MODEL_QGRSW) {

@@ -72,36 +72,36 @@ struct DevScalars {
     // Robert-Asselin filter coefficient of the leap-frog integrator
     // (param.py:50 RAgamma, integrators.py:39-55)
     double ragamma;
-    // time step of the step whose stage increments the warm start keeps
-    // (0: none yet), by which the next step scales them, and whether they may
-    // be extrapolated to second order (not right after a diag: the state may
-    // be a new one). Written at stage 3; *0: copies of the step under way
+    // time step of the step whose stage increments the warm start keeps (0: none
+    // yet, or a diag since, whose state may be a new one: the increments of a
+    // stronger flow are too far off to start from, those of a NaN never end),
+    // by which the next step scales them. Written at stage 3; dt_warm0: the
+    // copy of the step under way
     double dt_warm, dt_warm0;
-    int warm_ext, warm_ext0;
     // step lengths (FP32) of the inner iterations of the current refinement
     // round: the round's correction is sum alpha_i p_i (solver.cu)
     float ahist[32];
 };
 
 // The warm start's state as stage MODE + 1 of a step reads it, and its update
-// by one thread of the grid: a grid never reads what it writes.
+// by one thread of the grid: a grid never reads what it writes. Without hist
+// (no step before, or one of less than 1/64 of this step's size, whose
+// increments are mostly rounding) no array of the history may be read.
 struct WarmState {
-    bool hist, ext;
+    bool hist;
     double rho;
 };
 template <int MODE> __device__ __forceinline__ WarmState warm_state(DevScalars* sc, bool owner)
 {
     const double last = MODE == 0 ? sc->dt_warm : sc->dt_warm0;
-    const int ext = MODE == 0 ? sc->warm_ext : sc->warm_ext0;
-    if (MODE == 0 && owner) {
-        sc->dt_warm0 = last;
-        sc->warm_ext0 = ext;
-    } else if (MODE == 2 && owner) {
-        sc->dt_warm = sc->dt;
-        sc->warm_ext = 1;
-    }
-    return {last > 0.0, last > 0.0 && ext, last > 0.0 ? sc->dt / last : 0.0};
+    if (MODE == 0 && owner) sc->dt_warm0 = last;
+    if (MODE == 2 && owner) sc->dt_warm = sc->dt;
+    const double rho = last > 0.0 ? sc->dt / last : 0.0;
+    const bool hist = rho > 0.0 && rho <= 64.0;  // (false for NaN)
+    return {hist, hist ? rho : 0.0};
 }
+// Host: bytes to clear from dt_warm on to drop the history
+constexpr size_t WARM_BYTES = 2 * sizeof(double);
 
 // ---------------------------------------------------------------------------
 // Small PTX helpers: TMA tile loads through an mbarrier, with a time-bounded

@@ -878,8 +878,8 @@ int64_t f2d_ensemble_packed_size(f2d_ensemble e)
 int f2d_ensemble_diag(f2d_ensemble e)
 {
     if (!e) return f2d_internal_fail(1, "null ensemble");
-    // the states may be new ones: no second-order warm start of the next step
-    if (cudaMemset2DAsync(&e->scs->warm_ext, sizeof(DevScalars), 0, sizeof(int), e->n,
+    // the states may be new ones: the next step has no history to start from
+    if (cudaMemset2DAsync(&e->scs->dt_warm, sizeof(DevScalars), 0, WARM_BYTES, e->n,
                           e->stream) != cudaSuccess)
         return f2d_internal_fail(3, "cudaMemset2DAsync");
     return ens_run_graph(e, 0);

@@ -838,26 +838,28 @@ __global__ void __launch_bounds__(256) k_p_warm(WarmArrays w, const uint32_t* __
 {
     const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const WarmState ws = warm_state<MODE>(sc, k == 0);
+    const bool hist = ws.hist;
     const double rho = ws.rho;
     if (k < n && (code[k] & B_MSK)) {
         const double p = w.psi[k];
         if constexpr (MODE == 0) {
-            if (ws.hist) {
-                const double S2 = w.d1[k], e1 = ws.ext ? w.e1[k] : 0.0;
-                w.e3[k] = ws.ext ? fma(1.5, p, -0.375 * (w.s0[k] + S2)) : 0.0;
+            if (hist) {
+                const double S2 = w.d1[k], e1 = w.e1[k];
+                w.e3[k] = fma(1.5, p, -0.375 * (w.s0[k] + S2));
                 w.psi[k] = rho * (S2 + e1);
             }
         } else if constexpr (MODE == 1) {
-            const double d1 = w.d1[k], d2 = w.d2[k], e2 = ws.ext ? w.e2[k] : 0.0;
+            const double d1 = hist ? w.d1[k] : 0.0, d2 = hist ? w.d2[k] : 0.0;
+            const double e2 = hist ? w.e2[k] : 0.0;
             w.s0[k] = p;
-            w.e1[k] = ws.ext ? fma(-rho, d1, p) : 0.0;
+            w.e1[k] = hist ? fma(-rho, d1, p) : 0.0;
             w.psi[k] = fma(0.25 * rho, d2 + e2, -0.5 * p);
         } else {
-            const double S1 = w.s0[k], d2 = w.d2[k], e3 = w.e3[k];
+            const double S1 = w.s0[k], d2 = hist ? w.d2[k] : 0.0, e3 = hist ? w.e3[k] : 0.0;
             const double S2 = fma(4.0, p, 3.0 * S1), D = S2 - S1;
             w.d1[k] = S2;
             w.d2[k] = D;
-            w.e2[k] = ws.ext ? fma(-rho, d2, D) : 0.0;
+            w.e2[k] = hist ? fma(-rho, d2, D) : 0.0;
             w.psi[k] = fma(rho * (2.0 / 3.0), e3, 0.25 * (S1 + S2));
         }
     }

@@ -72,8 +72,9 @@ int launch_set_dt(DevScalars* sc, cudaStream_t s);
 // and 4.4e-6 to 1.7e-6, 9e-7 and 5.5e-7, on qg 128^2 turbulence from 1.3e-3,
 // 7.5e-4 and 4.7e-4 to 5.6e-4, 5.6e-4 and 3.2e-4. Where the increments of a
 // step come down to the FP32 rounding of the state (psi_warm_brackets) the
-// brackets are noise and left out. A guess only moves the solve's starting
-// point.
+// brackets are noise and left out. A guess moves the solve's starting point, and
+// the residual that its recurrence can attain by about eps times the largest
+// iterate: it must not be larger than the solution (no history across a diag).
 struct WarmArrays {
     double* psi;  // in: the last solution; out: the guess
     double* s0;   // psi at the step start
@@ -96,7 +97,7 @@ inline bool psi_warm_brackets(int prec, long long points)
 // there: 16-byte loads and stores, all the loads of the U pairs before any
 // store (the arrays do not overlap, but a store ahead of a load through
 // another pointer would hold the load back). ok[u] false skips pair u. The
-// brackets are 0 without ws.ext. The large grids are bound by the FP64
+// brackets are 0 without ws.hist. The large grids are bound by the FP64
 // pipe here too, so the mode and the brackets (EXT) are compile-time.
 // e3 holds t3 = 1.5 psi0 + 0.75 (S1 + S2) of the step between its stages 2
 // and 3 (S3 - (S1 + S2)/2 = 1.5 psi3 - t3).
@@ -111,14 +112,14 @@ __device__ __forceinline__ void psi_warm_pairs(const WarmArrays& w, const long l
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const double2 z = make_double2(0.0, 0.0);
-        const bool h = ok[u] && hist, hb = ok[u] && ws.ext;
+        const bool h = ok[u] && hist;
         a[u] = ok[u] ? *(const double2*)(w.psi + k[u]) : z;
         s0[u] = MODE >= 1 && ok[u] ? *(const double2*)(w.s0 + k[u]) : z;
         p1[u] = MODE == 2 && ok[u] ? *(const double2*)(w.p1 + k[u]) : z;
         d1[u] = (MODE == 0 || (MODE == 1 && EXT)) && h ? *(const double2*)(w.d1 + k[u]) : z;
         d2[u] = (MODE == 1 || (MODE == 2 && EXT)) && h ? *(const double2*)(w.d2 + k[u]) : z;
-        e[u] = EXT && hb ? *(const double2*)(ein + k[u]) : z;
-        t3[u] = EXT && MODE == 0 && hb ? *(const double2*)(w.e3 + k[u]) : z;
+        e[u] = EXT && h ? *(const double2*)(ein + k[u]) : z;
+        t3[u] = EXT && MODE == 0 && h ? *(const double2*)(w.e3 + k[u]) : z;
     }
     const double rq = 0.25 * rho, r23 = rho * (2.0 / 3.0);
     // one element: the guess g, the bracket en, mode 2: S2, D and t3
@@ -157,7 +158,7 @@ __device__ __forceinline__ void psi_warm_pairs(const WarmArrays& w, const long l
             n3.x);
         one(a[u].y, s0[u].y, p1[u].y, d1[u].y, d2[u].y, e[u].y, t3[u].y, g.y, en.y, n1.y, n2.y,
             n3.y);
-        if (!ws.ext) en = make_double2(0.0, 0.0);
+        if (!hist) en = make_double2(0.0, 0.0);
         if constexpr (MODE == 0) {
             *(double2*)(w.s0 + k[u]) = a[u];
             if (hist) *(double2*)(w.psi + k[u]) = g;
