@@ -873,12 +873,22 @@ __device__ __forceinline__ void nc_half(const NCoarse& C, int l, double* x, cons
 {
     // (the colour's cells only: an FP64 instruction takes as long for half a warp)
     const int nx = C.nxn[l], wc = (nx + 1) / 2, n = wc * C.nyn[l], o = C.off[l];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int J = i / wc, I = 2 * (i - J * wc) + ((J + color) & 1), k = J * nx + I;
-        if (I >= nx) continue;
+    // On an x-periodic level of odd width the cells at both ends of a row are
+    // neighbours of one colour: one thread forms both values before it writes
+    // either, which is Jacobi across the seam as in n_half_seam.
+    const bool seam = C.per && nx > 1 && nx % 2;
+    auto value = [&](int J, int I) {
+        const int k = o + J * nx + I;
         double cs;
         const double ax = nc_ax(C, l, x, fx, fy, J, I, cs);
-        if (cs > 0.0) x[o + k] += (ax - b[o + k]) / cs;
+        return cs > 0.0 ? x[k] + (ax - b[k]) / cs : x[k];
+    };
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int J = i / wc, I = 2 * (i - J * wc) + ((J + color) & 1), k = o + J * nx + I;
+        if (I >= nx || (seam && I == nx - 1)) continue;
+        const double v = value(J, I);
+        if (seam && I == 0) x[k + nx - 1] = value(J, nx - 1);
+        x[k] = v;
     }
     __syncthreads();
 }
