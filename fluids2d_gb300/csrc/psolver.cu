@@ -585,7 +585,9 @@ __device__ __forceinline__ void p_dense(const PSArgs& A, const PSegs& segs, unsi
     });
 }
 
-// r = b - A x of a tile; tot = <b, b>, <r, r>
+// r = b - A x of a tile; tot = <b, b>, <r, r>. CHECK: r is not stored, tot[0] =
+// <x, x>
+template <bool CHECK>
 __device__ __forceinline__ void p_init(const PSArgs& A, const PTile& t, double (&tot)[2],
                                        unsigned char* smem)
 {
@@ -602,10 +604,10 @@ __device__ __forceinline__ void p_init(const PSArgs& A, const PTile& t, double (
             const double xe = ke >= 0 && t.m[ke] ? A.x[ke] : 0.0;
             const double xs = s ? A.x[k - t.pitch] : 0.0, xn = n ? A.x[k + t.pitch] : 0.0;
             rv = b - ((t.cx * ((xw - c) + (xe - c)) + t.cy * ((xs - c) + (xn - c))) - t.md * c);
-            tot[0] += b * b;
+            tot[0] += CHECK ? c * c : b * b;
             tot[1] += rv * rv;
         }
-        A.r[0][k] = rv;
+        if constexpr (!CHECK) A.r[0][k] = rv;
     });
 }
 
@@ -614,9 +616,11 @@ __device__ __forceinline__ void p_init(const PSArgs& A, const PTile& t, double (
 // the same order: the same bits.
 struct PSlot {
     double alpha, beta, d, rz, irz, goal, bb, rr;
+    double checked;  // <r, r> of the last true residual, 0: none yet
+    double floor;    // (8 eps diagonal)^2
     int conv, zero, status;
+    int verify;      // the recurrence has ended, the true residual is not known
     int member, n0, nn, owner;  // owner: this block writes the member's state
-    int pad;
 };
 
 template <typename S>
@@ -660,7 +664,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
     // r = b - A x, <b, b>, <r, r>
     for (int i = 0; i < ns; ++i) {
         double v[2] = {0.0, 0.0};
-        p_init(A, rec[i], v, smem);
+        p_init<false>(A, rec[i], v, smem);
         ps_block_total<2>(v, pb + rec[i].tile, nt);
     }
     const int nslot = single ? 1 : ns;
@@ -682,6 +686,11 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
         c.zero = bb == 0.0;
         c.conv = c.zero || rr <= c.goal;
         c.status = 0;
+        c.verify = 0;
+        c.checked = 0.0;
+        // (one member: also in the blocks without a level-0 tile)
+        const double e8 = 8.0 * 2.220446049250313e-16 * (single ? A.dg : rec[i].dg);
+        c.floor = e8 * e8;
         if (c.owner && !single) {
             A.conv[c.member] = c.conv;
             if (!c.conv) atomicAdd(A.active, 1);
@@ -697,7 +706,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
             });
         }
     if (!ps_sync(g)) return;
-    int it = 0;
+    int it = 0, before = 0;  // iterations since and before the last start
     // The decision after the update of iteration `it`, by the idle warps of
     // the next barrier: the tiles' <r, r> are complete, the phase before that
     // barrier is lost when a solve is over, but the totals cost no time.
@@ -711,18 +720,19 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
             c.rr = rr;
             c.irz = 1.0 / c.rz;  // for the next beta
             if (!(rr == rr)) c.status = ST_NONFINITE;
-            else if (rr > c.goal && it >= maxit) c.status = ST_PCG_MAXIT;
+            else if (rr > c.goal && before + it >= maxit) c.status = ST_PCG_MAXIT;
             c.conv = c.status || rr <= c.goal;
+            c.verify = sizeof(S) == 4 && c.conv && c.status != ST_NONFINITE;
             if (!c.owner) continue;
             if (c.conv) {
                 if (!single) {
                     A.conv[c.member] = 1;
                     atomicSub(A.active, 1);
                 }
-                if (c.status) atomicOr(A.status, c.status);
+                if (c.status && !c.verify) atomicOr(A.status, c.status);
             }
             DevScalars& sc = A.scs[c.member];
-            sc.iter = it;
+            sc.iter = before + it;
             sc.total_iters += 1;
         }
     };
@@ -745,7 +755,68 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
         __syncthreads();
         return v > 0;
     };
-    while (go_on()) {
+    // The FP32 form's true residual, once the recurrences have ended: these
+    // solves are to end on it, as the refinement rounds of the larger ones do. x
+    // is rounded with every update, so the two differ by a few eps |diagonal| |x|
+    // of the largest iterate. Within 8 of the last one's the solve is done;
+    // beyond, the start was far larger than the solution: CG starts again from
+    // the true residual, as long as that reduces it 10x. False (in all blocks)
+    // when no member goes on.
+    __shared__ int s_check;
+    auto again = [&] {
+        if (threadIdx.x == 0) {
+            s_check = 0;
+            for (int i = 0; i < nslot; ++i) s_check |= slot[i].verify;
+        }
+        __syncthreads();
+        if (single && !s_check) return false;
+        for (int i = 0; i < ns; ++i) {
+            if (!slot[single ? 0 : i].verify) continue;
+            double v[2] = {0.0, 0.0};
+            p_init<true>(A, rec[i], v, smem);
+            ps_block_total<2>(v, pb + rec[i].tile, nt);
+        }
+        if (!ps_sync(g)) return false;
+        for (int i = w; i < nslot; i += PS_NT / 32) {
+            PSlot& c = slot[i];
+            if (!c.verify) continue;
+            double xx, rr;
+            ps_total2(pb + c.n0, pb + nt + c.n0, c.nn, xx, rr);
+            if (lane) continue;
+            const bool slow = c.checked > 0.0 && rr > 0.01 * c.checked;
+            const bool done = rr <= 4.0 * c.goal || rr <= c.floor * xx || slow;
+            c.verify = 0;
+            c.rr = rr;
+            c.checked = rr;
+            if (done) c.status = 0;
+            if (done || c.status) {
+                if (c.status && c.owner) atomicOr(A.status, c.status);
+                continue;
+            }
+            c.conv = 0;
+            c.alpha = c.beta = c.d = c.rz = c.irz = 0.0;
+            if (!c.owner) continue;
+            A.scs[c.member].total_outer += 1;
+            if (!single) {
+                A.conv[c.member] = 0;
+                atomicAdd(A.active, 1);
+            }
+        }
+        before += it;
+        it = 0;
+        __syncthreads();
+        if (single && slot[0].conv) return false;
+        for (int i = 0; i < ns; ++i) {
+            if (slot[single ? 0 : i].conv) continue;
+            double v[2] = {0.0, 0.0};
+            p_init<false>(A, rec[i], v, smem);
+        }
+        if (!ps_sync(g)) return false;
+        for (int k = threadIdx.x; k < nrec; k += PS_NT)
+            if (!single) rconv[k] = *(volatile int*)&A.conv[rec[k].member];
+        return go_on();
+    };
+    while (go_on() || (sizeof(S) == 4 && again())) {
         for (int i = 0; i < ns; ++i) {
             const PSlot& c = slot[single ? 0 : i];
             if (c.conv) continue;
@@ -763,18 +834,18 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
             told = true;
             if (single && slot[0].conv) break;
         }
-        if (single && slot[0].conv) break;
+        if (single && slot[0].conv) continue;
         if (A.dense0 && single && it > 0) {
             // no level leg to hide the decision behind, and the phase that
             // would be lost is the whole solve: decide first
             if (w > 0) decide();
             __syncthreads();
-            if (slot[0].conv) break;
+            if (slot[0].conv) continue;
             told = true;
         }
         p_dense<S>(A, segs, smem);
         if (!(told ? ps_sync(g, refresh) : ps_sync(g, decide))) return;
-        if (single && slot[0].conv) break;
+        if (single && slot[0].conv) continue;
         for (int l = A.ng - 1; l >= 1; --l) {
             for (int i = lev0[l] - base; i < lev0[l + 1] - base; ++i)
                 if (!rconv[i]) p_up<S>(rec[i], A.nu, smem);
@@ -814,7 +885,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
             }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         A.eg->loops_out += 1;
-        A.eg->loops_in += it;
+        A.eg->loops_in += before + it;
     }
 }
 
@@ -1233,6 +1304,7 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     a.eg = eg;
     a.status = status;
     s.prec = prec;
+    a.dg = mem[0].mg->lev[0].diag;
     s.grid = sms;
     s.smem = smem;
     for (const void* k : {(const void*)k_ps_solve<double>, (const void*)k_ps_solve<float>,

@@ -49,6 +49,7 @@ struct PSArgs {
     int dense0;          // one member whose level 0 is the dense level
     int ntiles;          // level-0 tiles
     int mkeep;           // offset in shared memory of the block's dense rows (0: not kept)
+    double dg;           // level-0 diagonal of the first member
     double *x, *b, *r[2], *s[2], *p, *w;  // arenas, FP64
     double* part;        // tile totals, 2 x 2 ntiles
     int* conv;           // per member
@@ -79,7 +80,9 @@ struct PSMember {
 int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long nelem,
              DevScalars* scs, BSGlobals* eg, int* status, int l0 = 0);
 void ps_free(PSolver& s);
-// Record one solve of every member on `st`: x and b are the arenas (FP64).
+// Record one solve of every member on `st`: x and b are the arenas (FP64). It
+// ends at |r| <= tol |b|, r the recurrence residual (FP64 form) or b - A x to
+// within its rounding (FP32 form, see k_ps_solve), or after maxit iterations.
 int ps_record(PSolver& s, double* x, double* b, int nu, double tol, int maxit, cudaStream_t st);
 // Record the V-cycle on the levels from l0 on (from its b to its x), skipped
 // when the member is not iterating (ir: its inner loop); ps_record_cycle_reset

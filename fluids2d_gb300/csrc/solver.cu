@@ -1481,7 +1481,9 @@ int bs_record(BatchSolver& s, cudaStream_t st, cudaStream_t st2, int* launches)
     if (s.ps.on) {
         s.body_launches = 0;
         if (launches) *launches = 2;
-        return ps_record(s.ps, (double*)s.v.x64, (double*)s.v.b64, s.nu, s.tol, s.maxit, st);
+        // (FP32: as many iterations as the refinement form's rounds may take)
+        const int maxit = s.mode == 0 ? s.maxit : s.maxit_in * s.maxouter;
+        return ps_record(s.ps, (double*)s.v.x64, (double*)s.v.b64, s.nu, s.tol, maxit, st);
     }
     return s.th == 64 ? bs_record_t<64>(s, st, st2, launches)
                       : bs_record_t<32>(s, st, st2, launches);

@@ -55,8 +55,12 @@ typedef struct f2d_params {
     int noslip;         /* F2D_SLIP_* */
     int noslip_sides;   /* F2D_SIDE_* bits when noslip == F2D_SLIP_SIDES */
     int precision;      /* F2D_PREC_* */
-    double poisson_tol; /* relative residual of the Poisson solve */
-    int poisson_maxit;
+    double poisson_tol; /* relative residual of the Poisson solve: of CG's
+                           recurrence (FP64 form, and the pressure of euler and
+                           boussinesq) or of b - A x (FP32 form), which stops at
+                           its rounding: a few eps |diagonal of A| |x| */
+    int poisson_maxit;  /* CG iterations of a solve; FP32 form (vertex solves):
+                           max(2, maxit / 10) times 30 of them */
     int integrator;     /* F2D_INTEG_* */
     double ragamma;     /* Robert-Asselin coefficient of LFRA (param.py:50) */
     int tracer;         /* 1: a passive tracer field "tracer" (param.py:57,

@@ -13,6 +13,8 @@ The FP32 divergence of two unconnected basins sums to 1e-7 in each instead of
 0, and only the mean of both is taken off, so that system has no solution: the
 solve reports its iteration limit.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -22,7 +24,7 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 from fluids2d_gb300 import workloads as wl  # noqa: E402
-from fluids2d_gb300._lib import F2DError  # noqa: E402
+from fluids2d_gb300._lib import F2DError, check, lib  # noqa: E402
 from test_gpu_parity import (_ensemble, _model, _oracle_like, compare,  # noqa: E402
                              rel_l2)
 
@@ -177,10 +179,12 @@ def test_uneven_ensemble(sizes, precision, tol):
 ])
 def test_fluid_at_rest_stays_at_rest(nx, ny, precision, xper):
     """A zero right-hand side has the pressure 0, whatever was there before:
-    a flow that is stopped does not start again."""
+    a flow that is stopped does not start again. (Without a speed the time step
+    is dtmax, whose default is beyond FP32's range.)"""
     case = wl.euler_case(n=nx, ny=ny, seed=8, nislands=1, xperiodic=xper)
     m = _model("euler", nx, ny, case["msk"], precision=precision, xperiodic=xper,
-               Lx=case["Lx"], Ly=case["Ly"], cfl=0.5, tend=1e300, maxite=10 ** 9)
+               Lx=case["Lx"], Ly=case["Ly"], cfl=0.5, dtmax=1.0, tend=1e300,
+               maxite=10 ** 9)
     s = m.state
     s.u.x[:], s.u.y[:] = case["fields"]["u.x"], case["fields"]["u.y"]
     m.integrator.diag(s)
@@ -222,3 +226,69 @@ def test_fp32_pressure_over_odd_periodic_widths(nx, ny):
         fl[:, :3] = fl[:, -3:] = False
         assert np.linalg.norm(d[fl]) <= 16 * 2.0 ** -24 * u0
     assert np.array_equal(*out)
+
+
+def _true_residual(m, model, b, x, msk, **kw):
+    om = O.Mesh(O.Param(model=model, nx=m.param.nx, ny=m.param.ny, **kw))
+    om.msk[:] = msk
+    om.finalize()
+    A, G = O.laplacian(om, om.maindiag if model == "qg" else 0.0)[:2]
+    sel = G >= 0
+    return np.linalg.norm(b[sel] - A @ x[sel]) / np.linalg.norm(b[sel])
+
+
+def _rounds(m):
+    n = ctypes.c_int64()
+    check(lib().f2d_refine_rounds(m._h, ctypes.byref(n)))
+    return n.value
+
+
+@pytest.mark.parametrize("model,nx,ny", [("eulerpsi", 40, 36), ("eulerpsi", 97, 131),
+                                         ("qg", 90, 61)])
+def test_fp32_vertex_solve_from_a_far_start(model, nx, ny):
+    """The FP32 form ends on the true residual: a start 1e10 times the
+    solution leaves rounding of its own size in x, which the recurrence does
+    not see. An ordinary start needs one check and no second start."""
+    kw = dict(f0=30.0 if model == "qg" else 0.0, g=1.0, H=1.0)
+    msk = _mask(nx, ny, islands=2)
+    m = _model(model, nx, ny, msk, precision="fp32", **kw)
+    solver = m.mesh.qg_helmholtz if model == "qg" else m.mesh.poisson_vertices
+    rng = np.random.default_rng(5)
+    wet = m.mesh.G_vertices >= 0
+    b = rng.standard_normal(m.mesh.shape) * wet
+    x = np.zeros(m.mesh.shape)
+    solver.solve(b, x)
+    assert _true_residual(m, model, b, x, msk, **kw) <= 1e-10
+    assert _rounds(m) == 0
+    x = 1e10 * np.abs(x).max() * rng.standard_normal(x.shape) * wet
+    solver.solve(b, x)
+    assert _true_residual(m, model, b, x, msk, **kw) <= 1e-10
+    assert solver.last_relres <= 1e-10
+    assert _rounds(m) >= 1
+    m.sync()
+
+
+def test_fp32_ensemble_from_a_far_start():
+    """The same for one member of a batch, the others being done."""
+    sizes = [(40, 36), (97, 131), (64, 64)]
+    cs = [wl.eulerpsi_case(n=nx, ny=ny, seed=20 + k, nislands=1)
+          for k, (nx, ny) in enumerate(sizes)]
+    e, far = _ensemble(cs, "fp32"), _ensemble(cs, "fp32")
+    rng = np.random.default_rng(6)
+    psi = far.get_field(1, "psi")
+    far.set_field(1, "psi", 1e10 * rng.standard_normal(psi.shape) * psi)
+    far.diag()
+    far.sync()
+    assert far.stats()["refine_rounds"] >= 1 and e.stats()["refine_rounds"] == 0
+    for b in range(len(cs)):
+        assert rel_l2(far.get_field(b, "psi"), e.get_field(b, "psi")) <= 1e-10, b
+
+
+def test_fp32_iteration_limit_counts_rounds():
+    """poisson_maxit = 5 allows the FP32 form two rounds of 30 iterations,
+    whichever kernels run it (a solve from zero takes 12 to 20)."""
+    case = wl.eulerpsi_case(n=96, ny=80, seed=3, nislands=2)
+    m = _model("eulerpsi", 96, 80, case["msk"], precision="fp32", poisson_maxit=5)
+    m.state.omega[:] = case["fields"]["omega"]
+    m.integrator.diag(m.state)
+    m.sync()
