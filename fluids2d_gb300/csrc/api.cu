@@ -1460,11 +1460,14 @@ int f2d_set_coriolis(f2d_model m, const double* f)
     return 0;
 }
 
-// diag of what may be a new state: the next step has no history to start from
+// diag of what may be a new state: then the next step has no history to start
+// from
 static int diag_state(f2d_model_s* m)
 {
-    CK(cudaMemsetAsync(&m->sc->dt_warm, 0, WARM_BYTES, m->stream));
-    return run_graph(m, 0);
+    const int e = run_graph(m, 0);
+    if (e) return e;
+    CKI(launch_warm_check(m->sc, 1, m->stream));
+    return 0;
 }
 
 int f2d_diag(f2d_model m)

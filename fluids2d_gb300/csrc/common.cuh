@@ -73,11 +73,12 @@ struct DevScalars {
     // (param.py:50 RAgamma, integrators.py:39-55)
     double ragamma;
     // time step of the step whose stage increments the warm start keeps (0: none
-    // yet, or a diag since, whose state may be a new one: the increments of a
+    // yet, or a diag of another state since, see warm_check: the increments of a
     // stronger flow are too far off to start from, those of a NaN never end),
     // by which the next step scales them. Written at stage 3; dt_warm0: the
     // copy of the step under way
     double dt_warm, dt_warm0;
+    double bb_last;   // <b, b> of the solve before the last one
     // step lengths (FP32) of the inner iterations of the current refinement
     // round: the round's correction is sum alpha_i p_i (solver.cu)
     float ahist[32];
@@ -100,8 +101,15 @@ template <int MODE> __device__ __forceinline__ WarmState warm_state(DevScalars* 
     const bool hist = rho > 0.0 && rho <= 64.0;  // (false for NaN)
     return {hist, hist ? rho : 0.0};
 }
-// Host: bytes to clear from dt_warm on to drop the history
-constexpr size_t WARM_BYTES = 2 * sizeof(double);
+// After the solve of a diag: drop the history unless its right-hand side has,
+// to the bit, the norm of the last step's (sums run in a fixed order: the same
+// state, whose increments still hold; a new one differs, and so does a NaN).
+// Models whose solve does not write bb here (euler, boussinesq) always drop it:
+// the diag replaces the pressure that theirs goes with.
+__device__ __forceinline__ void warm_check(DevScalars& sc)
+{
+    if (!(sc.bb > 0.0 && sc.bb == sc.bb_last)) sc.dt_warm = sc.dt_warm0 = 0.0;
+}
 
 // ---------------------------------------------------------------------------
 // Small PTX helpers: TMA tile loads through an mbarrier, with a time-bounded

@@ -878,11 +878,11 @@ int64_t f2d_ensemble_packed_size(f2d_ensemble e)
 int f2d_ensemble_diag(f2d_ensemble e)
 {
     if (!e) return f2d_internal_fail(1, "null ensemble");
-    // the states may be new ones: the next step has no history to start from
-    if (cudaMemset2DAsync(&e->scs->dt_warm, sizeof(DevScalars), 0, WARM_BYTES, e->n,
-                          e->stream) != cudaSuccess)
-        return f2d_internal_fail(3, "cudaMemset2DAsync");
-    return ens_run_graph(e, 0);
+    const int r = ens_run_graph(e, 0);
+    if (r) return r;
+    // new states have no history to start their next step from
+    ECK((cudaError_t)launch_warm_check(e->scs, e->n, e->stream));
+    return 0;
 }
 
 int f2d_ensemble_autotune(f2d_ensemble e, int reps, int* th, int* nu, double* tol_in,

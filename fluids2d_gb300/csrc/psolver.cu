@@ -949,6 +949,7 @@ __global__ void k_ps_setup(const __grid_constant__ PSArgs A, double tol2, int ma
     }
     if (b < A.nmem) {
         A.scs[b].tol2 = tol2;
+        A.scs[b].bb_last = A.scs[b].bb;
         A.scs[b].maxit = maxit;
         A.scs[b].converged = 0;
         A.scs[b].iter = 0;

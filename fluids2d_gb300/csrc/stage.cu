@@ -830,6 +830,19 @@ int launch_psi_warm(int mode, const WarmArrays& w, long long n, DevScalars* sc, 
     return (int)cudaGetLastError();
 }
 
+// warm_check of n models' scalars
+__global__ void k_warm_check(DevScalars* scs, int n)
+{
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < n) warm_check(scs[b]);
+}
+
+int launch_warm_check(DevScalars* scs, int n, cudaStream_t s)
+{
+    k_warm_check<<<(n + 127) / 128, 128, 0, s>>>(scs, n);
+    return (int)cudaGetLastError();
+}
+
 // Warm start of the pressure solves (launch_p_warm) at the fluid cells: the
 // others are never solved for.
 template <int MODE>

@@ -74,7 +74,8 @@ int launch_set_dt(DevScalars* sc, cudaStream_t s);
 // step come down to the FP32 rounding of the state (psi_warm_brackets) the
 // brackets are noise and left out. A guess moves the solve's starting point, and
 // the residual that its recurrence can attain by about eps times the largest
-// iterate: it must not be larger than the solution (no history across a diag).
+// iterate: it must not be larger than the solution (no history across a diag of another
+// state).
 struct WarmArrays {
     double* psi;  // in: the last solution; out: the guess
     double* s0;   // psi at the step start
@@ -183,6 +184,10 @@ __device__ __forceinline__ void psi_warm_pairs(const WarmArrays& w, const long l
 // stay 0)
 int launch_psi_warm(int mode, const WarmArrays& w, long long n, DevScalars* sc,
                     cudaStream_t s);
+
+// after a diag: keep the history of n models only where the state is still the
+// last step's (warm_check)
+int launch_warm_check(DevScalars* scs, int n, cudaStream_t s);
 
 // Warm start of the pressure solve of RK3 stage mode+1 (euler and boussinesq,
 // FP64 states). The stages add -3/4 L1 + 1/4 L2 and so on of the unprojected

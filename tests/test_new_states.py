@@ -124,3 +124,27 @@ def test_rewritten_ensemble_equals_fresh_one(precision):
     for b in range(len(members)):
         for k in ("omega", "psi"):
             assert np.array_equal(e.get_field(b, k), fresh.get_field(b, k)), (b, k)
+
+
+@pytest.mark.parametrize("kind,precision", [("eulerpsi", "fp64"), ("eulerpsi", "fp32"),
+                                            ("qg", "fp64")])
+def test_diag_of_the_same_state_keeps_the_history(kind, precision):
+    """A diag between steps costs its own solve, at most two iterations from
+    the solution, and none of the steps' iterations."""
+    case = CASES[kind](n=144, ny=128, seed=31, nislands=1)
+
+    def iterations(diag):
+        m = _make(kind, case, precision)
+        _write(m, case["fields"])
+        m.advance(4)
+        m.sync()
+        i0 = m.stats()[0]
+        for _ in range(8):
+            if diag:
+                m.integrator.diag(m.state)
+            m.advance(1)
+        m.sync()
+        return m.stats()[0] - i0
+
+    # (psi moves by rounding in a diag: an iteration more or less of a step)
+    assert iterations(True) <= iterations(False) + 8 * 3
