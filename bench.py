@@ -101,12 +101,12 @@ ENSEMBLE_DESC = ("ensemble of 256 eulerpsi closed basins, sizes uniform in "
                  "vortices, WENO5, SSP-RK3, per-member CFL 0.8")
 
 
-def solver_roofline(timer, pipelined, handle, workload, peak, peak_src):
-    """Roofline of the solver's level-0 down leg of the V-cycle (k_mgp_down when
-    the FP32 level arrays fit the pipelined kernels, else the leg of the FP64
-    persistent solve, k_ps_down0: b and mask read, the pre-smoothed x written, the restricted
-    right-hand side written at a quarter of the nodes = (2.25 es + 1) bytes
-    per level-0 node), timed alone with CUDA events, L2 flushed."""
+def solver_roofline(timer, solver_form, handle, workload, peak, peak_src):
+    """Roofline of the solver's level-0 down leg of the V-cycle (the kernel of
+    the form that the solve runs: b and mask read, the pre-smoothed x written,
+    the restricted right-hand side written at a quarter of the nodes =
+    (2.25 es + 1) bytes per level-0 node), timed alone with CUDA events, L2
+    flushed."""
     import ctypes
     avg = ctypes.c_double()
     nodes = ctypes.c_int64()
@@ -114,12 +114,12 @@ def solver_roofline(timer, pipelined, handle, workload, peak, peak_src):
     rc = timer(handle, 10, 1, ctypes.byref(avg), ctypes.byref(nodes), ctypes.byref(es))
     if rc != 0:
         return None
-    pipe = ctypes.c_int()
-    if pipelined(handle, ctypes.byref(pipe)) != 0:
+    form = ctypes.c_int()
+    if solver_form(handle, ctypes.byref(form)) != 0:
         return None
     alg = nodes.value * (2.25 * es.value + 1)
     achieved = alg / (avg.value * 1e-3) / 1e9
-    kname = "k_mgp_down" if pipe.value else "k_ps_down0"
+    kname = ("k_mg_down", "k_mgp_down", "k_ps_down0")[form.value]
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak,
             "traffic": read_profile_traffic(f"{kname}_{workload}"),
@@ -704,7 +704,7 @@ def run_gpu_ensemble(args, rank, world):
                 "steps": e2e_steps, "trials": trials,
                 "reported": "median of 3 trials"},
         "roofline": solver_roofline(L.f2d_ensemble_time_solver,
-                                    L.f2d_ensemble_solver_pipelined, h, args.workload,
+                                    L.f2d_ensemble_solver_form, h, args.workload,
                                     peak, peak_src),
         "roofline_stage": {"bound": "hbm", "achieved": achieved, "peak": peak,
                            "unit": "GB/s", "frac": achieved / peak,
@@ -983,7 +983,7 @@ def run_gpu(args, rank, world):
     if model != "rsw":
         # the Poisson solve dominates the step: its largest kernel is the
         # roofline kernel, the fused stage is reported beside it
-        sr = solver_roofline(L.f2d_time_solver, L.f2d_solver_pipelined, h, args.workload,
+        sr = solver_roofline(L.f2d_time_solver, L.f2d_solver_form, h, args.workload,
                              peak, peak_src)
         if sr is not None:
             line["roofline_stage"] = line["roofline"]

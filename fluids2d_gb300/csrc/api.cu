@@ -1917,6 +1917,16 @@ int f2d_solver_pipelined(f2d_model m, int* pipelined)
     return 0;
 }
 
+int f2d_solver_form(f2d_model m, int* form)
+{
+    if (!m || !form) return fail(1, "null argument");
+    int pipelined = 0;
+    const int e = f2d_solver_pipelined(m, &pipelined);
+    if (e) return e;
+    *form = m->bs[m->p.model == F2D_MODEL_EULERPSI ? 0 : 1].ps.on ? 2 : pipelined;
+    return 0;
+}
+
 // ---- discrete adjoint of the eulerpsi step ------------------------------------
 static int adj_check(f2d_model m)
 {

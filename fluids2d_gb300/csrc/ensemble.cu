@@ -1036,6 +1036,13 @@ int f2d_ensemble_solver_pipelined(f2d_ensemble e, int* pipelined)
     return 0;
 }
 
+int f2d_ensemble_solver_form(f2d_ensemble e, int* form)
+{
+    if (!e || !form) return f2d_internal_fail(1, "null argument");
+    *form = e->bs.ps.on ? 2 : e->bs.pipe ? 1 : 0;
+    return 0;
+}
+
 int f2d_ensemble_time_stage(f2d_ensemble e, int stage, int reps, int flush_l2,
                             double* avg_ms)
 {

@@ -889,13 +889,14 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
     }
 }
 
-// the level-0 down leg of every member by itself, FP64 (a measurement)
+// the level-0 down leg of every member by itself (a measurement)
+template <typename S>
 __global__ void __launch_bounds__(PS_NT, 1) k_ps_down0(const __grid_constant__ PSArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int* l0 = A.rec0 + blockIdx.x * (A.ng + 1);
     double t[1] = {0.0};
-    for (int i = l0[0]; i < l0[1]; ++i) p_phase_a<double>(A, A.recs[i], 0, 0.0, 0.0, t, smem);
+    for (int i = l0[0]; i < l0[1]; ++i) p_phase_a<S>(A, A.recs[i], 0, 0.0, 0.0, t, smem);
 }
 
 // The V-cycle of one member on the levels from A.l0 on, for the FP32 form's
@@ -1309,7 +1310,8 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     s.grid = sms;
     s.smem = smem;
     for (const void* k : {(const void*)k_ps_solve<double>, (const void*)k_ps_solve<float>,
-                          (const void*)k_ps_down0, (const void*)k_ps_cycle<float>})
+                          (const void*)k_ps_down0<double>, (const void*)k_ps_down0<float>,
+                          (const void*)k_ps_cycle<float>})
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS_SMEM) !=
             cudaSuccess)
             return 3;
@@ -1356,7 +1358,8 @@ int ps_record_cycle(PSolver& s, int nu, int ir, cudaStream_t st)
 int ps_time_down(PSolver& s, int nu, cudaStream_t st)
 {
     s.a.nu = nu;
-    k_ps_down0<<<s.grid, PS_NT, s.smem, st>>>(s.a);
+    if (s.prec == 0) k_ps_down0<double><<<s.grid, PS_NT, s.smem, st>>>(s.a);
+    else k_ps_down0<float><<<s.grid, PS_NT, s.smem, st>>>(s.a);
     return (int)cudaGetLastError();
 }
 

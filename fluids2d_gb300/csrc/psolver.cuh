@@ -89,7 +89,7 @@ int ps_record(PSolver& s, double* x, double* b, int nu, double tol, int maxit, c
 // before the first of a solve.
 int ps_record_cycle(PSolver& s, int nu, int ir, cudaStream_t st);
 int ps_record_cycle_reset(PSolver& s, cudaStream_t st);
-// Measurement hook (FP64): one launch of the level-0 down leg of every member.
+// Measurement hook: one launch of the level-0 down leg of every member.
 int ps_time_down(PSolver& s, int nu, cudaStream_t st);
 
 }  // namespace f2d

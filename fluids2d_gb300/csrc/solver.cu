@@ -1459,7 +1459,7 @@ int bs_time_down(BatchSolver& s, cudaStream_t st, int reps, int flush_l2, double
         if (fl) cudaMemsetAsync(fl, r & 0xff, flush_bytes, st);
         cudaEventRecord(a, st);
         const bool two = s.nu >= 2;
-        if (s.mode == 0 && s.ps.on) err = ps_time_down(s.ps, s.nu, st);
+        if (s.ps.on) err = ps_time_down(s.ps, s.nu, st);
         else if (s.mode == 0) two ? launch_down0<double, 2>(s, st, ir) : launch_down0<double, 1>(s, st, ir);
         else two ? launch_down0<float, 2>(s, st, ir) : launch_down0<float, 1>(s, st, ir);
         cudaEventRecord(b, st);

@@ -230,18 +230,24 @@ int f2d_autotune(f2d_model m, int reps, int *tile_rows, int *sweeps, double *tol
  * the FP64 form). Recorded graphs are dropped. No reference counterpart. */
 int f2d_set_schedule(f2d_model m, int tile_rows, int sweeps, double tol_in);
 /* Time `reps` launches of the Poisson solver's level-0 down leg
- * (pre-smoothing + residual + restriction of the V-cycle; FP64: the same leg of
- * the persistent solve kernel, launched by itself) on the current right-hand
- * side, L2 flushed between launches when flush_l2 != 0; *avg_ms = mean ms, *nodes = level-0 nodes, *elem_bytes = 4
- * or 8 (multigrid precision). Measurement hook of the benchmark; no
- * reference counterpart. The model must have solved once. */
+ * (pre-smoothing + residual + restriction of the V-cycle; the kernel that
+ * f2d_solver_form names) on the current right-hand side, L2 flushed between
+ * launches when flush_l2 != 0; *avg_ms = mean ms, *nodes = level-0 nodes,
+ * *elem_bytes = 4 or 8 (multigrid precision). Measurement hook of the
+ * benchmark; no reference counterpart. The model must have solved once. */
 int f2d_time_solver(f2d_model m, int reps, int flush_l2, double *avg_ms,
                     int64_t *nodes, int *elem_bytes);
-/* Which level kernels f2d_time_solver times: *pipelined = 1 for the persistent
- * TMA-staged FP32 kernels (k_mgp_down / k_mgp_up), 0 otherwise (the FP64 form,
- * or level arrays outside the pipelined kernels' layout). Instrumentation,
- * no reference counterpart. The model must have solved once. */
+/* Whether the level arrays fit the pipelined FP32 kernels: *pipelined = 1 for
+ * the persistent TMA-staged ones (k_mgp_down / k_mgp_up), 0 otherwise (the FP64
+ * form, or level arrays outside their layout). Instrumentation, no reference
+ * counterpart. The model must have solved once. */
 int f2d_solver_pipelined(f2d_model m, int *pipelined);
+/* Which kernels run the solve, and which f2d_time_solver times: *form = 2 for
+ * the whole solve in one kernel (k_ps_solve; its leg by itself: k_ps_down0), 1
+ * for the pipelined level kernels (k_mgp_down), 0 for the one-tile-per-block
+ * ones (k_mg_down). Instrumentation, no reference counterpart. The model must
+ * have solved once. */
+int f2d_solver_form(f2d_model m, int *form);
 /* Failure-detection test switch (no reference counterpart). enabled != 0:
  * every stage kernel, once its TMA tile has landed, also waits for a barrier
  * phase that nothing completes, gives up after limit_ms (0 < limit_ms <=
@@ -332,8 +338,9 @@ int f2d_ensemble_time_stage(f2d_ensemble e, int stage, int reps, int flush_l2,
 /* f2d_time_solver for the batched solver of all members. */
 int f2d_ensemble_time_solver(f2d_ensemble e, int reps, int flush_l2, double *avg_ms,
                              int64_t *nodes, int *elem_bytes);
-/* f2d_solver_pipelined for the batched solver of all members. */
+/* f2d_solver_pipelined, f2d_solver_form for the batched solver of all members. */
 int f2d_ensemble_solver_pipelined(f2d_ensemble e, int *pipelined);
+int f2d_ensemble_solver_form(f2d_ensemble e, int *form);
 
 /* ---- discrete adjoint (eulerpsi, closed basin, weno/upwind fluxes) ------ */
 

@@ -228,6 +228,32 @@ def test_fp32_pressure_over_odd_periodic_widths(nx, ny):
     assert np.array_equal(*out)
 
 
+@pytest.mark.parametrize("nx,ny,precision,xper,want", [
+    (256, 200, "fp64", False, 2), (256, 200, "fp32", False, 2),
+    (1450, 1400, "fp32", False, 1),
+    # 75 periodic columns: above the dense level (2048 unknowns; FP32 4096), or on it
+    (300, 200, "fp64", True, 0), (300, 200, "fp32", True, 2), (300, 300, "fp32", True, 1),
+])
+def test_timed_leg_is_of_the_form_that_runs(nx, ny, precision, xper, want):
+    m = _model("qg", nx, ny, _mask(nx, ny, xper), precision=precision, xperiodic=xper,
+               f0=1.0, g=1.0, H=1.0)
+    rng = np.random.default_rng(2)
+    m.state.pv[:] = rng.standard_normal(m.mesh.shape) * (m.mesh.msk > 0)
+    m.integrator.diag(m.state)
+    m.sync()
+    form, ms = ctypes.c_int(-1), ctypes.c_double()
+    nodes, es = ctypes.c_int64(), ctypes.c_int()
+    check(lib().f2d_solver_form(m._h, ctypes.byref(form)))
+    assert form.value == want
+    check(lib().f2d_time_solver(m._h, 3, 0, ctypes.byref(ms), ctypes.byref(nodes),
+                                ctypes.byref(es)))
+    assert ms.value > 0 and es.value == (8 if precision == "fp64" else 4)
+    psi = m.state.psi.copy()
+    m.integrator.diag(m.state)  # the hook leaves the solver as it was
+    m.sync()
+    assert rel_l2(m.state.psi, psi) <= 1e-10
+
+
 def _true_residual(m, model, b, x, msk, **kw):
     om = O.Mesh(O.Param(model=model, nx=m.param.nx, ny=m.param.ny, **kw))
     om.msk[:] = msk
