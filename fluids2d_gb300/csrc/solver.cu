@@ -1627,7 +1627,7 @@ static int bs_pipe_setup(BatchSolver& s, const std::vector<MGLevel>& levs,
     return 0;
 }
 
-constexpr long long PS_FP32_NODES = 2000000;
+constexpr long long PS_FP32_NODES = 2000000, PS_CROWD_NODES = 1300;
 // largest level of the coarse levels' launch: on larger ones its tiles are slower
 // than the pipelined legs with their launches (1024^2: 16 us a leg, against 9)
 constexpr long long PC_NODES = 300000;
@@ -1826,7 +1826,12 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
     // cost more at every size), and FP32 problems of up to PS_FP32_NODES nodes
     // (batches half of that):
     // above that the refinement form's FP32 Krylov vectors and pipelined legs
-    // move less and are the faster ones.
+    // move less and are the faster ones. Not with more members than SMs where
+    // the level kernels, several members to an SM at a time, beat a block that
+    // takes its members' tiles in turn: FP32 (200 64^2: 3.44 ms a step
+    // persistent, 2.68 with the level kernels; 152: 2.07 and 2.36), and FP64
+    // members of fewer than PS_CROWD_NODES nodes (1000 32^2: 9.52 and 7.94;
+    // 1000 40^2: 11.5 and 17.6).
     {
         long long n0 = 0;
         std::vector<PSMember> pm(s.n);
@@ -1837,7 +1842,9 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
             pm[b].mg = &s.mg[b];
             pm[b].ndense_cap = s.n == 1 ? PS_NDENSE32 : (int)sqrt((mode == 0 ? 1.5e6 : 6e6) / s.n);
         }
-        if (mode == 0 || n0 <= (s.n == 1 ? PS_FP32_NODES : PS_FP32_NODES / 2)) {
+        const bool crowd = s.n > ps_sms() && (mode == 1 || n0 < PS_CROWD_NODES * s.n);
+        if (!crowd &&
+            (mode == 0 || n0 <= (s.n == 1 ? PS_FP32_NODES : PS_FP32_NODES / 2))) {
             const int e = ps_build(s.ps, pm, mode, v.nelem, scs, s.eg, &s.eg->status);
             if (e) return e;
         }

@@ -254,6 +254,39 @@ def test_timed_leg_is_of_the_form_that_runs(nx, ny, precision, xper, want):
     assert rel_l2(m.state.psi, psi) <= 1e-10
 
 
+@pytest.mark.parametrize("n,size,precision,want", [
+    (152, (32, 32), "fp64", 2), (153, (32, 32), "fp64", 0), (153, (40, 36), "fp64", 2),
+    (152, (48, 40), "fp32", 2), (153, (48, 40), "fp32", 1), (153, (16, 12), "fp32", 0),
+    (1230, (40, 40), "fp64", 2),  # more than eight members to a block
+])
+def test_batches_around_the_number_of_sms(n, size, precision, want):
+    """The form of batches with as many members as SMs (152 of them here) and
+    one more, and their members against single models."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n += (sms - 152) * (n < 160)
+    cs = [wl.eulerpsi_case(n=size[0], ny=size[1], seed=20 + k, nislands=k % 2)
+          for k in range(4)]
+    e = _ensemble([cs[b % 4] for b in range(n)], precision)
+    form = ctypes.c_int(-1)
+    check(lib().f2d_ensemble_solver_form(e._h, ctypes.byref(form)))
+    assert form.value == want
+    e.run(3)
+    e.sync()
+    tol = 1e-10 if precision == "fp64" else 1e-6
+    for k, c in enumerate(cs):
+        m = _model("eulerpsi", c["nx"], c["ny"], c["msk"], cfl=0.8, tend=1e300,
+                   maxite=10 ** 9, precision=precision)
+        m.state.omega[:] = c["fields"]["omega"]
+        m.integrator.diag(m.state)
+        m.advance(3)
+        m.sync()
+        for b in (k, n // 2 // 4 * 4 + k, (n - 1 - k) // 4 * 4 + k):
+            if b >= n:
+                continue
+            assert rel_l2(e.get_field(b, "omega"), m.state.omega) <= tol, b
+            assert rel_l2(e.get_field(b, "psi"), m.state.psi) <= tol, b
+
+
 def _true_residual(m, model, b, x, msk, **kw):
     om = O.Mesh(O.Param(model=model, nx=m.param.nx, ny=m.param.ny, **kw))
     om.msk[:] = msk
