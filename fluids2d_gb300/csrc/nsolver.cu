@@ -834,7 +834,10 @@ static int dense_inverse(const std::vector<double>& fx, const std::vector<double
             h[(size_t)k * w1] += cx + cy;
         }
     }
-    return ps_invert(h, n, bw, part, -1.0, prec, out);
+    PSScratch scratch;
+    const int rc = ps_invert(h, n, bw, part, -1.0, prec, out, scratch);
+    if (rc) return rc;
+    return cudaDeviceSynchronize() == cudaSuccess ? 0 : 3;
 }
 
 // The FP32 form's dense level: not the inverse but the V-cycle on the levels

@@ -2,6 +2,7 @@
 // coarsest operator and the cooperative launch.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "persist.cuh"
@@ -108,7 +109,7 @@ __global__ void k_inverse_out(const double* __restrict__ X, const int* __restric
 static_assert(PS_NDENSE32 <= 2 * PS_NDENSE, "shared memory of k_band_inverse");
 
 int ps_invert(const std::vector<double>& band, int n, int bw, const std::vector<int>& part,
-              double scale, int prec, void* out)
+              double scale, int prec, void* out, PSScratch& scratch)
 {
     // Right-looking Cholesky in column bands, c[j w1 + k] = H(j + k, j), B
     // columns at a time: one update of the columns after them costs a load and
@@ -155,58 +156,55 @@ int ps_invert(const std::vector<double>& band, int n, int bw, const std::vector<
                 t[k] -= (f0 * s0[k] + f1 * s1[k]) + (f2 * s2[k] + f3 * s3[k]);
         }
     }
-    std::vector<void*> tmp;
-    auto dal = [&](size_t bytes, const void* src) -> void* {
-        void* p = nullptr;
-        if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
-        tmp.push_back(p);
-        if (src && cudaMemcpy(p, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
-        return p;
-    };
-    auto run = [&]() -> int {
-        double* dlc = (double*)dal(lc.size() * 8, lc.data());
-        double* dlr = (double*)dal(lr.size() * 8, lr.data());
-        double* did = (double*)dal(id.size() * 8, id.data());
-        double* X = (double*)dal((size_t)n * n * 8, nullptr);
-        if (!dlc || !dlr || !did || !X) return 2;
-        const int w = n <= PS_NDENSE ? BI_W : BI_W / 2;
-        const size_t smem = (size_t)w * n * sizeof(double);
-        if (cudaFuncSetAttribute(k_band_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 BI_W * PS_NDENSE * (int)sizeof(double)) != cudaSuccess)
-            return 3;
-        k_band_inverse<<<(n + w - 1) / w, 32 * w, smem>>>(dlc, dlr, did, n, bw, X);
-        int* dpart = nullptr;
-        double *dr = nullptr, *dm = nullptr;
-        if (!part.empty()) {
-            std::vector<double> isize(n, 0.0), cnt(n, 0.0), r(n), sum(n, 0.0), mean(n, 0.0);
-            for (int i = 0; i < n; ++i)
-                if (part[i] >= 0) cnt[part[i]] += 1.0;
-            for (int i = 0; i < n; ++i)
-                if (part[i] >= 0) isize[i] = 1.0 / cnt[part[i]];
-            dpart = (int*)dal((size_t)n * 4, part.data());
-            double* dsz = (double*)dal((size_t)n * 8, isize.data());
-            dr = (double*)dal((size_t)n * 8, nullptr);
-            if (!dpart || !dsz || !dr) return 2;
-            k_row_means<<<(n + 7) / 8, 256>>>(X, dpart, dsz, n, dr);
-            if (cudaMemcpy(r.data(), dr, (size_t)n * 8, cudaMemcpyDeviceToHost) != cudaSuccess)
-                return 2;
-            for (int i = 0; i < n; ++i)
-                if (part[i] >= 0) sum[part[i]] += r[i] * isize[i];
-            for (int i = 0; i < n; ++i)
-                if (part[i] >= 0) mean[i] = sum[part[i]];
-            dm = (double*)dal((size_t)n * 8, mean.data());
-            if (!dm) return 2;
-        }
-        const unsigned ng = (unsigned)(((size_t)n * (n + 4) + 255) / 256);
-        if (prec == 0)
-            k_inverse_out<double><<<ng, 256>>>(X, dpart, dr, dm, n, scale, (double*)out);
-        else
-            k_inverse_out<float><<<ng, 256>>>(X, dpart, dr, dm, n, scale, (float*)out);
-        return cudaDeviceSynchronize() == cudaSuccess ? 0 : 3;
-    };
-    const int rc = run();
-    for (void* p : tmp) cudaFree(p);
-    return rc;
+    // one allocation, one copy (an allocation per array and a synchronisation per
+    // member were half of the set-up of an ensemble of small members)
+    const size_t nb = (size_t)n * bw, nn = (size_t)n * n;
+    std::vector<double> host(2 * nb + 4 * (size_t)n, 0.0);
+    std::copy(lc.begin(), lc.end(), host.begin());
+    std::copy(lr.begin(), lr.end(), host.begin() + nb);
+    std::copy(id.begin(), id.end(), host.begin() + 2 * nb);
+    double* isize = &host[2 * nb + n];
+    if (!part.empty()) {
+        std::vector<double> cnt(n, 0.0);
+        for (int i = 0; i < n; ++i)
+            if (part[i] >= 0) cnt[part[i]] += 1.0;
+        for (int i = 0; i < n; ++i)
+            if (part[i] >= 0) isize[i] = 1.0 / cnt[part[i]];
+        memcpy(&host[2 * nb + 2 * (size_t)n], part.data(), (size_t)n * sizeof(int));
+    }
+    double* d = (double*)scratch.get((host.size() + nn) * 8);
+    if (!d) return 2;
+    if (cudaMemcpy(d, host.data(), host.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess)
+        return 2;
+    double *dlr = d + nb, *did = d + 2 * nb, *dsz = did + n, *dr = dsz + 2 * n;
+    int* dpart = part.empty() ? nullptr : (int*)(dsz + n);
+    double* X = d + host.size();
+    const int w = n <= PS_NDENSE ? BI_W : BI_W / 2;
+    const size_t smem = (size_t)w * n * sizeof(double);
+    if (cudaFuncSetAttribute(k_band_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             BI_W * PS_NDENSE * (int)sizeof(double)) != cudaSuccess)
+        return 3;
+    k_band_inverse<<<(n + w - 1) / w, 32 * w, smem>>>(d, dlr, did, n, bw, X);
+    double* dm = nullptr;
+    if (dpart) {
+        k_row_means<<<(n + 7) / 8, 256>>>(X, dpart, dsz, n, dr);
+        std::vector<double> r(n), sum(n, 0.0), mean(n, 0.0);
+        if (cudaMemcpy(r.data(), dr, (size_t)n * 8, cudaMemcpyDeviceToHost) != cudaSuccess)
+            return 2;
+        for (int i = 0; i < n; ++i)
+            if (part[i] >= 0) sum[part[i]] += r[i] * isize[i];
+        for (int i = 0; i < n; ++i)
+            if (part[i] >= 0) mean[i] = sum[part[i]];
+        dm = dsz;  // (the sizes are not needed any more)
+        if (cudaMemcpy(dm, mean.data(), (size_t)n * 8, cudaMemcpyHostToDevice) != cudaSuccess)
+            return 2;
+    }
+    const unsigned ng = (unsigned)(((size_t)n * (n + 4) + 255) / 256);
+    if (prec == 0)
+        k_inverse_out<double><<<ng, 256>>>(X, dpart, dr, dm, n, scale, (double*)out);
+    else
+        k_inverse_out<float><<<ng, 256>>>(X, dpart, dr, dm, n, scale, (float*)out);
+    return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
 int ps_launch(const void* kern, int grid, size_t smem, void** args, cudaStream_t st)

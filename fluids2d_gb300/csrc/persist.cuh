@@ -340,9 +340,28 @@ __device__ __forceinline__ void ps_copy16(void* dst, const void* src, size_t byt
 // n). Cholesky on the host (ps_band_ok
 // bounds its n bw^2 operations), the columns of the inverse on the GPU. part:
 // empty, or a part number per row: the constants of a part are projected out
-// of the result from both sides, and rows of part -1 become 0. 0 on success.
+// of the result from both sides, and rows of part -1 become 0. 0 on success: the
+// work is on the default stream, which the caller synchronises before the
+// scratch goes or another stream reads the result.
+struct PSScratch {  // device memory of the inversions of one set-up
+    void* p = nullptr;
+    size_t bytes = 0;
+    PSScratch() = default;
+    PSScratch(const PSScratch&) = delete;
+    PSScratch& operator=(const PSScratch&) = delete;
+    ~PSScratch() { cudaFree(p); }
+    void* get(size_t n)
+    {
+        if (n > bytes) {
+            cudaFree(p);  // (waits for its readers)
+            p = nullptr;
+            bytes = cudaMalloc(&p, n) == cudaSuccess ? n : 0;
+        }
+        return bytes ? p : nullptr;
+    }
+};
 int ps_invert(const std::vector<double>& band, int n, int bw, const std::vector<int>& part,
-              double scale, int prec, void* out);
+              double scale, int prec, void* out, PSScratch& scratch);
 // whether a level of n cells in rows of bw may be the dense one
 inline bool ps_band_ok(long long n, long long bw, int prec)
 {

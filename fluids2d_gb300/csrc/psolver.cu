@@ -1152,21 +1152,36 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     std::vector<std::vector<PTile>> tl(a.ng);
     std::vector<PDense> dense(n);
     size_t smem = 0, maxrow = 0;
+    PSScratch scratch;
+    // b, x and the inverse of every dense level, in one allocation
+    auto align = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+    size_t dbytes = 0;
+    auto sizes = [&](int b, size_t& nv, size_t& ni) {
+        const MGLevel& D = mem[b].mg->lev[ng[b]];
+        const int nd = (int)unknowns(D);
+        nv = align((size_t)D.nyn * D.nxn * es);
+        ni = align((size_t)nd * (prec == 0 ? ps_pitch<double>(nd) : ps_pitch<float>(nd)) * es);
+        return 2 * nv + ni;
+    };
+    size_t nv, ni;
+    for (int b = 0; b < n; ++b) dbytes += sizes(b, nv, ni);
+    char* dmem = (char*)dal(dbytes);
+    if (!dmem) return 2;
     for (int b = 0; b < n; ++b) {
         const MGLevel& D = mem[b].mg->lev[ng[b]];
         // the unknowns: all nodes but the closed edges' (no fluid node there)
         const int e0 = D.per ? 0 : 1, w = D.nxn - 2 * e0, nd = w * (D.nyn - 2);
-        const size_t nodes = (size_t)D.nyn * D.nxn;
         dense[b].n = nd;
         dense[b].row0 = b ? dense[b - 1].row0 + dense[b - 1].n : 0;
         dense[b].box = PSBox{w, D.nxn, D.nxn + e0, 1.0f / (float)w};
-        dense[b].b = dal(nodes * es);
-        dense[b].x = dal(nodes * es);
+        const size_t member = sizes(b, nv, ni);
+        dense[b].b = dmem;
+        dense[b].x = dmem + nv;
+        void* minv = dmem + 2 * nv;
+        dmem += member;
         const int np = prec == 0 ? ps_pitch<double>(nd) : ps_pitch<float>(nd);
-        void* minv = dal((size_t)nd * np * es);
         maxrow = std::max(maxrow, np * es);
         dense[b].minv = minv;
-        if (!dense[b].b || !dense[b].x || !minv) return 2;
         // -A of the dense level (identity rows at non-fluid nodes: their b is 0)
         const std::vector<uint8_t>& hm = mem[b].mg->hmask[ng[b]];
         const int w1 = w + 1;
@@ -1183,7 +1198,7 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
             if (J > 1 && fluid(J - 1, I)) r[w] -= D.cy;
             if (D.per && I == D.nxn - 1 && D.nxn > 1 && fluid(J, 0)) r[I] -= D.cx;
         }
-        const int rc = ps_invert(h, nd, w, {}, -1.0, prec, minv);
+        const int rc = ps_invert(h, nd, w, {}, -1.0, prec, minv, scratch);
         if (rc == 5) return 0;
         if (rc) return rc;
         const int rows = (nrows + sms - 1) / sms;  // of a block, at most
@@ -1316,6 +1331,7 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
             cudaSuccess)
             return 3;
     if (smem > PS_SMEM) return 0;
+    if (cudaDeviceSynchronize() != cudaSuccess) return 3;
     s.on = true;
     return 0;
 }
