@@ -619,7 +619,8 @@ struct PSlot {
     double checked;  // <r, r> of the last true residual, 0: none yet
     double floor;    // (8 eps diagonal)^2
     int conv, zero, status;
-    int verify;      // the recurrence has ended, the true residual is not known
+    int far;         // the start was worse than 0: <r, r> above <b, b>
+    int verify;      // the recurrence has ended, the true residual is to be formed
     int member, n0, nn, owner;  // owner: this block writes the member's state
 };
 
@@ -686,6 +687,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
         c.zero = bb == 0.0;
         c.conv = c.zero || rr <= c.goal;
         c.status = 0;
+        c.far = rr > bb;
         c.verify = 0;
         c.checked = 0.0;
         // (one member: also in the blocks without a level-0 tile)
@@ -694,6 +696,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
         if (c.owner && !single) {
             A.conv[c.member] = c.conv;
             if (!c.conv) atomicAdd(A.active, 1);
+            if (c.far) atomicAdd(A.active + 1, 1);
         }
     }
     __syncthreads();
@@ -722,7 +725,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
             if (!(rr == rr)) c.status = ST_NONFINITE;
             else if (rr > c.goal && before + it >= maxit) c.status = ST_PCG_MAXIT;
             c.conv = c.status || rr <= c.goal;
-            c.verify = sizeof(S) == 4 && c.conv && c.status != ST_NONFINITE;
+            c.verify = sizeof(S) == 4 && c.far && c.conv && c.status != ST_NONFINITE;
             if (!c.owner) continue;
             if (c.conv) {
                 if (!single) {
@@ -755,21 +758,16 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
         __syncthreads();
         return v > 0;
     };
-    // The FP32 form's true residual, once the recurrences have ended: these
-    // solves are to end on it, as the refinement rounds of the larger ones do. x
-    // is rounded with every update, so the two differ by a few eps |diagonal| |x|
-    // of the largest iterate. Within 8 of the last one's the solve is done;
-    // beyond, the start was far larger than the solution: CG starts again from
-    // the true residual, as long as that reduces it 10x. False (in all blocks)
-    // when no member goes on.
-    __shared__ int s_check;
+    // The FP32 form's true residual, once the recurrences have ended: x is
+    // rounded with every update, so the two differ by a few eps |diagonal| |x| of
+    // the largest iterate (0.7 to 4 on 256^2 .. 2000 x 40 from zero), and a start
+    // 1e10 times the solution left 2e-5 to 1e-4 |b| unseen. So where a start was
+    // worse than 0, b - A x is formed: within 8 eps |diagonal| |x| the solve is
+    // done, beyond, CG starts again from it, as long as that reduces it 10x (as
+    // the refinement rounds of the larger problems). False (in all blocks) when
+    // no member goes on. (For every solve the pass cost 2 to 5 % of a step.)
     auto again = [&] {
-        if (threadIdx.x == 0) {
-            s_check = 0;
-            for (int i = 0; i < nslot; ++i) s_check |= slot[i].verify;
-        }
-        __syncthreads();
-        if (single && !s_check) return false;
+        if (single && !slot[0].verify) return false;
         for (int i = 0; i < ns; ++i) {
             if (!slot[single ? 0 : i].verify) continue;
             double v[2] = {0.0, 0.0};
@@ -816,7 +814,10 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
             if (!single) rconv[k] = *(volatile int*)&A.conv[rec[k].member];
         return go_on();
     };
-    while (go_on() || (sizeof(S) == 4 && again())) {
+    __shared__ int s_far;
+    if (threadIdx.x == 0) s_far = single ? slot[0].far : *(volatile int*)(A.active + 1);
+    __syncthreads();
+    while (go_on() || (sizeof(S) == 4 && s_far && again())) {
         for (int i = 0; i < ns; ++i) {
             const PSlot& c = slot[single ? 0 : i];
             if (c.conv) continue;
@@ -946,7 +947,7 @@ __global__ void k_ps_setup(const __grid_constant__ PSArgs A, double tol2, int ma
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b == 0) {
         ps_reset(A.bar);
-        *A.active = 0;
+        A.active[0] = A.active[1] = 0;
     }
     if (b < A.nmem) {
         A.scs[b].tol2 = tol2;
@@ -1299,7 +1300,7 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
         if (l0 == 0 && !(p = (double*)dal((size_t)nelem * 8))) return 2;
     a.part = (double*)dal((size_t)5 * std::max(1, a.ntiles) * sizeof(double));
     a.conv = (int*)dal(n * sizeof(int));
-    a.active = (int*)dal(sizeof(int));
+    a.active = (int*)dal(2 * sizeof(int));
     a.bar = (PSBar*)dal(sizeof(PSBar));
     if (!drec || !d0 || !dd || !a.part || !a.conv || !a.active || !a.bar) return 2;
     if (cudaMemcpy(drec, recs.data(), recs.size() * sizeof(PTile), cudaMemcpyHostToDevice) !=

@@ -53,7 +53,7 @@ struct PSArgs {
     double *x, *b, *r[2], *s[2], *p, *w;  // arenas, FP64
     double* part;        // tile totals, 2 x 2 ntiles
     int* conv;           // per member
-    int* active;         // members still iterating
+    int* active;         // members still iterating, members whose start was worse than 0
     DevScalars* scs;
     BSGlobals* eg;
     int* status;
@@ -81,8 +81,9 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
              DevScalars* scs, BSGlobals* eg, int* status, int l0 = 0);
 void ps_free(PSolver& s);
 // Record one solve of every member on `st`: x and b are the arenas (FP64). It
-// ends at |r| <= tol |b|, r the recurrence residual (FP64 form) or b - A x to
-// within its rounding (FP32 form, see k_ps_solve), or after maxit iterations.
+// ends at |r| <= tol |b|, r the recurrence residual (FP32 form from a start worse
+// than 0: b - A x to within its rounding, see k_ps_solve), or after maxit
+// iterations.
 int ps_record(PSolver& s, double* x, double* b, int nu, double tol, int maxit, cudaStream_t st);
 // Record the V-cycle on the levels from l0 on (from its b to its x), skipped
 // when the member is not iterating (ir: its inner loop); ps_record_cycle_reset

@@ -55,10 +55,11 @@ typedef struct f2d_params {
     int noslip;         /* F2D_SLIP_* */
     int noslip_sides;   /* F2D_SIDE_* bits when noslip == F2D_SLIP_SIDES */
     int precision;      /* F2D_PREC_* */
-    double poisson_tol; /* relative residual of the Poisson solve: of CG's
-                           recurrence (FP64 form, and the pressure of euler and
-                           boussinesq) or of b - A x (FP32 form), which stops at
-                           its rounding: a few eps |diagonal of A| |x| */
+    double poisson_tol; /* relative residual of the Poisson solve, of CG's
+                           recurrence; b - A x differs from it by its rounding,
+                           a few eps |diagonal of A| |x| of the largest iterate.
+                           FP32 form: of b - A x where the grid is large or the
+                           start was worse than 0 */
     int poisson_maxit;  /* CG iterations of a solve; FP32 form (vertex solves):
                            max(2, maxit / 10) times 30 of them */
     int integrator;     /* F2D_INTEG_* */
