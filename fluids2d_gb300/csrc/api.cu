@@ -1438,8 +1438,8 @@ int f2d_field_names(f2d_model m, char* buf, size_t len)
         // the state's fields (not the integrator's scratch, the warm-start
         // history, the rhs and forcing fields)
         const std::string& n = kv.first;
-        if (n.rfind("ds", 0) == 0 || n.rfind("psi.", 0) == 0 || n.rfind("rhs.", 0) == 0 ||
-            n.rfind("frc.", 0) == 0)
+        if (n.rfind("ds", 0) == 0 || n.rfind("psi.", 0) == 0 || n.rfind("p.", 0) == 0 ||
+            n.rfind("rhs.", 0) == 0 || n.rfind("frc.", 0) == 0)
             continue;
         if (!s.empty()) s += ",";
         s += kv.first;

@@ -5,6 +5,8 @@ the steps of a state that was written since. The kernels sum in fixed orders,
 so a model whose fields are all written anew, after a stronger flow or after a
 NaN, repeats a fresh model's steps to the bit.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -13,6 +15,7 @@ torch = pytest.importorskip("torch")
 
 import fluids2d_gb300 as f2d  # noqa: E402
 from fluids2d_gb300 import workloads as wl  # noqa: E402
+from fluids2d_gb300._lib import check, lib  # noqa: E402
 from test_gpu_parity import _ensemble, _model  # noqa: E402
 
 
@@ -95,6 +98,23 @@ def test_rewritten_model_equals_fresh_model(kind, precision, dt, before):
     for k, a in _arrays(m.state):
         if not k.startswith("flx"):
             assert np.array_equal(a, want[k]), k
+
+
+@pytest.mark.parametrize("kind", list(CASES))
+def test_field_names_are_the_state(kind):
+    """f2d_field_names lists the state's fields, none of the history's, so the
+    same ones in both precisions."""
+    names = {}
+    for precision in ("fp64", "fp32"):
+        m = _make(kind, CASES[kind](n=32, ny=24, seed=1, nislands=0), precision)
+        buf = ctypes.create_string_buffer(4096)
+        check(lib().f2d_field_names(m._h, buf, len(buf)))
+        names[precision] = set(buf.value.decode().split(","))
+        assert not [n for n in names[precision]
+                    if "." in n and n.split(".")[1] not in ("x", "y")]
+        state = {k for k, _ in _arrays(m.state) if not k.startswith("flx")}
+        assert state <= names[precision]
+    assert names["fp64"] == names["fp32"]
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
