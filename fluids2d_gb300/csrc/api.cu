@@ -729,7 +729,7 @@ static int rec_stage(f2d_model_s* m, int k, int par, cudaStream_t s)
     if (e) return e;
     const bool warm = m->p.integrator == F2D_INTEG_RK3 &&
                       (m->p.model == F2D_MODEL_EULERPSI || m->p.model == F2D_MODEL_QG ||
-                       (projected(m->p.model) && m->prec == 0));
+                       fb(m, "p.s0"));
     return rec_diag(m, 1 - par, s, warm ? k - 1 : -1);
 }
 
@@ -1216,7 +1216,8 @@ int f2d_model_create(const f2d_params* p, const int8_t* msk, f2d_model* out)
             if ((f[4] != 'e' || psi_warm_brackets(m->prec, (long long)m->g.P * m->g.NY)) &&
                 (e = add_field(m, f, false, 8)))
                 return bail(e);
-    if (projected(p->model) && m->prec == 0)
+    if (projected(p->model) && m->prec == 0 &&
+        (long long)m->g.P * m->g.NY <= WARM_POINTS)
         for (const char* f : {"p.s0", "p.d1", "p.d2", "p.e1", "p.e2", "p.e3"})
             if ((e = add_field(m, f, false, 8))) return bail(e);
     // qgrsw keeps the third stage's (or LFRA's) tendency too: it is

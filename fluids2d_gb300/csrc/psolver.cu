@@ -1100,10 +1100,9 @@ static std::vector<TileDim> pick_tiles(const std::vector<std::pair<int, int>>& n
     return best;
 }
 
-int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long nelem,
-             DevScalars* scs, BSGlobals* eg, int* status, int l0)
+static int ps_try(PSolver& s, const std::vector<PSMember>& mem, int prec, long long nelem,
+                  double* const (&work)[4], DevScalars* scs, BSGlobals* eg, int* status, int l0)
 {
-    ps_free(s);
     const int n = (int)mem.size(), sms = ps_sms();
     if (n < 1 || sms < 1 || (l0 == 0 && nelem <= 0) || (l0 > 0 && n > 1)) return 0;
     const size_t es = prec == 0 ? 8 : 4;
@@ -1295,9 +1294,10 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     PTile* drec = (PTile*)dal(recs.size() * sizeof(PTile));
     int* d0 = (int*)dal(rec0.size() * sizeof(int));
     PDense* dd = (PDense*)dal(n * sizeof(PDense));
-    double* vec[6] = {};
-    for (auto& p : vec)
-        if (l0 == 0 && !(p = (double*)dal((size_t)nelem * 8))) return 2;
+    // r and s in the caller's vectors (no value is read before it is written)
+    double* vec[6] = {work[0], work[1], work[2], work[3], nullptr, nullptr};
+    for (double*& p : vec)
+        if (l0 == 0 && !p && !(p = (double*)dal((size_t)nelem * 8))) return 2;
     a.part = (double*)dal((size_t)5 * std::max(1, a.ntiles) * sizeof(double));
     a.conv = (int*)dal(n * sizeof(int));
     a.active = (int*)dal(2 * sizeof(int));
@@ -1334,6 +1334,18 @@ int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long n
     if (smem > PS_SMEM) return 0;
     if (cudaDeviceSynchronize() != cudaSuccess) return 3;
     s.on = true;
+    return 0;
+}
+
+int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long nelem,
+             double* const (&work)[4], DevScalars* scs, BSGlobals* eg, int* status, int l0)
+{
+    ps_free(s);
+    const int rc = ps_try(s, mem, prec, nelem, work, scs, eg, status, l0);
+    if (s.on) return 0;
+    ps_free(s);
+    if (rc != 2) return rc;
+    cudaGetLastError();  // out of memory: the level kernels need less
     return 0;
 }
 

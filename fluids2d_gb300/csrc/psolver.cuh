@@ -75,10 +75,11 @@ struct PSMember {
 
 // Build for the members' hierarchies: on = false (and no error) where the
 // kernel does not apply (no level small enough for the dense inverse, more
-// tiles than a block has records). l0 > 0: one member, for ps_record_cycle
-// alone, on the levels from l0 on (nelem is not used).
+// tiles than a block has records) or its memory is not to be had. work: FP64
+// vectors of nelem elements that the solves may use. l0 > 0: one member, for
+// ps_record_cycle alone, on the levels from l0 on (nelem and work are not used).
 int ps_build(PSolver& s, const std::vector<PSMember>& mem, int prec, long long nelem,
-             DevScalars* scs, BSGlobals* eg, int* status, int l0 = 0);
+             double* const (&work)[4], DevScalars* scs, BSGlobals* eg, int* status, int l0 = 0);
 void ps_free(PSolver& s);
 // Record one solve of every member on `st`: x and b are the arenas (FP64). It
 // ends at |r| <= tol |b|, r the recurrence residual (FP32 form from a start worse

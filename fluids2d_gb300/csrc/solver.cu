@@ -1845,7 +1845,10 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
         const bool crowd = s.n > ps_sms() && (mode == 1 || n0 < PS_CROWD_NODES * s.n);
         if (!crowd &&
             (mode == 0 || n0 <= (s.n == 1 ? PS_FP32_NODES : PS_FP32_NODES / 2))) {
-            const int e = ps_build(s.ps, pm, mode, v.nelem, scs, s.eg, &s.eg->status);
+            // (arenas of 8 bytes an element in both forms, which only the level
+            // kernels use otherwise)
+            double* const work[4] = {(double*)v.r64, (double*)v.p, (double*)v.p2, (double*)v.q};
+            const int e = ps_build(s.ps, pm, mode, v.nelem, work, scs, s.eg, &s.eg->status);
             if (e) return e;
         }
     }
@@ -1856,7 +1859,8 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
         while (s.lc < s.maxl && (long long)lev[s.lc].nyn * lev[s.lc].nxn > PC_NODES) ++s.lc;
         if (s.lc < s.maxl) {
             const std::vector<PSMember> pm = {{&s.mg[0], PS_NDENSE}};
-            const int e = ps_build(s.pc, pm, mode, 0, scs, s.eg, &s.eg->status, s.lc);
+            double* const none[4] = {};
+            const int e = ps_build(s.pc, pm, mode, 0, none, scs, s.eg, &s.eg->status, s.lc);
             if (e) return e;
         }
     }

@@ -88,10 +88,13 @@ struct WarmArrays {
 // points. (A CFL step's change shrinks with the grid spacing, its rounding
 // does not. FP32 CG iterations per solve without and with them: 9.67 and 8.36
 // on the 256-member ensemble of 64^2 .. 512^2, 8.33 and 8.64 on qg 4096^2;
-// 2048^2 gains what the extra arrays cost.)
+// 2048^2 gains what the extra arrays cost.) Beyond 1e8 points a model is to fit
+// the memory as it did without them: 2.4 GB and more of arrays (the pressure's
+// whole history, 4.8 GB), which only shorten the solves.
+constexpr long long WARM_POINTS = 100000000ll;
 inline bool psi_warm_brackets(int prec, long long points)
 {
-    return prec == 0 || points <= 3000000ll;
+    return points <= (prec == 0 ? WARM_POINTS : 3000000ll);
 }
 
 // U pairs of elements (k, k + 1), k even and every array 16-byte aligned

@@ -351,3 +351,25 @@ def test_fp32_iteration_limit_counts_rounds():
     m.state.omega[:] = case["fields"]["omega"]
     m.integrator.diag(m.state)
     m.sync()
+
+
+def test_memory_of_an_fp64_model():
+    """Of its grid's arrays of 8 bytes an FP64 eulerpsi model holds 24.6 of its
+    own, one for the coarse levels, and two of the persistent solve (its others
+    are the level kernels'), with its dense inverse half of one: 28.3, and 1.7
+    for small buffers and the driver."""
+    m = _model("eulerpsi", 32, 32)
+    m.integrator.diag(m.state)  # (the library's own memory)
+    m.sync()
+    n = 3072
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    m = _model("eulerpsi", n, n)
+    check(lib().f2d_diag(m._h))
+    check(lib().f2d_run(m._h, 1))
+    m.sync()
+    form = ctypes.c_int(-1)
+    check(lib().f2d_solver_form(m._h, ctypes.byref(form)))
+    assert form.value == 2
+    used = free - torch.cuda.mem_get_info()[0]
+    assert used <= 30 * 8 * ((n + 6 + 15) // 16 * 16) * (n + 6)
