@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_solve(const __grid_constant__ P
     const int nt = A.ntiles;
     // totals per tile: <r, z>, <z, w> | <r, r> | <b, b>, <r, r>
     double *pz = A.part, *pr = A.part + 2 * nt, *pb = A.part + 3 * nt;
-    PSGrid g = {A.bar, A.status, 0u};
+    PSGrid g = ps_grid(A.bar, A.status, 0u);
     const double tol2 = A.scs[0].tol2;
     const int maxit = A.scs[0].maxit;
     // r = b - A x, <b, b>, <r, r>
@@ -916,7 +916,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ps_cycle(const __grid_constant__ P
     __shared__ PSegs segs;
     const DevScalars& sc = A.scs[0];
     const int skip = sc.converged | (ir ? sc.conv_in : 0);
-    PSGrid g = {A.bar, A.status, A.bar->base};
+    PSGrid g = ps_grid(A.bar, A.status, A.bar->base);
     const int nl = A.ng + 1;
     if (threadIdx.x < nl) lev0[threadIdx.x] = A.rec0[blockIdx.x * nl + threadIdx.x];
     if (skip) return;  // (the same in every block: no barrier is left waiting)
@@ -952,6 +952,7 @@ __global__ void k_ps_setup(const __grid_constant__ PSArgs A, double tol2, int ma
     if (b < A.nmem) {
         A.scs[b].tol2 = tol2;
         A.scs[b].bb_last = A.scs[b].bb;
+        A.scs[b].bb = 0.0;  // (of a solve that does not finish, too)
         A.scs[b].maxit = maxit;
         A.scs[b].converged = 0;
         A.scs[b].iter = 0;

@@ -1034,6 +1034,7 @@ __global__ void k_bs_setup(DevScalars* scs, int n, double tol2, int maxit, doubl
     if (b < n) {
         DevScalars& s = scs[b];
         s.bb_last = s.bb;
+        s.bb = 0.0;
         s.tol2 = tol2;
         s.maxit = maxit;
         s.tol_in2 = tol_in2;
