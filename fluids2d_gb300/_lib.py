@@ -122,6 +122,7 @@ _SIGS = {
                                   ctypes.POINTER(c_i64), ctypes.POINTER(c_int)], c_int),
     "f2d_solver_pipelined": ([c_void_p, ctypes.POINTER(c_int)], c_int),
     "f2d_ensemble_solver_pipelined": ([c_void_p, ctypes.POINTER(c_int)], c_int),
+    "f2d_test_grid_wait": ([c_void_p, c_int, c_dbl], c_int),
     "f2d_solver_form": ([c_void_p, ctypes.POINTER(c_int)], c_int),
     "f2d_ensemble_solver_form": ([c_void_p, ctypes.POINTER(c_int)], c_int),
     "f2d_adjoint_forward": ([c_void_p, c_void_p, c_void_p, c_int, c_dbl, c_int], c_int),

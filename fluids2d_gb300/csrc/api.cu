@@ -1768,6 +1768,19 @@ int f2d_test_tma_wait(int enabled, double limit_ms)
     return 0;
 }
 
+int f2d_test_grid_wait(f2d_model m, int enabled, double limit_ms)
+{
+    if (!m) return fail(1, "null model");
+    if (enabled && !(limit_ms >= 0.001 && limit_ms <= 1000))
+        return fail(1, "f2d_test_grid_wait: limit_ms must be in [0.001, 1000]");
+    const unsigned int us = enabled ? (unsigned int)(limit_ms * 1e3) : 0u;
+    CK(cudaStreamSynchronize(m->stream));
+    for (PSBar* bar : {m->bs[0].ps.a.bar, m->bs[0].pc.a.bar, m->bs[1].ps.a.bar,
+                       m->bs[1].pc.a.bar, (PSBar*)m->ns.a.bar})
+        CKI(ps_test_wait(bar, us));
+    return 0;
+}
+
 int f2d_refine_rounds(f2d_model m, int64_t* rounds)
 {
     if (!m || !rounds) return fail(1, "null argument");

@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(PS_NT, 1) k_ns_solve(const __grid_constant__ N
         int done, status;
     } c;
     DevScalars* sc = (DevScalars*)A.sc;
-    PSGrid g = {(PSBar*)A.bar, &A.eg->status, 0u};
+    PSGrid g = ps_grid((PSBar*)A.bar, &A.eg->status, 0u);
     const NLevel& L = A.lev[0];
     const unsigned G = gridDim.x;
     // the block's rows of the dense level, kept in shared memory if they fit

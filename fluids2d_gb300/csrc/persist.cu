@@ -207,6 +207,13 @@ int ps_invert(const std::vector<double>& band, int n, int bw, const std::vector<
     return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
+int ps_test_wait(PSBar* bar, unsigned int limit_us)
+{
+    if (!bar) return 0;
+    const unsigned int v[2] = {limit_us ? 1u : 0u, limit_us};
+    return (int)cudaMemcpy(&bar->hold, v, sizeof(v), cudaMemcpyHostToDevice);
+}
+
 int ps_launch(const void* kern, int grid, size_t smem, void** args, cudaStream_t st)
 {
     cudaLaunchConfig_t cfg = {};

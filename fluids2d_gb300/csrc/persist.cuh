@@ -23,19 +23,29 @@ constexpr int PS_NT = 512;  // threads of a block (one block per SM)
 // each reaches k times its number of blocks. (One counter for all 152 blocks:
 // 2840 cycles with writes in flight, four: 2660. A flag per block that all
 // blocks poll: 5000 to 8500; clusters with one arrival each: 3500 and more.) The wait
-// is bounded: after limit_ns without progress the block sets the abort word
+// is bounded: after 2 s without progress the block sets the abort word
 // and the kernel's status, and every block returns from the kernel.
 struct PSBar {
     unsigned int count[4][32];  // arrivals
     int abort;                  // a wait ran out
     unsigned int base;          // barriers passed by the launches before (k_ps_cycle)
+    // test hook (f2d_test_grid_wait): one arrival more than there are blocks
+    // (hold = 1), and the limit of the wait (0: 2 s). Never reset by a solve
+    unsigned int hold;
+    unsigned int limit_us;
 };
 
 struct PSGrid {
     PSBar* bar;
     int* status;
-    unsigned int round;
+    unsigned int round, hold, limit_us;
 };
+
+__device__ __forceinline__ PSGrid ps_grid(PSBar* bar, int* status, unsigned int round)
+{
+    const unsigned int limit = bar->limit_us;
+    return {bar, status, round, bar->hold, limit ? limit : 2000000u};
+}
 
 // zero the counters (before the launch)
 __device__ __forceinline__ void ps_reset(PSBar* b)
@@ -74,13 +84,13 @@ __device__ __forceinline__ bool ps_sync(PSGrid& g, F idle)
                          : "memory");
         if (lane < 4) {
             // blocks of counter `lane`
-            const unsigned target = g.round * ((gridDim.x + 3 - lane) / 4);
+            const unsigned target = g.round * ((gridDim.x + 3 - lane) / 4) + g.hold;
             uint64_t t0 = 0;
             for (unsigned spin = 0; (int)(ld_acquire(g.bar->count[lane]) - target) < 0; ++spin) {
                 if ((spin & 255u) != 255u) continue;
                 const uint64_t t = globaltimer_ns();
                 if (t0 == 0) t0 = t;
-                if (t - t0 > 2000000000ull || *(volatile int*)&g.bar->abort) {
+                if (t - t0 > g.limit_us * 1000ull || *(volatile int*)&g.bar->abort) {
                     *(volatile int*)&g.bar->abort = 1;
                     atomicOr(g.status, ST_GRID_TIMEOUT);
                     dead = 1;
@@ -367,6 +377,9 @@ inline bool ps_band_ok(long long n, long long bw, int prec)
 {
     return n <= (prec == 0 ? PS_NDENSE : PS_NDENSE32) && n * bw * bw <= 50000000ll;
 }
+// The test hook of the barrier's wait: limit_us > 0 makes every one run out
+// after it, 0 ends that.
+int ps_test_wait(PSBar* bar, unsigned int limit_us);
 // Launch a cooperative kernel of PS_NT threads per block.
 int ps_launch(const void* kern, int grid, size_t smem, void** args, cudaStream_t st);
 // SMs of the current device.

@@ -257,6 +257,13 @@ int f2d_solver_form(f2d_model m, int *form);
  * enabled == 0 restores normal operation. Applies to every model and
  * ensemble of the process; synchronises the device. For tests only. */
 int f2d_test_tma_wait(int enabled, double limit_ms);
+/* The same for the grid barriers of this model's persistent solve kernels (the
+ * model must have solved once; a rebuild of its solver ends it): enabled != 0
+ * makes each wait for an arrival that no block makes, give up after limit_ms
+ * (0.001 <= limit_ms <= 1000) and record the barrier's time-out status, which
+ * the next f2d_sync reports; the solve's output is then unfinished. For tests
+ * only. */
+int f2d_test_grid_wait(f2d_model m, int enabled, double limit_ms);
 /* Test hook (no reference counterpart): the library's integer-pipe
  * binary64 -> binary32 (round to nearest even) and binary32 -> binary64
  * conversions next to the hardware conversions, on the device, for host

@@ -6,6 +6,7 @@ so a model whose fields are all written anew, after a stronger flow or after a
 NaN, repeats a fresh model's steps to the bit.
 """
 import ctypes
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
@@ -144,6 +145,73 @@ def test_rewritten_ensemble_equals_fresh_one(precision):
     for b in range(len(members)):
         for k in ("omega", "psi"):
             assert np.array_equal(e.get_field(b, k), fresh.get_field(b, k)), (b, k)
+
+
+@pytest.mark.parametrize("kind,precision,n", [("eulerpsi", "fp64", 72), ("eulerpsi", "fp32", 72),
+                                              ("euler", "fp64", 72), ("boussinesq", "fp32", 72),
+                                              ("qg", "fp32", 1450)])
+def test_grid_barrier_timeout_reports_then_recovers(kind, precision, n):
+    """A grid barrier that one arrival is missing from gives up after its limit
+    (5 ms here), in the solves' kernels and the coarse levels' (qg 1450^2); the
+    status is reported, and the model is as good as new afterwards."""
+    case = CASES[kind](n=n, ny=n - 8, seed=31, nislands=1)
+    fresh = _make(kind, case, precision)
+    _write(fresh, case["fields"])
+    fresh.advance(1)
+    fresh.sync()
+    m = _make(kind, case, precision)
+    _write(m, case["fields"])
+    m.sync()
+    check(lib().f2d_test_grid_wait(m._h, 1, 5.0))
+    m.advance(1)
+    with pytest.raises(f2d.F2DError, match="grid barrier timed out"):
+        m.sync()
+    check(lib().f2d_test_grid_wait(m._h, 0, 0.0))
+    _write(m, case["fields"])
+    m.advance(1)
+    m.sync()
+    want = dict(_arrays(fresh.state))
+    for k, a in _arrays(m.state):
+        if not k.startswith("flx"):
+            assert np.array_equal(a, want[k]), k
+
+
+@pytest.mark.parametrize("threads", [False, True])
+def test_models_solving_at_the_same_time(threads):
+    """Models on streams of their own, whose solves take the whole GPU, stepped
+    in turn from one thread and at once from several: the results of each alone."""
+    kinds = [("eulerpsi", "fp64", 160), ("euler", "fp64", 96), ("qg", "fp32", 200),
+             ("boussinesq", "fp32", 72)]
+    cases = [CASES[k](n=n, ny=n - 10, seed=7, nislands=1) for k, _, n in kinds]
+
+    def models():
+        out = [_make(k, c, p) for (k, p, _), c in zip(kinds, cases)]
+        for m, c in zip(out, cases):
+            _write(m, c["fields"])
+        return out
+
+    def steps(m, n):
+        for _ in range(n):
+            m.advance(1)
+        m.sync()
+
+    alone = models()
+    for m in alone:
+        steps(m, 12)
+    both = models()
+    if threads:
+        with ThreadPoolExecutor(len(both)) as ex:
+            list(ex.map(lambda m: steps(m, 12), both))
+    else:
+        for _ in range(12):
+            for m in both:
+                m.advance(1)
+    for m, a in zip(both, alone):
+        m.sync()
+        want = dict(_arrays(a.state))
+        for k, v in _arrays(m.state):
+            if not k.startswith("flx"):
+                assert np.array_equal(v, want[k]), k
 
 
 @pytest.mark.parametrize("kind,precision", [("eulerpsi", "fp64"), ("eulerpsi", "fp32"),
