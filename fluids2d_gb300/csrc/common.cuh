@@ -87,7 +87,7 @@ struct DevScalars {
 // The warm start's state as stage MODE + 1 of a step reads it, and its update
 // by one thread of the grid: a grid never reads what it writes. Without hist
 // (no step before, or one of less than 1/64 of this step's size, whose
-// increments are mostly rounding) no array of the history may be read.
+// increments are mostly rounding) no value of the history may be used.
 struct WarmState {
     bool hist;
     double rho;

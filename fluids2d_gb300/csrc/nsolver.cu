@@ -12,7 +12,11 @@
 // so the right-hand side is projected to zero mean over the fluid cells (the
 // compatibility condition; for a divergence it is zero up to rounding) and
 // the solution is returned with zero mean: the pressure is defined up to a
-// constant, and only its gradient enters the model.
+// constant, and only its gradient enters the model. One connected fluid region
+// is assumed: the mean is that of all fluid cells. Unconnected basins are
+// solvable where each one's sum of b is 0 to rounding by itself (the divergence
+// of an FP64 velocity); an FP32 velocity leaves 1e-7 of it in each, that system
+// has no solution, and the solve reports its iteration limit.
 //
 // Preconditioner: cell-centred V-cycle with red-black Gauss-Seidel (2 sweeps
 // per leg, symmetric order), coarse cells = 2x2 agglomerates (fluid if any
@@ -45,11 +49,11 @@
 // A leg works on a tile and a halo of the 4 (B: 5) cells its half sweeps
 // reach over, in shared memory, so a leg needs one barrier; tile sizes are
 // chosen per level so that the chip is filled (pick_tile).
-// What bounds it: at 40^2 (one iteration on the dense level, 48 us) the latency
+// What bounds it: at 40^2 (one iteration on the dense level, 42 us) the latency
 // of its phases and barriers; at 512^2 FP64 (75 us an iteration) the FP64 pipe,
 // 40 % busy, and between its bursts the loads of a phase and the barriers (2.6k
-// cycles each). One launch per sweep and level before it: 11.4 ms a step of
-// euler 512^2, now 2.1 ms with the warm start.
+// cycles each). One launch per sweep and level before it: 11.8 ms a step of
+// euler 512^2, now 1.84 with the warm start.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -1145,8 +1149,8 @@ int ns_build(NSolver& s, int nyn, int nxn, long long pitch, long long off, int p
     if (rc) return rc;
     a.minv = minv;
     // every SM also for small problems: the rows of the dense level are dealt
-    // to all blocks, and a barrier of 152 blocks (1.36 us) costs hardly more
-    // than one of 25 (1.28 us)
+    // to all blocks, and a barrier of 152 blocks costs hardly more than one of 25
+    // (1.36 us and 1.28, timed by barriers alone)
     s.grid = sms;
     const int rows = (a.nd + sms - 1) / sms;  // of a block, at most
     s.smem = (prec == 0 ? ps_dense_elems<double>(a.nd, rows) : ps_dense_elems<float>(a.nd, rows)) *

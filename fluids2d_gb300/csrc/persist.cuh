@@ -7,7 +7,7 @@
 // dependent steps. As kernels in a graph each costs its launch gap, the
 // dependent loads of its descriptors and the drain of its last blocks (5 to
 // 8 us for a few hundred ns of work); a grid barrier on GB300 costs about
-// 1.5 us and the descriptors stay in the kernel's parameters.
+// 1.3 us (2.7k cycles) and the descriptors stay in the kernel's parameters.
 #pragma once
 #include <vector>
 
@@ -43,8 +43,7 @@ struct PSGrid {
 
 __device__ __forceinline__ PSGrid ps_grid(PSBar* bar, int* status, unsigned int round)
 {
-    const unsigned int limit = bar->limit_us;
-    return {bar, status, round, bar->hold, limit ? limit : 2000000u};
+    return {bar, status, round, bar->hold, bar->limit_us};
 }
 
 // zero the counters (before the launch)
@@ -90,7 +89,9 @@ __device__ __forceinline__ bool ps_sync(PSGrid& g, F idle)
                 if ((spin & 255u) != 255u) continue;
                 const uint64_t t = globaltimer_ns();
                 if (t0 == 0) t0 = t;
-                if (t - t0 > g.limit_us * 1000ull || *(volatile int*)&g.bar->abort) {
+                // (here: used any earlier, the loads would hold the kernel's start up)
+                const uint64_t limit = g.limit_us ? g.limit_us * 1000ull : 2000000000ull;
+                if (t - t0 > limit || *(volatile int*)&g.bar->abort) {
                     *(volatile int*)&g.bar->abort = 1;
                     atomicOr(g.status, ST_GRID_TIMEOUT);
                     dead = 1;

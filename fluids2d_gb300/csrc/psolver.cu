@@ -8,8 +8,9 @@
 // Operator, hierarchy and cycle are mg.cu's: red-black Gauss-Seidel with nu
 // sweeps per leg, bilinear prolongation and its transpose, coarse masks by
 // injection, re-discretised coarse operators. The first level with few enough
-// nodes is solved exactly with its dense inverse (a single model: up to 2048
-// nodes, level 0 itself if it is that small). S is the cycle's precision;
+// unknowns (nodes off the closed edges) is solved exactly with its dense inverse
+// (a single model: up to 2048 unknowns, FP32 4096, level 0 itself if it is that
+// small). S is the cycle's precision;
 // the CG vectors, the operator product and the inner products are FP64 in
 // both forms (FP32 form: the cycle's right-hand side is the FP64 residual
 // rounded).

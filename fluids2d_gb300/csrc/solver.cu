@@ -956,7 +956,8 @@ k_bs_correct(const int4* __restrict__ tiles, const MGLevel* __restrict__ levs,
     }
 }
 
-// k_bs_correct in the same layout: qg 4096^2, eight directions: 236 -> 187 us.
+// k_bs_correct in the same layout: qg 4096^2, eight directions: 201 -> 155 us;
+// 256 members: 246 -> 186.
 // (The FP64 residual gains nothing from it, 293 -> 309 us: its pipe is busy
 // either way, and the side lanes cost it a fifteenth of its instructions.)
 __global__ void __launch_bounds__(256, 2)

@@ -855,25 +855,25 @@ __global__ void __launch_bounds__(256) k_p_warm(WarmArrays w, const uint32_t* __
     const double rho = ws.rho;
     if (k < n && (code[k] & B_MSK)) {
         const double p = w.psi[k];
+        // (the history's loads do not wait for hist: only their values do)
         if constexpr (MODE == 0) {
+            const double S2 = w.d1[k], e1 = w.e1[k], s0 = w.s0[k];
             if (hist) {
-                const double S2 = w.d1[k], e1 = w.e1[k];
-                w.e3[k] = fma(1.5, p, -0.375 * (w.s0[k] + S2));
+                w.e3[k] = fma(1.5, p, -0.375 * (s0 + S2));
                 w.psi[k] = rho * (S2 + e1);
             }
         } else if constexpr (MODE == 1) {
-            const double d1 = hist ? w.d1[k] : 0.0, d2 = hist ? w.d2[k] : 0.0;
-            const double e2 = hist ? w.e2[k] : 0.0;
+            const double d1 = w.d1[k], d2 = w.d2[k], e2 = w.e2[k];
             w.s0[k] = p;
             w.e1[k] = hist ? fma(-rho, d1, p) : 0.0;
-            w.psi[k] = fma(0.25 * rho, d2 + e2, -0.5 * p);
+            w.psi[k] = hist ? fma(0.25 * rho, d2 + e2, -0.5 * p) : -0.5 * p;
         } else {
-            const double S1 = w.s0[k], d2 = hist ? w.d2[k] : 0.0, e3 = hist ? w.e3[k] : 0.0;
-            const double S2 = fma(4.0, p, 3.0 * S1), D = S2 - S1;
+            const double S1 = w.s0[k], d2 = w.d2[k], e3 = w.e3[k];
+            const double S2 = fma(4.0, p, 3.0 * S1), D = S2 - S1, h = 0.25 * (S1 + S2);
             w.d1[k] = S2;
             w.d2[k] = D;
             w.e2[k] = hist ? fma(-rho, d2, D) : 0.0;
-            w.psi[k] = fma(rho * (2.0 / 3.0), e3, 0.25 * (S1 + S2));
+            w.psi[k] = hist ? fma(rho * (2.0 / 3.0), e3, h) : h;
         }
     }
 }

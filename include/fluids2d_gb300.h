@@ -221,8 +221,8 @@ int f2d_time_stage(f2d_model m, int stage, int reps, int flush_l2,
  * reaches the tolerance is kept (the step graphs are re-captured). The state
  * is unchanged. Outputs may be NULL. Models with a vertex Poisson/Helmholtz
  * solve (eulerpsi, qg, qgrsw) and ensembles. Where the whole solve is one
- * persistent kernel (FP64; FP32 up to 2M nodes, ensembles 1M) only the sweeps
- * matter and only they are tried. */
+ * persistent kernel (f2d_solver_form 2) only the sweeps matter and only they
+ * are tried. */
 int f2d_autotune(f2d_model m, int reps, int *tile_rows, int *sweeps, double *tol_in,
                  double *ms_per_solve);
 /* Set the multigrid schedule directly (what f2d_autotune would pick):
@@ -271,7 +271,8 @@ int f2d_test_grid_wait(f2d_model m, int enabled, double limit_ms);
 int f2d_test_conversions(const double *x64, int64_t n64, float *sw32, float *hw32,
                          const float *x32, int64_t n32, double *sw64, double *hw64);
 /* Refinement rounds of the FP32 form's solves summed since creation (see
- * f2d_ensemble_refine_rounds; a persistent solve has none). Instrumentation. */
+ * f2d_ensemble_refine_rounds; a persistent solve counts its starts after the
+ * first). Instrumentation. */
 int f2d_refine_rounds(f2d_model m, int64_t *rounds);
 /* Counters: Poisson iterations summed over all solves since creation; the
  * kernels one time step launches outside the Poisson loops; the kernels one
