@@ -1826,7 +1826,9 @@ int bs_build(BatchSolver& s, const std::vector<BSMemberDesc>& members, const uin
         s.wide = s.wide && (uintptr_t)p % 16 == 0;
     // The persistent solve: every FP64 problem (its level kernels and loops
     // cost more at every size), and FP32 problems of up to PS_FP32_NODES nodes
-    // (batches half of that):
+    // (batches half of that: 15 256^2, 1.0M nodes, 2.44 ms a step persistent, 2.79
+    // with the level kernels; 22, 1.5M: 3.34 and 3.07; 4 512^2 2.38 and 2.95, 6
+    // 3.40 and 3.31):
     // above that the refinement form's FP32 Krylov vectors and pipelined legs
     // move less and are the faster ones. Not with more members than SMs where
     // the level kernels, several members to an SM at a time, beat a block that
